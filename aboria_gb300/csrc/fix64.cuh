@@ -1,0 +1,339 @@
+// FP64-accurate kernel values from integer and FP32 arithmetic.
+//
+// GB300 issues 2 FP64 operations per clock and SM (measured 1.7-1.8) against
+// 58 32x32+64-bit multiply-adds, 62 integer ALU operations and 115 FP32 FMAs,
+// so one double-precision operation costs as much as about 32 integer ones.
+// A pair's kernel value takes ~30 of the former (distance 6-8, sqrt or exp
+// 10-20, the rest the polynomial and the product); here everything but the
+// last multiply-add into the row's FP64 sum runs on the integer pipe:
+//
+//  * coordinates are 64-bit fixed point, X = x * 2^K modulo 2^64.  A double's
+//    bits are shifted, not rounded, down to 2^-K, and differences that fit in
+//    62 bits are exact whatever wrapped on the way (to_fixed);
+//  * the squared distance keeps 63 fractional bits of the unit R^2,
+//    R = 2^(62-K) >= |dx| (sq_acc, sq_sum): each dx = h 2^32 + l with a signed
+//    low half; h^2 and h l are summed exactly and l^2 (below 2^-62) is left
+//    out;
+//  * sqrt starts from the hardware's FP32 reciprocal square root and takes
+//    two corrections from exact integer residuals (sqrt60);
+//  * 2^-t splits t into an exponent, an index of a 256-entry table and a rest
+//    below 2^-8 whose Taylor series (ln 2 powers) is a Horner chain of
+//    multiply-adds (exp2_neg).  Table-driven exponentials: P.T.P. Tang, ACM
+//    TOMS 15 (1989).
+//
+// Relative errors, against 50 digits (tests/test_fix64.py): below 2^-52 for
+// every value, 2^-54 rms, where the FP64 formulas have 2^-49.4 (Gaussian), 2^-51
+// (1/(d + p0)) and 2^-51.5 (sqrt(d^2 + p0)) at worst and about 2^-53 rms, the
+// Gaussian 2^-52; a Wendland value near its cut-off keeps 6 bits more than in
+// FP64.
+#pragma once
+
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#ifdef __CUDACC__
+#define FX_HD __host__ __device__ __forceinline__
+#else
+#define FX_HD inline
+#endif
+
+namespace abx {
+namespace fx {
+
+typedef uint64_t u64;
+typedef int64_t i64;
+typedef uint32_t u32;
+
+FX_HD u32 hi32(u64 a) { return (u32)(a >> 32); }
+
+// a b / 2^64 to within 1 unit for a, b <= 2^63: the low x low product is left
+// out and the constant makes up for it and for the floor on average (the two
+// middle products and the constant cannot overflow their sum).
+FX_HD u64 mulhi63(u64 a, u64 b) {
+  const u64 w = ((u64)(u32)a * hi32(b) + 0xc0000000ull) + (u64)hi32(a) * (u32)b;
+  return (u64)hi32(a) * hi32(b) + (w >> 32);
+}
+
+FX_HD u64 bits_of(double x) {
+#ifdef __CUDA_ARCH__
+  return (u64)__double_as_longlong(x);
+#else
+  u64 u;
+  memcpy(&u, &x, 8);
+  return u;
+#endif
+}
+FX_HD double from_bits(u64 u) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((i64)u);
+#else
+  double x;
+  memcpy(&x, &u, 8);
+  return x;
+#endif
+}
+
+// x * 2^K modulo 2^64, rounded to nearest (half away from zero); x finite.
+// Differences of two such numbers are exact modulo 2^64 up to those roundings,
+// and bits of x at or above 2^-K are never lost.
+FX_HD i64 to_fixed(double x, int K) {
+  const u64 u = bits_of(x);
+  const int e = (int)((u >> 52) & 0x7ff);
+  const u64 m = (u & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+  const int sh = (e ? e : 1) - 1075 + K;  // value = m * 2^(sh) in units of 2^-K
+  u64 v;
+  if (sh >= 64)
+    v = 0;
+  else if (sh >= 0)
+    v = m << sh;
+  else if (sh > -64)
+    v = ((m >> (-sh - 1)) + 1) >> 1;
+  else
+    v = 0;
+  return (i64)((u >> 63) ? 0 - v : v);
+}
+
+// Adds dx^2 to the split sum: dx = h 2^32 + l, |l| <= 2^31.
+FX_HD void sq_acc(i64 d, i64 &S, i64 &T) {
+  const int32_t l = (int32_t)d;
+  const int32_t h = (int32_t)(d >> 32) - (l >> 31);
+  S += (i64)h * h;
+  T += (i64)h * l;
+}
+FX_HD u64 sq_low(i64 d) {
+  const int32_t l = (int32_t)d;
+  return (u64)((i64)l * l);
+}
+// |dx|^2 in units of 2^-63 R^2 (dx in units of 2^-62 R, |dx| <= R): 2^-60 S + 2^-91 T.
+FX_HD u64 sq_sum(i64 S, i64 T) { return ((u64)S << 3) + (u64)(T >> 28); }
+
+FX_HD float rsqrt32(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return 1.0f / sqrtf(x);
+#endif
+}
+FX_HD float rcp32(float x) {
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+#else
+  return 1.0f / x;
+#endif
+}
+FX_HD int f2i(float x) {  // to nearest
+#ifdef __CUDA_ARCH__
+  return __float2int_rn(x);
+#else
+  return (int)lrintf(x);
+#endif
+}
+FX_HD float fma32(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
+  return __fmaf_rn(a, b, c);
+#else
+  return fmaf(a, b, c);
+#endif
+}
+FX_HD int clz32(u32 x) {
+#ifdef __CUDA_ARCH__
+  return __clz((int)x);
+#else
+  return x ? __builtin_clz(x) : 32;
+#endif
+}
+
+// sqrt(u 2^-60) in units of 2^-62 for u <= 3 2^60 (a root up to 1.74); the
+// error is below 2^-60 for u >= 2^40.  q0 = the FP32 root as an integer (units
+// 2^-30, relative error below 2^-21.5); with res = u - q0^2 exact, the
+// correction is d - d^2 / (2 q0), d = res / (2 q0): D1 is d in units of 2^-50
+// to FP32 accuracy, R1 what D1 leaves of res (exact), and the last FP32 term
+// carries R1's and d^2's share.  u = 0 gives 0.
+FX_HD u64 sqrt60(u64 u) {
+  const float uf = fma32((float)hi32(u), 4294967296.0f, (float)(u32)u);
+  const float rs = rsqrt32(fmaxf(uf, 1.0f));
+  const int q0 = f2i(uf * rs);
+  const i64 res = (i64)u - (i64)q0 * q0;
+  const float d1 = (float)(int32_t)(res >> 11) * (rs * 1073741824.0f);  // 2^11 2^20 / 2
+  const int D1 = f2i(d1);
+  const i64 R1 = (i64)((u64)res << 20) - (i64)q0 * (2 * D1);
+  const float r1 = (float)(int32_t)(R1 >> 10);
+  const float c = fma32(d1 * d1, -9.3132257461547852e-10f, r1) * (rs * 2097152.0f);
+  const i64 low = (i64)D1 * 4096 + f2i(c);
+  return (((u64)(u32)q0) << 32) + (u64)low;
+}
+
+// m * 2^-s as a double, rounded to nearest; m != 0, the result normal.
+FX_HD double make_double(u64 m, int s) {
+  const u32 h = hi32(m);
+  const int z = h ? clz32(h) : 32 + clz32((u32)m);
+  const u64 n = m << z;  // top bit set
+  // 53 significant bits; the sum carries into the exponent where it rounds up
+  const u64 r = (n >> 11) + ((n >> 10) & 1);
+  return from_bits(r + ((u64)(1085 - z - s) << 52));
+}
+
+// ------------------------------------------------------------ exponential ---
+constexpr int EXP_TAB = 256;
+// 2^(-i/256) in units of 2^-63, from repeated integer square roots of 1/2 and
+// their products: within 3.4 units (2^-61), and the same on every compiler.
+struct ExpTable {
+  u64 v[EXP_TAB];
+};
+constexpr ExpTable make_exp_table() {
+  typedef unsigned __int128 u128;
+  u64 root[8] = {};  // 2^(-2^k/256) in units of 2^-64
+  u128 v = (u128)1 << 63;
+  for (int k = 7; k >= 0; --k) {
+    const u128 n = v << 64;
+    u128 s = 0;
+    for (int b = 63; b >= 0; --b) {
+      const u128 t = s | ((u128)1 << b);
+      if (t * t <= n) s = t;
+    }
+    v = s;
+    root[k] = (u64)s;
+  }
+  ExpTable T{};
+  for (int i = 0; i < EXP_TAB; ++i) {
+    u128 p = (u128)1 << 64;
+    for (int k = 0; k < 8; ++k)
+      if ((i >> k) & 1) p = (p * root[k]) >> 64;
+    T.v[i] = (u64)(p >> 1);
+  }
+  return T;
+}
+#ifdef __CUDACC__
+static __device__ const ExpTable exp_table = make_exp_table();
+#endif
+
+// 2^-t for t in units of 2^-54 (t < 2^64: below 1024, the result normal below
+// 1020), as a double.
+// t = n + i/256 + g, g < 2^-8 as y = 2^8 g in units of 2^-63 (G);
+// 1 - 2^-g = g (L1 - g (L2 - g (L3 - g (L4 - g L5)))), Lk = ln(2)^k / k!,
+// the first neglected term below 2^-60.  Every Horner step is one 32x32+64
+// multiply-add whose scale is folded into the constants:
+// E = 2^64 (1 - 2^-g).
+FX_HD double exp2_neg(u64 t, const u64 *tab) {
+  const u32 th = hi32(t);
+  const u64 G = (t & 0x3fffffffffffull) << 17;
+  const int32_t g = (int32_t)hi32(G);  // y in units of 2^-31
+  // n4 = -(L4 - g L5) in units of 2^-28; a3 = L3 - g(...) in units of 2^-35
+  const int32_t n4 = (int32_t)((((i64)g * 2796) - ((i64)2581847 << 32)) >> 32);
+  const int32_t a3 = (int32_t)((((i64)g * n4) + ((i64)1907106652 << 32)) >> 32);
+  const int32_t ga3 = (int32_t)(((i64)g * a3) >> 32);  // y a3 in units of 2^-34
+  // A2 = L2 - g a3 in units of 2^-50, A1 = L1 - g A2 in units of 2^-57
+  const u64 A2 = (u64)((i64)ga3 * -256 + (i64)270471001806380ll);
+  const u64 A1 = 99893036290645747ull - mulhi63(G, A2);
+  const u64 E = mulhi63(G, A1);
+  const u64 T = tab[(th >> 14) & (EXP_TAB - 1)];
+  const u64 M = T - mulhi63(T, E);  // in (2^62, 2^63]
+  const u64 m = (M + 512) >> 10;
+  return from_bits(m + ((u64)(1021u - (th >> 22)) << 52));
+}
+
+// ---------------------------------------------------------- kernel values ---
+// Kernel constants.  A product of two doubles keeps 106 bits as a pair hi + lo
+// (lo = fma(a, b, -a b)); scaled to an integer below 2^63.
+FX_HD u64 scaled(double hi, double lo, int shift) {
+  // hi 2^shift + lo 2^shift, hi >= 0: both parts are exact integers plus a rest
+  return (u64)(to_fixed(hi, shift) + to_fixed(lo, shift));
+}
+// a log2(e) in units of 2^-55, a < 177: log2(e) as the sum of two doubles
+FX_HD u64 gaussian_constant(double a) {
+  const double l = 1.4426950408889634, m = 2.0355273740931033e-17;
+  const double hi = a * l;
+  return scaled(hi, fma(a, l, -hi) + a * m, 55);
+}
+// (p0 2^r)^2 in units of 2^-61
+FX_HD u64 wendland_constant(double p0, int r) {
+  const double p = ldexp(p0, r), hi = p * p;
+  return scaled(hi, fma(p, p, -hi), 61);
+}
+// p0 / 2^r = pm 2^-62 2^-pe, pm in [2^62, 2^63) or 0; 0 <= p0 < 2^r
+FX_HD void laplace_constant(double p0, int r, u64 &pm, int &pe) {
+  pm = 0;
+  pe = 0;
+  if (p0 > 0.0) {
+    int e;
+    frexp(p0, &e);
+    pe = r + 1 - e;
+    pm = (u64)to_fixed(ldexp(p0, -e), 63);
+  }
+}
+
+// exp(-p0 d^2) = 2^-(s c): s = d^2 / R^2 <= 1 in units of 2^-63, c = p0 R^2
+// log2(e) < 256 in units of 2^-55.
+FX_HD double gaussian(u64 s, u64 c, const u64 *tab) { return exp2_neg(mulhi63(s, c), tab); }
+
+// Wendland C2 (1-q)^4 (4q+1) = t^4 (5 - 4t), t = 1 - q, for q^2 in units of
+// 2^-60; 0 for q >= 1.  t is normalised, so that the value keeps its relative
+// accuracy where t is small.
+FX_HD double wendland(u64 q2) {
+  if (q2 >= (1ull << 60)) return 0.0;
+  const i64 td = (i64)(1ull << 62) - (i64)sqrt60(q2);
+  const u64 t = ((u64)td << 1) - (u64)(td >> 62);  // units of 2^-63, below 2^63
+  const u32 th = hi32(t);
+  if (td <= 0 || th == 0) return 0.0;  // t < 2^-31: the value is below 2^-121
+  const int z = clz32(th) - 1;
+  const u64 tn = t << z;                // in [2^62, 2^63)
+  const u64 t2 = mulhi63(tn, tn) << 1;  // t^2 in units of 2^-63, >= 2^61
+  const u64 t4 = mulhi63(t2, t2) << 1;  // t^4 in units of 2^-63, >= 2^59
+  const u64 p = (5ull << 60) - (t >> 1);
+  return make_double(mulhi63(t4, p), 59 + 4 * z);
+}
+
+// |dx|^2 of a split sum with its low part U = sum l^2, normalised: the value
+// is n 2^-62 2^-z R^2 with n in [2^62, 2^64), z even; n = 0 when d < 2^-30 R.
+FX_HD u64 norm_d2(i64 S, i64 T, u64 U, int &z) {
+  const u64 lo = U + ((u64)T << 33);
+  const u64 hi = (u64)S + (u64)(T >> 31) + (lo < U ? 1u : 0u);  // units of 2^-60
+  const int k = (hi32(hi) ? clz32(hi32(hi)) : 32 + clz32((u32)hi)) & ~1;
+  z = k - 2;
+  return k < 64 ? (hi << k) | ((lo >> 1) >> (63 - k)) : 0;
+}
+
+// d >= 2^-7 R: the coordinates' rounding to 2^-62 R is below 2^-54 of d.  Closer
+// pairs are left to the FP64 formula on the double coordinates.
+FX_HD bool laplace_far(i64 S) { return S >= (i64)1 << 46; }
+// 1 / (d + p0) for laplace_far pairs: n, z as norm_d2 gives them (n != 0), p0 / R = pm 2^-62 2^-pe
+// with pm in [2^62, 2^63) (or 0) and pe >= 0, R = 2^r.
+FX_HD double laplace(u64 n, int z, u64 pm, int pe, int r) {
+  const u64 q = sqrt60(n >> 4);  // d = q 2^-62 2^(1 - z/2) R, q in [2^61, 2^62)
+  // a = d + p0 at the scale of the larger, a 2^-62 2^E R
+  const int sh = pe + 1 - (z >> 1);
+  u64 a;
+  int E;
+  if (sh >= 0) {
+    a = q + (sh < 64 ? pm >> sh : 0);
+    E = 1 - (z >> 1);
+  } else {
+    a = pm + (sh > -64 ? q >> -sh : 0);
+    E = -pe;
+  }
+  const int y = clz32(hi32(a)) - 1;  // a in [2^61, 2^64)
+  const u64 A = y < 0 ? a >> 1 : a << y;
+  // reciprocal of A 2^-62 in [1, 2): FP32 seed, then 1 + e + e^2
+  const u32 Y0 = (u32)f2i(rcp32((float)hi32(A) * 9.3132257461547852e-10f) * 1073741824.0f);
+  const u64 w = (u64)(u32)A * Y0;
+  const i64 er = (i64)((1ull << 60) - ((u64)hi32(A) * Y0 + (w >> 32)));
+  const i64 es = er >> 20;
+  const i64 e2 = er + ((es * es) >> 20);
+  const i64 add = ((i64)Y0 * (int32_t)(e2 >> 8) + (i64)(((u64)Y0 * (u32)(e2 & 255)) >> 8)) >> 20;
+  return make_double(((u64)Y0 << 32) + (u64)add, 62 + E - y + r);
+}
+
+// sqrt(d^2 + c): v = (d^2 + c) / R^2 in units of 2^-63, 2^-8 <= v 2^-63 < 1;
+// R = 2^r.
+FX_HD double multiquadric(u64 v, int r) {
+  const int k = (clz32(hi32(v)) - 1) | 1;
+  return make_double(sqrt60((v << k) >> 4), 62 + (k >> 1) - r);
+}
+
+}  // namespace fx
+}  // namespace abx

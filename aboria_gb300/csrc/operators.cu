@@ -11,6 +11,7 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "fix64.cuh"
 #include "handles.cuh"
 
 namespace abx {
@@ -72,7 +73,12 @@ template <int KIND> __device__ __forceinline__ float dk32(float d2, float p0f, f
   return 0.f;
 }
 
-template <int KIND> __global__ void __launch_bounds__(DT) k_dense_fp64(DenseParams P) {
+// `F` (may be null): leave at once where k_dense_fix has done the product.
+struct DenseFix;
+__device__ bool dense_fix_done(const DenseFix *F);
+template <int KIND>
+__global__ void __launch_bounds__(DT) k_dense_fp64(DenseParams P, const DenseFix *F) {
+  if (F && dense_fix_done(F)) return;
   __shared__ double sx[DT], sy[DT], sz[DT], sb[DT], ss[DT];
   const int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x;
   const bool act = i < P.nr;
@@ -187,6 +193,217 @@ __global__ void __launch_bounds__(DT) k_dense_mixed(DenseParams P, int64_t chunk
   }
 }
 
+// ---------------------------------------------------- FP64 on integer units ---
+// The default (FP64) dense product, for kernels and sizes that fix64.cuh
+// covers: every pair costs one FP64 multiply-add instead of ~30 FP64
+// operations.  Bounds: integer ALU (about 50 operations a pair at 62 a clock
+// and SM) next to the one FP64 multiply-add (at 1.8).  Rows stay one a
+// thread; columns, as fixed-point coordinates with their weights, are staged
+// 256 at a time and read by broadcast; column chunks (blockIdx.y) fill the GPU
+// when there are few rows and are added in order.  N = 32,768 x 30,011
+// Gaussian: 57.6 -> 4.4 ms (error against 64 bits 5.2e-15 -> 1.2e-15).
+//
+// The unit R of the fixed-point coordinates (a power of two no smaller than
+// the diagonal of both sets' bounding box) is found on the device by
+// k_dense_range; k_dense_prep checks what it allows and writes `ok`.  Where it
+// does not allow the integer path (a coordinate that is not finite, a Gaussian
+// narrower than c = p0 R^2 log2(e) = 255, whose argument would lose bits; a
+// Wendland support below R / 2; a multiquadric with p0 < R^2 / 256; a Laplace
+// softening of R and above or negative), k_dense_fix leaves at once and
+// k_dense_fp64 does the work; otherwise k_dense_fp64 leaves at once.
+struct DenseFix {
+  int ok, K, r;    // X = x 2^K, R = 2^r
+  int pe;          // Laplace: p0 / R = pm 2^-62 2^-pe
+  fx::u64 c;       // kernel constant, pm for Laplace
+  unsigned long long range[6];  // ordered bits: max of x_d, then max of -x_d
+};
+struct alignas(32) FixCol {
+  long long x, y, z;
+  double b;
+};
+
+__device__ bool dense_fix_done(const DenseFix *F) { return F->ok != 0; }
+
+__device__ __forceinline__ unsigned long long ordered_bits(unsigned long long u) {
+  return (u >> 63) ? ~u : u | 0x8000000000000000ull;
+}
+__device__ __forceinline__ double from_ordered(unsigned long long k) {
+  return __longlong_as_double((long long)((k >> 63) ? k & 0x7fffffffffffffffull : ~k));
+}
+
+// Maxima of x_d and -x_d over a point set, on the bits in an order-preserving
+// form: a NaN of either sign sorts beyond the infinities and is caught with
+// them (floating-point negation and comparison would lose its sign).
+__global__ void __launch_bounds__(DT) k_dense_range(const double *__restrict__ a, int64_t na,
+                                                    const double *__restrict__ b, int64_t nb,
+                                                    int dim, DenseFix *__restrict__ F) {
+  __shared__ unsigned long long red[DT / 32];
+  const int64_t step = (int64_t)gridDim.x * DT;
+  for (int d = 0; d < dim; ++d) {
+    unsigned long long hi = 0, lo = 0;
+    for (int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x; i < na + nb; i += step) {
+      const unsigned long long u = (unsigned long long)__double_as_longlong(
+          i < na ? a[d * na + i] : b[d * nb + (i - na)]);
+      hi = max(hi, ordered_bits(u));
+      lo = max(lo, ordered_bits(u ^ 0x8000000000000000ull));
+    }
+    for (int s = 0; s < 2; ++s) {
+      unsigned long long v = s ? lo : hi;
+      for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int w = 1; w < DT / 32; ++w) v = max(v, red[w]);
+        atomicMax(&F->range[3 * s + d], v);
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// The unit and the kernel's constant from the ranges (one thread's work, done
+// by every CTA that needs it before its columns).
+template <int KIND> __device__ void dense_unit(const DenseParams &P, DenseFix &F) {
+  double ext2 = 0.0;
+  bool ok = true;
+  for (int d = 0; d < P.dim; ++d) {
+    const double hi = from_ordered(F.range[d]), lo = -from_ordered(F.range[3 + d]);
+    ok = ok && isfinite(hi) && isfinite(lo);
+    ext2 += (hi - lo) * (hi - lo);
+  }
+  double r2 = ext2;
+  if (KIND == ABX_K_MULTIQUADRIC) r2 += P.p0;
+  ok = ok && r2 < 1e200 && (r2 > 1e-200 || ext2 == 0.0) && isfinite(P.p0);
+  int e = 0;
+  frexp(sqrt(ext2 == 0.0 && KIND != ABX_K_MULTIQUADRIC ? 1.0 : r2) * (1.0 + 1e-12), &e);
+  F.r = e;  // R = 2^e > sqrt(r2)
+  F.K = 62 - e;
+  const double R2 = ldexp(1.0, 2 * e);
+  F.pe = 0;
+  F.c = 0;
+  if (KIND == ABX_K_GAUSSIAN || KIND == ABX_K_COMPACT_GAUSSIAN) {
+    ok = ok && P.p0 >= 0.0 && P.p0 * R2 * 1.4426950408889634 < 255.0;
+    if (ok) F.c = fx::gaussian_constant(P.p0 * R2);
+  } else if (KIND == ABX_K_WENDLAND_C2) {
+    ok = ok && P.p0 >= 0.0 && P.p0 * P.p0 * R2 < 3.99;
+    if (ok) F.c = fx::wendland_constant(P.p0, e);
+  } else if (KIND == ABX_K_MULTIQUADRIC) {
+    ok = ok && P.p0 >= R2 * (1.0 / 256.0);
+    if (ok) F.c = (fx::u64)ldexp(P.p0, 63 - 2 * e);
+  } else if (KIND == ABX_K_LAPLACE) {
+    ok = ok && P.p0 >= 0.0 && P.p0 < ldexp(1.0, e);
+    if (ok) fx::laplace_constant(P.p0, e, F.c, F.pe);
+  } else
+    ok = false;
+  F.ok = ok ? 1 : 0;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(DT) k_dense_prep(DenseParams P, DenseFix *__restrict__ Fg,
+                                                   FixCol *__restrict__ cols) {
+  __shared__ DenseFix F;
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < 6; ++k) F.range[k] = Fg->range[k];
+    dense_unit<KIND>(P, F);
+    if (blockIdx.x == 0) {
+      Fg->ok = F.ok;
+      Fg->K = F.K;
+      Fg->r = F.r;
+      Fg->pe = F.pe;
+      Fg->c = F.c;
+    }
+  }
+  __syncthreads();
+  const int64_t j = (int64_t)blockIdx.x * DT + threadIdx.x;
+  if (!F.ok || j >= P.nc) return;
+  FixCol c;
+  c.x = fx::to_fixed(P.cpos[j], F.K);
+  c.y = P.dim > 1 ? fx::to_fixed(P.cpos[P.nc + j], F.K) : 0;
+  c.z = P.dim > 2 ? fx::to_fixed(P.cpos[2 * P.nc + j], F.K) : 0;
+  c.b = P.b[j];
+  cols[j] = c;
+}
+
+// Kernel value of one pair from its fixed-point differences; `far` false: too
+// close for the Laplace kernel's fixed point, the caller evaluates in FP64.
+template <int KIND>
+__device__ __forceinline__ double dense_value(long long dx, long long dy, long long dz, int dim,
+                                              const DenseFix &F, const fx::u64 *tab, bool &far) {
+  fx::i64 S = 0, T = 0;
+  fx::sq_acc(dx, S, T);
+  if (dim > 1) fx::sq_acc(dy, S, T);
+  if (dim > 2) fx::sq_acc(dz, S, T);
+  far = true;
+  if (KIND == ABX_K_LAPLACE) {
+    fx::u64 U = fx::sq_low(dx);
+    if (dim > 1) U += fx::sq_low(dy);
+    if (dim > 2) U += fx::sq_low(dz);
+    far = fx::laplace_far(S);
+    int z;
+    const fx::u64 n = fx::norm_d2(S, T, U, z);
+    return fx::laplace(n, z, F.c, F.pe, F.r);
+  }
+  const fx::u64 s = fx::sq_sum(S, T);
+  if (KIND == ABX_K_WENDLAND_C2) return fx::wendland(fx::mulhi63(s, F.c));
+  if (KIND == ABX_K_MULTIQUADRIC) return fx::multiquadric(s + F.c, F.r);
+  return fx::gaussian(s, F.c, tab);
+}
+
+template <int KIND, int DIM>
+__global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix *__restrict__ Fg,
+                                                  const FixCol *__restrict__ cols,
+                                                  int64_t chunk_cols, double *__restrict__ partial) {
+  __shared__ FixCol sc[DT];
+  __shared__ fx::u64 tab[fx::EXP_TAB];
+  DenseFix F;
+  F.ok = Fg->ok;
+  F.K = Fg->K;
+  F.r = Fg->r;
+  F.pe = Fg->pe;
+  F.c = Fg->c;
+  if (!F.ok) return;
+  if (KIND == ABX_K_GAUSSIAN) tab[threadIdx.x] = fx::exp_table.v[threadIdx.x];
+  const int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x;
+  const bool act = i < P.nr;
+  long long x = 0, y = 0, z = 0;
+  if (act) {
+    x = fx::to_fixed(P.rpos[i], F.K);
+    if (DIM > 1) y = fx::to_fixed(P.rpos[P.nr + i], F.K);
+    if (DIM > 2) z = fx::to_fixed(P.rpos[2 * P.nr + i], F.K);
+  }
+  double acc = 0.0;
+  const int64_t c0 = (int64_t)blockIdx.y * chunk_cols;
+  const int64_t c1 = c0 + chunk_cols < P.nc ? c0 + chunk_cols : P.nc;
+  for (int64_t t = c0; t < c1; t += DT) {
+    __syncthreads();
+    if (t + threadIdx.x < c1) sc[threadIdx.x] = cols[t + threadIdx.x];
+    __syncthreads();
+    const int nt = (int)((c1 - t) < DT ? (c1 - t) : DT);
+#pragma unroll 2
+    for (int jj = 0; jj < nt; ++jj) {
+      const FixCol q = sc[jj];
+      bool far;
+      double v = dense_value<KIND>((long long)((fx::u64)q.x - (fx::u64)x),
+                                   (long long)((fx::u64)q.y - (fx::u64)y),
+                                   (long long)((fx::u64)q.z - (fx::u64)z), DIM, F, tab, far);
+      if (KIND == ABX_K_LAPLACE && !far) {
+        double d2 = 0.0;
+        if (act)
+          for (int d = 0; d < DIM; ++d) {
+            const double dx = P.cpos[d * P.nc + t + jj] - P.rpos[d * P.nr + i];
+            d2 = __dadd_rn(d2, __dmul_rn(dx, dx));
+          }
+        v = dk64<KIND>(d2, P.p0, 0.0, 0.0);
+      }
+      acc = fma(v, q.b, acc);
+    }
+  }
+  if (act) {
+    if (partial) partial[(int64_t)blockIdx.y * P.nr + i] = acc;
+    else P.c[i] = acc;
+  }
+}
+
 __global__ void k_dense_reduce(const double *__restrict__ partial, int64_t nr, int chunks,
                                double *__restrict__ c) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -196,18 +413,52 @@ __global__ void k_dense_reduce(const double *__restrict__ partial, int64_t nr, i
   c[i] = s;
 }
 
+// Columns in chunks of whole tiles when the rows alone give fewer than about
+// per_sm CTAs per SM; returns the number of chunks, at least 1.
+int dense_chunks(abx_context *ctx, int64_t nc, unsigned blocks, int per_sm, int64_t &chunk_cols) {
+  const int64_t tiles = (nc + DT - 1) / DT;
+  const int64_t want = (per_sm * (int64_t)std::max(ctx->num_sms, 1) + blocks - 1) / blocks;
+  const int chunks = (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min<int64_t>(tiles, 65535)));
+  // no columns: one chunk that writes zeros
+  chunk_cols = tiles > 0 ? ((tiles + chunks - 1) / chunks) * DT : DT;
+  return tiles > 0 ? (int)((nc + chunk_cols - 1) / chunk_cols) : 1;
+}
+
+template <int KIND>
+int launch_dense_fix(abx_context *ctx, const DenseParams &P, abx_operator *op) {
+  cudaStream_t s = ctx->stream;
+  const unsigned blocks = ceil_div(P.nr, DT);
+  int64_t chunk_cols;
+  const int used = dense_chunks(ctx, P.nc, blocks, 16, chunk_cols);
+  // one buffer: the unit, the columns, the chunks' row sums
+  const size_t nf = sizeof(DenseFix) / 8 + 4, nb = (sizeof(FixCol) / 8) * (size_t)P.nc;
+  ABX_TRY(op->partial.reserve(nf + nb + (used > 1 ? (size_t)used * P.nr : 0)));
+  DenseFix *F = reinterpret_cast<DenseFix *>(op->partial.ptr);
+  FixCol *cols = reinterpret_cast<FixCol *>(op->partial.ptr + (nf / 4) * 4);
+  double *partial = used > 1 ? op->partial.ptr + (nf / 4) * 4 + nb : nullptr;
+  ABX_CHECK_CUDA(cudaMemsetAsync(F, 0, sizeof(DenseFix), s));
+  const unsigned rb = std::min(ceil_div(P.nr + P.nc, DT), 2u * (unsigned)std::max(ctx->num_sms, 1));
+  k_dense_range<<<rb, DT, 0, s>>>(P.rpos, P.nr, P.cpos, P.nc, P.dim, F);
+  k_dense_prep<KIND><<<std::max(1u, ceil_div(P.nc, DT)), DT, 0, s>>>(P, F, cols);
+  const dim3 grid(blocks, used);
+  if (P.dim == 3)
+    k_dense_fix<KIND, 3><<<grid, DT, 0, s>>>(P, F, cols, chunk_cols, partial);
+  else if (P.dim == 2)
+    k_dense_fix<KIND, 2><<<grid, DT, 0, s>>>(P, F, cols, chunk_cols, partial);
+  else
+    k_dense_fix<KIND, 1><<<grid, DT, 0, s>>>(P, F, cols, chunk_cols, partial);
+  if (partial) k_dense_reduce<<<ceil_div(P.nr, 256), 256, 0, s>>>(partial, P.nr, used, P.c);
+  k_dense_fp64<KIND><<<blocks, DT, 0, s>>>(P, F);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  return ABX_OK;
+}
+
 template <int KIND>
 int launch_dense(abx_context *ctx, const DenseParams &P, bool mixed, abx_operator *op) {
   const unsigned blocks = ceil_div(P.nr, DT);
   if (mixed && KIND != ABX_K_SCALAR_SUM) {
-    // about 32 CTAs per SM in all: split the columns when the rows alone
-    // give fewer
-    const int64_t tiles = (P.nc + DT - 1) / DT;
-    const int64_t want = (32 * (int64_t)std::max(ctx->num_sms, 1) + blocks - 1) / blocks;
-    const int chunks = (int)std::max<int64_t>(1, std::min<int64_t>(want, std::min<int64_t>(tiles, 65535)));
-    // no columns: one chunk that writes zeros
-    const int64_t chunk_cols = tiles > 0 ? ((tiles + chunks - 1) / chunks) * DT : DT;
-    const int used = tiles > 0 ? (int)((P.nc + chunk_cols - 1) / chunk_cols) : 1;
+    int64_t chunk_cols;
+    const int used = dense_chunks(ctx, P.nc, blocks, 32, chunk_cols);
     double *partial = nullptr;
     if (used > 1) {
       ABX_TRY(op->partial.reserve((size_t)used * P.nr));
@@ -217,8 +468,15 @@ int launch_dense(abx_context *ctx, const DenseParams &P, bool mixed, abx_operato
                                                                                partial);
     if (partial)
       k_dense_reduce<<<ceil_div(P.nr, 256), 256, 0, ctx->stream>>>(partial, P.nr, used, P.c);
-  } else
-    k_dense_fp64<KIND><<<blocks, DT, 0, ctx->stream>>>(P);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
+  if constexpr (KIND != ABX_K_CONST && KIND != ABX_K_SCALAR_SUM) {
+    // the two Gaussians share one instantiation
+    if (P.nc > 0)
+      return launch_dense_fix<KIND == ABX_K_COMPACT_GAUSSIAN ? ABX_K_GAUSSIAN : KIND>(ctx, P, op);
+  }
+  k_dense_fp64<KIND><<<blocks, DT, 0, ctx->stream>>>(P, nullptr);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }

@@ -1,0 +1,113 @@
+"""FP64-accurate kernel values from integer arithmetic (csrc/fix64.cuh), on the
+CPU against 50-digit decimals: the same header the GPU kernels include."""
+import ctypes as C
+import random
+import subprocess
+from decimal import Decimal, getcontext
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+getcontext().prec = 50
+SRC = r"""
+#include "fix64.cuh"
+using namespace abx::fx;
+static constexpr ExpTable TAB = make_exp_table();
+static void sums(const double *x, const double *y, int dim, int K, i64 &S, i64 &T, u64 &U) {
+  S = T = 0; U = 0;
+  for (int d = 0; d < dim; ++d) {
+    const i64 dx = (i64)((u64)to_fixed(y[d], K) - (u64)to_fixed(x[d], K));
+    sq_acc(dx, S, T);
+    U += sq_low(dx);
+  }
+}
+extern "C" {
+double v_gauss(const double *x, const double *y, int dim, int r, double p0) {
+  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
+  return gaussian(sq_sum(S, T), gaussian_constant(ldexp(p0, 2 * r)), TAB.v);
+}
+double v_wend(const double *x, const double *y, int dim, int r, double p0) {
+  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
+  return wendland(mulhi63(sq_sum(S, T), wendland_constant(p0, r)));
+}
+double v_lap(const double *x, const double *y, int dim, int r, double p0) {
+  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
+  u64 pm; int pe, z; laplace_constant(p0, r, pm, pe);
+  const u64 n = norm_d2(S, T, U, z);
+  return laplace_far(S) ? laplace(n, z, pm, pe, r) : -1.0;
+}
+double v_mq(const double *x, const double *y, int dim, int r, double p0) {
+  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
+  return multiquadric(sq_sum(S, T) + (u64)ldexp(p0, 63 - 2 * r), r);
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("fix64")
+    (d / "fix64_host.cpp").write_text(SRC)
+    so = d / "fix64_host.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I",
+                    str(ROOT / "aboria_gb300" / "csrc"), str(d / "fix64_host.cpp"), "-o", str(so)],
+                   check=True)
+    lib = C.CDLL(str(so))
+    for f in ("v_gauss", "v_wend", "v_lap", "v_mq"):
+        getattr(lib, f).restype = C.c_double
+    return lib
+
+
+def _exact(kind, x, y, p0):
+    d2 = sum((Decimal(b) - Decimal(a)) ** 2 for a, b in zip(x, y))
+    p = Decimal(p0)
+    if kind == "gauss":
+        return (-d2 * p).exp(), Decimal(0)
+    if kind == "lap":
+        return 1 / (d2.sqrt() + p), Decimal(0)
+    if kind == "mq":
+        return (d2 + p).sqrt(), Decimal(0)
+    q = d2.sqrt() * p
+    t = 1 - q
+    # the slope of the value times the root's error
+    return (t ** 4 * (4 * q + 1), 20 * q * abs(t) ** 3 * Decimal(2) ** -59) if t > 0 else (Decimal(0), Decimal(0))
+
+
+@pytest.mark.parametrize("kind,p0r2", [("gauss", 4.0), ("gauss", 21.0), ("wend", 1.0),
+                                       ("lap", 0.0), ("lap", 1e-11), ("lap", 0.02), ("lap", 0.4),
+                                       ("mq", 0.02), ("mq", 0.7)])
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_values_within_an_ulp(lib, kind, p0r2, dim):
+    rng = random.Random(7 * dim + len(kind))
+    for case in range(300):
+        radius = rng.choice([0.02, 0.05, 1.0, 37.0])
+        # points of [-4, 4] radii, pairs from nearly touching to the radius
+        x = [rng.uniform(-4, 4) * radius for _ in range(dim)]
+        dist = radius * 2.0 ** -rng.uniform(0, 9)
+        v = [rng.gauss(0, 1) for _ in range(dim)]
+        n = sum(c * c for c in v) ** 0.5
+        y = [a + dist * 0.999 * c / n for a, c in zip(x, v)]
+        p0 = {"gauss": p0r2 / radius ** 2, "wend": p0r2 / radius, "lap": p0r2 * radius,
+              "mq": p0r2 * radius ** 2}[kind]
+        reach = radius if kind != "mq" else (radius ** 2 + p0) ** 0.5
+        r = 0
+        while 2.0 ** r < reach * 1.0001:
+            r += 1
+        while 2.0 ** (r - 1) >= reach * 1.0001:
+            r -= 1
+        X, Y = (C.c_double * dim)(*x), (C.c_double * dim)(*y)
+        got = Decimal(getattr(lib, "v_" + kind)(X, Y, dim, r, C.c_double(p0)))
+        want, slack = _exact(kind, x, y, p0)
+        if got == -1:  # left to the FP64 formula: closer than R / 128
+            assert kind == "lap" and dist < 2.0 ** (r - 7)
+            continue
+        assert abs(got - want) <= want * Decimal(2) ** -52 + slack, (case, x, y, p0, got, want)
+
+
+def test_limits(lib):
+    x, far = (C.c_double * 1)(0.25), (C.c_double * 1)(0.25 + 0.5)
+    assert lib.v_gauss(x, x, 1, 0, C.c_double(3.0)) == 1.0
+    assert lib.v_wend(x, x, 1, -1, C.c_double(2.0)) == 1.0
+    assert lib.v_wend(x, far, 1, -1, C.c_double(2.0)) == 0.0     # q = 1
+    assert lib.v_mq(x, x, 1, 0, C.c_double(0.25)) == 0.5
