@@ -7,13 +7,15 @@
 // 10-20, the rest the polynomial and the product); here everything but the
 // last multiply-add into the row's FP64 sum runs on the integer pipe:
 //
-//  * coordinates are 64-bit fixed point, X = x * 2^K modulo 2^64.  A double's
-//    bits are shifted, not rounded, down to 2^-K, and differences that fit in
-//    62 bits are exact whatever wrapped on the way (to_fixed);
-//  * the squared distance keeps 63 fractional bits of the unit R^2,
-//    R = 2^(62-K) >= |dx| (sq_acc, sq_sum): each dx = h 2^32 + l with a signed
-//    low half; h^2 and h l are summed exactly and l^2 (below 2^-62) is left
-//    out;
+//  * coordinates are 64-bit fixed point modulo 2^64, X = x f in a unit 2^-k
+//    (to_fixed): differences that fit in 63 bits are exact whatever wrapped on
+//    the way.  f is a power of two, so that a double's bits are shifted and
+//    not rounded down to the unit, or, where that saves the pair a product,
+//    the kernel's own scale: sqrt(p0 log2(e)) for the Gaussian, p0 for the
+//    Wendland kernel, held to 100 bits (Unit);
+//  * each difference is split as h 2^32 + l with a signed low half; h^2 and h l
+//    are summed exactly, l^2 (below the unit of the sum) is left out except
+//    where the kernel is singular (sq_acc);
 //  * sqrt starts from the hardware's FP32 reciprocal square root and takes
 //    two corrections from exact integer residuals (sqrt60);
 //  * 2^-t splits t into an exponent, an index of a 256-entry table and a rest
@@ -74,39 +76,82 @@ FX_HD double from_bits(u64 u) {
 #endif
 }
 
-// x * 2^K modulo 2^64, rounded to nearest (half away from zero); x finite.
-// Differences of two such numbers are exact modulo 2^64 up to those roundings,
-// and bits of x at or above 2^-K are never lost.
-FX_HD i64 to_fixed(double x, int K) {
+FX_HD u64 mulhi64(u64 a, u64 b) {
+#ifdef __CUDA_ARCH__
+  return __umul64hi(a, b);
+#else
+  return (u64)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// A positive factor f = F 2^-ef, F = fh 2^64 + fl with the top bit set.
+struct Factor {
+  u64 fh, fl;
+  int ef;
+};
+// f = hi + lo, hi > 0 normal, |lo| <= ulp(hi)
+FX_HD Factor make_factor(double hi, double lo) {
+  const u64 u = bits_of(hi);
+  const int e = (int)(u >> 52) - 1023;
+  Factor F;
+  F.fh = (u << 11) | (1ull << 63);
+  F.fl = 0;
+  F.ef = 127 - e;
+  // lo in units of 2^(e - 127): 75 bits at most
+  const double l1 = ldexp(lo, 63 - e);  // units of 2^64 F units
+  const double w = floor(l1);
+  F.fh += (u64)(i64)w;
+  F.fl = (u64)ldexp(l1 - w, 63) << 1;
+  return F;
+}
+
+// x f 2^k modulo 2^64, rounded to nearest; x finite.
+FX_HD i64 to_fixed(double x, const Factor &F, int k) {
   const u64 u = bits_of(x);
   const int e = (int)((u >> 52) & 0x7ff);
   const u64 m = (u & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
-  const int sh = (e ? e : 1) - 1075 + K;  // value = m * 2^(sh) in units of 2^-K
+  // |x| = m 2^(max(e, 1) - 1075); m F as three words
+  const u64 p0 = m * F.fl, t = mulhi64(m, F.fl), a = m * F.fh;
+  const u64 p1 = a + t, p2 = mulhi64(m, F.fh) + (p1 < a ? 1u : 0u);
+  const int s = (e ? e : 1) - 1075 - F.ef + k;  // value = m F 2^s
   u64 v;
-  if (sh >= 64)
+  if (s >= 64)
     v = 0;
-  else if (sh >= 0)
-    v = m << sh;
-  else if (sh > -64)
-    v = ((m >> (-sh - 1)) + 1) >> 1;
-  else
-    v = 0;
+  else if (s >= 0)
+    v = p0 << s;
+  else {
+    const int r = -s, w = r >> 6, b = r & 63;
+    const u64 lo = w == 0 ? p0 : w == 1 ? p1 : w == 2 ? p2 : 0;
+    const u64 hi = w == 0 ? p1 : w == 1 ? p2 : 0;
+    v = b ? (lo >> b) | (hi << (64 - b)) : lo;
+    // the bit below the unit rounds
+    const int rb = r - 1, rw = rb >> 6;
+    const u64 below = rw == 0 ? p0 : rw == 1 ? p1 : rw == 2 ? p2 : 0;
+    v += (below >> (rb & 63)) & 1;
+  }
   return (i64)((u >> 63) ? 0 - v : v);
 }
 
-// Adds dx^2 to the split sum: dx = h 2^32 + l, |l| <= 2^31.
+// A query's coordinate is kept shifted by 2^31 (biased), so that the upper half
+// of a difference comes out rounded and its lower half as a signed number with
+// the top bit inverted.
+FX_HD i64 biased(i64 q) { return (i64)((u64)q - 0x80000000ull); }
+FX_HD i64 diff(i64 x, i64 q_biased) { return (i64)((u64)x - (u64)q_biased); }
+FX_HD int32_t low_of(i64 d) { return (int32_t)((u32)d ^ 0x80000000u); }
+// Adds dx^2 to the split sum (d as diff() gives it).
 FX_HD void sq_acc(i64 d, i64 &S, i64 &T) {
-  const int32_t l = (int32_t)d;
-  const int32_t h = (int32_t)(d >> 32) - (l >> 31);
+  const int32_t h = (int32_t)(d >> 32), l = low_of(d);
   S += (i64)h * h;
   T += (i64)h * l;
 }
 FX_HD u64 sq_low(i64 d) {
-  const int32_t l = (int32_t)d;
+  const int32_t l = low_of(d);
   return (u64)((i64)l * l);
 }
-// |dx|^2 in units of 2^-63 R^2 (dx in units of 2^-62 R, |dx| <= R): 2^-60 S + 2^-91 T.
-FX_HD u64 sq_sum(i64 S, i64 T) { return ((u64)S << 3) + (u64)(T >> 28); }
+// The sum in units of u^2 2^64 for coordinates in units of u ...
+FX_HD u64 sq_sum(i64 S, i64 T) { return (u64)S + (u64)(T >> 31); }
+// ... and with three bits more (a sum below 2^60 of those units).
+FX_HD u64 sq_sum8(i64 S, i64 T) { return ((u64)S << 3) + (u64)(T >> 28); }
 
 FX_HD float rsqrt32(float x) {
 #ifdef __CUDA_ARCH__
@@ -181,7 +226,9 @@ FX_HD double make_double(u64 m, int s) {
 // ------------------------------------------------------------ exponential ---
 constexpr int EXP_TAB = 256;
 // 2^(-i/256) in units of 2^-63, from repeated integer square roots of 1/2 and
-// their products: within 3.4 units (2^-61), and the same on every compiler.
+// their products: within 3.4 units (2^-61), and the same on every compiler;
+// plus the half unit (512) that rounds a value to 53 bits, less what the
+// products' floors leave out on average (3e-17 of the value).
 struct ExpTable {
   u64 v[EXP_TAB];
 };
@@ -204,7 +251,7 @@ constexpr ExpTable make_exp_table() {
     u128 p = (u128)1 << 64;
     for (int k = 0; k < 8; ++k)
       if ((i >> k) & 1) p = (p * root[k]) >> 64;
-    T.v[i] = (u64)(p >> 1);
+    T.v[i] = (u64)(p >> 1) + 305;
   }
   return T;
 }
@@ -232,45 +279,11 @@ FX_HD double exp2_neg(u64 t, const u64 *tab) {
   const u64 A1 = 99893036290645747ull - mulhi63(G, A2);
   const u64 E = mulhi63(G, A1);
   const u64 T = tab[(th >> 14) & (EXP_TAB - 1)];
-  const u64 M = T - mulhi63(T, E);  // in (2^62, 2^63]
-  const u64 m = (M + 512) >> 10;
+  const u64 m = (T - mulhi63(T, E)) >> 10;  // 53 bits; 2^53 carries into the exponent
   return from_bits(m + ((u64)(1021u - (th >> 22)) << 52));
 }
 
 // ---------------------------------------------------------- kernel values ---
-// Kernel constants.  A product of two doubles keeps 106 bits as a pair hi + lo
-// (lo = fma(a, b, -a b)); scaled to an integer below 2^63.
-FX_HD u64 scaled(double hi, double lo, int shift) {
-  // hi 2^shift + lo 2^shift, hi >= 0: both parts are exact integers plus a rest
-  return (u64)(to_fixed(hi, shift) + to_fixed(lo, shift));
-}
-// a log2(e) in units of 2^-55, a < 177: log2(e) as the sum of two doubles
-FX_HD u64 gaussian_constant(double a) {
-  const double l = 1.4426950408889634, m = 2.0355273740931033e-17;
-  const double hi = a * l;
-  return scaled(hi, fma(a, l, -hi) + a * m, 55);
-}
-// (p0 2^r)^2 in units of 2^-61
-FX_HD u64 wendland_constant(double p0, int r) {
-  const double p = ldexp(p0, r), hi = p * p;
-  return scaled(hi, fma(p, p, -hi), 61);
-}
-// p0 / 2^r = pm 2^-62 2^-pe, pm in [2^62, 2^63) or 0; 0 <= p0 < 2^r
-FX_HD void laplace_constant(double p0, int r, u64 &pm, int &pe) {
-  pm = 0;
-  pe = 0;
-  if (p0 > 0.0) {
-    int e;
-    frexp(p0, &e);
-    pe = r + 1 - e;
-    pm = (u64)to_fixed(ldexp(p0, -e), 63);
-  }
-}
-
-// exp(-p0 d^2) = 2^-(s c): s = d^2 / R^2 <= 1 in units of 2^-63, c = p0 R^2
-// log2(e) < 256 in units of 2^-55.
-FX_HD double gaussian(u64 s, u64 c, const u64 *tab) { return exp2_neg(mulhi63(s, c), tab); }
-
 // Wendland C2 (1-q)^4 (4q+1) = t^4 (5 - 4t), t = 1 - q, for q^2 in units of
 // 2^-60; 0 for q >= 1.  t is normalised, so that the value keeps its relative
 // accuracy where t is small.
@@ -333,6 +346,102 @@ FX_HD double laplace(u64 n, int z, u64 pm, int pe, int r) {
 FX_HD double multiquadric(u64 v, int r) {
   const int k = (clz32(hi32(v)) - 1) | 1;
   return make_double(sqrt60((v << k) >> 4), 62 + (k >> 1) - r);
+}
+
+// ------------------------------------------------------------------- units ---
+// The fixed point of one kernel for pairs up to `reach` apart: coordinates
+// X = x f 2^k, and the kernel's constant (c, pe).  ok false: the kernel's
+// parameter or the reach is outside what the value functions cover --
+//   Gaussian      t = p0 d^2 log2(e) must stay below 255 (at 16 and above the
+//                 coordinates' 63 bits overflow);
+//   Wendland      q must stay below 1.99 (the same);
+//   multiquadric  p0 >= R^2 / 256: sqrt60 loses relative accuracy below;
+//   Laplace       0 <= p0 < R.
+// R = 2^r: the power of two above the reach (above sqrt(reach^2 + p0)).
+struct Unit {
+  int ok, k, r, pe;
+  u64 c;
+  Factor f;
+};
+enum { GAUSSIAN = 1, WENDLAND = 2, LAPLACE = 4, MULTIQUADRIC = 5 };  // as abx.h numbers them
+
+template <int KIND> FX_HD Unit make_unit(double p0, double reach) {
+  Unit U;
+  U.ok = 0;
+  U.k = U.r = U.pe = 0;
+  U.c = 0;
+  U.f = make_factor(1.0, 0.0);
+  double reach2 = reach * reach;
+  if (KIND == MULTIQUADRIC) reach2 += p0;
+  if (!(p0 >= 0.0) || !(p0 < 1e200) || !(reach2 > 1e-200) || !(reach2 < 1e200)) return U;
+  int e = 0;
+  frexp(sqrt(reach2) * (1.0 + 1e-12), &e);
+  U.r = e;
+  if (KIND == GAUSSIAN) {
+    if (!(p0 > 1e-200) || p0 * reach2 * 1.4426950408889634 >= 255.0) return U;
+    // sqrt(p0 log2(e)) as hi + lo: log2(e) as a sum of two doubles, one
+    // Newton step on the square root
+    const double l = 1.4426950408889634, m = 2.0355273740931033e-17;
+    const double ah = p0 * l, al = fma(p0, l, -ah) + p0 * m;
+    const double s = sqrt(ah), lo = (fma(-s, s, ah) + al) / (2.0 * s);
+    U.f = make_factor(s + lo, lo - ((s + lo) - s));
+    U.k = 59;  // t = sum X^2 in units of 2^-54
+  } else if (KIND == WENDLAND) {
+    if (!(p0 > 1e-100) || p0 * p0 * reach2 >= 3.96) return U;
+    U.f = make_factor(p0, 0.0);
+    U.k = 62;  // q^2 in units of 2^-60
+  } else {
+    U.k = 62 - e;
+    if (KIND == MULTIQUADRIC) {
+      if (p0 < ldexp(1.0, 2 * e - 8)) return U;
+      U.c = (u64)ldexp(p0, 63 - 2 * e);
+    } else if (KIND == LAPLACE) {
+      if (p0 >= ldexp(1.0, e)) return U;
+      if (p0 > 0.0) {  // p0 / R = c 2^-62 2^-pe, c in [2^62, 2^63)
+        int g;
+        const double fr = frexp(p0, &g);
+        U.pe = e + 1 - g;
+        U.c = (u64)ldexp(fr, 63);
+      }
+    } else
+      return U;
+  }
+  U.ok = 1;
+  return U;
+}
+template <int KIND> FX_HD i64 fixed(double x, const Unit &U) { return to_fixed(x, U.f, U.k); }
+
+// What a kernel needs of the unit.
+struct Consts {
+  u64 c;
+  int pe, r;
+  double k0;  // value at distance 0 (Laplace)
+};
+FX_HD Consts consts(const Unit &U, double k0) { return {U.c, U.pe, U.r, k0}; }
+
+// Kernel value of one pair from its differences (diff(); the first dims of
+// them).  near: a Laplace pair closer than R / 128, left to the FP64 formula on
+// the double coordinates (except coincident points, which are exact).
+template <int KIND>
+FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 *tab, bool &near) {
+  i64 S = 0, T = 0;
+  sq_acc(dx, S, T);
+  if (dims > 1) sq_acc(dy, S, T);
+  if (dims > 2) sq_acc(dz, S, T);
+  near = false;
+  if (KIND == LAPLACE) {
+    u64 U = sq_low(dx);
+    if (dims > 1) U += sq_low(dy);
+    if (dims > 2) U += sq_low(dz);
+    if ((S | T) == 0 && U == 0) return C.k0;
+    near = !laplace_far(S);
+    int z;
+    const u64 n = norm_d2(S, T, U, z);
+    return laplace(n, z, C.c, C.pe, C.r);
+  }
+  if (KIND == WENDLAND) return wendland(sq_sum(S, T));
+  if (KIND == MULTIQUADRIC) return multiquadric(sq_sum8(S, T) + C.c, C.r);
+  return exp2_neg(sq_sum(S, T), tab);
 }
 
 }  // namespace fx

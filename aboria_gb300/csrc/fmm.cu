@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fix64.cuh"
 #include "handles.cuh"
 
 namespace abx {
@@ -93,6 +94,11 @@ struct FmmPlan {
   ChebTab32 tab32{};    // the same in FP32 (mixed-precision P2M / L2P)
   DevBuf<float4> posf;  // mixed near field: FP32 position relative to the leaf centre
   DevBuf<float> b32;    // mixed near field: FP32 weights of the current matvec
+  // FP64 near field on the integer units (fix64.cuh), where unit.ok: the
+  // positions in fixed point, written by every matvec
+  fx::Unit unit{};
+  DevBuf<longlong2> fxy;
+  DevBuf<long long> fz;
   DevBuf<int> mi_d;                 // ncheb x 3 multi-indices
   DevBuf<int> tile_mat, tile_first; // tensor-core M2L tiles
   int ntiles = 0;
@@ -1153,6 +1159,131 @@ __global__ void __launch_bounds__(PT * PW) k_l2p_p2p32(
   }
 }
 
+// ------------------------------------------- FP64 near field on integers ---
+__global__ void k_fixed_pos(int D, const double *__restrict__ pos, int64_t n, fx::Unit U,
+                            longlong2 *__restrict__ fxy, long long *__restrict__ fz) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  fxy[i] = make_longlong2(fx::to_fixed(pos[i], U.f, U.k),
+                          D > 1 ? fx::to_fixed(pos[n + i], U.f, U.k) : 0);
+  fz[i] = D > 2 ? fx::to_fixed(pos[2 * n + i], U.f, U.k) : 0;
+}
+
+// L2P in FP64: one warp per leaf, one lane per target, the tensor-product sum
+// nested by dimension (n^3 + n^2 + n multiply-adds a target instead of 3 n^3
+// products).
+__global__ void __launch_bounds__(PT * PW) k_l2p64(
+    int D, int n, int ncheb, int nleaves, const int *__restrict__ leaves, const int *__restrict__ nb,
+    const int *__restrict__ ne, const double *__restrict__ box, const double *__restrict__ pos,
+    int64_t npos, const double *__restrict__ G, const ChebTab tab, double *__restrict__ c) {
+  __shared__ double sS_all[PW][3][MAXN][PT];
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int li = blockIdx.x * PW + wl;
+  if (li >= nleaves) return;  // whole warps: each lane reads its own column of sS only
+  const int leaf = leaves[li];
+  const double *bx = box + (size_t)leaf * 6;
+  const double *g = G + (size_t)leaf * ncheb;
+  double(*sS)[MAXN][PT] = sS_all[wl];
+  for (int i = nb[leaf] + lane; i < ne[leaf]; i += PT) {
+    for (int d = 0; d < D; ++d) {
+      double S[MAXN];
+      cheb_sn_tab(shift_coord(pos[(int64_t)d * npos + i], bx[d], bx[3 + d]), n, tab, S);
+      for (int m = 0; m < n; ++m) sS[d][m][lane] = S[m];
+    }
+    double acc = 0.0;
+    for (int m0 = 0; m0 < n; ++m0) {
+      double p1 = 0.0;
+      if (D == 1) {
+        p1 = g[m0];
+      } else {
+        for (int m1 = 0; m1 < n; ++m1) {
+          double p2 = 0.0;
+          if (D == 2) {
+            p2 = g[m0 * n + m1];
+          } else {
+            const double *gg = g + (m0 * n + m1) * n;
+            for (int m2 = 0; m2 < n; ++m2) p2 = fma(gg[m2], sS[2][m2][lane], p2);
+          }
+          p1 = fma(p2, sS[1][m1][lane], p1);
+        }
+      }
+      acc = fma(p1, sS[0][m0][lane], acc);
+    }
+    c[i] = acc;
+  }
+}
+
+// P2P in FP64 accuracy on the integer units, added to the L2P result: one warp
+// per target leaf, one lane per target.  Leaves hold 32 targets on average and
+// a third of them a few more than 32: a last tile of r <= 16 targets is worked
+// by 32 / p lanes a target (p the power of two above r), each taking every
+// (32 / p)-th source, and the lanes' sums are added.  N = 1,048,576 uniform,
+// Laplace, order 3: the whole product @F_OLD@ -> @F_NEW@ ms.
+template <int KIND>
+__global__ void __launch_bounds__(PT * PW) k_p2p_fix(
+    int D, int nleaves, const int *__restrict__ leaves, const int *__restrict__ nb,
+    const int *__restrict__ ne, const double *__restrict__ pos, int64_t npos,
+    const longlong2 *__restrict__ fxy, const long long *__restrict__ fz,
+    const double *__restrict__ b, const int *__restrict__ rp, const int *__restrict__ src, double p0,
+    const fx::Consts C, double *__restrict__ c) {
+  __shared__ longlong2 sxy_all[PW][PT], szb_all[PW][PT];
+  __shared__ fx::u64 tab[KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
+  if (KIND == ABX_K_GAUSSIAN) {
+    for (int i = threadIdx.x; i < fx::EXP_TAB; i += PT * PW) tab[i] = fx::exp_table.v[i];
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+  const int li = blockIdx.x * PW + wl;
+  if (li >= nleaves) return;  // whole warps: only warp-level synchronisation below
+  longlong2 *sxy = sxy_all[wl], *szb = szb_all[wl];
+  const int leaf = leaves[li];
+  for (int i0 = nb[leaf]; i0 < ne[leaf]; i0 += PT) {
+    const int r = min(PT, ne[leaf] - i0);
+    const int p = r > 16 ? 32 : r > 8 ? 16 : r > 4 ? 8 : 4;
+    const int i = i0 + (lane & (p - 1)), grp = lane / p, ngrp = 32 / p;
+    const bool act = (lane & (p - 1)) < r;
+    long long x = 0, y = 0, z = 0;
+    if (act) {
+      const longlong2 f = fxy[i];
+      x = fx::biased(f.x);
+      y = fx::biased(f.y);
+      z = fx::biased(fz[i]);
+    }
+    double acc = 0.0;
+    for (int e = rp[li]; e < rp[li + 1]; ++e) {
+      const int sl = src[e];
+      for (int j0 = nb[sl]; j0 < ne[sl]; j0 += PT) {
+        const int cnt = min(PT, ne[sl] - j0);
+        __syncwarp();
+        if (lane < cnt) {
+          sxy[lane] = fxy[j0 + lane];
+          szb[lane] = make_longlong2(fz[j0 + lane], __double_as_longlong(b[j0 + lane]));
+        }
+        __syncwarp();
+        if (act) {
+          for (int q = grp; q < cnt; q += ngrp) {
+            const longlong2 s0 = sxy[q], s1 = szb[q];
+            bool near;
+            double v = fx::value<KIND>(fx::diff(s0.x, x), fx::diff(s0.y, y), fx::diff(s1.x, z), D, C,
+                                       tab, near);
+            if (KIND == ABX_K_LAPLACE && near) {
+              double d2 = 0.0;
+              for (int d = 0; d < D; ++d) {
+                const double dx = pos[(int64_t)d * npos + j0 + q] - pos[(int64_t)d * npos + i];
+                d2 += dx * dx;
+              }
+              v = fmm_k64<KIND>(d2, p0);
+            }
+            acc = fma(v, __longlong_as_double(s1.y), acc);
+          }
+        }
+      }
+    }
+    for (int o = p; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (act && grp == 0) c[i] += acc;
+  }
+}
+
 // M2L matrices: for each (level box size, offset) K[i][j] = kernel(x_i^t, x_j^s)
 template <int KIND>
 __global__ void k_m2l_mats(int D, int n, int ncheb, const double *__restrict__ mat_desc,
@@ -1294,6 +1425,28 @@ int fmm_plan_build(abx_operator *op, int order, FmmPlan *&out, double eta = 1.0)
   P->mat_off = lists.mat_off;
   std::vector<int> leaves = T.leaves;
   P->nleaves = (int)leaves.size();
+  // near field in fixed point: two near boxes of one level are no larger than
+  // the largest leaf (of sides s_d) and less than max(s) / eta apart, so their
+  // points differ by less than 2 s_d + max(s) / eta in every dimension
+  {
+    double side[3] = {0, 0, 0}, reach2 = 0.0;
+    for (int leaf : leaves)
+      for (int d = 0; d < D; ++d)
+        side[d] = std::max(side[d], boxes[leaf * 6 + 3 + d] - boxes[leaf * 6 + d]);
+    const double gap = std::max(side[0], std::max(side[1], side[2])) / std::min(eta, 1.0);
+    for (int d = 0; d < D; ++d) {
+      const double most = std::min(2.0 * side[d] + gap, p->grid.hi[d] - p->grid.lo[d]);
+      reach2 += most * most;
+    }
+    const double reach = std::sqrt(reach2) * (1.0 + 1e-6);
+    switch (P->kind) {
+    case ABX_K_LAPLACE: P->unit = fx::make_unit<fx::LAPLACE>(P->p0, reach); break;
+    case ABX_K_GAUSSIAN:
+    case ABX_K_COMPACT_GAUSSIAN: P->unit = fx::make_unit<fx::GAUSSIAN>(P->p0, reach); break;
+    case ABX_K_MULTIQUADRIC: P->unit = fx::make_unit<fx::MULTIQUADRIC>(P->p0, reach); break;
+    default: break;
+    }
+  }
   // ---- child interpolation matrices Tc[o][i][j] = R_i(node j of child o; parent box)
   std::vector<double> Tc((size_t)P->nchild * nc * nc);
   for (int o = 0; o < P->nchild; ++o)
@@ -1416,6 +1569,20 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
         P->D, P->n, P->ncheb, P->nleaves, P->leaf_ids.ptr, P->node_begin.ptr, P->node_end.ptr,
         P->box.ptr, P->posf.ptr, P->b32.ptr, b, P->G.ptr, P->p2p_rowptr.ptr, P->p2p_src.ptr,
         P->p0, P->tab32, c);
+  } else if (KIND != ABX_K_CONST && P->unit.ok) {
+    constexpr int FK = KIND == ABX_K_COMPACT_GAUSSIAN || KIND == ABX_K_CONST ? ABX_K_GAUSSIAN : KIND;
+    ABX_TRY(P->fxy.reserve((size_t)npos));
+    ABX_TRY(P->fz.reserve((size_t)npos));
+    const unsigned lb = ceil_div((size_t)P->nleaves, PW);
+    k_fixed_pos<<<ceil_div((size_t)npos, 256), 256, 0, s>>>(P->D, pos, npos, P->unit, P->fxy.ptr,
+                                                            P->fz.ptr);
+    k_l2p64<<<lb, PT * PW, 0, s>>>(P->D, P->n, P->ncheb, P->nleaves, P->leaf_ids.ptr,
+                                   P->node_begin.ptr, P->node_end.ptr, P->box.ptr, pos, npos,
+                                   P->G.ptr, P->tab, c);
+    k_p2p_fix<FK><<<lb, PT * PW, 0, s>>>(P->D, P->nleaves, P->leaf_ids.ptr, P->node_begin.ptr,
+                                         P->node_end.ptr, pos, npos, P->fxy.ptr, P->fz.ptr, b,
+                                         P->p2p_rowptr.ptr, P->p2p_src.ptr, P->p0,
+                                         fx::consts(P->unit, 1.0 / P->p0), c);
   } else
     k_l2p_p2p<KIND, false><<<P->nleaves, FT, 0, s>>>(
         P->D, P->n, P->ncheb, P->leaf_ids.ptr, P->node_begin.ptr, P->node_end.ptr, P->box.ptr, pos,

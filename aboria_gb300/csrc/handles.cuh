@@ -69,6 +69,10 @@ struct FmmLists {
   int64_t n_m2l = 0;
 };
 
+struct SearchSpace;  // pairs.cu: workspace of a particle set's searches
+SearchSpace *search_space_new();
+void search_space_free(SearchSpace *w);
+
 }  // namespace abx
 
 struct abx_particles {
@@ -95,6 +99,7 @@ struct abx_particles {
   abx::OctTree tree;
   uint64_t version = 0;  // bumped by every rebuild; operators check it
   abx::HostStage stage_a, stage_b;
+  abx::SearchSpace *search = nullptr;
   // cell-list build (celllist.cu): per-dimension cell boundaries of the
   // grid they were computed for, look-back status words, pass epoch
   abx::DevBuf<uint64_t> cl_bnd;

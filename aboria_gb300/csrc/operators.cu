@@ -203,18 +203,13 @@ __global__ void __launch_bounds__(DT) k_dense_mixed(DenseParams P, int64_t chunk
 // when there are few rows and are added in order.  N = 32,768 x 30,011
 // Gaussian: 57.6 -> 4.4 ms (error against 64 bits 5.2e-15 -> 1.2e-15).
 //
-// The unit R of the fixed-point coordinates (a power of two no smaller than
-// the diagonal of both sets' bounding box) is found on the device by
-// k_dense_range; k_dense_prep checks what it allows and writes `ok`.  Where it
-// does not allow the integer path (a coordinate that is not finite, a Gaussian
-// narrower than c = p0 R^2 log2(e) = 255, whose argument would lose bits; a
-// Wendland support below R / 2; a multiquadric with p0 < R^2 / 256; a Laplace
-// softening of R and above or negative), k_dense_fix leaves at once and
-// k_dense_fp64 does the work; otherwise k_dense_fp64 leaves at once.
+// The unit of the fixed-point coordinates follows from the diagonal of both
+// sets' bounding box, which k_dense_range finds on the device.  Where
+// make_unit does not allow the integer path, or a coordinate is not finite,
+// k_dense_fix leaves at once and k_dense_fp64 does the work; otherwise
+// k_dense_fp64 leaves at once.
 struct DenseFix {
-  int ok, K, r;    // X = x 2^K, R = 2^r
-  int pe;          // Laplace: p0 / R = pm 2^-62 2^-pe
-  fx::u64 c;       // kernel constant, pm for Laplace
+  fx::Unit U;
   unsigned long long range[6];  // ordered bits: max of x_d, then max of -x_d
 };
 struct alignas(32) FixCol {
@@ -222,7 +217,7 @@ struct alignas(32) FixCol {
   double b;
 };
 
-__device__ bool dense_fix_done(const DenseFix *F) { return F->ok != 0; }
+__device__ bool dense_fix_done(const DenseFix *F) { return F->U.ok != 0; }
 
 __device__ __forceinline__ unsigned long long ordered_bits(unsigned long long u) {
   return (u >> 63) ? ~u : u | 0x8000000000000000ull;
@@ -261,92 +256,39 @@ __global__ void __launch_bounds__(DT) k_dense_range(const double *__restrict__ a
   }
 }
 
-// The unit and the kernel's constant from the ranges (one thread's work, done
-// by every CTA that needs it before its columns).
-template <int KIND> __device__ void dense_unit(const DenseParams &P, DenseFix &F) {
+// The kernel's unit from the ranges (one thread's work, done by every CTA that
+// needs it before its columns).
+template <int KIND> __device__ fx::Unit dense_unit(const DenseParams &P,
+                                                   const unsigned long long *range) {
   double ext2 = 0.0;
   bool ok = true;
   for (int d = 0; d < P.dim; ++d) {
-    const double hi = from_ordered(F.range[d]), lo = -from_ordered(F.range[3 + d]);
+    const double hi = from_ordered(range[d]), lo = -from_ordered(range[3 + d]);
     ok = ok && isfinite(hi) && isfinite(lo);
     ext2 += (hi - lo) * (hi - lo);
   }
-  double r2 = ext2;
-  if (KIND == ABX_K_MULTIQUADRIC) r2 += P.p0;
-  ok = ok && r2 < 1e200 && (r2 > 1e-200 || ext2 == 0.0) && isfinite(P.p0);
-  int e = 0;
-  frexp(sqrt(ext2 == 0.0 && KIND != ABX_K_MULTIQUADRIC ? 1.0 : r2) * (1.0 + 1e-12), &e);
-  F.r = e;  // R = 2^e > sqrt(r2)
-  F.K = 62 - e;
-  const double R2 = ldexp(1.0, 2 * e);
-  F.pe = 0;
-  F.c = 0;
-  if (KIND == ABX_K_GAUSSIAN || KIND == ABX_K_COMPACT_GAUSSIAN) {
-    ok = ok && P.p0 >= 0.0 && P.p0 * R2 * 1.4426950408889634 < 255.0;
-    if (ok) F.c = fx::gaussian_constant(P.p0 * R2);
-  } else if (KIND == ABX_K_WENDLAND_C2) {
-    ok = ok && P.p0 >= 0.0 && P.p0 * P.p0 * R2 < 3.99;
-    if (ok) F.c = fx::wendland_constant(P.p0, e);
-  } else if (KIND == ABX_K_MULTIQUADRIC) {
-    ok = ok && P.p0 >= R2 * (1.0 / 256.0);
-    if (ok) F.c = (fx::u64)ldexp(P.p0, 63 - 2 * e);
-  } else if (KIND == ABX_K_LAPLACE) {
-    ok = ok && P.p0 >= 0.0 && P.p0 < ldexp(1.0, e);
-    if (ok) fx::laplace_constant(P.p0, e, F.c, F.pe);
-  } else
-    ok = false;
-  F.ok = ok ? 1 : 0;
+  fx::Unit U = fx::make_unit<KIND>(P.p0, ext2 > 0.0 ? sqrt(ext2) : 1e-30);
+  U.ok = U.ok && ok;
+  return U;
 }
 
 template <int KIND>
 __global__ void __launch_bounds__(DT) k_dense_prep(DenseParams P, DenseFix *__restrict__ Fg,
                                                    FixCol *__restrict__ cols) {
-  __shared__ DenseFix F;
+  __shared__ fx::Unit U;
   if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) F.range[k] = Fg->range[k];
-    dense_unit<KIND>(P, F);
-    if (blockIdx.x == 0) {
-      Fg->ok = F.ok;
-      Fg->K = F.K;
-      Fg->r = F.r;
-      Fg->pe = F.pe;
-      Fg->c = F.c;
-    }
+    U = dense_unit<KIND>(P, Fg->range);
+    if (blockIdx.x == 0) Fg->U = U;
   }
   __syncthreads();
   const int64_t j = (int64_t)blockIdx.x * DT + threadIdx.x;
-  if (!F.ok || j >= P.nc) return;
+  if (!U.ok || j >= P.nc) return;
   FixCol c;
-  c.x = fx::to_fixed(P.cpos[j], F.K);
-  c.y = P.dim > 1 ? fx::to_fixed(P.cpos[P.nc + j], F.K) : 0;
-  c.z = P.dim > 2 ? fx::to_fixed(P.cpos[2 * P.nc + j], F.K) : 0;
+  c.x = fx::fixed<KIND>(P.cpos[j], U);
+  c.y = P.dim > 1 ? fx::fixed<KIND>(P.cpos[P.nc + j], U) : 0;
+  c.z = P.dim > 2 ? fx::fixed<KIND>(P.cpos[2 * P.nc + j], U) : 0;
   c.b = P.b[j];
   cols[j] = c;
-}
-
-// Kernel value of one pair from its fixed-point differences; `far` false: too
-// close for the Laplace kernel's fixed point, the caller evaluates in FP64.
-template <int KIND>
-__device__ __forceinline__ double dense_value(long long dx, long long dy, long long dz, int dim,
-                                              const DenseFix &F, const fx::u64 *tab, bool &far) {
-  fx::i64 S = 0, T = 0;
-  fx::sq_acc(dx, S, T);
-  if (dim > 1) fx::sq_acc(dy, S, T);
-  if (dim > 2) fx::sq_acc(dz, S, T);
-  far = true;
-  if (KIND == ABX_K_LAPLACE) {
-    fx::u64 U = fx::sq_low(dx);
-    if (dim > 1) U += fx::sq_low(dy);
-    if (dim > 2) U += fx::sq_low(dz);
-    far = fx::laplace_far(S);
-    int z;
-    const fx::u64 n = fx::norm_d2(S, T, U, z);
-    return fx::laplace(n, z, F.c, F.pe, F.r);
-  }
-  const fx::u64 s = fx::sq_sum(S, T);
-  if (KIND == ABX_K_WENDLAND_C2) return fx::wendland(fx::mulhi63(s, F.c));
-  if (KIND == ABX_K_MULTIQUADRIC) return fx::multiquadric(s + F.c, F.r);
-  return fx::gaussian(s, F.c, tab);
 }
 
 template <int KIND, int DIM>
@@ -355,21 +297,17 @@ __global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix 
                                                   int64_t chunk_cols, double *__restrict__ partial) {
   __shared__ FixCol sc[DT];
   __shared__ fx::u64 tab[fx::EXP_TAB];
-  DenseFix F;
-  F.ok = Fg->ok;
-  F.K = Fg->K;
-  F.r = Fg->r;
-  F.pe = Fg->pe;
-  F.c = Fg->c;
-  if (!F.ok) return;
+  if (!Fg->U.ok) return;
   if (KIND == ABX_K_GAUSSIAN) tab[threadIdx.x] = fx::exp_table.v[threadIdx.x];
+  const fx::Consts C = fx::consts(Fg->U, 1.0 / P.p0);
   const int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x;
   const bool act = i < P.nr;
   long long x = 0, y = 0, z = 0;
   if (act) {
-    x = fx::to_fixed(P.rpos[i], F.K);
-    if (DIM > 1) y = fx::to_fixed(P.rpos[P.nr + i], F.K);
-    if (DIM > 2) z = fx::to_fixed(P.rpos[2 * P.nr + i], F.K);
+    const fx::Unit U = Fg->U;
+    x = fx::biased(fx::fixed<KIND>(P.rpos[i], U));
+    if (DIM > 1) y = fx::biased(fx::fixed<KIND>(P.rpos[P.nr + i], U));
+    if (DIM > 2) z = fx::biased(fx::fixed<KIND>(P.rpos[2 * P.nr + i], U));
   }
   double acc = 0.0;
   const int64_t c0 = (int64_t)blockIdx.y * chunk_cols;
@@ -382,11 +320,10 @@ __global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix 
 #pragma unroll 2
     for (int jj = 0; jj < nt; ++jj) {
       const FixCol q = sc[jj];
-      bool far;
-      double v = dense_value<KIND>((long long)((fx::u64)q.x - (fx::u64)x),
-                                   (long long)((fx::u64)q.y - (fx::u64)y),
-                                   (long long)((fx::u64)q.z - (fx::u64)z), DIM, F, tab, far);
-      if (KIND == ABX_K_LAPLACE && !far) {
+      bool near;
+      double v = fx::value<KIND>(fx::diff(q.x, x), fx::diff(q.y, y), fx::diff(q.z, z), DIM, C, tab,
+                                 near);
+      if (KIND == ABX_K_LAPLACE && near) {
         double d2 = 0.0;
         if (act)
           for (int d = 0; d < DIM; ++d) {

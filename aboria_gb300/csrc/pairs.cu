@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fix64.cuh"
 #include "handles.cuh"
 
 namespace abx {
@@ -42,7 +43,7 @@ struct alignas(32) D4 {
 struct FineGrid {
   int dim, eoff;
   int m[3];
-  double h[3];
+  double h[3], inv[3];
   float hf[3];
   double lo[3];
   double L[3];
@@ -59,6 +60,11 @@ struct PointLayout {
   DevBuf<float4> loc;     // FP32 offset from the clamped cell corner; .w = clamped c2 bits
   DevBuf<D4> posk;        // FP64 position in kernel order (internal dims, pad = 0)
   DevBuf<uint32_t> keys;  // sorted clamped cell keys
+  // fixed-point positions in kernel order (fix64.cuh), where the operator's
+  // FP64 product runs on the integer units
+  DevBuf<longlong2> fxy;
+  DevBuf<long long> fz;
+  DevBuf<uint32_t> tmp;   // sort scratch
 };
 
 struct PairLayout {
@@ -70,24 +76,51 @@ struct PairLayout {
   PointLayout rows_own;
   PointLayout *rows = nullptr;
   DevBuf<uint32_t> cell_start;  // fg.ncells + 1
-  DevBuf<int2> units;           // (first query in kernel order, count <= 32)
-  int nunits = 0;
+  // Query units (first query in kernel order, count <= 32): full ones from the
+  // front of the array, those of fewer than `split` queries from its back, and
+  // the latter's queries once more as a list (k_units).
+  DevBuf<int2> units;
+  DevBuf<int> singles;
+  int split = 0;
+  DevBuf<int> counts;  // full units, small units, singles, work counters
   DevBuf<float> bk32;
   DevBuf<double> bk64;
   DevBuf<double> sk;  // column scalar in kernel order
   DevBuf<double> sq;  // row scalar in kernel order
   DevBuf<double> ck;  // result in row kernel order
-  DevBuf<int> counter;
-  DevBuf<int> ext;  // e2 extent table
+  DevBuf<int> ext;        // e2 extent table
+  DevBuf<float4> bands;   // rounding bands by tile span (k_tables)
+  DevBuf<int4> stencil;   // unpruned rows of a cell's stencil (k_tables)
+  DevBuf<uint32_t> tmp;   // scan scratch
+  fx::Unit unit{};  // FP64 on the integer units, where unit.ok
 };
 
 void pair_layout_free(PairLayout *L) { delete L; }
+
+// Workspace of a particle set's searches: a search builds its layout anew in
+// buffers that only grow and go with the set.  One search at a time holds it.
+struct SearchSpace {
+  std::mutex m;
+  PairLayout L;
+  DevBuf<double> qsoa, dxd;
+  DevBuf<int32_t> cnt_k, cnt, cols;
+  DevBuf<int64_t> rowptr, rpk, sums;
+};
+constexpr size_t KEEP_BYTES = size_t(256) << 20;
+SearchSpace *search_space_new() { return new SearchSpace(); }
+void search_space_free(SearchSpace *w) { delete w; }
 
 namespace {
 
 constexpr int TPB = 256;
 constexpr int WARPS_PER_CTA = 4;
 constexpr int GROUP_E2 = 4;  // a unit spans at most this many fine cells along e2
+// Units of fewer queries are walked one query a thread.  Measured (N = 100,000
+// with 50 neighbours / the clustered 4M set): FP64 4: 423, 7: 315, 12: 246 us /
+// no difference; counts 4: 698, 7: 669, 12: 658 us / 25.2, 25.4, 25.6 ms; mixed
+// at 4M 4: 20.6, 7: 20.9, 12: 21.5 ms (its unit kernel spends little on a
+// query, so fewer make a unit worth while).
+constexpr int SPLIT_FP64 = 12, SPLIT_COUNT = 7, SPLIT_MIXED = 4;
 
 enum { POL_COUNT = 0, POL_LIST = 1, POL_MATVEC = 2 };
 
@@ -130,19 +163,21 @@ FineGrid make_fine_grid(const GridDesc &g, double r, int64_t npts, int F) {
     const int d = e - fg.eoff;
     fg.h[e] = d < 0 ? 1.0 : fg.L[e] / fg.m[e];
     fg.hf[e] = (float)fg.h[e];
+    fg.inv[e] = 1.0 / fg.h[e];
     fg.K[e] = d < 0 ? 0 : (int)std::ceil(r / fg.h[e] * (1.0 + 1e-9));
     if (fg.K[e] > 2 * fg.m[e] + 1) fg.K[e] = 2 * fg.m[e] + 1;
   }
   return fg;
 }
 
-__device__ __forceinline__ int fine_coord(double x, double lo, double h, int m) {
-  // floor((x - lo)/h) computed as in the layout; unclamped
-  const double t = floor((x - lo) / h);
-  if (!(t == t)) return 1000000000;  // NaN: far outside, never a neighbour
-  if (t < -1e9) return -1000000000;
-  if (t > 1e9) return 1000000000;
-  return (int)t;
+// floor((x - lo) / h), unclamped; NaN: far outside, never a neighbour.  inv =
+// 1 / h rounded: a coordinate on a cell boundary may land in the cell beside
+// it, which the pruning margin (1e-9 of a cell) covers.  (A division here and
+// in the layout made both kernels FP64-bound: 440 us each at N = 4M.)
+__device__ __forceinline__ int fine_coord(double x, double lo, double inv) {
+  const double t = (x - lo) * inv;
+  if (!(fabs(t) < 1e9)) return t < 0.0 ? -1000000000 : 1000000000;
+  return __double2int_rd(t);
 }
 
 // Sort key of a point: clamped fine cell (row-major, e2 fastest) times 8 plus
@@ -161,7 +196,7 @@ __global__ void k_fine_keys(const double *__restrict__ src, int64_t n, int64_t s
       continue;
     }
     const double x = src[(int64_t)d * stride + i];
-    int u = fine_coord(x, fg.lo[e], fg.h[e], fg.m[e]);
+    const int u = fine_coord(x, fg.lo[e], fg.inv[e]);
     c[e] = min(max(u, 0), fg.m[e] - 1);
     const double f = x - (fg.lo[e] + (double)c[e] * fg.h[e]);
     sub |= (f >= 0.5 * fg.h[e] ? 1u : 0u) << (2 - e);
@@ -195,7 +230,7 @@ __global__ void k_fill_layout(const double *__restrict__ src, int64_t stride, Fi
       continue;
     }
     x[e] = src[(int64_t)d * stride + i];
-    u[e] = fine_coord(x[e], fg.lo[e], fg.h[e], fg.m[e]);
+    u[e] = fine_coord(x[e], fg.lo[e], fg.inv[e]);
     c[e] = clamp_anchor ? min(max(u[e], 0), fg.m[e] - 1) : u[e];
     const double corner = fg.lo[e] + (double)c[e] * fg.h[e];
     f[e] = (float)(x[e] - corner);
@@ -219,6 +254,16 @@ __global__ void k_sub(const uint32_t *__restrict__ a, uint32_t n, uint32_t *__re
   if (c < n) b[c] -= a[c];
 }
 
+// Fixed-point positions of a point set in kernel order.
+__global__ void k_fill_fixed(const D4 *__restrict__ posk, int64_t n, fx::Unit U,
+                             longlong2 *__restrict__ fxy, long long *__restrict__ fz) {
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const D4 x = posk[k];
+  fxy[k] = make_longlong2(fx::to_fixed(x.x, U.f, U.k), fx::to_fixed(x.y, U.f, U.k));
+  fz[k] = fx::to_fixed(x.z, U.f, U.k);
+}
+
 int build_points(abx_context *ctx, const double *src_soa, int64_t n, int64_t stride,
                  const FineGrid &fg, bool clamp_anchor, PointLayout &P) {
   cudaStream_t s = ctx->stream;
@@ -229,20 +274,18 @@ int build_points(abx_context *ctx, const double *src_soa, int64_t n, int64_t str
   ABX_TRY(P.loc.reserve(n ? n : 1));
   ABX_TRY(P.posk.reserve(n ? n : 1));
   if (n == 0) return ABX_OK;
-  DevBuf<uint32_t> tmp;
   const size_t rt = radix_temp_u32(n);
-  ABX_TRY(tmp.reserve(2 * (size_t)n + rt + 64));
+  ABX_TRY(P.tmp.reserve(2 * (size_t)n + rt + 64));
   k_fine_keys<<<ceil_div(n, TPB), TPB, 0, s>>>(src_soa, n, stride, fg, P.keys.ptr, P.perm.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
   int bits = 0;
   while (bits < 32 && (((uint64_t)fg.ncells * 8 - 1) >> bits) != 0) ++bits;
-  ABX_TRY(radix_sort_pairs(P.keys.ptr, P.perm.ptr, n, bits, tmp.ptr, tmp.ptr + n, tmp.ptr + 2 * n,
-                           s));
+  ABX_TRY(radix_sort_pairs(P.keys.ptr, P.perm.ptr, n, bits, P.tmp.ptr, P.tmp.ptr + n,
+                           P.tmp.ptr + 2 * n, s));
   k_fill_layout<<<ceil_div(n, TPB), TPB, 0, s>>>(src_soa, stride, fg, P.perm.ptr, n,
                                                  clamp_anchor ? 1 : 0, P.cell.ptr, P.loc.ptr,
                                                  P.posk.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
-  ABX_CHECK_CUDA(cudaStreamSynchronize(s));
   return ABX_OK;
 }
 
@@ -250,57 +293,142 @@ int build_cell_start(abx_context *ctx, PairLayout &L) {
   cudaStream_t s = ctx->stream;
   const uint32_t nc = L.fg.ncells;
   ABX_TRY(L.cell_start.reserve((size_t)nc + 1));
-  DevBuf<uint32_t> first;
-  ABX_TRY(first.reserve((size_t)nc + 1 + scan_temp_elems((size_t)nc + 1)));
-  uint32_t *cs = L.cell_start.ptr;
+  ABX_TRY(L.tmp.reserve((size_t)nc + 1 + scan_temp_elems((size_t)nc + 1)));
+  uint32_t *cs = L.cell_start.ptr, *first = L.tmp.ptr;
   ABX_CHECK_CUDA(cudaMemsetAsync(cs, 0, ((size_t)nc + 1) * 4, s));
-  ABX_CHECK_CUDA(cudaMemsetAsync(first.ptr, 0, ((size_t)nc + 1) * 4, s));
+  ABX_CHECK_CUDA(cudaMemsetAsync(first, 0, ((size_t)nc + 1) * 4, s));
   const int64_t n = L.cols.n;
   if (n > 0) {
-    k_mark_runs_fine<<<ceil_div(n, TPB), TPB, 0, s>>>(L.cols.keys.ptr, n, first.ptr, cs);
+    k_mark_runs_fine<<<ceil_div(n, TPB), TPB, 0, s>>>(L.cols.keys.ptr, n, first, cs);
     ABX_CHECK_CUDA(cudaGetLastError());
-    k_sub<<<ceil_div(nc, TPB), TPB, 0, s>>>(first.ptr, nc, cs);
+    k_sub<<<ceil_div(nc, TPB), TPB, 0, s>>>(first, nc, cs);
     ABX_CHECK_CUDA(cudaGetLastError());
   }
   // counts -> exclusive scan over nc+1 entries (last entry 0 -> total)
-  ABX_TRY(exclusive_scan_u32(cs, (size_t)nc + 1, first.ptr + nc + 1, s));
-  ABX_CHECK_CUDA(cudaStreamSynchronize(s));
+  ABX_TRY(exclusive_scan_u32(cs, (size_t)nc + 1, first + nc + 1, s));
   return ABX_OK;
 }
 
+// First index of keys[0, n) whose value is >= key, by a 32-way search (whole
+// warps).
+__device__ __forceinline__ int64_t warp_lower_bound(const uint32_t *__restrict__ keys, int64_t n,
+                                                    uint64_t key, int lane) {
+  int64_t lo = 0, hi = n;  // the answer lies in [lo, hi]
+  while (hi - lo > 32) {
+    const int64_t step = (hi - lo + 32) / 33;
+    const int64_t i = lo + (int64_t)(lane + 1) * step;
+    const unsigned m = __ballot_sync(0xffffffffu, i < hi && (uint64_t)keys[i < hi ? i : lo] < key);
+    const int c = __popc(m);  // probes below the key form a prefix
+    const int64_t nlo = c ? lo + (int64_t)c * step + 1 : lo;
+    hi = c < 32 && lo + (int64_t)(c + 1) * step < hi ? lo + (int64_t)(c + 1) * step : hi;
+    lo = nlo;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, lo + lane < hi && (uint64_t)keys[lo + lane] < key);
+  return lo + __popc(m);
+}
+
 // Units: greedy runs of <= 32 consecutive queries (kernel order) whose anchor
-// cells share (e0, e1) and span fewer than GROUP_E2 cells along e2.
-int build_units(abx_context *ctx, PairLayout &L) {
+// cells share (e0, e1) and span fewer than GROUP_E2 cells along e2.  One warp
+// per (e0, e1) column walks its queries 32 at a time with the next 32 already
+// loaded; the unit that starts at query s is the run of lanes that continue
+// it.  A unit of at least `split` queries goes to the front of `units`; a smaller
+// one (low density, where a warp of 32 lanes would hold few queries) to the
+// back, and its queries to `singles`, which the one-query-a-thread kernels
+// walk.  Built on the host before, from a 16 B/point copy of the cells: 14 of
+// the 39 ms of a search at N = 4M.
+constexpr int UNIT_WARPS = 4;
+__global__ void __launch_bounds__(UNIT_WARPS * 32)
+    k_units(const int4 *__restrict__ cell, const uint32_t *__restrict__ keys,
+            const uint32_t *__restrict__ cell_start, int64_t n, uint32_t ncol, int m2, int64_t cap,
+            int split, int2 *__restrict__ units, int *__restrict__ singles, int *__restrict__ counts) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * UNIT_WARPS;
+  for (uint32_t col = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); col < ncol; col += warps) {
+    int64_t s, end;
+    if (cell_start) {
+      s = cell_start[(uint64_t)col * m2];
+      end = cell_start[(uint64_t)(col + 1) * m2];
+    } else {
+      s = warp_lower_bound(keys, n, (uint64_t)col * m2 * 8, lane);
+      end = warp_lower_bound(keys, n, (uint64_t)(col + 1) * m2 * 8, lane);
+    }
+    const int4 none = make_int4(0, 0, 0, 0);
+    int64_t base = s;  // A holds queries [base, base + 32), B the 32 after them
+    int4 A = base + lane < end ? cell[base + lane] : none;
+    int4 B = base + 32 + lane < end ? cell[base + 32 + lane] : none;
+    int2 mine = make_int2(0, 0);  // lane i keeps the i-th unit not written out yet
+    int held = 0;
+    while (s < end || held > 0) {
+      if (s < end) {
+        if (s - base >= 32) {
+          base += 32;
+          A = B;
+          B = base + 32 + lane < end ? cell[base + 32 + lane] : none;
+        }
+        const int o = (int)(s - base), src = (o + lane) & 31;
+        const int ax = __shfl_sync(0xffffffffu, A.x, src), bx = __shfl_sync(0xffffffffu, B.x, src);
+        const int ay = __shfl_sync(0xffffffffu, A.y, src), by = __shfl_sync(0xffffffffu, B.y, src);
+        const int az = __shfl_sync(0xffffffffu, A.z, src), bz = __shfl_sync(0xffffffffu, B.z, src);
+        const bool a = o + lane < 32;
+        const int x = a ? ax : bx, y = a ? ay : by, z = a ? az : bz;
+        const int x0 = __shfl_sync(0xffffffffu, x, 0), y0 = __shfl_sync(0xffffffffu, y, 0),
+                  z0 = __shfl_sync(0xffffffffu, z, 0);
+        const bool go = s + lane < end && x == x0 && y == y0 && z >= z0 && z - z0 < GROUP_E2;
+        const unsigned stop = ~__ballot_sync(0xffffffffu, go);
+        const int count = stop ? __ffs(stop) - 1 : 32;
+        if (lane == held) mine = make_int2((int)s, count);
+        ++held;
+        s += count;
+      }
+      if (held == 32 || s >= end) {
+        const bool full = lane < held && mine.y >= split, small = lane < held && mine.y < split;
+        const unsigned mf = __ballot_sync(0xffffffffu, full), ms = __ballot_sync(0xffffffffu, small);
+        const unsigned lt = (1u << lane) - 1u;
+        int tot = small ? mine.y : 0, incl = tot;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, d);
+          if (lane >= d) incl += v;
+        }
+        const int nsing = __shfl_sync(0xffffffffu, incl, 31);
+        int bf = 0, bs = 0, bq = 0;
+        if (lane == 0) {
+          if (mf) bf = atomicAdd(&counts[0], __popc(mf));
+          if (ms) {
+            bs = atomicAdd(&counts[1], __popc(ms));
+            bq = atomicAdd(&counts[2], nsing);
+          }
+        }
+        bf = __shfl_sync(0xffffffffu, bf, 0);
+        bs = __shfl_sync(0xffffffffu, bs, 0);
+        bq = __shfl_sync(0xffffffffu, bq, 0);
+        if (full) units[bf + __popc(mf & lt)] = mine;
+        if (small) {
+          units[cap - 1 - (bs + __popc(ms & lt))] = mine;
+          for (int k = 0; k < mine.y; ++k) singles[bq + incl - tot + k] = mine.x + k;
+        }
+        held = 0;
+      }
+    }
+  }
+}
+
+int build_units(abx_context *ctx, PairLayout &L, int split) {
   PointLayout &Q = *L.rows;
+  L.split = split;
   const int64_t n = Q.n;
   ABX_REQUIRE(n < (int64_t)0x7fffffff, ABX_ERR_INVALID, "too many query points");
-  std::vector<int4> cell(n);
-  if (n) ABX_CHECK_CUDA(cudaMemcpy(cell.data(), Q.cell.ptr, n * sizeof(int4), cudaMemcpyDeviceToHost));
-  std::vector<int2> units;
-  units.reserve(n / 16 + 16);
-  int64_t i = 0;
-  while (i < n) {
-    const int4 c0 = cell[i];
-    int zmin = c0.z, zmax = c0.z;
-    int64_t j = i + 1;
-    while (j < n && j - i < 32) {
-      const int4 cj = cell[j];
-      if (cj.x != c0.x || cj.y != c0.y) break;
-      const int nz0 = std::min(zmin, cj.z), nz1 = std::max(zmax, cj.z);
-      if (nz1 - nz0 >= GROUP_E2) break;
-      zmin = nz0;
-      zmax = nz1;
-      ++j;
-    }
-    units.push_back(make_int2((int)i, (int)(j - i)));
-    i = j;
-  }
-  L.nunits = (int)units.size();
-  ABX_TRY(L.units.reserve(units.size() ? units.size() : 1));
-  if (!units.empty())
-    ABX_CHECK_CUDA(cudaMemcpy(L.units.ptr, units.data(), units.size() * sizeof(int2),
-                              cudaMemcpyHostToDevice));
-  ABX_TRY(L.counter.reserve(4));
+  ABX_TRY(L.units.reserve(n ? n : 1));
+  ABX_TRY(L.singles.reserve(n ? n : 1));
+  ABX_TRY(L.counts.reserve(8));
+  ABX_CHECK_CUDA(cudaMemsetAsync(L.counts.ptr, 0, 3 * sizeof(int), ctx->stream));
+  if (n == 0) return ABX_OK;
+  const uint32_t ncol = (uint32_t)L.fg.m[0] * L.fg.m[1];
+  const unsigned blocks = std::min(ceil_div(ncol, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
+  k_units<<<blocks, UNIT_WARPS * 32, 0, ctx->stream>>>(
+      Q.cell.ptr, Q.keys.ptr, L.self ? L.cell_start.ptr : nullptr, n, ncol, L.fg.m[2], n,
+      split, L.units.ptr, L.singles.ptr, L.counts.ptr);
+  ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
 
@@ -333,11 +461,22 @@ struct KParams {
   const float4 *qloc;
   const D4 *qpos;
   const double *s_row;
-  const int2 *units;
-  int nunits;
-  int *counter;
+  const int2 *units;     // full units from the front, small ones from the back
+  int64_t units_cap;
+  const int *singles;    // queries of the small units
+  const int *counts;     // full units, small units, singles
+  int all_units;         // 1: the small units too (searches that write lists)
+  int *counter;          // work counters: units, singles
+  const float4 *bands;   // two entries a span: r2lo, r2hi, r2box, rbox_inf; r2mid, r2half
+  const int4 *stencil;   // unpruned rows of a cell's stencil, counts[3] of them
+  int lanes;             // lanes a query of the singles
+  // fixed point (fix64.cuh): column and query positions, box lengths, constants
+  const longlong2 *fxy, *qfxy;
+  const long long *fz, *qfz;
+  long long Lfix[3];
+  fx::Consts fixc;
   // outputs (query kernel order)
-  int32_t *counts;
+  int32_t *counts_out;
   const int64_t *rowptr;  // for LIST: query kernel order -> output offset
   int32_t *cols_out;      // storage index of the column particle
   double *dx_out;         // for LIST (optional): x_j - (x_i + image*L), D per pair
@@ -560,16 +699,6 @@ __device__ __forceinline__ int build_segments(const KParams &P, const int lo[3],
   return base;
 }
 
-// Segment holding flattened candidate t (off[s] <= t < off[s+1]).
-__device__ __forceinline__ int find_seg(const WarpSeg &ws, int nseg, int t) {
-  int lo = 0, hi = nseg - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (ws.off[mid] <= t) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 constexpr int STAGE = 64;  // candidates staged per round (two per lane)
 
 // Internal kernel tag: Wendland C2 in a mixed-precision matvec whose kernel
@@ -680,6 +809,99 @@ __device__ __forceinline__ void unit_box(const KParams &P, const int4 qc, bool a
   nrows = (R0 > 0 && R1 > 0) ? R0 * R1 : 0;
 }
 
+// Rounding band of a tile whose FP32 offsets reach `span` cells from their
+// reference corner: an offset carries < (3*span+2)*h*2^-24 error and a
+// difference of two < edx = (span+2)*h*2^-20; |d2_f32 - d2| <= band.
+struct TileBand {
+  float4 a;  // r2lo, r2hi: accepted up to r2lo, rejected beyond r2hi; r2box, rbox_inf
+  float4 b;  // r2mid, r2half: the band as |d2 - r2mid| <= r2half
+};
+constexpr int BAND_TAB = 64;
+__device__ __forceinline__ TileBand tile_band(int span, const FineGrid &fg, double r, double r2,
+                                              double thr, int norm) {
+  const double hmax = fmax(fmax(fg.h[0] * (fg.eoff <= 0), fg.h[1] * (fg.eoff <= 1)), fg.h[2]);
+  const double edx = (double)(span + 2) * hmax * 9.5367431640625e-07;
+  const double band = 2.0 * 1.7320508075688772 * (r + edx) * edx + 3.0 * edx * edx +
+                      4.0 * 5.960464477539063e-08 * r2 + 1e-300;
+  // manhattan / chebyshev: each FP32 |d_e| is within edx of the exact one,
+  // the sum of three adds <= 2 roundings of a value below 3 r
+  const double nband = norm == 1 ? 3.0 * edx + 6.0 * 5.960464477539063e-08 * 3.0 * r + 1e-300
+                                 : edx + 2.0 * 5.960464477539063e-08 * r + 1e-300;
+  // (when the band reaches below 0 nothing is accepted outright: two
+  // distinct points may share an FP32 offset, d = 0, yet lie outside a
+  // radius smaller than the band)
+  const double lo_thr = norm == 2 ? r2 - band : thr - nband;
+  const float r2lo = lo_thr > 0.0 ? __double2float_rd(lo_thr) : -1.0f;
+  const float r2hi = norm == 2 ? __double2float_ru(r2 + band) : __double2float_ru(thr + nband);
+  // box test: euclidean for norms 2 and 1 (the manhattan ball lies inside
+  // the euclidean one), a max-norm test for the chebyshev ball
+  const float r2box = __double2float_ru((r2 + band) * (1.0 + 1e-6) + 1e-300);
+  const float rbox_inf = __double2float_ru((thr + nband) * (1.0 + 1e-6) + 1e-300);
+  // the band around its middle, widened by a few ulps so that the FP32
+  // subtraction never shrinks it below (r2lo, r2hi]
+  const float r2mid = (float)(0.5 * ((double)r2lo + (double)r2hi));
+  const float r2half =
+      __double2float_ru(0.5 * ((double)r2hi - (double)r2lo) + 8.0 * 5.960464477539063e-08 * r2);
+  return {make_float4(r2lo, r2hi, r2box, rbox_inf), make_float4(r2mid, r2half, 0.f, 0.f)};
+}
+
+// Largest e2 gap (in cells) that keeps a cell within the pruning distance, for
+// every pair of e0/e1 gaps below EXT_TAB cells (-1: pruned), and the bands by
+// span: ~30 FP64 operations a unit otherwise, 0.4 of a unit's time where it
+// holds few queries.
+//
+// rows: the rows (e0, e1 offsets) of a single cell's stencil that are not
+// pruned, in row-major order, as (o0, o1, reach along e2); their number goes
+// to *nrows (k_pairs_thread).  By block 0.
+constexpr int TABLE_TPB = 256;
+constexpr int ROWS_MAX = 1024;  // (2 K0 + 1)(2 K1 + 1), K <= 7 (make_fine_grid)
+__device__ __forceinline__ int row_reach(int a, int b, const FineGrid &fg, double prune2, int norm) {
+  if (norm == -1) return fg.K[2];  // the chebyshev ball is the whole stencil box
+  const int g0c = max(abs(a) - 1, 0), g1c = max(abs(b) - 1, 0);
+  const double g0 = g0c * fg.h[0], g1 = g1c * fg.h[1];
+  const double rem = __dsub_rn(__dsub_rn(prune2, __dmul_rn(g0, g0)), __dmul_rn(g1, g1));
+  return rem < 0.0 ? -1 : min((int)fmin(floor(sqrt(rem) / fg.h[2]), (double)fg.K[2]) + 1, fg.K[2]);
+}
+__global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2, double r,
+                                                      double thr, int norm, int *__restrict__ ext,
+                                                      float4 *__restrict__ bands,
+                                                      int4 *__restrict__ rows,
+                                                      int *__restrict__ nrows) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0) {
+    __shared__ int wsum[TABLE_TPB / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int R1 = 2 * fg.K[1] + 1, NR = (2 * fg.K[0] + 1) * R1;
+    int done = 0;
+    for (int i0 = 0; i0 < NR; i0 += TABLE_TPB) {
+      const int i = i0 + threadIdx.x;
+      const int a = i / R1 - fg.K[0], b = i % R1 - fg.K[1];
+      const int reach = i < NR ? row_reach(a, b, fg, prune2, norm) : -1;
+      const unsigned m = __ballot_sync(0xffffffffu, reach >= 0);
+      if (lane == 0) wsum[w] = __popc(m);
+      __syncthreads();
+      int at = done + __popc(m & ((1u << lane) - 1u));
+      for (int k = 0; k < TABLE_TPB / 32; ++k) {
+        if (k < w) at += wsum[k];
+        done += wsum[k];
+      }
+      if (reach >= 0 && at < ROWS_MAX) rows[at] = make_int4(a, b, reach, 0);
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *nrows = min(done, ROWS_MAX);
+  }
+  if (t < EXT_TAB * EXT_TAB) {
+    const double g0 = (t / EXT_TAB) * fg.h[0], g1 = (t % EXT_TAB) * fg.h[1];
+    const double rem = __dsub_rn(__dsub_rn(prune2, __dmul_rn(g0, g0)), __dmul_rn(g1, g1));
+    ext[t] = rem < 0.0 ? -1 : (int)fmin(floor(sqrt(rem) / fg.h[2]), (double)fg.K[2]);
+  }
+  if (t < BAND_TAB) {
+    const TileBand b = tile_band(t, fg, r, r * r, thr, norm);
+    bands[2 * t] = b.a;
+    bands[2 * t + 1] = b.b;
+  }
+}
+
 // Mixed-precision pair kernel.  Per unit (one warp, <= 32 queries):
 //   rows of the stencil -> segment list -> flattened candidate stream, 32 at a
 //   time -> each lane stages one candidate (FP32 offset from the unit's
@@ -709,12 +931,13 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
   const unsigned lt = (1u << lane) - 1u;
   constexpr bool WCUT = KIND == K_WEND_CUT;
   const float sc = WCUT ? P.p0f : 1.f;  // staging scale (d^2 = q^2 for WCUT)
+  const int nfull = P.counts[0], nunits = nfull + (P.all_units ? P.counts[1] : 0);
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = atomicAdd(P.counter, 1);
     unit = __shfl_sync(0xffffffffu, unit, 0);
-    if (unit >= P.nunits) break;
-    const int2 U = P.units[unit];
+    if (unit >= nunits) break;
+    const int2 U = unit < nfull ? P.units[unit] : P.units[P.units_cap - 1 - (unit - nfull)];
     const bool active = lane < U.y;
     const int qi = U.x + (active ? lane : 0);
     const int4 qc = P.qcell[qi];
@@ -734,34 +957,14 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
     const float bc1 = 0.5f * (bl1 + bh1), bw1 = __fadd_ru(0.5f * (bh1 - bl1), 1e-6f * (fabsf(bl1) + fabsf(bh1)));
     const float bc2 = 0.5f * (bl2 + bh2), bw2 = __fadd_ru(0.5f * (bh2 - bl2), 1e-6f * (fabsf(bl2) + fabsf(bh2)));
     // rounding band: every staged coordinate lies within `span` cells of the
-    // reference corner, so an FP32 offset carries < (3*span+2)*h*2^-24 error
-    // and a difference of two < edx = (span+2)*h*2^-20; |d2_f32 - d2| <= band.
+    // reference corner (tile_band)
     int span = 0;
 #pragma unroll
     for (int e = 0; e < 3; ++e) span = max(span, hi[e] - lo[e] + 2 * fg.K[e] + 2);
-    const double hmax = fmax(fmax(fg.h[0] * (fg.eoff <= 0), fg.h[1] * (fg.eoff <= 1)), fg.h[2]);
-    const double edx = (double)(span + 2) * hmax * 9.5367431640625e-07;
-    const double band = 2.0 * 1.7320508075688772 * (P.r + edx) * edx + 3.0 * edx * edx +
-                        4.0 * 5.960464477539063e-08 * P.r2 + 1e-300;
-    // manhattan / chebyshev: each FP32 |d_e| is within edx of the exact one,
-    // the sum of three adds <= 2 roundings of a value below 3 r
-    const double nband = NORM == 1 ? 3.0 * edx + 6.0 * 5.960464477539063e-08 * 3.0 * P.r + 1e-300
-                                   : edx + 2.0 * 5.960464477539063e-08 * P.r + 1e-300;
-    // (when the band reaches below 0 nothing is accepted outright: two
-    // distinct points may share an FP32 offset, d = 0, yet lie outside a
-    // radius smaller than the band)
-    const double lo_thr = NORM == 2 ? P.r2 - band : P.thr - nband;
-    const float r2lo = lo_thr > 0.0 ? __double2float_rd(lo_thr) : -1.0f;
-    const float r2hi = NORM == 2 ? __double2float_ru(P.r2 + band) : __double2float_ru(P.thr + nband);
-    // box test: euclidean for norms 2 and 1 (the manhattan ball lies inside
-    // the euclidean one), a max-norm test for the chebyshev ball
-    const float r2box = __double2float_ru((P.r2 + band) * (1.0 + 1e-6) + 1e-300);
-    const float rbox_inf = __double2float_ru((P.thr + nband) * (1.0 + 1e-6) + 1e-300);
-    // band as |d2 - r2mid| <= r2half, widened by a few ulps so that the FP32
-    // subtraction never shrinks it below (r2lo, r2hi]
-    const float r2mid = (float)(0.5 * ((double)r2lo + (double)r2hi));
-    const float r2half =
-        __double2float_ru(0.5 * ((double)r2hi - (double)r2lo) + 8.0 * 5.960464477539063e-08 * P.r2);
+    const TileBand bd = span < BAND_TAB ? TileBand{P.bands[2 * span], P.bands[2 * span + 1]}
+                                        : tile_band(span, fg, P.r, P.r2, P.thr, NORM);
+    const float r2lo = bd.a.x, r2hi = bd.a.y, r2box = bd.a.z, rbox_inf = bd.a.w;
+    const float r2mid = bd.b.x, r2half = bd.b.y;
     D4 xq;
     bool have_xq = false;
     double acc64 = 0.0;
@@ -919,8 +1122,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
               // the kernel vanishes for q >= 1: the clamp is the cut-off for
               // every pair outside the rounding band (d2 > r2hi means q > 1),
               // and band pairs are flagged for the exact test below
-              const float2 bd = __fadd2_rn(dd, make_float2(-r2mid, -r2mid));
-              need |= (fabsf(bd.x) <= r2half) | (fabsf(bd.y) <= r2half);
+              const float2 off = __fadd2_rn(dd, make_float2(-r2mid, -r2mid));
+              need |= (fabsf(off.x) <= r2half) | (fabsf(off.y) <= r2half);
               w = kern32x2_wendland_clamped(dd, P);
             } else {
               const bool ia = dd.x <= r2lo, ib = dd.y <= r2lo;
@@ -991,7 +1194,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
     }
     if (active) {
       if (POL == POL_MATVEC) P.c[qi] = acc64;
-      if (POL == POL_COUNT) P.counts[qi] = count;
+      if (POL == POL_COUNT) P.counts_out[qi] = count;
     }
   }
 }
@@ -1002,9 +1205,29 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
 // value), with their weights and (column index, segment) for the exact test.
 struct WarpTile64 {
   float4 pf[STAGE];
-  double ux[STAGE], uy[STAGE], uz[STAGE], b[STAGE], s[STAGE];
+  // (bits of) the position: double, or fixed point (FIX)
+  long long ux[STAGE], uy[STAGE], uz[STAGE];
+  double b[STAGE], s[STAGE];
   int2 meta[STAGE];
 };
+
+// FP64-accurate kernel value of one accepted pair from its fixed-point
+// differences (fix64.cuh); the padding dimensions come first.
+template <int KIND>
+__device__ __forceinline__ double fix_value(long long dx, long long dy, long long dz,
+                                            const KParams &P, const fx::u64 *tab, bool &near) {
+  return fx::value<KIND>(dz, dy, dx, 3 - P.fg.eoff, P.fixc, tab, near);
+}
+
+// FP64 distance and kernel value of one accepted pair, dx = (x_j - image*L) - x_i.
+template <int KIND>
+__device__ __forceinline__ double pair64(const D4 &xq, const D4 &xj, const int *img,
+                                         const KParams &P, double si, double sj) {
+  const double dx = __dsub_rn(xj.x, (double)img[0] * P.fg.L[0]) - xq.x;
+  const double dy = __dsub_rn(xj.y, (double)img[1] * P.fg.L[1]) - xq.y;
+  const double dz = __dsub_rn(xj.z, (double)img[2] * P.fg.L[2]) - xq.z;
+  return kern64<KIND>(fma(dz, dz, fma(dy, dy, dx * dx)), P, si, sj);
+}
 
 // FP64 sparse matvec: the reference's arithmetic for every accepted pair,
 // FP64 work only for accepted pairs.  Per staged tile of <= 64 candidates:
@@ -1014,12 +1237,14 @@ struct WarpTile64 {
 //      64-bit mask of this lane's neighbours among the candidates;
 //  (2) every lane walks its own mask and evaluates the FP64 distance, kernel
 //      and product for those pairs only.
-// The warp then pays FP64 issue for max over lanes of its neighbour count,
-// not for every (query, candidate) combination.  The distance for the kernel
+// The warp then pays for max over lanes of its neighbour count, not for every
+// (query, candidate) combination.  With FIX the values come from the integer
+// units (fix64.cuh) and the FP64 pipe is left with one multiply-add a pair: N =
+// 1,048,576 clustered, 1,250 neighbours a row, Wendland: @U_OLD@ -> @U_NEW@ ms.  The distance for the kernel
 // value is |(x_j - image*L) - x_i|, which differs from the reference's
 // x_j - (x_i + image*L) by at most an ulp of the box length (the acceptance
 // decision itself is exact); the row sum order differs from the reference's.
-template <int POL, int KIND>
+template <int POL, int KIND, bool FIX>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
     k_pairs_fp64(KParams P) {
   __shared__ WarpSeg seg_all[WARPS_PER_CTA];
@@ -1030,12 +1255,18 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
   WarpTile64 &sm = tile_all[wid];
   const FineGrid &fg = P.fg;
   const unsigned lt = (1u << lane) - 1u;
+  const int nfull = P.counts[0], nunits = nfull + (P.all_units ? P.counts[1] : 0);
+  __shared__ fx::u64 tab[FIX && KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
+  if (FIX && KIND == ABX_K_GAUSSIAN) {
+    for (int i = threadIdx.x; i < fx::EXP_TAB; i += WARPS_PER_CTA * 32) tab[i] = fx::exp_table.v[i];
+    __syncthreads();
+  }
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = atomicAdd(P.counter, 1);
     unit = __shfl_sync(0xffffffffu, unit, 0);
-    if (unit >= P.nunits) break;
-    const int2 U = P.units[unit];
+    if (unit >= nunits) break;
+    const int2 U = unit < nfull ? P.units[unit] : P.units[P.units_cap - 1 - (unit - nfull)];
     const bool active = lane < U.y;
     const int qi = U.x + (active ? lane : 0);
     const int4 qc = P.qcell[qi];
@@ -1051,18 +1282,21 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
     const float bc0 = 0.5f * (bl0 + bh0), bw0 = __fadd_ru(0.5f * (bh0 - bl0), 1e-6f * (fabsf(bl0) + fabsf(bh0)));
     const float bc1 = 0.5f * (bl1 + bh1), bw1 = __fadd_ru(0.5f * (bh1 - bl1), 1e-6f * (fabsf(bl1) + fabsf(bh1)));
     const float bc2 = 0.5f * (bl2 + bh2), bw2 = __fadd_ru(0.5f * (bh2 - bl2), 1e-6f * (fabsf(bl2) + fabsf(bh2)));
-    // rounding band of the FP32 d2 (the same bound as the mixed kernel's)
+    // rounding band of the FP32 d2
     int span = 0;
 #pragma unroll
     for (int e = 0; e < 3; ++e) span = max(span, hi[e] - lo[e] + 2 * fg.K[e] + 2);
-    const double hmax = fmax(fmax(fg.h[0] * (fg.eoff <= 0), fg.h[1] * (fg.eoff <= 1)), fg.h[2]);
-    const double edx = (double)(span + 2) * hmax * 9.5367431640625e-07;
-    const double band = 2.0 * 1.7320508075688772 * (P.r + edx) * edx + 3.0 * edx * edx +
-                        4.0 * 5.960464477539063e-08 * P.r2 + 1e-300;
-    const float r2lo = P.r2 - band > 0.0 ? __double2float_rd(P.r2 - band) : -1.0f;
-    const float r2hi = __double2float_ru(P.r2 + band);
-    const float r2box = __double2float_ru((P.r2 + band) * (1.0 + 1e-6) + 1e-300);
+    const float4 bd = span < BAND_TAB ? P.bands[2 * span]
+                                      : tile_band(span, fg, P.r, P.r2, P.r2, 2).a;
+    const float r2lo = bd.x, r2hi = bd.y, r2box = bd.z;
     const D4 xq = P.qpos[qi];
+    longlong2 fq = make_longlong2(0, 0);
+    long long fqz = 0;
+    if (FIX) {
+      fq = P.qfxy[qi];
+      fq = make_longlong2(fx::biased(fq.x), fx::biased(fq.y));
+      fqz = fx::biased(P.qfz[qi]);
+    }
     const double si = (KIND == ABX_K_SCALAR_SUM) ? P.s_row[qi] : 0.0;
     double acc = 0.0;
 
@@ -1113,11 +1347,18 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
             const int slot = nt + __popc(km & lt);
             int img[3], du0, du1;
             unpack_seg(ws.seg[sx[sub]].z, img, du0, du1);
-            const D4 pj = P.cpos[k];
             sm.pf[slot] = st;
-            sm.ux[slot] = __dsub_rn(pj.x, (double)img[0] * fg.L[0]);
-            sm.uy[slot] = __dsub_rn(pj.y, (double)img[1] * fg.L[1]);
-            sm.uz[slot] = __dsub_rn(pj.z, (double)img[2] * fg.L[2]);
+            if (FIX) {
+              const longlong2 f = P.fxy[k];
+              sm.ux[slot] = fx::diff(f.x, img[0] * P.Lfix[0]);
+              sm.uy[slot] = fx::diff(f.y, img[1] * P.Lfix[1]);
+              sm.uz[slot] = fx::diff(P.fz[k], img[2] * P.Lfix[2]);
+            } else {
+              const D4 pj = P.cpos[k];
+              sm.ux[slot] = __double_as_longlong(__dsub_rn(pj.x, (double)img[0] * fg.L[0]));
+              sm.uy[slot] = __double_as_longlong(__dsub_rn(pj.y, (double)img[1] * fg.L[1]));
+              sm.uz[slot] = __double_as_longlong(__dsub_rn(pj.z, (double)img[2] * fg.L[2]));
+            }
             sm.b[slot] = P.b64[k];
             if (KIND == ABX_K_SCALAR_SUM) sm.s[slot] = P.s_col[k];
             sm.meta[slot] = make_int2(k, sx[sub]);
@@ -1154,18 +1395,215 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
             if (j < 32) m0 |= 1u << j; else m1 |= 1u << (j - 32);
           }
         }
-        // (2) FP64 distance, kernel and product for this lane's neighbours
+        // (2) distance, kernel and product for this lane's neighbours
         while (m0 | m1) {
           const int j = m0 ? __ffs(m0) - 1 : 32 + __ffs(m1) - 1;
           if (j < 32) m0 &= m0 - 1u; else m1 &= m1 - 1u;
-          const double dx = sm.ux[j] - xq.x, dy = sm.uy[j] - xq.y, dz = sm.uz[j] - xq.z;
-          const double d2 = fma(dz, dz, fma(dy, dy, dx * dx));
-          acc = fma(kern64<KIND>(d2, P, si, sm.s[j]), sm.b[j], acc);
+          double v;
+          if (FIX) {
+            bool near;
+            v = fix_value<KIND>(fx::diff(sm.ux[j], fq.x), fx::diff(sm.uy[j], fq.y),
+                                fx::diff(sm.uz[j], fqz), P, tab, near);
+            if (KIND == ABX_K_LAPLACE && near) {
+              const int2 mt = sm.meta[j];
+              int img[3], du0, du1;
+              unpack_seg(ws.seg[mt.y].z, img, du0, du1);
+              v = pair64<KIND>(xq, P.cpos[mt.x], img, P, 0.0, 0.0);
+            }
+          } else {
+            const double dx = __longlong_as_double(sm.ux[j]) - xq.x,
+                         dy = __longlong_as_double(sm.uy[j]) - xq.y,
+                         dz = __longlong_as_double(sm.uz[j]) - xq.z;
+            v = kern64<KIND>(fma(dz, dz, fma(dy, dy, dx * dx)), P, si, sm.s[j]);
+          }
+          acc = fma(v, sm.b[j], acc);
         }
         __syncwarp();
       }
     }
     if (active) P.c[qi] = acc;
+  }
+}
+
+// ----------------------------------------------- few lanes a query ---
+// The pair work of the small units (few queries in GROUP_E2 cells: up to ~150
+// neighbours a ball in 3-D), where a warp of the unit kernels would keep most
+// lanes idle.  A query has P.lanes lanes (a power of two), which share the rows
+// of its stencil: one where there are queries enough to fill the GPU, up to a
+// whole warp for small sets, whose time is the latency of one query's rows.
+// The FP32 test is as cheap as the loads; FP64 values (~100 instructions) are
+// not evaluated where they are found but queued per lane in shared memory and
+// evaluated when a queue is full, as long as DRAIN lanes have one.  N = 100,000,
+// 50 neighbours a row: counts @C_OLD@ -> @C_NEW@, FP64 Gaussian product @S_OLD@
+// -> @S_NEW@ us.
+enum { VAL_FP64 = 0, VAL_MIXED = 1, VAL_FIX = 2 };
+constexpr int QCAP = 16;   // queued pairs per lane
+constexpr int DRAIN = 22;  // lanes that make an evaluation worth its issue
+
+template <int POL, int KIND, int VAL, int NORM = 2>
+__global__ void __launch_bounds__(WARPS_PER_CTA * 32)
+    k_pairs_thread(KParams P) {
+  constexpr bool QUEUE = POL == POL_MATVEC && VAL != VAL_MIXED;
+  constexpr bool WCUT = KIND == K_WEND_CUT;
+  __shared__ unsigned long long queue[QUEUE ? WARPS_PER_CTA * QCAP * 32 : 1];
+  __shared__ fx::u64 tab[VAL == VAL_FIX && KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long *qu = queue + (QUEUE ? wid * QCAP * 32 + lane : 0);
+  const FineGrid &fg = P.fg;
+  if (VAL == VAL_FIX && KIND == ABX_K_GAUSSIAN) {
+    for (int i = threadIdx.x; i < fx::EXP_TAB; i += WARPS_PER_CTA * 32) tab[i] = fx::exp_table.v[i];
+    __syncthreads();
+  }
+  const int nsing = P.counts[2], nrows = P.counts[3];
+  const int sub = lane & (P.lanes - 1);
+  const int span = 2 * max(max(fg.K[0], fg.K[1]), fg.K[2]) + 2;
+  const float4 bd = span < BAND_TAB ? P.bands[2 * span]
+                                    : tile_band(span, fg, P.r, P.r2, P.thr, NORM).a;
+  const float r2lo = bd.x, r2hi = bd.y;
+  const float p0f2 = WCUT ? P.p0f * P.p0f : 0.f;
+  for (;;) {
+    int base = 0;
+    if (lane == 0) base = atomicAdd(P.counter + 1, 32 / P.lanes);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base >= nsing) break;
+    const int mine = base + lane / P.lanes;
+    const bool act = mine < nsing;
+    const int qi = P.singles[act ? mine : base];
+    const int4 qc = P.qcell[qi];
+    const float4 ql = P.qloc[qi];
+    D4 xq;
+    if (QUEUE && VAL == VAL_FP64) xq = P.qpos[qi];
+    longlong2 fq = make_longlong2(0, 0);
+    long long fqz = 0;
+    if (VAL == VAL_FIX) {
+      fq = P.qfxy[qi];
+      fq = make_longlong2(fx::biased(fq.x), fx::biased(fq.y));
+      fqz = fx::biased(P.qfz[qi]);
+    }
+    const double si = (QUEUE && KIND == ABX_K_SCALAR_SUM) ? P.s_row[qi] : 0.0;
+    double acc = 0.0;
+    float acc32 = 0.f;
+    int count = 0, nq = 0, rows32 = 0;
+    auto evaluate = [&]() {  // one queued pair of every lane that has one
+      if (nq > 0) {
+        --nq;
+        const unsigned long long ent = qu[nq * 32];
+        const unsigned k = (unsigned)ent;
+        const int code = (int)(ent >> 32);
+        const int img[3] = {(code & 3) - 1, ((code >> 2) & 3) - 1, ((code >> 4) & 3) - 1};
+        double v;
+        if (VAL == VAL_FIX) {
+          const longlong2 f = P.fxy[k];
+          long long dx = fx::diff(f.x, fq.x), dy = fx::diff(f.y, fq.y), dz = fx::diff(P.fz[k], fqz);
+          if (code != 21) {  // 21: the centre image in every dimension
+            dx = fx::diff(dx, img[0] * P.Lfix[0]);
+            dy = fx::diff(dy, img[1] * P.Lfix[1]);
+            dz = fx::diff(dz, img[2] * P.Lfix[2]);
+          }
+          bool near;
+          v = fix_value<KIND>(dx, dy, dz, P, tab, near);
+          if (KIND == ABX_K_LAPLACE && near)
+            v = pair64<KIND>(P.qpos[qi], P.cpos[k], img, P, 0.0, 0.0);
+        } else
+          v = pair64<KIND>(xq, P.cpos[k], img, P, si, KIND == ABX_K_SCALAR_SUM ? P.s_col[k] : 0.0);
+        acc = fma(v, P.b64[k], acc);
+      }
+    };
+    for (int t0 = 0; t0 < nrows; t0 += P.lanes) {
+      const bool has = t0 + sub < nrows;
+      const int4 st = P.stencil[has ? t0 + sub : 0];  // o0, o1, reach along e2
+      {
+        int w0 = qc.x + st.x, i0 = 1, w1 = qc.y + st.y, i1 = 1;
+        bool ok = act && has;
+        if (w0 < 0) {
+          ok = ok && fg.periodic[0] && w0 >= -fg.m[0];
+          w0 += fg.m[0];
+          i0 = 2;
+        } else if (w0 >= fg.m[0]) {
+          ok = ok && fg.periodic[0] && w0 < 2 * fg.m[0];
+          w0 -= fg.m[0];
+          i0 = 0;
+        }
+        if (w1 < 0) {
+          ok = ok && fg.periodic[1] && w1 >= -fg.m[1];
+          w1 += fg.m[1];
+          i1 = 2;
+        } else if (w1 >= fg.m[1]) {
+          ok = ok && fg.periodic[1] && w1 < 2 * fg.m[1];
+          w1 -= fg.m[1];
+          i1 = 0;
+        }
+        const int a2 = qc.z - st.z, b2 = qc.z + st.z;
+        const int m2 = fg.m[2];
+        const uint32_t row = ok ? ((uint32_t)w0 * fg.m[1] + w1) * (uint32_t)m2 : 0u;
+        const float rx = fmaf((float)st.x, fg.hf[0], -ql.x), ry = fmaf((float)st.y, fg.hf[1], -ql.y);
+        // the domain itself, then (periodic e2) its images below and above
+        for (int part = 0; part < 3; ++part) {
+          const int i2 = part == 0 ? 0 : (part == 1 ? 1 : -1);  // image; wrapped w2 = u2 + i2 m2
+          const int sa = max(a2 + i2 * m2, 0), sb = min(b2 + i2 * m2, m2 - 1);
+          const bool some = ok && sa <= sb;
+          if (part > 0) {
+            if (!fg.periodic[2]) break;
+            if (!__any_sync(0xffffffffu, some)) continue;
+          }
+          uint32_t k = 0, e = 0;
+          if (some) {
+            k = P.cell_start[row + (uint32_t)sa];
+            e = P.cell_start[row + (uint32_t)sb + 1];
+          }
+          const float zs = (float)(-i2 * m2 - qc.z);
+          const int code = i0 | (i1 << 2) | ((i2 + 1) << 4);
+          while (__any_sync(0xffffffffu, k < e)) {
+            if (k < e) {
+              const float4 cl = __ldg(&P.cloc[k]);
+              const float dx = cl.x + rx, dy = cl.y + ry,
+                          dz = fmaf(cl.w + zs, fg.hf[2], cl.z) - ql.z;
+              float dd = norm32<NORM>(dx, dy, dz);
+              if (WCUT) {
+                // the clamp is the cut-off (see K_WEND_CUT)
+                dd = fmaf(dd, p0f2, 1e-30f);
+                const float t = __saturatef(fmaf(-dd, rsqrt_approx(dd), 1.f));
+                const float t2 = t * t;
+                if (t > 0.f) acc32 = fmaf(t2 * t2 * fmaf(t, -4.f, 5.f), __ldg(&P.b32[k]), acc32);
+              } else {
+                bool in = dd <= r2lo;
+                if (!in && dd <= r2hi) {  // rare: the reference's FP64 test
+                  const int img[3] = {i0 - 1, i1 - 1, i2};
+                  in = !(exact_norm(P.qpos[qi], P.cpos[k], img, fg, NORM) > P.thr);
+                }
+                if (POL == POL_COUNT) count += in ? 1 : 0;
+                if (POL == POL_MATVEC && VAL == VAL_MIXED && in)
+                  acc32 = fmaf(kern32<KIND>(dd, P), __ldg(&P.b32[k]), acc32);
+                if (QUEUE && in) {
+                  qu[nq * 32] = (unsigned long long)k | ((unsigned long long)code << 32);
+                  ++nq;
+                }
+              }
+              ++k;
+            }
+            if (QUEUE && __any_sync(0xffffffffu, nq == QCAP)) {
+              do evaluate();
+              while (__popc(__ballot_sync(0xffffffffu, nq > 0)) >= DRAIN);
+            }
+          }
+        }
+      }
+      if (VAL == VAL_MIXED && POL == POL_MATVEC && (++rows32 & 3) == 0) {
+        acc += (double)acc32;
+        acc32 = 0.f;
+      }
+    }
+    if (QUEUE)
+      while (__any_sync(0xffffffffu, nq > 0)) evaluate();
+    if (POL == POL_MATVEC && VAL == VAL_MIXED) acc += (double)acc32;
+    for (int d = 1; d < P.lanes; d <<= 1) {
+      if (POL == POL_MATVEC) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+      if (POL == POL_COUNT) count += __shfl_xor_sync(0xffffffffu, count, d);
+    }
+    if (act && sub == 0) {
+      if (POL == POL_MATVEC) P.c[qi] = acc;
+      if (POL == POL_COUNT) P.counts_out[qi] = count;
+    }
   }
 }
 
@@ -1193,23 +1631,6 @@ __global__ void k_scatter(const T *__restrict__ src, const uint32_t *__restrict_
   dst[perm[k]] = src[k];
 }
 
-// Largest e2 gap (in cells) that keeps a cell within the pruning distance,
-// for every pair of e0/e1 gaps below EXT_TAB cells (-1: pruned).
-int build_ext_table(PairLayout &L, double prune2) {
-  std::vector<int> tab(EXT_TAB * EXT_TAB);
-  const FineGrid &fg = L.fg;
-  for (int a = 0; a < EXT_TAB; ++a)
-    for (int b = 0; b < EXT_TAB; ++b) {
-      const double g0 = a * fg.h[0], g1 = b * fg.h[1];
-      const double rem = prune2 - g0 * g0 - g1 * g1;
-      tab[a * EXT_TAB + b] =
-          rem < 0.0 ? -1 : std::min((int)std::floor(std::sqrt(rem) / fg.h[2]), fg.K[2]);
-    }
-  ABX_TRY(L.ext.reserve(tab.size()));
-  ABX_CHECK_CUDA(cudaMemcpy(L.ext.ptr, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice));
-  return ABX_OK;
-}
-
 double prune_distance2(const PairLayout &L) {
   double hmax = 0;
   for (int e = 0; e < 3; ++e)
@@ -1218,9 +1639,22 @@ double prune_distance2(const PairLayout &L) {
   return (L.r + margin) * (L.r + margin);
 }
 
+int build_tables(abx_context *ctx, PairLayout &L, int norm, double thr) {
+  ABX_TRY(L.ext.reserve(EXT_TAB * EXT_TAB));
+  ABX_TRY(L.bands.reserve(2 * BAND_TAB));
+  ABX_TRY(L.stencil.reserve(ROWS_MAX));
+  k_tables<<<EXT_TAB * EXT_TAB / TABLE_TPB, TABLE_TPB, 0, ctx->stream>>>(
+      L.fg, prune_distance2(L), L.r, thr, norm, L.ext.ptr, L.bands.ptr, L.stencil.ptr,
+      L.counts.ptr + 3);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  return ABX_OK;
+}
+
 KParams base_params(const PairLayout &L) {
   KParams P{};
   P.ext = L.ext.ptr;
+  P.bands = L.bands.ptr;
+  P.stencil = L.stencil.ptr;
   P.fg = L.fg;
   P.r = L.r;
   P.r2 = L.r * L.r;
@@ -1235,83 +1669,141 @@ KParams base_params(const PairLayout &L) {
   P.qloc = L.rows->loc.ptr;
   P.qpos = L.rows->posk.ptr;
   P.units = L.units.ptr;
-  P.nunits = L.nunits;
-  P.counter = L.counter.ptr;
+  P.units_cap = L.rows->n;
+  P.singles = L.singles.ptr;
+  P.counts = L.counts.ptr;
+  P.counter = L.counts.ptr + 4;
+  P.fxy = L.cols.fxy.ptr;
+  P.fz = L.cols.fz.ptr;
+  P.qfxy = L.rows->fxy.ptr;
+  P.qfz = L.rows->fz.ptr;
+  if (L.unit.ok)
+    for (int e = 0; e < 3; ++e) P.Lfix[e] = fx::to_fixed(L.fg.L[e], L.unit.f, L.unit.k);
   return P;
 }
 
-int grid_blocks(abx_context *ctx, int nunits) {
-  int blocks = ctx->num_sms * 8;
-  const int need = (nunits + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
-  return std::max(1, std::min(blocks, need));
+// CTAs of the kernels that take their work from a counter: as many as there
+// can be work for, 8 an SM at most.
+int grid_blocks(abx_context *ctx, const KParams &P) {
+  const int64_t need = (P.units_cap + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms * 8, need));
+}
+// Lanes a query of the singles: enough queries x lanes for LANES_FILL an SM.
+constexpr int64_t LANES_FILL = 2048;
+int query_lanes(abx_context *ctx, int64_t nq) {
+  int g = 1;
+  while (g < 32 && nq * g < ctx->num_sms * LANES_FILL) g *= 2;
+  return g;
+}
+int thread_blocks(abx_context *ctx, const KParams &P) {
+  const int64_t need = (P.units_cap * P.lanes + WARPS_PER_CTA * 32 - 1) / (WARPS_PER_CTA * 32);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms * 12, need));
+}
+int reset_counters(abx_context *ctx, const KParams &P) {
+  ABX_CHECK_CUDA(cudaMemsetAsync(P.counter, 0, 2 * sizeof(int), ctx->stream));
+  return ABX_OK;
 }
 
-template <int POL, int KIND> int launch_pairs(abx_context *ctx, const KParams &P, bool mixed) {
-  const int blocks = grid_blocks(ctx, P.nunits);
-  ABX_CHECK_CUDA(cudaMemsetAsync(P.counter, 0, sizeof(int), ctx->stream));
+// The full units by a warp each, the small units' queries by a thread each.
+template <int KIND> int launch_matvec(abx_context *ctx, KParams P, bool mixed, bool fix) {
+  cudaStream_t s = ctx->stream;
+  P.lanes = query_lanes(ctx, P.units_cap);
+  const int ub = grid_blocks(ctx, P), tb = thread_blocks(ctx, P), T = WARPS_PER_CTA * 32;
+  // the two Gaussians are one kernel where it matters
+  constexpr int FK = KIND == ABX_K_COMPACT_GAUSSIAN ? ABX_K_GAUSSIAN : KIND;
+  constexpr bool CAN_FIX = FK == ABX_K_GAUSSIAN || FK == ABX_K_WENDLAND_C2 ||
+                           FK == ABX_K_LAPLACE || FK == ABX_K_MULTIQUADRIC;
+  ABX_TRY(reset_counters(ctx, P));
   if (mixed) {
-    k_pairs_mixed<POL, KIND><<<blocks, WARPS_PER_CTA * 32, 0, ctx->stream>>>(P);
+    k_pairs_mixed<POL_MATVEC, FK><<<ub, T, 0, s>>>(P);
+    k_pairs_thread<POL_MATVEC, FK, VAL_MIXED><<<tb, T, 0, s>>>(P);
   } else {
-    if constexpr (POL == POL_MATVEC) {
-      k_pairs_fp64<POL, KIND><<<blocks, WARPS_PER_CTA * 32, 0, ctx->stream>>>(P);
-    } else {
-      set_error("the FP64 pair kernel computes matvecs only");
-      return ABX_ERR_INVALID;
+    if constexpr (CAN_FIX) {
+      if (fix) {
+        k_pairs_fp64<POL_MATVEC, FK, true><<<ub, T, 0, s>>>(P);
+        k_pairs_thread<POL_MATVEC, FK, VAL_FIX><<<tb, T, 0, s>>>(P);
+        ABX_CHECK_CUDA(cudaGetLastError());
+        return ABX_OK;
+      }
+    }
+    if constexpr (KIND != K_WEND_CUT) {
+      k_pairs_fp64<POL_MATVEC, FK, false><<<ub, T, 0, s>>>(P);
+      k_pairs_thread<POL_MATVEC, FK, VAL_FP64><<<tb, T, 0, s>>>(P);
     }
   }
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
 
-// The radius search (count or list) in the norm P.lnorm.
+// The radius search (count or list) in the norm P.lnorm.  Lists keep one
+// kernel for all units: their order within a row is the unit kernel's.
+template <int POL, int NORM> int launch_search_norm(abx_context *ctx, KParams P) {
+  cudaStream_t s = ctx->stream;
+  const int T = WARPS_PER_CTA * 32;
+  P.all_units = POL == POL_LIST ? 1 : 0;
+  P.lanes = query_lanes(ctx, P.units_cap);
+  ABX_TRY(reset_counters(ctx, P));
+  k_pairs_mixed<POL, ABX_K_CONST, NORM><<<grid_blocks(ctx, P), T, 0, s>>>(P);
+  if (POL == POL_COUNT)
+    k_pairs_thread<POL_COUNT, ABX_K_CONST, VAL_MIXED, NORM><<<thread_blocks(ctx, P), T, 0, s>>>(P);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  return ABX_OK;
+}
 template <int POL> int launch_search(abx_context *ctx, const KParams &P) {
-  const int blocks = grid_blocks(ctx, P.nunits);
-  ABX_CHECK_CUDA(cudaMemsetAsync(P.counter, 0, sizeof(int), ctx->stream));
-  if (P.lnorm == 1)
-    k_pairs_mixed<POL, ABX_K_CONST, 1><<<blocks, WARPS_PER_CTA * 32, 0, ctx->stream>>>(P);
-  else if (P.lnorm == -1)
-    k_pairs_mixed<POL, ABX_K_CONST, -1><<<blocks, WARPS_PER_CTA * 32, 0, ctx->stream>>>(P);
-  else
-    k_pairs_mixed<POL, ABX_K_CONST, 2><<<blocks, WARPS_PER_CTA * 32, 0, ctx->stream>>>(P);
-  ABX_CHECK_CUDA(cudaGetLastError());
-  return ABX_OK;
+  if (P.lnorm == 1) return launch_search_norm<POL, 1>(ctx, P);
+  if (P.lnorm == -1) return launch_search_norm<POL, -1>(ctx, P);
+  return launch_search_norm<POL, 2>(ctx, P);
 }
 
-int launch_wend_cut(abx_context *ctx, const KParams &P) {
-  const int blocks = grid_blocks(ctx, P.nunits);
-  ABX_CHECK_CUDA(cudaMemsetAsync(P.counter, 0, sizeof(int), ctx->stream));
-  k_pairs_mixed<POL_MATVEC, K_WEND_CUT><<<blocks, WARPS_PER_CTA * 32, 0, ctx->stream>>>(P);
-  ABX_CHECK_CUDA(cudaGetLastError());
-  return ABX_OK;
-}
-
-template <int POL> int launch_pairs_kind(abx_context *ctx, const KParams &P, bool mixed) {
+int launch_matvec_kind(abx_context *ctx, const KParams &P, bool mixed, bool fix) {
   switch (P.kind) {
-  case ABX_K_CONST: return launch_pairs<POL, ABX_K_CONST>(ctx, P, mixed);
-  case ABX_K_GAUSSIAN: return launch_pairs<POL, ABX_K_GAUSSIAN>(ctx, P, mixed);
+  case ABX_K_CONST: return launch_matvec<ABX_K_CONST>(ctx, P, mixed, fix);
+  case ABX_K_GAUSSIAN:
+  case ABX_K_COMPACT_GAUSSIAN: return launch_matvec<ABX_K_GAUSSIAN>(ctx, P, mixed, fix);
   case ABX_K_WENDLAND_C2:
     // support 1/p0 <= r up to rounding of p0 = 1/r (a support wider by a
     // relative 1e-9 adds pairs of weight <= 5e-36)
-    if (POL == POL_MATVEC && mixed && P.p0 * P.r >= 1.0 - 1e-9) return launch_wend_cut(ctx, P);
-    return launch_pairs<POL, ABX_K_WENDLAND_C2>(ctx, P, mixed);
-  case ABX_K_COMPACT_GAUSSIAN: return launch_pairs<POL, ABX_K_COMPACT_GAUSSIAN>(ctx, P, mixed);
-  case ABX_K_LAPLACE: return launch_pairs<POL, ABX_K_LAPLACE>(ctx, P, mixed);
-  case ABX_K_MULTIQUADRIC: return launch_pairs<POL, ABX_K_MULTIQUADRIC>(ctx, P, mixed);
-  case ABX_K_SCALAR_SUM: return launch_pairs<POL, ABX_K_SCALAR_SUM>(ctx, P, false);
+    if (mixed && P.p0 * P.r >= 1.0 - 1e-9) return launch_matvec<K_WEND_CUT>(ctx, P, true, false);
+    return launch_matvec<ABX_K_WENDLAND_C2>(ctx, P, mixed, fix);
+  case ABX_K_LAPLACE: return launch_matvec<ABX_K_LAPLACE>(ctx, P, mixed, fix);
+  case ABX_K_MULTIQUADRIC: return launch_matvec<ABX_K_MULTIQUADRIC>(ctx, P, mixed, fix);
+  case ABX_K_SCALAR_SUM: return launch_matvec<ABX_K_SCALAR_SUM>(ctx, P, false, false);
   }
   set_error("unknown kernel kind %d", P.kind);
   return ABX_ERR_INVALID;
 }
 
+// The unit of an operator's FP64 product on the integer units (fix64.cuh).
+fx::Unit fix_unit(const abx_kernel &k, double r) {
+  switch (k.kind) {
+  case ABX_K_GAUSSIAN:
+  case ABX_K_COMPACT_GAUSSIAN: return fx::make_unit<fx::GAUSSIAN>(k.p[0], r);
+  case ABX_K_WENDLAND_C2: return fx::make_unit<fx::WENDLAND>(k.p[0], r);
+  case ABX_K_LAPLACE: return fx::make_unit<fx::LAPLACE>(k.p[0], r);
+  case ABX_K_MULTIQUADRIC: return fx::make_unit<fx::MULTIQUADRIC>(k.p[0], r);
+  default: return fx::Unit{};
+  }
+}
+
+int fill_fixed(abx_context *ctx, PointLayout &P, const fx::Unit &U) {
+  ABX_TRY(P.fxy.reserve(P.n ? P.n : 1));
+  ABX_TRY(P.fz.reserve(P.n ? P.n : 1));
+  if (P.n)
+    k_fill_fixed<<<ceil_div(P.n, TPB), TPB, 0, ctx->stream>>>(P.posk.ptr, P.n, U, P.fxy.ptr,
+                                                              P.fz.ptr);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  return ABX_OK;
+}
+
 // Build a layout for cols (a searchable particle set) and a query set given as
 // SoA FP64 (qsrc, nq, stride) -- or the column set itself when qsrc == null.
+// All on the context's stream, nothing waited for; norm and thr as KParams'.
 int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *qsrc, int64_t nq,
-                 int64_t qstride, PairLayout &L) {
+                 int64_t qstride, PairLayout &L, int split, int norm = 2) {
   GridDesc g;
   ABX_TRY(particles_grid_desc(cols, &g));
   L.r = r;
   L.fg = make_fine_grid(g, r, std::max<int64_t>(cols->n, 1), 3);
-  L.cols_version = cols->version;
   ABX_TRY(build_points(ctx, cols->pos.ptr, cols->n, cols->n, L.fg, true, L.cols));
   ABX_TRY(build_cell_start(ctx, L));
   if (!qsrc) {
@@ -1322,22 +1814,31 @@ int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *
     ABX_TRY(build_points(ctx, qsrc, nq, qstride, L.fg, false, L.rows_own));
     L.rows = &L.rows_own;
   }
-  ABX_TRY(build_units(ctx, L));
-  ABX_TRY(build_ext_table(L, prune_distance2(L)));
+  ABX_TRY(build_units(ctx, L, split));
+  ABX_TRY(build_tables(ctx, L, norm, norm == 2 ? r * r : std::fabs(r)));
   return ABX_OK;
 }
 
 }  // namespace
 
+static int matvec_split(const abx_operator *op) {
+  return op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM ? SPLIT_MIXED : SPLIT_FP64;
+}
+
 int pair_layout_build(abx_operator *op) {
   abx_context *ctx = op->rows->ctx;
-  if (op->pairs) delete op->pairs;
-  op->pairs = new PairLayout();
-  PairLayout &L = *op->pairs;
+  if (!op->pairs) op->pairs = new PairLayout();
+  PairLayout &L = *op->pairs;  // a rebuild keeps the buffers
+  L.cols_version = ~uint64_t(0);  // valid once everything below has succeeded
   const bool self = op->rows == op->cols;
   ABX_TRY(layout_build(ctx, op->cols, op->radius, self ? nullptr : op->rows->pos.ptr,
-                       op->rows->n, op->rows->n, L));
+                       op->rows->n, op->rows->n, L, matvec_split(op)));
   L.rows_version = op->rows->version;
+  L.unit = fix_unit(op->k, L.r);
+  if (L.unit.ok) {
+    ABX_TRY(fill_fixed(ctx, L.cols, L.unit));
+    if (!L.self) ABX_TRY(fill_fixed(ctx, L.rows_own, L.unit));
+  }
   const int64_t nr = L.rows->n, nc = L.cols.n;
   ABX_TRY(L.bk32.reserve(nc ? nc : 1));
   ABX_TRY(L.bk64.reserve(nc ? nc : 1));
@@ -1355,7 +1856,7 @@ int pair_layout_build(abx_operator *op) {
                                                              nr, nullptr, L.sq.ptr);
     ABX_CHECK_CUDA(cudaGetLastError());
   }
-  ABX_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+  L.cols_version = op->cols->version;
   return ABX_OK;
 }
 
@@ -1367,6 +1868,7 @@ int sparse_matvec_device(abx_operator *op, const double *b, double *c) {
   PairLayout &L = *op->pairs;
   const int64_t nr = L.rows->n, nc = L.cols.n;
   if (nr == 0) return ABX_OK;
+  if (L.split != matvec_split(op)) ABX_TRY(build_units(ctx, L, matvec_split(op)));
   const bool mixed = op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM;
   if (nc > 0)
     k_gather_b<<<ceil_div(nc, TPB), TPB, 0, ctx->stream>>>(
@@ -1377,6 +1879,7 @@ int sparse_matvec_device(abx_operator *op, const double *b, double *c) {
   P.p0 = op->k.p[0];
   P.p0f = (float)op->k.p[0];
   P.c_exp2 = (float)(-op->k.p[0] * 1.4426950408889634);
+  P.fixc = fx::consts(L.unit, 1.0 / P.p0);
   P.b32 = L.bk32.ptr;
   P.b64 = L.bk64.ptr;
   P.s_col = L.sk.ptr;
@@ -1386,7 +1889,7 @@ int sparse_matvec_device(abx_operator *op, const double *b, double *c) {
     ABX_CHECK_CUDA(cudaMemsetAsync(c, 0, nr * sizeof(double), ctx->stream));
     return ABX_OK;
   }
-  ABX_TRY(launch_pairs_kind<POL_MATVEC>(ctx, P, mixed));
+  ABX_TRY(launch_matvec_kind(ctx, P, mixed, L.unit.ok));
   k_scatter_c<<<ceil_div(nr, TPB), TPB, 0, ctx->stream>>>(L.ck.ptr, L.rows->perm.ptr, nr, c);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
@@ -1400,11 +1903,71 @@ __global__ void k_aos_to_soa_q(const double *__restrict__ aos, int64_t n, int di
   for (int d = 0; d < dim; ++d) soa[(int64_t)d * n + i] = aos[i * dim + d];
 }
 
-__global__ void k_count_to_i64(const int32_t *__restrict__ counts, const uint32_t *__restrict__ perm,
-                               int64_t n, int64_t *__restrict__ rowcnt) {
-  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  rowcnt[perm[k]] = counts[k];
+// Exclusive prefix sum of n counts as 64-bit row pointers (n + 1 entries):
+// sums of tiles, one CTA's scan of the sums, then the tiles.  (The counts were
+// summed on the host before: 8 B a row out and back.)
+constexpr int RP_TPB = 256, RP_ITEMS = 8, RP_TILE = RP_TPB * RP_ITEMS;
+__device__ __forceinline__ int64_t block_exclusive(int64_t v, int64_t *warp_sums, int64_t &total) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int64_t incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int64_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
+  }
+  if (lane == 31) warp_sums[w] = incl;
+  __syncthreads();
+  int64_t before = 0;
+  total = 0;
+  for (int i = 0; i < RP_TPB / 32; ++i) {
+    if (i < w) before += warp_sums[i];
+    total += warp_sums[i];
+  }
+  __syncthreads();
+  return before + incl - v;
+}
+__global__ void __launch_bounds__(RP_TPB) k_rp_sums(const int32_t *__restrict__ counts, int64_t n,
+                                                    int64_t *__restrict__ sums) {
+  __shared__ int64_t ws[RP_TPB / 32];
+  int64_t s = 0;
+  for (int i = 0; i < RP_ITEMS; ++i) {
+    const int64_t g = (int64_t)blockIdx.x * RP_TILE + i * RP_TPB + threadIdx.x;
+    if (g < n) s += counts[g];
+  }
+  int64_t total;
+  block_exclusive(s, ws, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(RP_TPB) k_rp_scan(int64_t *__restrict__ sums, int64_t nb,
+                                                    int64_t *__restrict__ last) {
+  __shared__ int64_t ws[RP_TPB / 32];
+  int64_t run = 0;
+  for (int64_t i0 = 0; i0 < nb; i0 += RP_TPB) {
+    const int64_t i = i0 + threadIdx.x;
+    int64_t total;
+    const int64_t ex = block_exclusive(i < nb ? sums[i] : 0, ws, total);
+    if (i < nb) sums[i] = run + ex;
+    run += total;
+  }
+  if (threadIdx.x == 0) *last = run;
+}
+__global__ void __launch_bounds__(RP_TPB) k_rp_write(const int32_t *__restrict__ counts, int64_t n,
+                                                     const int64_t *__restrict__ sums,
+                                                     int64_t *__restrict__ rowptr) {
+  __shared__ int64_t ws[RP_TPB / 32];
+  const int64_t base = (int64_t)blockIdx.x * RP_TILE + (int64_t)threadIdx.x * RP_ITEMS;
+  int32_t c[RP_ITEMS];
+  int64_t s = 0;
+  for (int i = 0; i < RP_ITEMS; ++i) {
+    c[i] = base + i < n ? counts[base + i] : 0;
+    s += c[i];
+  }
+  int64_t total;
+  int64_t run = sums[blockIdx.x] + block_exclusive(s, ws, total);
+  for (int i = 0; i < RP_ITEMS; ++i) {
+    if (base + i < n) rowptr[base + i] = run;
+    run += c[i];
+  }
 }
 
 __global__ void k_rowptr_to_kernel(const int64_t *__restrict__ rowptr,
@@ -1413,6 +1976,24 @@ __global__ void k_rowptr_to_kernel(const int64_t *__restrict__ rowptr,
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   rowptr_k[k] = rowptr[perm[k]];
+}
+
+// Row pointers (input order, W.rowptr, n + 1 entries) from the counts in
+// kernel order, and their total on the host.
+int rowptr_device(abx_context *ctx, SearchSpace &W, const uint32_t *perm, int64_t n, int64_t &nnz) {
+  cudaStream_t s = ctx->stream;
+  const unsigned nb = ceil_div(n, RP_TILE);
+  ABX_TRY(W.cnt.reserve(n + 1));
+  ABX_TRY(W.rowptr.reserve(n + 1));
+  ABX_TRY(W.sums.reserve(nb + 1));
+  k_scatter<int32_t><<<ceil_div(n, TPB), TPB, 0, s>>>(W.cnt_k.ptr, perm, n, W.cnt.ptr);
+  k_rp_sums<<<nb, RP_TPB, 0, s>>>(W.cnt.ptr, n, W.sums.ptr);
+  k_rp_scan<<<1, RP_TPB, 0, s>>>(W.sums.ptr, nb, W.rowptr.ptr + n);
+  k_rp_write<<<nb, RP_TPB, 0, s>>>(W.cnt.ptr, n, W.sums.ptr, W.rowptr.ptr);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  ABX_CHECK_CUDA(cudaMemcpyAsync(&nnz, W.rowptr.ptr + n, 8, cudaMemcpyDeviceToHost, s));
+  ABX_CHECK_CUDA(cudaStreamSynchronize(s));
+  return ABX_OK;
 }
 }  // namespace
 
@@ -1429,13 +2010,14 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
   const int D = p->dim;
   const void *qd;
   ABX_TRY(p->stage_b.in(ctx, q_host_or_dev, (size_t)nq * D * sizeof(double), &qd));
-  DevBuf<double> qsoa;
-  ABX_TRY(qsoa.reserve((size_t)D * (nq ? nq : 1)));
+  std::lock_guard<std::mutex> hold(p->search->m);
+  SearchSpace &W = *p->search;
+  PairLayout &L = W.L;
+  ABX_TRY(W.qsoa.reserve((size_t)D * (nq ? nq : 1)));
   if (nq)
-    k_aos_to_soa_q<<<ceil_div(nq, TPB), TPB, 0, s>>>((const double *)qd, nq, D, qsoa.ptr);
+    k_aos_to_soa_q<<<ceil_div(nq, TPB), TPB, 0, s>>>((const double *)qd, nq, D, W.qsoa.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
-  PairLayout L;
-  ABX_TRY(layout_build(ctx, p, r, qsoa.ptr, nq, nq, L));
+  ABX_TRY(layout_build(ctx, p, r, W.qsoa.ptr, nq, nq, L, SPLIT_COUNT, lnorm));
   if (nq == 0) {
     if (rowptr_user) {
       int64_t z = 0;
@@ -1443,66 +2025,55 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
     }
     return ABX_OK;
   }
-  DevBuf<int32_t> cnt_k;
-  ABX_TRY(cnt_k.reserve(nq));
+  ABX_TRY(W.cnt_k.reserve(nq + 1));
   KParams P = base_params(L);
   P.kind = ABX_K_CONST;
   P.lnorm = lnorm;
   P.thr = lnorm == 2 ? r * r : std::fabs(r);
-  P.counts = cnt_k.ptr;
-  ABX_CHECK_CUDA(cudaMemsetAsync(cnt_k.ptr, 0, nq * 4, s));
-  if (p->n > 0) ABX_TRY(launch_search<POL_COUNT>(ctx, P));
+  P.counts_out = W.cnt_k.ptr;
+  if (p->n > 0)
+    ABX_TRY(launch_search<POL_COUNT>(ctx, P));
+  else
+    ABX_CHECK_CUDA(cudaMemsetAsync(W.cnt_k.ptr, 0, nq * 4, s));
   if (counts_user) {
-    DevBuf<int32_t> cnt;
-    ABX_TRY(cnt.reserve(nq));
-    k_scatter<int32_t><<<ceil_div(nq, TPB), TPB, 0, s>>>(cnt_k.ptr, L.rows->perm.ptr, nq, cnt.ptr);
+    const int where = device_ptr_usable(counts_user, ctx->device);
+    int32_t *out = counts_user;
+    if (where != 1) {
+      ABX_TRY(W.cnt.reserve(nq + 1));
+      out = W.cnt.ptr;
+    }
+    k_scatter<int32_t><<<ceil_div(nq, TPB), TPB, 0, s>>>(W.cnt_k.ptr, L.rows->perm.ptr, nq, out);
     ABX_CHECK_CUDA(cudaGetLastError());
-    ABX_CHECK_CUDA(cudaMemcpyAsync(counts_user, cnt.ptr, nq * 4, cudaMemcpyDefault, s));
-    ABX_CHECK_CUDA(cudaStreamSynchronize(s));
+    if (where != 1) ABX_CHECK_CUDA(cudaMemcpyAsync(counts_user, out, nq * 4, cudaMemcpyDefault, s));
   }
   if (rowptr_user) {
-    // rowptr in input order: counts -> int64 -> exclusive scan (host: nq+1)
-    DevBuf<int64_t> rc;
-    ABX_TRY(rc.reserve(nq));
-    k_count_to_i64<<<ceil_div(nq, TPB), TPB, 0, s>>>(cnt_k.ptr, L.rows->perm.ptr, nq, rc.ptr);
-    ABX_CHECK_CUDA(cudaGetLastError());
-    std::vector<int64_t> h(nq + 1);
-    ABX_CHECK_CUDA(cudaMemcpyAsync(h.data(), rc.ptr, nq * 8, cudaMemcpyDeviceToHost, s));
-    ABX_CHECK_CUDA(cudaStreamSynchronize(s));
-    int64_t run = 0;
-    for (int64_t i = 0; i < nq; ++i) {
-      const int64_t c = h[i];
-      h[i] = run;
-      run += c;
-    }
-    h[nq] = run;
-    ABX_CHECK_CUDA(cudaMemcpy(rowptr_user, h.data(), (nq + 1) * 8, cudaMemcpyDefault));
+    int64_t nnz = 0;
+    ABX_TRY(rowptr_device(ctx, W, L.rows->perm.ptr, nq, nnz));
+    ABX_CHECK_CUDA(cudaMemcpyAsync(rowptr_user, W.rowptr.ptr, (nq + 1) * 8, cudaMemcpyDefault, s));
     if (cols_user) {
-      ABX_REQUIRE(cap >= run, ABX_ERR_CAPACITY, "cols capacity %lld < nnz %lld", (long long)cap,
-                  (long long)run);
-      DevBuf<int64_t> rp, rpk;
-      DevBuf<int32_t> colsd;
-      DevBuf<double> dxd;
-      ABX_TRY(rp.reserve(nq));
-      ABX_TRY(rpk.reserve(nq));
-      ABX_TRY(colsd.reserve(run ? run : 1));
+      ABX_REQUIRE(cap >= nnz, ABX_ERR_CAPACITY, "cols capacity %lld < nnz %lld", (long long)cap,
+                  (long long)nnz);
+      ABX_TRY(W.rpk.reserve(nq));
+      ABX_TRY(W.cols.reserve(nnz ? nnz : 1));
       if (dx_user) {
-        ABX_TRY(dxd.reserve((size_t)(run ? run : 1) * D));
-        P.dx_out = dxd.ptr;
+        ABX_TRY(W.dxd.reserve((size_t)(nnz ? nnz : 1) * D));
+        P.dx_out = W.dxd.ptr;
       }
-      ABX_CHECK_CUDA(cudaMemcpyAsync(rp.ptr, h.data(), nq * 8, cudaMemcpyHostToDevice, s));
-      k_rowptr_to_kernel<<<ceil_div(nq, TPB), TPB, 0, s>>>(rp.ptr, L.rows->perm.ptr, nq, rpk.ptr);
+      k_rowptr_to_kernel<<<ceil_div(nq, TPB), TPB, 0, s>>>(W.rowptr.ptr, L.rows->perm.ptr, nq,
+                                                           W.rpk.ptr);
       ABX_CHECK_CUDA(cudaGetLastError());
-      P.rowptr = rpk.ptr;
-      P.cols_out = colsd.ptr;
-      if (p->n > 0 && run > 0) ABX_TRY(launch_search<POL_LIST>(ctx, P));
-      ABX_CHECK_CUDA(cudaMemcpyAsync(cols_user, colsd.ptr, run * 4, cudaMemcpyDefault, s));
-      if (dx_user && run)
-        ABX_CHECK_CUDA(cudaMemcpyAsync(dx_user, dxd.ptr, (size_t)run * D * 8, cudaMemcpyDefault, s));
-      ABX_CHECK_CUDA(cudaStreamSynchronize(s));
+      P.rowptr = W.rpk.ptr;
+      P.cols_out = W.cols.ptr;
+      if (p->n > 0 && nnz > 0) ABX_TRY(launch_search<POL_LIST>(ctx, P));
+      ABX_CHECK_CUDA(cudaMemcpyAsync(cols_user, W.cols.ptr, nnz * 4, cudaMemcpyDefault, s));
+      if (dx_user && nnz)
+        ABX_CHECK_CUDA(cudaMemcpyAsync(dx_user, W.dxd.ptr, (size_t)nnz * D * 8, cudaMemcpyDefault, s));
     }
   }
   ABX_CHECK_CUDA(cudaStreamSynchronize(s));
+  // lists can be larger than everything else: the large ones are not kept
+  if (W.cols.cap * sizeof(int32_t) > KEEP_BYTES) W.cols.release();
+  if (W.dxd.cap * sizeof(double) > KEEP_BYTES) W.dxd.release();
   return ABX_OK;
 }
 
@@ -1513,39 +2084,30 @@ int self_csr_device(abx_particles *p, double r, DevBuf<int64_t> &rowptr, DevBuf<
   abx_context *ctx = p->ctx;
   cudaStream_t s = ctx->stream;
   const int64_t n = p->n;
-  PairLayout L;
-  ABX_TRY(layout_build(ctx, p, r, nullptr, n, n, L));
+  std::lock_guard<std::mutex> hold(p->search->m);
+  SearchSpace &W = *p->search;
+  PairLayout &L = W.L;
+  ABX_TRY(layout_build(ctx, p, r, nullptr, n, n, L, SPLIT_COUNT));
   ABX_TRY(rowptr.reserve(n + 1));
-  DevBuf<int32_t> cnt_k;
-  ABX_TRY(cnt_k.reserve(n + 1));
+  nnz = 0;
+  if (n == 0) {
+    ABX_CHECK_CUDA(cudaMemsetAsync(rowptr.ptr, 0, 8, s));
+    return cols.reserve(1);
+  }
+  ABX_TRY(W.cnt_k.reserve(n + 1));
   KParams P = base_params(L);
   P.kind = ABX_K_CONST;
-  P.counts = cnt_k.ptr;
-  ABX_CHECK_CUDA(cudaMemsetAsync(cnt_k.ptr, 0, (n + 1) * 4, s));
-  if (n > 0) ABX_TRY(launch_pairs<POL_COUNT, ABX_K_CONST>(ctx, P, true));
-  DevBuf<int64_t> rc;
-  ABX_TRY(rc.reserve(n + 1));
-  if (n) k_count_to_i64<<<ceil_div(n, TPB), TPB, 0, s>>>(cnt_k.ptr, L.rows->perm.ptr, n, rc.ptr);
-  std::vector<int64_t> h(n + 1);
-  if (n) ABX_CHECK_CUDA(cudaMemcpyAsync(h.data(), rc.ptr, n * 8, cudaMemcpyDeviceToHost, s));
-  ABX_CHECK_CUDA(cudaStreamSynchronize(s));
-  int64_t run = 0;
-  for (int64_t i = 0; i < n; ++i) {
-    const int64_t c = h[i];
-    h[i] = run;
-    run += c;
-  }
-  h[n] = run;
-  nnz = run;
-  ABX_CHECK_CUDA(cudaMemcpy(rowptr.ptr, h.data(), (n + 1) * 8, cudaMemcpyHostToDevice));
-  ABX_TRY(cols.reserve(run + 1));
-  if (n > 0 && run > 0) {
-    DevBuf<int64_t> rpk;
-    ABX_TRY(rpk.reserve(n));
-    k_rowptr_to_kernel<<<ceil_div(n, TPB), TPB, 0, s>>>(rowptr.ptr, L.rows->perm.ptr, n, rpk.ptr);
-    P.rowptr = rpk.ptr;
+  P.counts_out = W.cnt_k.ptr;
+  ABX_TRY(launch_search<POL_COUNT>(ctx, P));
+  ABX_TRY(rowptr_device(ctx, W, L.rows->perm.ptr, n, nnz));
+  ABX_CHECK_CUDA(cudaMemcpyAsync(rowptr.ptr, W.rowptr.ptr, (n + 1) * 8, cudaMemcpyDeviceToDevice, s));
+  ABX_TRY(cols.reserve(nnz + 1));
+  if (nnz > 0) {
+    ABX_TRY(W.rpk.reserve(n));
+    k_rowptr_to_kernel<<<ceil_div(n, TPB), TPB, 0, s>>>(W.rowptr.ptr, L.rows->perm.ptr, n, W.rpk.ptr);
+    P.rowptr = W.rpk.ptr;
     P.cols_out = cols.ptr;
-    ABX_TRY(launch_pairs<POL_LIST, ABX_K_CONST>(ctx, P, true));
+    ABX_TRY(launch_search<POL_LIST>(ctx, P));
     ABX_CHECK_CUDA(cudaStreamSynchronize(s));
   }
   return ABX_OK;
@@ -1632,8 +2194,9 @@ int knn_device(abx_particles *p, int k, int32_t *idx, double *d2) {
   double vol = 1.0;
   for (int d = 0; d < p->dim; ++d) vol *= g.hi[d] - g.lo[d];
   const double h = std::pow(std::max(1.0, k / 4.0) * vol / (double)n, 1.0 / p->dim);
-  PairLayout L;
-  ABX_TRY(layout_build(ctx, p, 3.0 * h, nullptr, n, n, L));
+  std::lock_guard<std::mutex> hold(p->search->m);
+  PairLayout &L = p->search->L;
+  ABX_TRY(layout_build(ctx, p, 3.0 * h, nullptr, n, n, L, SPLIT_COUNT));
   KParams P = base_params(L);
   k_knn<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(P, k, n, idx, d2);
   ABX_CHECK_CUDA(cudaGetLastError());
@@ -2023,6 +2586,8 @@ extern "C" int abx_operator_matvec_noalloc(abx_operator *op, const double *b, do
   int *counter = (int *)(base + bbytes + align256((size_t)nr * sizeof(double)));
   cudaStream_t s = ctx->stream;
   PairLayout &L = *op->pairs;
+  // (precision changed since: the units are listed anew, in the same buffers)
+  if (L.split != matvec_split(op)) ABX_TRY(build_units(ctx, L, matvec_split(op)));
   if (nc == 0) {
     ABX_CHECK_CUDA(cudaMemsetAsync(c, 0, nr * sizeof(double), s));
     return ABX_OK;
@@ -2036,13 +2601,14 @@ extern "C" int abx_operator_matvec_noalloc(abx_operator *op, const double *b, do
   P.p0 = op->k.p[0];
   P.p0f = (float)op->k.p[0];
   P.c_exp2 = (float)(-op->k.p[0] * 1.4426950408889634);
+  P.fixc = fx::consts(L.unit, 1.0 / P.p0);
   P.b32 = mixed ? (const float *)bk : nullptr;
   P.b64 = mixed ? nullptr : (const double *)bk;
   P.s_col = L.sk.ptr;
   P.s_row = L.sq.ptr;
   P.c = ck;
   P.counter = counter;  // zeroed by the launch helper before every launch
-  ABX_TRY(launch_pairs_kind<POL_MATVEC>(ctx, P, mixed));
+  ABX_TRY(launch_matvec_kind(ctx, P, mixed, L.unit.ok));
   k_scatter_c<<<ceil_div(nr, TPB), TPB, 0, s>>>(ck, L.rows->perm.ptr, nr, c);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;

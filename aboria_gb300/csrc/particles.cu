@@ -502,6 +502,7 @@ void particles_release(abx_particles *p) {
   abx_context *ctx = p->ctx;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
+  search_space_free(p->search);
   delete p;
   ctx_release(ctx);
 }
@@ -525,6 +526,7 @@ int abx_particles_create(abx_context *ctx, int dim, abx_particles **out) {
   abx_particles *p = new abx_particles();
   p->ctx = ctx;
   p->dim = dim;
+  p->search = search_space_new();
   for (int d = 0; d < 3; ++d) {
     p->grid.size[d] = 1;
     p->grid.side[d] = 1.0;

@@ -11,6 +11,9 @@
 // 16 slots in order visits the warp's items in input order; ranking with
 // __match_any_sync then gives a stable per-warp rank without a block-wide
 // local sort.
+#include <algorithm>
+#include <utility>
+
 #include "common.cuh"
 
 namespace abx {
@@ -189,6 +192,208 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(
   }
 }
 
+// ---- few tiles: the digit offsets without scan launches
+//
+// Up to RF_TILES tiles (524,288 items) a pass is two launches, counts per tile
+// and the scatter, whose CTAs each add up the whole (tile, digit) table from L2
+// (at most 1 MB) instead of three scan launches between them; with so few
+// tiles an 11-bit digit costs little, so that 22-bit keys take two passes.  N =
+// 100,000, 21-bit keys: 3 x (hist, 3 scan kernels, scatter) + 2 copies -> 2 x 2
+// launches, @RS_OLD@ -> @RS_NEW@ us.
+constexpr int RF_TILES = 128;
+template <int RB>
+__global__ void __launch_bounds__(RS_THREADS) k_rf_hist(const uint32_t *__restrict__ keys, size_t n,
+                                                        int shift, uint32_t *__restrict__ hist) {
+  constexpr int RADIX = 1 << RB;
+  __shared__ uint32_t h[RADIX];
+  for (int i = threadIdx.x; i < RADIX; i += RS_THREADS) h[i] = 0;
+  __syncthreads();
+  const size_t base = (size_t)blockIdx.x * RS_TILE;
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const size_t g = base + i * RS_THREADS + threadIdx.x;
+    if (g < n) atomicAdd(&h[(keys[g] >> shift) & (RADIX - 1)], 1u);
+  }
+  __syncthreads();
+  for (int d = threadIdx.x; d < RADIX; d += RS_THREADS) hist[(size_t)blockIdx.x * RADIX + d] = h[d];
+}
+
+// Stable rank of every item of a tile among the items of its digit: warps own
+// consecutive runs of 32 x ITEMS items, lane l the items l, l + 32, ... (see
+// the top of this file).  wcount: [warp][RADIX + 1], zeroed.
+template <int RADIX, int ITEMS, typename C>
+__device__ __forceinline__ void rank_items(const int (&dig)[ITEMS], C *wc, uint32_t (&rank)[ITEMS]) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const uint32_t peers = __match_any_sync(0xffffffffu, dig[i]);
+    const int leader = 31 - __clz(peers);
+    const uint32_t cnt = wc[dig[i]];
+    rank[i] = cnt + __popc(peers & lt_mask);
+    __syncwarp();
+    if (lane == leader) wc[dig[i]] = (C)(cnt + __popc(peers));
+    __syncwarp();
+  }
+}
+
+// Exclusive scan of RADIX values in shared memory by the CTA, THREADS at least
+// 32 and a power of two.
+template <int RADIX, int THREADS>
+__device__ __forceinline__ void scan_digits(uint32_t *v, uint32_t *warp_tot) {
+  constexpr int PER = RADIX / THREADS > 0 ? RADIX / THREADS : 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t loc[PER], sum = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    loc[k] = tid * PER + k < RADIX ? v[tid * PER + k] : 0u;
+    sum += loc[k];
+  }
+  const uint32_t incl = warp_incl_scan(sum);
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  uint32_t run = incl - sum;
+  for (int w = 0; w < warp; ++w) run += warp_tot[w];
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    if (tid * PER + k < RADIX) v[tid * PER + k] = run;
+    run += loc[k];
+  }
+  __syncthreads();
+}
+
+template <int RB>
+__global__ void __launch_bounds__(RS_THREADS) k_rf_scatter(
+    const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
+    uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, size_t n, int shift,
+    const uint32_t *__restrict__ hist) {
+  constexpr int RADIX = 1 << RB;
+  __shared__ uint16_t wcount[RS_WARPS][RADIX + 2];
+  __shared__ uint32_t first[RADIX];
+  __shared__ uint32_t warp_tot[RS_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < RS_WARPS * (RADIX + 2); i += RS_THREADS) (&wcount[0][0])[i] = 0;
+  const size_t base = (size_t)blockIdx.x * RS_TILE + (size_t)warp * (32 * RS_ITEMS);
+  uint32_t key[RS_ITEMS], val[RS_ITEMS], rank[RS_ITEMS];
+  int dig[RS_ITEMS];
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const size_t g = base + (size_t)i * 32 + lane;
+    key[i] = g < n ? keys_in[g] : 0u;
+    val[i] = g < n ? vals_in[g] : 0u;
+    dig[i] = g < n ? (int)((key[i] >> shift) & (RADIX - 1)) : RADIX;  // RADIX: never written out
+  }
+  // this tile's and all tiles' counts of every digit
+  uint32_t before[RADIX / RS_THREADS > 0 ? RADIX / RS_THREADS : 1];
+#pragma unroll
+  for (int q = 0; q * RS_THREADS < RADIX; ++q) {
+    const int d = tid + q * RS_THREADS;
+    uint32_t pre = 0, tot = 0;
+    if (d < RADIX) {
+#pragma unroll 8
+      for (unsigned t = 0; t < gridDim.x; ++t) {
+        const uint32_t c = hist[(size_t)t * RADIX + d];
+        tot += c;
+        pre += t < blockIdx.x ? c : 0u;
+      }
+      first[d] = tot;
+    }
+    before[q] = pre;
+  }
+  __syncthreads();
+  scan_digits<RADIX, RS_THREADS>(first, warp_tot);
+  rank_items<RADIX, RS_ITEMS>(dig, wcount[warp], rank);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q * RS_THREADS < RADIX; ++q) {
+    const int d = tid + q * RS_THREADS;
+    if (d < RADIX) {
+      first[d] += before[q];
+      uint32_t run = 0;
+#pragma unroll
+      for (int w = 0; w < RS_WARPS; ++w) {
+        const uint32_t c = wcount[w][d];
+        wcount[w][d] = (uint16_t)run;
+        run += c;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    if (dig[i] < RADIX) {
+      const uint32_t dst = first[dig[i]] + wcount[warp][dig[i]] + rank[i];
+      keys_out[dst] = key[i];
+      vals_out[dst] = val[i];
+    }
+  }
+}
+
+// ---- one tile: all passes in one launch, the items in shared memory between
+// them.
+constexpr int R1_THREADS = 512, R1_ITEMS = 8, R1_TILE = R1_THREADS * R1_ITEMS, R1_RB = 8;
+__global__ void __launch_bounds__(R1_THREADS) k_r1_sort(uint32_t *__restrict__ keys,
+                                                        uint32_t *__restrict__ vals, int n,
+                                                        int bits) {
+  constexpr int RADIX = 1 << R1_RB, WARPS = R1_THREADS / 32;
+  __shared__ uint32_t sk[R1_TILE], sv[R1_TILE];
+  __shared__ uint16_t wcount[WARPS][RADIX + 2];
+  __shared__ uint32_t first[RADIX], warp_tot[WARPS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < n; i += R1_THREADS) {
+    sk[i] = keys[i];
+    sv[i] = vals[i];
+  }
+  for (int shift = 0; shift < bits; shift += R1_RB) {
+    for (int i = tid; i < WARPS * (RADIX + 2); i += R1_THREADS) (&wcount[0][0])[i] = 0;
+    __syncthreads();
+    uint32_t key[R1_ITEMS], val[R1_ITEMS], rank[R1_ITEMS];
+    int dig[R1_ITEMS];
+#pragma unroll
+    for (int i = 0; i < R1_ITEMS; ++i) {
+      const int g = warp * (32 * R1_ITEMS) + i * 32 + lane;
+      key[i] = g < n ? sk[g] : 0u;
+      val[i] = g < n ? sv[g] : 0u;
+      dig[i] = g < n ? (int)((key[i] >> shift) & (RADIX - 1)) : RADIX;
+    }
+    rank_items<RADIX, R1_ITEMS>(dig, wcount[warp], rank);
+    __syncthreads();
+    if (tid < RADIX) {
+      uint32_t run = 0;
+      for (int w = 0; w < WARPS; ++w) {
+        const uint32_t c = wcount[w][tid];
+        wcount[w][tid] = (uint16_t)run;
+        run += c;
+      }
+      first[tid] = run;
+    }
+    __syncthreads();
+    scan_digits<RADIX, R1_THREADS>(first, warp_tot);
+#pragma unroll
+    for (int i = 0; i < R1_ITEMS; ++i) {
+      if (dig[i] < RADIX) {
+        const uint32_t dst = first[dig[i]] + wcount[warp][dig[i]] + rank[i];
+        sk[dst] = key[i];
+        sv[dst] = val[i];
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < n; i += R1_THREADS) {
+    keys[i] = sk[i];
+    vals[i] = sv[i];
+  }
+}
+
+template <int RB>
+int rf_pass(const uint32_t *ki, const uint32_t *vi, uint32_t *ko, uint32_t *vo, size_t n, int shift,
+            uint32_t *hist, int ntiles, cudaStream_t s) {
+  k_rf_hist<RB><<<ntiles, RS_THREADS, 0, s>>>(ki, n, shift, hist);
+  k_rf_scatter<RB><<<ntiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, shift, hist);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  return ABX_OK;
+}
+
 }  // namespace
 
 size_t scan_temp_elems(size_t n) {
@@ -221,15 +426,40 @@ int exclusive_scan_u32(uint32_t *data, size_t n, uint32_t *temp, cudaStream_t s)
 size_t radix_temp_u32(size_t n) {
   const size_t ntiles = (n + RS_TILE - 1) / RS_TILE;
   const size_t hist = ntiles * RADIX_MAX;
-  return hist + 64 + scan_temp_elems(hist);
+  // (the passes over few tiles: 2048 digits)
+  return std::max(hist + 64 + scan_temp_elems(hist), std::min<size_t>(ntiles, RF_TILES) * 2048);
 }
 
 int radix_sort_pairs(uint32_t *keys, uint32_t *vals, size_t n, int bits, uint32_t *keys_alt,
                      uint32_t *vals_alt, uint32_t *temp, cudaStream_t s) {
   if (n <= 1 || bits <= 0) return ABX_OK;
-  // digit width: 10 bits where that saves a pass (17..20-bit keys)
-  const int rb = (bits > 16 && bits <= 20) ? 10 : 8;
   const int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
+  if (n <= (size_t)R1_TILE) {
+    k_r1_sort<<<1, R1_THREADS, 0, s>>>(keys, vals, (int)n, bits);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
+  if (ntiles <= RF_TILES) {
+    uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
+    const int passes = (bits + 10) / 11, rb = (bits + passes - 1) / passes;
+    for (int shift = 0; shift < bits; shift += rb) {
+      if (rb <= 8)
+        ABX_TRY(rf_pass<8>(ki, vi, ko, vo, n, shift, temp, ntiles, s));
+      else if (rb <= 10)
+        ABX_TRY(rf_pass<10>(ki, vi, ko, vo, n, shift, temp, ntiles, s));
+      else
+        ABX_TRY(rf_pass<11>(ki, vi, ko, vo, n, shift, temp, ntiles, s));
+      std::swap(ki, ko);
+      std::swap(vi, vo);
+    }
+    if (ki != keys) {
+      ABX_CHECK_CUDA(cudaMemcpyAsync(keys, ki, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+      ABX_CHECK_CUDA(cudaMemcpyAsync(vals, vi, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+    }
+    return ABX_OK;
+  }
+  // digit width: 9 or 10 bits where that saves a pass (17..20- and 25..27-bit keys)
+  const int rb = (bits > 16 && bits <= 20) ? 10 : (bits > 24 && bits <= 27) ? 9 : 8;
   const size_t hist_n = (size_t)ntiles << rb;
   uint32_t *hist = temp;
   uint32_t *scan_tmp = temp + hist_n + 64;
@@ -239,12 +469,16 @@ int radix_sort_pairs(uint32_t *keys, uint32_t *vals, size_t n, int bits, uint32_
     const uint32_t mask = (1u << nb) - 1u;
     if (rb == 10)
       k_radix_hist<10><<<ntiles, RS_THREADS, 0, s>>>(ki, n, shift, mask, hist, ntiles);
+    else if (rb == 9)
+      k_radix_hist<9><<<ntiles, RS_THREADS, 0, s>>>(ki, n, shift, mask, hist, ntiles);
     else
       k_radix_hist<8><<<ntiles, RS_THREADS, 0, s>>>(ki, n, shift, mask, hist, ntiles);
     ABX_CHECK_CUDA(cudaGetLastError());
     ABX_TRY(exclusive_scan_u32(hist, hist_n, scan_tmp, s));
     if (rb == 10)
       k_radix_scatter<10><<<ntiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, shift, mask, hist, ntiles);
+    else if (rb == 9)
+      k_radix_scatter<9><<<ntiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, shift, mask, hist, ntiles);
     else
       k_radix_scatter<8><<<ntiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, shift, mask, hist, ntiles);
     ABX_CHECK_CUDA(cudaGetLastError());

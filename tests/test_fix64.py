@@ -14,32 +14,29 @@ SRC = r"""
 #include "fix64.cuh"
 using namespace abx::fx;
 static constexpr ExpTable TAB = make_exp_table();
-static void sums(const double *x, const double *y, int dim, int K, i64 &S, i64 &T, u64 &U) {
-  S = T = 0; U = 0;
-  for (int d = 0; d < dim; ++d) {
-    const i64 dx = (i64)((u64)to_fixed(y[d], K) - (u64)to_fixed(x[d], K));
-    sq_acc(dx, S, T);
-    U += sq_low(dx);
-  }
+template <int KIND> static double run(const double *x, const double *y, int dim, double reach,
+                                      double p0) {
+  const Unit U = make_unit<KIND>(p0, reach);
+  if (!U.ok) return -2.0;
+  i64 d[3] = {0, 0, 0};
+  for (int k = 0; k < dim; ++k)
+    d[k] = diff(fixed<KIND>(y[k], U), biased(fixed<KIND>(x[k], U)));
+  bool near;
+  const double v = value<KIND>(d[0], d[1], d[2], dim, consts(U, 1.0 / p0), TAB.v, near);
+  return near ? -1.0 : v;
 }
 extern "C" {
-double v_gauss(const double *x, const double *y, int dim, int r, double p0) {
-  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
-  return gaussian(sq_sum(S, T), gaussian_constant(ldexp(p0, 2 * r)), TAB.v);
+double v_gauss(const double *x, const double *y, int dim, double reach, double p0) {
+  return run<GAUSSIAN>(x, y, dim, reach, p0);
 }
-double v_wend(const double *x, const double *y, int dim, int r, double p0) {
-  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
-  return wendland(mulhi63(sq_sum(S, T), wendland_constant(p0, r)));
+double v_wend(const double *x, const double *y, int dim, double reach, double p0) {
+  return run<WENDLAND>(x, y, dim, reach, p0);
 }
-double v_lap(const double *x, const double *y, int dim, int r, double p0) {
-  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
-  u64 pm; int pe, z; laplace_constant(p0, r, pm, pe);
-  const u64 n = norm_d2(S, T, U, z);
-  return laplace_far(S) ? laplace(n, z, pm, pe, r) : -1.0;
+double v_lap(const double *x, const double *y, int dim, double reach, double p0) {
+  return run<LAPLACE>(x, y, dim, reach, p0);
 }
-double v_mq(const double *x, const double *y, int dim, int r, double p0) {
-  i64 S, T; u64 U; sums(x, y, dim, 62 - r, S, T, U);
-  return multiquadric(sq_sum(S, T) + (u64)ldexp(p0, 63 - 2 * r), r);
+double v_mq(const double *x, const double *y, int dim, double reach, double p0) {
+  return run<MULTIQUADRIC>(x, y, dim, reach, p0);
 }
 }
 """
@@ -97,7 +94,7 @@ def test_values_within_an_ulp(lib, kind, p0r2, dim):
         while 2.0 ** (r - 1) >= reach * 1.0001:
             r -= 1
         X, Y = (C.c_double * dim)(*x), (C.c_double * dim)(*y)
-        got = Decimal(getattr(lib, "v_" + kind)(X, Y, dim, r, C.c_double(p0)))
+        got = Decimal(getattr(lib, "v_" + kind)(X, Y, dim, C.c_double(radius), C.c_double(p0)))
         want, slack = _exact(kind, x, y, p0)
         if got == -1:  # left to the FP64 formula: closer than R / 128
             assert kind == "lap" and dist < 2.0 ** (r - 7)
@@ -107,7 +104,8 @@ def test_values_within_an_ulp(lib, kind, p0r2, dim):
 
 def test_limits(lib):
     x, far = (C.c_double * 1)(0.25), (C.c_double * 1)(0.25 + 0.5)
-    assert lib.v_gauss(x, x, 1, 0, C.c_double(3.0)) == 1.0
-    assert lib.v_wend(x, x, 1, -1, C.c_double(2.0)) == 1.0
-    assert lib.v_wend(x, far, 1, -1, C.c_double(2.0)) == 0.0     # q = 1
-    assert lib.v_mq(x, x, 1, 0, C.c_double(0.25)) == 0.5
+    assert lib.v_gauss(x, x, 1, C.c_double(1.0), C.c_double(3.0)) == 1.0
+    assert lib.v_wend(x, x, 1, C.c_double(0.5), C.c_double(2.0)) == 1.0
+    assert lib.v_wend(x, far, 1, C.c_double(0.5), C.c_double(2.0)) == 0.0     # q = 1
+    assert lib.v_mq(x, x, 1, C.c_double(0.5), C.c_double(0.25)) == 0.5
+    assert lib.v_lap(x, x, 1, C.c_double(0.5), C.c_double(0.125)) == 8.0
