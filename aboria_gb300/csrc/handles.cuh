@@ -5,6 +5,7 @@
 #include <array>
 
 #include "common.cuh"
+#include "fix64.cuh"
 
 namespace abx {
 
@@ -168,6 +169,7 @@ int octree_build_device(abx_particles *p, const uint32_t *tags, int64_t na);
 int fmm_traverse_device(abx_particles *p, const double *boxes, double eta, FmmLists &out);
 // pairs.cu
 int pair_layout_build(abx_operator *op);
+fx::Unit fix_unit(const abx_kernel &k, double reach);  // fix64.cuh's unit of a kernel
 void pair_layout_free(PairLayout *L);
 int sparse_matvec_device(abx_operator *op, const double *b, double *c);
 // operators.cu

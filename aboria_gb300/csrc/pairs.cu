@@ -67,6 +67,12 @@ struct PointLayout {
   DevBuf<uint32_t> tmp;   // sort scratch
 };
 
+// Written by k_tables into pinned host memory: seq last.
+struct HostCounts {
+  int full, singles;
+  int seq;
+};
+
 struct PairLayout {
   FineGrid fg;
   double r = 0;
@@ -82,16 +88,24 @@ struct PairLayout {
   DevBuf<int2> units;
   DevBuf<int> singles;
   int split = 0;
-  DevBuf<int> counts;  // full units, small units, singles, work counters
+  // full units, small units, their queries, stencil rows; work counters of a
+  // count or product (4, 5) and of a list search (6, 7); small units and single
+  // queries that a count or product works (8, 9)
+  DevBuf<int> counts;
+  // the first three on the host, once the device has written them: one of the
+  // two pair kernels has no work at uniform density, and is not launched then
+  HostCounts *host = nullptr;
+  int host_seq = 0;
+  ~PairLayout() {
+    if (host) cudaFreeHost(host);
+  }
   DevBuf<float> bk32;
   DevBuf<double> bk64;
   DevBuf<double> sk;  // column scalar in kernel order
   DevBuf<double> sq;  // row scalar in kernel order
-  DevBuf<double> ck;  // result in row kernel order
   DevBuf<int> ext;        // e2 extent table
   DevBuf<float4> bands;   // rounding bands by tile span (k_tables)
   DevBuf<int4> stencil;   // unpruned rows of a cell's stencil (k_tables)
-  DevBuf<uint32_t> tmp;   // scan scratch
   fx::Unit unit{};  // FP64 on the integer units, where unit.ok
 };
 
@@ -103,7 +117,7 @@ struct SearchSpace {
   std::mutex m;
   PairLayout L;
   DevBuf<double> qsoa, dxd;
-  DevBuf<int32_t> cnt_k, cnt, cols;
+  DevBuf<int32_t> cnt, cols;
   DevBuf<int64_t> rowptr, rpk, sums;
 };
 constexpr size_t KEEP_BYTES = size_t(256) << 20;
@@ -121,6 +135,8 @@ constexpr int GROUP_E2 = 4;  // a unit spans at most this many fine cells along 
 // at 4M 4: 20.6, 7: 20.9, 12: 21.5 ms (its unit kernel spends little on a
 // query, so fewer make a unit worth while).
 constexpr int SPLIT_FP64 = 12, SPLIT_COUNT = 7, SPLIT_MIXED = 4;
+
+constexpr int COUNTS = 16;
 
 enum { POL_COUNT = 0, POL_LIST = 1, POL_MATVEC = 2 };
 
@@ -240,18 +256,48 @@ __global__ void k_fill_layout(const double *__restrict__ src, int64_t stride, Fi
   posk[k] = D4{x[0], x[1], x[2], 0.0};
 }
 
-__global__ void k_mark_runs_fine(const uint32_t *__restrict__ keys, int64_t n,
-                                 uint32_t *__restrict__ first, uint32_t *__restrict__ last) {
-  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const uint32_t key = keys[k] >> 3;
-  if (k == 0 || (keys[k - 1] >> 3) != key) first[key] = (uint32_t)k;
-  if (k == n - 1 || (keys[k + 1] >> 3) != key) last[key] = (uint32_t)(k + 1);
+// First index of keys[0, n) whose value is >= key, by a 32-way search (whole
+// warps).
+__device__ __forceinline__ int64_t warp_lower_bound(const uint32_t *__restrict__ keys, int64_t n,
+                                                    uint64_t key, int lane) {
+  int64_t lo = 0, hi = n;  // the answer lies in [lo, hi]
+  while (hi - lo > 32) {
+    const int64_t step = (hi - lo + 32) / 33;
+    const int64_t i = lo + (int64_t)(lane + 1) * step;
+    const unsigned m = __ballot_sync(0xffffffffu, i < hi && (uint64_t)keys[i < hi ? i : lo] < key);
+    const int c = __popc(m);  // probes below the key form a prefix
+    const int64_t nlo = c ? lo + (int64_t)c * step + 1 : lo;
+    hi = c < 32 && lo + (int64_t)(c + 1) * step < hi ? lo + (int64_t)(c + 1) * step : hi;
+    lo = nlo;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, lo + lane < hi && (uint64_t)keys[lo + lane] < key);
+  return lo + __popc(m);
 }
 
-__global__ void k_sub(const uint32_t *__restrict__ a, uint32_t n, uint32_t *__restrict__ b) {
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < n) b[c] -= a[c];
+// cell_start[c] = first of the n sorted keys in cell c or beyond, c <= ncells:
+// a CTA's cells are consecutive, so its threads search only between the first
+// keys of its first and last cell, which two warps find.  (Marking, counting
+// and scanning took six launches.)
+__global__ void __launch_bounds__(TPB) k_cell_start(const uint32_t *__restrict__ keys, int64_t n,
+                                                    uint32_t ncells,
+                                                    uint32_t *__restrict__ cell_start) {
+  __shared__ int64_t range[2];
+  const int64_t c0 = (int64_t)blockIdx.x * TPB;
+  const int w = threadIdx.x >> 5;
+  if (w < 2) {
+    const int64_t c = w ? min(c0 + TPB, (int64_t)ncells) : c0;
+    const int64_t at = warp_lower_bound(keys, n, (uint64_t)c * 8, threadIdx.x & 31);
+    if ((threadIdx.x & 31) == 0) range[w] = at;
+  }
+  __syncthreads();
+  const int64_t c = c0 + threadIdx.x;
+  if (c > (int64_t)ncells) return;
+  int64_t lo = range[0], hi = range[1];
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if ((uint64_t)keys[mid] < (uint64_t)c * 8) lo = mid + 1; else hi = mid;
+  }
+  cell_start[c] = (uint32_t)lo;
 }
 
 // Fixed-point positions of a point set in kernel order.
@@ -290,41 +336,12 @@ int build_points(abx_context *ctx, const double *src_soa, int64_t n, int64_t str
 }
 
 int build_cell_start(abx_context *ctx, PairLayout &L) {
-  cudaStream_t s = ctx->stream;
   const uint32_t nc = L.fg.ncells;
   ABX_TRY(L.cell_start.reserve((size_t)nc + 1));
-  ABX_TRY(L.tmp.reserve((size_t)nc + 1 + scan_temp_elems((size_t)nc + 1)));
-  uint32_t *cs = L.cell_start.ptr, *first = L.tmp.ptr;
-  ABX_CHECK_CUDA(cudaMemsetAsync(cs, 0, ((size_t)nc + 1) * 4, s));
-  ABX_CHECK_CUDA(cudaMemsetAsync(first, 0, ((size_t)nc + 1) * 4, s));
-  const int64_t n = L.cols.n;
-  if (n > 0) {
-    k_mark_runs_fine<<<ceil_div(n, TPB), TPB, 0, s>>>(L.cols.keys.ptr, n, first, cs);
-    ABX_CHECK_CUDA(cudaGetLastError());
-    k_sub<<<ceil_div(nc, TPB), TPB, 0, s>>>(first, nc, cs);
-    ABX_CHECK_CUDA(cudaGetLastError());
-  }
-  // counts -> exclusive scan over nc+1 entries (last entry 0 -> total)
-  ABX_TRY(exclusive_scan_u32(cs, (size_t)nc + 1, first + nc + 1, s));
+  k_cell_start<<<ceil_div((size_t)nc + 1, TPB), TPB, 0, ctx->stream>>>(L.cols.keys.ptr, L.cols.n, nc,
+                                                                       L.cell_start.ptr);
+  ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
-}
-
-// First index of keys[0, n) whose value is >= key, by a 32-way search (whole
-// warps).
-__device__ __forceinline__ int64_t warp_lower_bound(const uint32_t *__restrict__ keys, int64_t n,
-                                                    uint64_t key, int lane) {
-  int64_t lo = 0, hi = n;  // the answer lies in [lo, hi]
-  while (hi - lo > 32) {
-    const int64_t step = (hi - lo + 32) / 33;
-    const int64_t i = lo + (int64_t)(lane + 1) * step;
-    const unsigned m = __ballot_sync(0xffffffffu, i < hi && (uint64_t)keys[i < hi ? i : lo] < key);
-    const int c = __popc(m);  // probes below the key form a prefix
-    const int64_t nlo = c ? lo + (int64_t)c * step + 1 : lo;
-    hi = c < 32 && lo + (int64_t)(c + 1) * step < hi ? lo + (int64_t)(c + 1) * step : hi;
-    lo = nlo;
-  }
-  const unsigned m = __ballot_sync(0xffffffffu, lo + lane < hi && (uint64_t)keys[lo + lane] < key);
-  return lo + __popc(m);
 }
 
 // Units: greedy runs of <= 32 consecutive queries (kernel order) whose anchor
@@ -420,8 +437,8 @@ int build_units(abx_context *ctx, PairLayout &L, int split) {
   ABX_REQUIRE(n < (int64_t)0x7fffffff, ABX_ERR_INVALID, "too many query points");
   ABX_TRY(L.units.reserve(n ? n : 1));
   ABX_TRY(L.singles.reserve(n ? n : 1));
-  ABX_TRY(L.counts.reserve(8));
-  ABX_CHECK_CUDA(cudaMemsetAsync(L.counts.ptr, 0, 3 * sizeof(int), ctx->stream));
+  ABX_TRY(L.counts.reserve(COUNTS));
+  ABX_CHECK_CUDA(cudaMemsetAsync(L.counts.ptr, 0, COUNTS * sizeof(int), ctx->stream));
   if (n == 0) return ABX_OK;
   const uint32_t ncol = (uint32_t)L.fg.m[0] * L.fg.m[1];
   const unsigned blocks = std::min(ceil_div(ncol, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
@@ -467,6 +484,7 @@ struct KParams {
   const int *counts;     // full units, small units, singles
   int all_units;         // 1: the small units too (searches that write lists)
   int *counter;          // work counters: units, singles
+  int known_full, known_singles;  // work of the two kernels, -1: not known (yet)
   const float4 *bands;   // two entries a span: r2lo, r2hi, r2box, rbox_inf; r2mid, r2half
   const int4 *stencil;   // unpruned rows of a cell's stencil, counts[3] of them
   int lanes;             // lanes a query of the singles
@@ -475,12 +493,13 @@ struct KParams {
   const long long *fz, *qfz;
   long long Lfix[3];
   fx::Consts fixc;
-  // outputs (query kernel order)
+  // outputs (by row)
   int32_t *counts_out;
   const int64_t *rowptr;  // for LIST: query kernel order -> output offset
   int32_t *cols_out;      // storage index of the column particle
   double *dx_out;         // for LIST (optional): x_j - (x_i + image*L), D per pair
   const uint32_t *cperm;  // column kernel order -> storage index
+  const uint32_t *qperm;  // query kernel order -> row
   double *c;
 };
 
@@ -852,8 +871,11 @@ __device__ __forceinline__ TileBand tile_band(int span, const FineGrid &fg, doub
 //
 // rows: the rows (e0, e1 offsets) of a single cell's stencil that are not
 // pruned, in row-major order, as (o0, o1, reach along e2); their number goes
-// to *nrows (k_pairs_thread).  By block 0.
+// to counts[3] (k_pairs_thread).  By block 0, which also decides whether the
+// small units are worked by the unit kernel after all and tells the host which
+// of the two kernels have work.
 constexpr int TABLE_TPB = 256;
+constexpr int FOLD = 16;        // fewer than 1 / FOLD of the queries: no second kernel
 constexpr int ROWS_MAX = 1024;  // (2 K0 + 1)(2 K1 + 1), K <= 7 (make_fine_grid)
 __device__ __forceinline__ int row_reach(int a, int b, const FineGrid &fg, double prune2, int norm) {
   if (norm == -1) return fg.K[2];  // the chebyshev ball is the whole stencil box
@@ -866,7 +888,8 @@ __global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2
                                                       double thr, int norm, int *__restrict__ ext,
                                                       float4 *__restrict__ bands,
                                                       int4 *__restrict__ rows,
-                                                      int *__restrict__ nrows) {
+                                                      int *__restrict__ counts, int nq,
+                                                      HostCounts *host, int seq) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x == 0) {
     __shared__ int wsum[TABLE_TPB / 32];
@@ -888,7 +911,19 @@ __global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2
       if (reach >= 0 && at < ROWS_MAX) rows[at] = make_int4(a, b, reach, 0);
       __syncthreads();
     }
-    if (threadIdx.x == 0) *nrows = min(done, ROWS_MAX);
+    if (threadIdx.x == 0) {
+      counts[3] = min(done, ROWS_MAX);
+      // a second kernel is not worth its launch for few queries
+      const bool fold = (int64_t)counts[2] * FOLD < nq;
+      counts[8] = fold ? counts[1] : 0;
+      counts[9] = fold ? 0 : counts[2];
+      if (host) {
+        host->full = counts[0] + counts[8];
+        host->singles = counts[9];
+        __threadfence_system();
+        *(volatile int *)&host->seq = seq;
+      }
+    }
   }
   if (t < EXT_TAB * EXT_TAB) {
     const double g0 = (t / EXT_TAB) * fg.h[0], g1 = (t % EXT_TAB) * fg.h[1];
@@ -931,7 +966,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
   const unsigned lt = (1u << lane) - 1u;
   constexpr bool WCUT = KIND == K_WEND_CUT;
   const float sc = WCUT ? P.p0f : 1.f;  // staging scale (d^2 = q^2 for WCUT)
-  const int nfull = P.counts[0], nunits = nfull + (P.all_units ? P.counts[1] : 0);
+  const int nfull = P.counts[0], nunits = nfull + P.counts[P.all_units ? 1 : 8];
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = atomicAdd(P.counter, 1);
@@ -1193,8 +1228,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
       }
     }
     if (active) {
-      if (POL == POL_MATVEC) P.c[qi] = acc64;
-      if (POL == POL_COUNT) P.counts_out[qi] = count;
+      if (POL == POL_MATVEC) P.c[P.qperm[qi]] = acc64;
+      if (POL == POL_COUNT) P.counts_out[P.qperm[qi]] = count;
     }
   }
 }
@@ -1255,7 +1290,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
   WarpTile64 &sm = tile_all[wid];
   const FineGrid &fg = P.fg;
   const unsigned lt = (1u << lane) - 1u;
-  const int nfull = P.counts[0], nunits = nfull + (P.all_units ? P.counts[1] : 0);
+  const int nfull = P.counts[0], nunits = nfull + P.counts[P.all_units ? 1 : 8];
   __shared__ fx::u64 tab[FIX && KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
   if (FIX && KIND == ABX_K_GAUSSIAN) {
     for (int i = threadIdx.x; i < fx::EXP_TAB; i += WARPS_PER_CTA * 32) tab[i] = fx::exp_table.v[i];
@@ -1421,7 +1456,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
         __syncwarp();
       }
     }
-    if (active) P.c[qi] = acc;
+    if (active) P.c[P.qperm[qi]] = acc;
   }
 }
 
@@ -1454,7 +1489,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
     for (int i = threadIdx.x; i < fx::EXP_TAB; i += WARPS_PER_CTA * 32) tab[i] = fx::exp_table.v[i];
     __syncthreads();
   }
-  const int nsing = P.counts[2], nrows = P.counts[3];
+  const int nsing = P.counts[9], nrows = P.counts[3];
   const int sub = lane & (P.lanes - 1);
   const int span = 2 * max(max(fg.K[0], fg.K[1]), fg.K[2]) + 2;
   const float4 bd = span < BAND_TAB ? P.bands[2 * span]
@@ -1601,34 +1636,22 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
       if (POL == POL_COUNT) count += __shfl_xor_sync(0xffffffffu, count, d);
     }
     if (act && sub == 0) {
-      if (POL == POL_MATVEC) P.c[qi] = acc;
-      if (POL == POL_COUNT) P.counts_out[qi] = count;
+      if (POL == POL_MATVEC) P.c[P.qperm[qi]] = acc;
+      if (POL == POL_COUNT) P.counts_out[P.qperm[qi]] = count;
     }
   }
 }
 
+// b in the columns' kernel order; zeroes the pair kernels' work counters.
 __global__ void k_gather_b(const double *__restrict__ b, const uint32_t *__restrict__ perm,
-                           int64_t n, float *__restrict__ b32, double *__restrict__ b64) {
+                           int64_t n, float *__restrict__ b32, double *__restrict__ b64,
+                           int *__restrict__ counters) {
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0 && counters) counters[0] = counters[1] = 0;
   if (k >= n) return;
   const double v = b[perm[k]];
   if (b32) b32[k] = (float)v;
   if (b64) b64[k] = v;
-}
-
-__global__ void k_scatter_c(const double *__restrict__ ck, const uint32_t *__restrict__ perm,
-                            int64_t n, double *__restrict__ c) {
-  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  c[perm[k]] = ck[k];
-}
-
-template <class T>
-__global__ void k_scatter(const T *__restrict__ src, const uint32_t *__restrict__ perm, int64_t n,
-                          T *__restrict__ dst) {
-  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  dst[perm[k]] = src[k];
 }
 
 double prune_distance2(const PairLayout &L) {
@@ -1645,9 +1668,15 @@ int build_tables(abx_context *ctx, PairLayout &L, int norm, double thr) {
   ABX_TRY(L.stencil.reserve(ROWS_MAX));
   k_tables<<<EXT_TAB * EXT_TAB / TABLE_TPB, TABLE_TPB, 0, ctx->stream>>>(
       L.fg, prune_distance2(L), L.r, thr, norm, L.ext.ptr, L.bands.ptr, L.stencil.ptr,
-      L.counts.ptr + 3);
+      L.counts.ptr, (int)L.rows->n, L.host, ++L.host_seq);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
+}
+
+// The units anew for another split, in the same buffers.
+int relist_units(abx_context *ctx, PairLayout &L, int split) {
+  ABX_TRY(build_units(ctx, L, split));
+  return build_tables(ctx, L, 2, L.r * L.r);
 }
 
 KParams base_params(const PairLayout &L) {
@@ -1673,6 +1702,10 @@ KParams base_params(const PairLayout &L) {
   P.singles = L.singles.ptr;
   P.counts = L.counts.ptr;
   P.counter = L.counts.ptr + 4;
+  P.qperm = L.rows->perm.ptr;
+  const bool known = L.host && *(volatile int *)&L.host->seq == L.host_seq;
+  P.known_full = known ? L.host->full : -1;
+  P.known_singles = known ? L.host->singles : -1;
   P.fxy = L.cols.fxy.ptr;
   P.fz = L.cols.fz.ptr;
   P.qfxy = L.rows->fxy.ptr;
@@ -1699,12 +1732,7 @@ int thread_blocks(abx_context *ctx, const KParams &P) {
   const int64_t need = (P.units_cap * P.lanes + WARPS_PER_CTA * 32 - 1) / (WARPS_PER_CTA * 32);
   return (int)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms * 12, need));
 }
-int reset_counters(abx_context *ctx, const KParams &P) {
-  ABX_CHECK_CUDA(cudaMemsetAsync(P.counter, 0, 2 * sizeof(int), ctx->stream));
-  return ABX_OK;
-}
-
-// The full units by a warp each, the small units' queries by a thread each.
+// The full units by a warp each, the small units' queries by P.lanes lanes each.
 template <int KIND> int launch_matvec(abx_context *ctx, KParams P, bool mixed, bool fix) {
   cudaStream_t s = ctx->stream;
   P.lanes = query_lanes(ctx, P.units_cap);
@@ -1713,22 +1741,22 @@ template <int KIND> int launch_matvec(abx_context *ctx, KParams P, bool mixed, b
   constexpr int FK = KIND == ABX_K_COMPACT_GAUSSIAN ? ABX_K_GAUSSIAN : KIND;
   constexpr bool CAN_FIX = FK == ABX_K_GAUSSIAN || FK == ABX_K_WENDLAND_C2 ||
                            FK == ABX_K_LAPLACE || FK == ABX_K_MULTIQUADRIC;
-  ABX_TRY(reset_counters(ctx, P));
+  const bool units = P.known_full != 0, singles = P.known_singles != 0;
   if (mixed) {
-    k_pairs_mixed<POL_MATVEC, FK><<<ub, T, 0, s>>>(P);
-    k_pairs_thread<POL_MATVEC, FK, VAL_MIXED><<<tb, T, 0, s>>>(P);
+    if (units) k_pairs_mixed<POL_MATVEC, FK><<<ub, T, 0, s>>>(P);
+    if (singles) k_pairs_thread<POL_MATVEC, FK, VAL_MIXED><<<tb, T, 0, s>>>(P);
   } else {
     if constexpr (CAN_FIX) {
       if (fix) {
-        k_pairs_fp64<POL_MATVEC, FK, true><<<ub, T, 0, s>>>(P);
-        k_pairs_thread<POL_MATVEC, FK, VAL_FIX><<<tb, T, 0, s>>>(P);
+        if (units) k_pairs_fp64<POL_MATVEC, FK, true><<<ub, T, 0, s>>>(P);
+        if (singles) k_pairs_thread<POL_MATVEC, FK, VAL_FIX><<<tb, T, 0, s>>>(P);
         ABX_CHECK_CUDA(cudaGetLastError());
         return ABX_OK;
       }
     }
     if constexpr (KIND != K_WEND_CUT) {
-      k_pairs_fp64<POL_MATVEC, FK, false><<<ub, T, 0, s>>>(P);
-      k_pairs_thread<POL_MATVEC, FK, VAL_FP64><<<tb, T, 0, s>>>(P);
+      if (units) k_pairs_fp64<POL_MATVEC, FK, false><<<ub, T, 0, s>>>(P);
+      if (singles) k_pairs_thread<POL_MATVEC, FK, VAL_FP64><<<tb, T, 0, s>>>(P);
     }
   }
   ABX_CHECK_CUDA(cudaGetLastError());
@@ -1742,7 +1770,7 @@ template <int POL, int NORM> int launch_search_norm(abx_context *ctx, KParams P)
   const int T = WARPS_PER_CTA * 32;
   P.all_units = POL == POL_LIST ? 1 : 0;
   P.lanes = query_lanes(ctx, P.units_cap);
-  ABX_TRY(reset_counters(ctx, P));
+  if (POL == POL_LIST) P.counter += 2;  // (zeroed by the layout, as the count's are)
   k_pairs_mixed<POL, ABX_K_CONST, NORM><<<grid_blocks(ctx, P), T, 0, s>>>(P);
   if (POL == POL_COUNT)
     k_pairs_thread<POL_COUNT, ABX_K_CONST, VAL_MIXED, NORM><<<thread_blocks(ctx, P), T, 0, s>>>(P);
@@ -1771,18 +1799,6 @@ int launch_matvec_kind(abx_context *ctx, const KParams &P, bool mixed, bool fix)
   }
   set_error("unknown kernel kind %d", P.kind);
   return ABX_ERR_INVALID;
-}
-
-// The unit of an operator's FP64 product on the integer units (fix64.cuh).
-fx::Unit fix_unit(const abx_kernel &k, double r) {
-  switch (k.kind) {
-  case ABX_K_GAUSSIAN:
-  case ABX_K_COMPACT_GAUSSIAN: return fx::make_unit<fx::GAUSSIAN>(k.p[0], r);
-  case ABX_K_WENDLAND_C2: return fx::make_unit<fx::WENDLAND>(k.p[0], r);
-  case ABX_K_LAPLACE: return fx::make_unit<fx::LAPLACE>(k.p[0], r);
-  case ABX_K_MULTIQUADRIC: return fx::make_unit<fx::MULTIQUADRIC>(k.p[0], r);
-  default: return fx::Unit{};
-  }
 }
 
 int fill_fixed(abx_context *ctx, PointLayout &P, const fx::Unit &U) {
@@ -1821,6 +1837,18 @@ int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *
 
 }  // namespace
 
+// The unit of an operator's FP64 product on the integer units (fix64.cuh).
+fx::Unit fix_unit(const abx_kernel &k, double reach) {
+  switch (k.kind) {
+  case ABX_K_GAUSSIAN:
+  case ABX_K_COMPACT_GAUSSIAN: return fx::make_unit<fx::GAUSSIAN>(k.p[0], reach);
+  case ABX_K_WENDLAND_C2: return fx::make_unit<fx::WENDLAND>(k.p[0], reach);
+  case ABX_K_LAPLACE: return fx::make_unit<fx::LAPLACE>(k.p[0], reach);
+  case ABX_K_MULTIQUADRIC: return fx::make_unit<fx::MULTIQUADRIC>(k.p[0], reach);
+  default: return fx::Unit{};
+  }
+}
+
 static int matvec_split(const abx_operator *op) {
   return op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM ? SPLIT_MIXED : SPLIT_FP64;
 }
@@ -1829,6 +1857,10 @@ int pair_layout_build(abx_operator *op) {
   abx_context *ctx = op->rows->ctx;
   if (!op->pairs) op->pairs = new PairLayout();
   PairLayout &L = *op->pairs;  // a rebuild keeps the buffers
+  if (!L.host) {
+    ABX_CHECK_CUDA(cudaHostAlloc((void **)&L.host, sizeof(HostCounts), cudaHostAllocMapped));
+    *L.host = HostCounts{};
+  }
   L.cols_version = ~uint64_t(0);  // valid once everything below has succeeded
   const bool self = op->rows == op->cols;
   ABX_TRY(layout_build(ctx, op->cols, op->radius, self ? nullptr : op->rows->pos.ptr,
@@ -1842,7 +1874,6 @@ int pair_layout_build(abx_operator *op) {
   const int64_t nr = L.rows->n, nc = L.cols.n;
   ABX_TRY(L.bk32.reserve(nc ? nc : 1));
   ABX_TRY(L.bk64.reserve(nc ? nc : 1));
-  ABX_TRY(L.ck.reserve(nr ? nr : 1));
   if (op->k.kind == ABX_K_SCALAR_SUM) {
     ABX_REQUIRE(op->rows->has_scalar && op->cols->has_scalar, ABX_ERR_STATE,
                 "ABX_K_SCALAR_SUM needs a scalar column on both particle sets");
@@ -1850,10 +1881,10 @@ int pair_layout_build(abx_operator *op) {
     ABX_TRY(L.sq.reserve(nr ? nr : 1));
     if (nc)
       k_gather_b<<<ceil_div(nc, TPB), TPB, 0, ctx->stream>>>(op->cols->scalar.ptr, L.cols.perm.ptr,
-                                                             nc, nullptr, L.sk.ptr);
+                                                             nc, nullptr, L.sk.ptr, nullptr);
     if (nr)
       k_gather_b<<<ceil_div(nr, TPB), TPB, 0, ctx->stream>>>(op->rows->scalar.ptr, L.rows->perm.ptr,
-                                                             nr, nullptr, L.sq.ptr);
+                                                             nr, nullptr, L.sq.ptr, nullptr);
     ABX_CHECK_CUDA(cudaGetLastError());
   }
   L.cols_version = op->cols->version;
@@ -1868,11 +1899,12 @@ int sparse_matvec_device(abx_operator *op, const double *b, double *c) {
   PairLayout &L = *op->pairs;
   const int64_t nr = L.rows->n, nc = L.cols.n;
   if (nr == 0) return ABX_OK;
-  if (L.split != matvec_split(op)) ABX_TRY(build_units(ctx, L, matvec_split(op)));
+  if (L.split != matvec_split(op)) ABX_TRY(relist_units(ctx, L, matvec_split(op)));
   const bool mixed = op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM;
   if (nc > 0)
     k_gather_b<<<ceil_div(nc, TPB), TPB, 0, ctx->stream>>>(
-        b, L.cols.perm.ptr, nc, mixed ? L.bk32.ptr : nullptr, mixed ? nullptr : L.bk64.ptr);
+        b, L.cols.perm.ptr, nc, mixed ? L.bk32.ptr : nullptr, mixed ? nullptr : L.bk64.ptr,
+        L.counts.ptr + 4);
   ABX_CHECK_CUDA(cudaGetLastError());
   KParams P = base_params(L);
   P.kind = op->k.kind;
@@ -1884,15 +1916,12 @@ int sparse_matvec_device(abx_operator *op, const double *b, double *c) {
   P.b64 = L.bk64.ptr;
   P.s_col = L.sk.ptr;
   P.s_row = L.sq.ptr;
-  P.c = L.ck.ptr;
+  P.c = c;
   if (nc == 0) {
     ABX_CHECK_CUDA(cudaMemsetAsync(c, 0, nr * sizeof(double), ctx->stream));
     return ABX_OK;
   }
-  ABX_TRY(launch_matvec_kind(ctx, P, mixed, L.unit.ok));
-  k_scatter_c<<<ceil_div(nr, TPB), TPB, 0, ctx->stream>>>(L.ck.ptr, L.rows->perm.ptr, nr, c);
-  ABX_CHECK_CUDA(cudaGetLastError());
-  return ABX_OK;
+  return launch_matvec_kind(ctx, P, mixed, L.unit.ok);
 }
 
 namespace {
@@ -1978,15 +2007,13 @@ __global__ void k_rowptr_to_kernel(const int64_t *__restrict__ rowptr,
   rowptr_k[k] = rowptr[perm[k]];
 }
 
-// Row pointers (input order, W.rowptr, n + 1 entries) from the counts in
-// kernel order, and their total on the host.
-int rowptr_device(abx_context *ctx, SearchSpace &W, const uint32_t *perm, int64_t n, int64_t &nnz) {
+// Row pointers (W.rowptr, n + 1 entries) from the counts W.cnt, and their total
+// on the host.
+int rowptr_device(abx_context *ctx, SearchSpace &W, int64_t n, int64_t &nnz) {
   cudaStream_t s = ctx->stream;
   const unsigned nb = ceil_div(n, RP_TILE);
-  ABX_TRY(W.cnt.reserve(n + 1));
   ABX_TRY(W.rowptr.reserve(n + 1));
   ABX_TRY(W.sums.reserve(nb + 1));
-  k_scatter<int32_t><<<ceil_div(n, TPB), TPB, 0, s>>>(W.cnt_k.ptr, perm, n, W.cnt.ptr);
   k_rp_sums<<<nb, RP_TPB, 0, s>>>(W.cnt.ptr, n, W.sums.ptr);
   k_rp_scan<<<1, RP_TPB, 0, s>>>(W.sums.ptr, nb, W.rowptr.ptr + n);
   k_rp_write<<<nb, RP_TPB, 0, s>>>(W.cnt.ptr, n, W.sums.ptr, W.rowptr.ptr);
@@ -2025,30 +2052,27 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
     }
     return ABX_OK;
   }
-  ABX_TRY(W.cnt_k.reserve(nq + 1));
+  // counts go by row, straight to the caller's device memory where it is that
+  const bool direct = counts_user && !rowptr_user && device_ptr_usable(counts_user, ctx->device) == 1;
+  int32_t *cnt = counts_user;
+  if (!direct) {
+    ABX_TRY(W.cnt.reserve(nq + 1));
+    cnt = W.cnt.ptr;
+  }
   KParams P = base_params(L);
   P.kind = ABX_K_CONST;
   P.lnorm = lnorm;
   P.thr = lnorm == 2 ? r * r : std::fabs(r);
-  P.counts_out = W.cnt_k.ptr;
+  P.counts_out = cnt;
   if (p->n > 0)
     ABX_TRY(launch_search<POL_COUNT>(ctx, P));
   else
-    ABX_CHECK_CUDA(cudaMemsetAsync(W.cnt_k.ptr, 0, nq * 4, s));
-  if (counts_user) {
-    const int where = device_ptr_usable(counts_user, ctx->device);
-    int32_t *out = counts_user;
-    if (where != 1) {
-      ABX_TRY(W.cnt.reserve(nq + 1));
-      out = W.cnt.ptr;
-    }
-    k_scatter<int32_t><<<ceil_div(nq, TPB), TPB, 0, s>>>(W.cnt_k.ptr, L.rows->perm.ptr, nq, out);
-    ABX_CHECK_CUDA(cudaGetLastError());
-    if (where != 1) ABX_CHECK_CUDA(cudaMemcpyAsync(counts_user, out, nq * 4, cudaMemcpyDefault, s));
-  }
+    ABX_CHECK_CUDA(cudaMemsetAsync(cnt, 0, nq * 4, s));
+  if (counts_user && !direct)
+    ABX_CHECK_CUDA(cudaMemcpyAsync(counts_user, cnt, nq * 4, cudaMemcpyDefault, s));
   if (rowptr_user) {
     int64_t nnz = 0;
-    ABX_TRY(rowptr_device(ctx, W, L.rows->perm.ptr, nq, nnz));
+    ABX_TRY(rowptr_device(ctx, W, nq, nnz));
     ABX_CHECK_CUDA(cudaMemcpyAsync(rowptr_user, W.rowptr.ptr, (nq + 1) * 8, cudaMemcpyDefault, s));
     if (cols_user) {
       ABX_REQUIRE(cap >= nnz, ABX_ERR_CAPACITY, "cols capacity %lld < nnz %lld", (long long)cap,
@@ -2094,12 +2118,12 @@ int self_csr_device(abx_particles *p, double r, DevBuf<int64_t> &rowptr, DevBuf<
     ABX_CHECK_CUDA(cudaMemsetAsync(rowptr.ptr, 0, 8, s));
     return cols.reserve(1);
   }
-  ABX_TRY(W.cnt_k.reserve(n + 1));
+  ABX_TRY(W.cnt.reserve(n + 1));
   KParams P = base_params(L);
   P.kind = ABX_K_CONST;
-  P.counts_out = W.cnt_k.ptr;
+  P.counts_out = W.cnt.ptr;
   ABX_TRY(launch_search<POL_COUNT>(ctx, P));
-  ABX_TRY(rowptr_device(ctx, W, L.rows->perm.ptr, n, nnz));
+  ABX_TRY(rowptr_device(ctx, W, n, nnz));
   ABX_CHECK_CUDA(cudaMemcpyAsync(rowptr.ptr, W.rowptr.ptr, (n + 1) * 8, cudaMemcpyDeviceToDevice, s));
   ABX_TRY(cols.reserve(nnz + 1));
   if (nnz > 0) {
@@ -2512,9 +2536,8 @@ extern "C" int abx_radius_query_csr_transform(abx_particles *p, int64_t nq, cons
 // pre-sizes everything at start-up), or a time-stepping loop that must not
 // pay cudaMalloc/cudaFree's implicit device-wide synchronisation.  For them
 // this entry point keeps the per-call scratch of the sparse matvec -- b
-// gathered into the operator's internal order, the result before it is
-// scattered back to storage order, and the work counter of the pair kernel
-// -- in one file-scope device array of fixed size instead of in buffers
+// gathered into the operator's internal order and the work counters of the pair
+// kernels -- in one file-scope device array of fixed size instead of in buffers
 // owned by the operator.  Every GPU that loads the library holds this array
 // until the process exits.
 namespace abx {
@@ -2582,19 +2605,19 @@ extern "C" int abx_operator_matvec_noalloc(abx_operator *op, const double *b, do
   ABX_TRY(noalloc_scratch(ctx->device, &base));
   const size_t bbytes = align256((size_t)nc * (mixed ? sizeof(float) : sizeof(double)));
   void *bk = base;
-  double *ck = (double *)(base + bbytes);
+  // (8 B a row held the result before it was written in place: the limit stays)
   int *counter = (int *)(base + bbytes + align256((size_t)nr * sizeof(double)));
   cudaStream_t s = ctx->stream;
   PairLayout &L = *op->pairs;
   // (precision changed since: the units are listed anew, in the same buffers)
-  if (L.split != matvec_split(op)) ABX_TRY(build_units(ctx, L, matvec_split(op)));
+  if (L.split != matvec_split(op)) ABX_TRY(relist_units(ctx, L, matvec_split(op)));
   if (nc == 0) {
     ABX_CHECK_CUDA(cudaMemsetAsync(c, 0, nr * sizeof(double), s));
     return ABX_OK;
   }
   k_gather_b<<<ceil_div(nc, TPB), TPB, 0, s>>>(b, L.cols.perm.ptr, nc,
                                                mixed ? (float *)bk : nullptr,
-                                               mixed ? nullptr : (double *)bk);
+                                               mixed ? nullptr : (double *)bk, counter);
   ABX_CHECK_CUDA(cudaGetLastError());
   KParams P = base_params(L);
   P.kind = op->k.kind;
@@ -2606,12 +2629,9 @@ extern "C" int abx_operator_matvec_noalloc(abx_operator *op, const double *b, do
   P.b64 = mixed ? nullptr : (const double *)bk;
   P.s_col = L.sk.ptr;
   P.s_row = L.sq.ptr;
-  P.c = ck;
-  P.counter = counter;  // zeroed by the launch helper before every launch
-  ABX_TRY(launch_matvec_kind(ctx, P, mixed, L.unit.ok));
-  k_scatter_c<<<ceil_div(nr, TPB), TPB, 0, s>>>(ck, L.rows->perm.ptr, nr, c);
-  ABX_CHECK_CUDA(cudaGetLastError());
-  return ABX_OK;
+  P.c = c;
+  P.counter = counter;  // zeroed by the gather
+  return launch_matvec_kind(ctx, P, mixed, L.unit.ok);
 }
 
 extern "C" int abx_knn(abx_particles *p, int k, int32_t *idx, double *d2) {

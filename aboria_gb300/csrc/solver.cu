@@ -128,9 +128,11 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
                                                   const int64_t *__restrict__ dom_mat,
                                                   const int *__restrict__ dom_size,
                                                   const int *__restrict__ dom_off,
-                                                  int *__restrict__ piv, int *__restrict__ info) {
+                                                  int *__restrict__ piv, int *__restrict__ info,
+                                                  int above) {
   const int d = blockIdx.x;
   const int n = dom_size[d];
+  if (n <= above) return;  // k_lu_fix's
   double *A = mat + dom_mat[d];
   int *pv = piv + dom_off[d];
   __shared__ double red_v[LU_T / 32];
@@ -238,6 +240,219 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
         __syncthreads();
       }
     }
+  }
+  if (tid == 0) info[d] = status;
+}
+
+// ------------------------------------------- LU with an integer update ---
+// The same factorisation (partial pivoting, panels of PW columns, LAPACK's
+// pivot convention) for blocks of kernel values of one size (Gaussian,
+// Wendland: at most 1, 1 on the diagonal), where the trailing update, n^3 / 3
+// multiply-adds, need not run at 2 FP64 operations a clock and SM: the panel's
+// rows and the block row's columns are scaled by powers of two to 56-bit
+// integers, x = (h 2^28 + l) 2^(e - 56) with signed halves, and a product sum
+// over the panel's 32 columns is two exact 64-bit sums, hi += h h and mid +=
+// h l + l h: three 32x32+64 multiply-adds (58 a clock and SM) for one FP64
+// multiply-add (1.8).  l l is below the scaled values' own 2^-57.  A row of L is
+// scaled by its largest entry in the panel and a column of U likewise, so the
+// error of a product is 2^-56 of the largest product of its row and column, where
+// FP64's partial sums round at 2^-53 of themselves.
+//
+// One CTA a domain.  The panel is factorised in shared memory (rows below the
+// diagonal block x 32 columns), row swaps of the other columns are deferred to
+// its end, the block row is solved a column a thread, and the update takes
+// UTR x UTC tiles, a 4 x 4 piece a thread.  Blocks of more rows than the shared
+// panel holds keep k_lu_fp64.  256 domains of 703 rows on average: @LU_OLD@ ->
+// @LU_NEW@ ms.
+constexpr int FL_T = 512;              // threads
+constexpr int UTR = 64, UTC = 128;     // update tile: rows, columns (4 x 4 a thread)
+constexpr int PLD = PW + 1;            // panel row stride
+constexpr int FL_MAX = 832;            // rows of a block: 832 * 33 * 8 B = 220 KB
+static_assert((UTR / 4) * (UTC / 4) == FL_T, "one 4 x 4 piece a thread");
+struct LuTiles {
+  int2 L[PW][UTR];  // (h, l) of the panel's rows, of the block row's columns
+  int2 U[PW][UTC];
+};
+static_assert(sizeof(LuTiles) <= (size_t)FL_MAX * PLD * 8, "tiles fit the panel's memory");
+
+// x 2^(56 - e) as h 2^28 + l, |l| <= 2^27; |x| <= 2^e, e in scale_exp's range
+__device__ __forceinline__ int2 split56(double x, int e) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)((u >> 52) & 0x7ff);
+  const unsigned long long m = (u & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
+  const int sh = (ex ? ex : 1) - 1075 + 56 - e;  // |x| 2^(56 - e) = m 2^sh, sh <= 4
+  long long f = sh >= 0 ? (long long)(m << sh)
+                        : (sh > -63 ? (long long)(((m >> (-sh - 1)) + 1) >> 1) : 0ll);
+  if (u >> 63) f = -f;
+  const int l = (int)((unsigned)f << 4) >> 4;  // the low 28 bits, signed
+  return make_int2((int)((f - l) >> 28), l);
+}
+// smallest e with |x| <= 2^e from the bits of the largest |x| (0: any)
+__device__ __forceinline__ int scale_exp(unsigned long long maxbits) {
+  const int ex = (int)((maxbits >> 52) & 0x7ff);
+  return ex - 1022;
+}
+
+__global__ void __launch_bounds__(FL_T) k_lu_fix(double *__restrict__ mat,
+                                                 const int64_t *__restrict__ dom_mat,
+                                                 const int *__restrict__ dom_size,
+                                                 const int *__restrict__ dom_off,
+                                                 int *__restrict__ piv, int *__restrict__ info) {
+  extern __shared__ __align__(16) unsigned char lu_raw[];
+  double *Pn = reinterpret_cast<double *>(lu_raw);  // panel: rows k0..n-1 x PW, stride PLD
+  LuTiles &T = *reinterpret_cast<LuTiles *>(lu_raw);
+  __shared__ double red_v[FL_T / 32];
+  __shared__ int red_i[FL_T / 32];
+  __shared__ double L11[PW][PW + 1];
+  __shared__ int swaps[PW];
+  __shared__ short le[FL_MAX], ue[FL_MAX];  // exponents of the panel's rows, the block row's columns
+  const int d = blockIdx.x;
+  const int n = dom_size[d];
+  if (n > FL_MAX) return;  // k_lu_fp64's
+  double *A = mat + dom_mat[d];
+  int *pv = piv + dom_off[d];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int status = 0;
+  for (int k0 = 0; k0 < n; k0 += PW) {
+    const int kw = min(PW, n - k0), k1 = k0 + kw, rows = n - k0;
+    // ---- the panel, in shared memory
+    for (int c = warp; c < kw; c += FL_T / 32)
+      for (int r = lane; r < rows; r += 32) Pn[r * PLD + c] = M(A, n, k0 + r, k0 + c);
+    __syncthreads();
+    for (int c = 0; c < kw; ++c) {
+      // pivot: the first row of largest |entry| at or below the diagonal
+      double best = -1.0;
+      int bi = c;
+      for (int r = c + tid; r < rows; r += FL_T) {
+        const double v = fabs(Pn[r * PLD + c]);
+        if (v > best) { best = v; bi = r; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ov = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+      }
+      if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
+      __syncthreads();
+      best = red_v[0];
+      bi = red_i[0];
+      for (int w = 1; w < FL_T / 32; ++w)
+        if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) { best = red_v[w]; bi = red_i[w]; }
+      if (tid == 0) {
+        swaps[c] = k0 + bi;
+        pv[k0 + c] = k0 + bi;
+        if (best == 0.0 && status == 0) status = k0 + c + 1;
+      }
+      if (bi != c && tid < kw) {
+        const double t = Pn[c * PLD + tid];
+        Pn[c * PLD + tid] = Pn[bi * PLD + tid];
+        Pn[bi * PLD + tid] = t;
+      }
+      __syncthreads();
+      const double dpiv = Pn[c * PLD + c];
+      const double inv = dpiv != 0.0 ? 1.0 / dpiv : 0.0;
+      for (int r = c + 1 + tid; r < rows; r += FL_T) {
+        const double l = Pn[r * PLD + c] * inv;
+        Pn[r * PLD + c] = l;
+        for (int cc = c + 1; cc < kw; ++cc)
+          Pn[r * PLD + cc] = fma(-l, Pn[c * PLD + cc], Pn[r * PLD + cc]);
+      }
+      __syncthreads();
+    }
+    for (int e = tid; e < kw * kw; e += FL_T) L11[e / kw][e % kw] = Pn[(e / kw) * PLD + e % kw];
+    // scale of every row below the diagonal block; the panel back to the matrix
+    for (int r = kw + tid; r < rows; r += FL_T) {
+      unsigned long long mx = 0;
+      for (int c = 0; c < kw; ++c)
+        mx = max(mx, (unsigned long long)__double_as_longlong(Pn[r * PLD + c]) & 0x7fffffffffffffffull);
+      le[r] = (short)scale_exp(mx);
+    }
+    for (int c = warp; c < kw; c += FL_T / 32)
+      for (int r = lane; r < rows; r += 32) M(A, n, k0 + r, k0 + c) = Pn[r * PLD + c];
+    __syncthreads();
+    // ---- the other columns: row swaps; right of the panel U12 = L11^{-1} A12
+    for (int j = tid; j < n; j += FL_T) {
+      if (j >= k0 && j < k1) continue;
+      double *col = A + (int64_t)j * n;
+      for (int c = 0; c < kw; ++c) {
+        const int p = swaps[c];
+        if (p != k0 + c) {
+          const double t = col[k0 + c];
+          col[k0 + c] = col[p];
+          col[p] = t;
+        }
+      }
+      if (j < k1) continue;
+      // (a panel with columns to its right has all its PW columns)
+      double x[PW];
+#pragma unroll
+      for (int c = 0; c < PW; ++c) x[c] = col[k0 + c];
+      unsigned long long mx = 0;
+#pragma unroll
+      for (int c = 0; c < PW; ++c) {
+        mx = max(mx, (unsigned long long)__double_as_longlong(x[c]) & 0x7fffffffffffffffull);
+#pragma unroll
+        for (int q = c + 1; q < PW; ++q) x[q] = fma(-L11[q][c], x[c], x[q]);
+        col[k0 + c] = x[c];
+      }
+      ue[j] = (short)scale_exp(mx);
+    }
+    __syncthreads();
+    if (k1 >= n) break;
+    // ---- A22 -= L21 U12
+    for (int ti = k1; ti < n; ti += UTR) {
+      __syncthreads();
+      for (int e = tid; e < PW * UTR; e += FL_T) {
+        const int r = e % UTR, c = e / UTR;
+        T.L[c][r] = ti + r < n ? split56(M(A, n, ti + r, k0 + c), le[ti + r - k0])
+                                         : make_int2(0, 0);
+      }
+      for (int tj = k1; tj < n; tj += UTC) {
+        __syncthreads();
+        for (int e = tid; e < PW * UTC; e += FL_T) {
+          const int c = e % PW, j = e / PW;
+          T.U[c][j] = tj + j < n ? split56(M(A, n, k0 + c, tj + j), ue[tj + j])
+                                           : make_int2(0, 0);
+        }
+        __syncthreads();
+        const int tr = (tid % (UTR / 4)) * 4, tc = (tid / (UTR / 4)) * 4;
+        if (ti + tr >= n || tj + tc >= n) continue;
+        long long hi[4][4] = {}, mid[4][4] = {};
+#pragma unroll 2
+        for (int c = 0; c < PW; ++c) {
+          int2 a[4], b[4];
+          *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&T.L[c][tr]);
+          *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&T.L[c][tr + 2]);
+          *reinterpret_cast<int4 *>(&b[0]) = *reinterpret_cast<const int4 *>(&T.U[c][tc]);
+          *reinterpret_cast<int4 *>(&b[2]) = *reinterpret_cast<const int4 *>(&T.U[c][tc + 2]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              hi[i][j] += (long long)a[i].x * b[j].x;
+              mid[i][j] += (long long)a[i].x * b[j].y;
+              mid[i][j] += (long long)a[i].y * b[j].x;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int cj = tj + tc + j;
+          if (cj >= n) continue;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int ri = ti + tr + i;
+            if (ri >= n) continue;
+            // (hi 2^56 + mid 2^28) 2^(le - 56) 2^(ue - 56)
+            const long long t = hi[i][j] + ((mid[i][j] + (1ll << 27)) >> 28);
+            const int ex = max(le[ri - k0] + ue[cj] - 56 + 1023, 1);
+            const double sc = __longlong_as_double((long long)ex << 52);
+            M(A, n, ri, cj) = fma(-(double)t, sc, M(A, n, ri, cj));
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
   if (tid == 0) info[d] = status;
 }
@@ -506,8 +721,24 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
     cudaMemcpyAsync(S->dom_mat.ptr, moff.data(), moff.size() * 8, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(S->idx.ptr, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, s);
     if ((st = launch_assemble(ctx, *S, p, op->k, op->radius, size))) return fail(st);
-    k_lu_fp64<<<S->ndom, LU_T, 0, s>>>(S->mat.ptr, S->dom_mat.ptr, S->dom_size.ptr,
-                                        S->dom_off.ptr, S->piv.ptr, S->info.ptr);
+    // blocks of kernel values of one size: integer update (k_lu_fix); kernels
+    // whose values span many magnitudes, and blocks beyond its panel: FP64
+    const bool flat = op->k.kind == ABX_K_GAUSSIAN || op->k.kind == ABX_K_COMPACT_GAUSSIAN ||
+                      op->k.kind == ABX_K_WENDLAND_C2;
+    if (flat) {
+      const size_t smem = std::max(sizeof(LuTiles), (size_t)std::min(S->max_size, FL_MAX) * PLD * 8);
+      if (cudaFuncSetAttribute(k_lu_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess) {
+        set_error("LU: %zu bytes of shared memory refused", smem);
+        return fail(ABX_ERR_CUDA);
+      }
+      k_lu_fix<<<S->ndom, FL_T, smem, s>>>(S->mat.ptr, S->dom_mat.ptr, S->dom_size.ptr,
+                                           S->dom_off.ptr, S->piv.ptr, S->info.ptr);
+    }
+    if (!flat || S->max_size > FL_MAX)
+      k_lu_fp64<<<S->ndom, LU_T, 0, s>>>(S->mat.ptr, S->dom_mat.ptr, S->dom_size.ptr,
+                                          S->dom_off.ptr, S->piv.ptr, S->info.ptr,
+                                          flat ? FL_MAX : 0);
     if (cudaGetLastError() != cudaSuccess) {
       set_error("LU launch failed");
       return fail(ABX_ERR_CUDA);

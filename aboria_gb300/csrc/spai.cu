@@ -5,6 +5,7 @@
 #include <chrono>
 
 #include "common.cuh"
+#include "fix64.cuh"
 #include "handles.cuh"
 
 namespace abx {
@@ -120,6 +121,9 @@ struct LsParams {
   int local;           // 1: U = S (row of the local block inverse)
   const int32_t *subset;  // rows to solve (null: all n rows)
   int64_t nrows;          // rows to solve
+  fx::Unit unit;          // local mode on the integer units, where unit.ok
+  fx::Consts fixc;
+  long long Lfix[3];
 };
 
 template <int KIND> __device__ __forceinline__ double ls_coeff(const LsParams &P, int a, int b) {
@@ -325,6 +329,90 @@ template <int KIND> __global__ void __launch_bounds__(LS_T) k_spai_ls(LsParams P
   }
 }
 
+// 1 / sqrt(x) and 1 / x in FP64 from the FP32 units' seed (22 bits) and two
+// Newton steps: 8 and 4 FP64 operations; x within FP32's range.
+__device__ __forceinline__ double rsqrt64(double x) {
+  double y = (double)fx::rsqrt32((float)x);
+  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
+  return fma(0.5 * y, fma(-x * y, y, 1.0), y);
+}
+__device__ __forceinline__ double rcp64(double x) {
+  double y = (double)fx::rcp32((float)x);
+  y = fma(fma(-x, y, 1.0), y, y);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+
+// Entry (s_lane, s_u) of a support's matrix for every u, in col: FP64
+// coefficients, or (FIX) the same values from the integer units (fix64.cuh).
+// Which entries lie inside the radius is the reference's strict FP64 test: FP32
+// offsets from the row's own point decide it except within `band` of r^2.
+template <int KIND, bool FIX>
+__device__ __forceinline__ void local_matrix(const LsParams &P, int64_t i, int s, int lane,
+                                             const fx::u64 *tab, float4 *rel, longlong2 *fxy,
+                                             long long *fz, double *col) {
+  bool wide = false;  // a support that reaches across a quarter of a periodic box
+  float far2 = 0.f;
+  if (FIX) {
+    float f[3] = {0.f, 0.f, 0.f};
+    long long X[3] = {0, 0, 0};
+    if (s >= 0)
+      for (int d = 0; d < P.dim; ++d) {
+        const double x = P.pos[(int64_t)d * P.n + s];
+        double dx = __dsub_rn(x, P.pos[(int64_t)d * P.n + i]);
+        X[d] = fx::to_fixed(x, P.unit.f, P.unit.k);
+        if (P.periodic[d]) {
+          const double w = P.L[d];
+          if (dx > w / 2) {
+            dx -= w;
+            X[d] = fx::diff(X[d], P.Lfix[d]);
+          } else if (dx <= -w / 2) {
+            dx += w;
+            X[d] = fx::diff(X[d], -P.Lfix[d]);
+          }
+          wide |= fabs(dx) > 0.25 * w;
+        }
+        f[d] = (float)dx;
+      }
+    far2 = f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
+    wide = __any_sync(0xffffffffu, wide || !(far2 < 1e30f));
+    far2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(far2)));
+    __syncwarp();
+    rel[lane] = make_float4(f[0], f[1], f[2], __int_as_float(s));
+    fxy[lane] = make_longlong2(X[0], X[1]);
+    fz[lane] = X[2];
+    __syncwarp();
+  }
+  if (FIX && !wide) {
+    const float r = sqrtf((float)P.r2);
+    const float band = 2e-6f * r * (sqrtf(far2) + r), lo = (float)P.r2 - band, hi = (float)P.r2 + band;
+    const float4 me = rel[lane];
+    const longlong2 mxy = fxy[lane];
+    const long long qx = fx::biased(mxy.x), qy = fx::biased(mxy.y), qz = fx::biased(fz[lane]);
+#pragma unroll
+    for (int u = 0; u < LS_K; ++u) {
+      const float4 o = rel[u];
+      const int su = __float_as_int(o.w);
+      const float dx = o.x - me.x, dy = o.y - me.y, dz = o.z - me.z;
+      const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      double v = 0.0;
+      if (s >= 0 && su >= 0 && d2 <= hi) {
+        const longlong2 oxy = fxy[u];
+        bool near;
+        v = fx::value<KIND>(fx::diff(oxy.x, qx), fx::diff(oxy.y, qy), fx::diff(fz[u], qz), P.dim,
+                            P.fixc, tab, near);
+        if (near || d2 >= lo) v = ls_coeff<KIND>(P, s, su);
+      }
+      col[u] = v;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < LS_K; ++u) {
+      const int su = __shfl_sync(0xffffffffu, s, u);
+      col[u] = (s >= 0 && su >= 0) ? ls_coeff<KIND>(P, s, su) : 0.0;
+    }
+  }
+}
+
 // Local mode (U = S, the k x k system of the row's support) with one warp
 // per row: lane c holds column c of B, B(u, c) = coeff(S[c], S[u]), in
 // registers, and lane u the rhs entry e_u.  The same Householder QR with
@@ -332,9 +420,25 @@ template <int KIND> __global__ void __launch_bounds__(LS_T) k_spai_ls(LsParams P
 // the remaining rows; stop at a norm <= 1e-13 |R00|), then the back
 // substitution over the rank; the Householder vector passes through a
 // per-warp shared-memory row.
-template <int KIND> __global__ void __launch_bounds__(LS_LOCAL_T) k_spai_local(LsParams P) {
+//
+// FP64 operations bound it (about 2 lanes a clock and SM, whatever the lanes
+// do), so they are spent on the two loops over the columns (d and the update):
+// the matrix comes from the integer units; column norms are downdated, and
+// computed anew when little of one is left (as LAPACK's xLAQP2 does); the norm
+// of x and its product with e share one reduction; square root and reciprocals
+// are Newton steps; the back substitution works by columns.  45,000 rows (2-D
+// RBF system of 200,000 points): 19.2 -> @SP_NEW@ ms.
+template <int KIND, bool FIX> __global__ void __launch_bounds__(LS_LOCAL_T) k_spai_local(LsParams P) {
   constexpr int WPB = LS_LOCAL_T / 32;
   __shared__ double vsh[WPB][LS_K];
+  __shared__ float4 rel_all[FIX ? WPB : 1][LS_K];
+  __shared__ longlong2 fxy_all[FIX ? WPB : 1][LS_K];
+  __shared__ long long fz_all[FIX ? WPB : 1][LS_K];
+  __shared__ fx::u64 tab[FIX && KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
+  if (FIX && KIND == ABX_K_GAUSSIAN) {
+    for (int t = threadIdx.x; t < fx::EXP_TAB; t += LS_LOCAL_T) tab[t] = fx::exp_table.v[t];
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int k = P.k;
   double *v = vsh[wib];
@@ -342,62 +446,70 @@ template <int KIND> __global__ void __launch_bounds__(LS_LOCAL_T) k_spai_local(L
     const int64_t i = P.subset ? P.subset[r] : r;
     const int s = lane < k ? P.knn[i * k + lane] : -1;
     double col[LS_K];
-#pragma unroll
-    for (int u = 0; u < LS_K; ++u) {
-      const int su = __shfl_sync(0xffffffffu, s, u);
-      col[u] = (s >= 0 && su >= 0) ? ls_coeff<KIND>(P, s, su) : 0.0;
-    }
+    local_matrix<KIND, FIX>(P, i, s, lane, tab, rel_all[FIX ? wib : 0], fxy_all[FIX ? wib : 0],
+                            fz_all[FIX ? wib : 0], col);
     double eu = (s >= 0 && s == i) ? 1.0 : 0.0;
     int perm = lane;
     int rank = k;
     double r00 = 0.0;
+    double cn = 0.0, cref = 0.0;  // squared norm over rows j..k-1, and when it was computed
+    bool anew = true;
     for (int j = 0; j < k; ++j) {
-      // norms of the remaining columns over rows j..k-1
-      double cn = 0.0;
+      if (__any_sync(0xffffffffu, anew)) {
+        cn = 0.0;
 #pragma unroll
-      for (int u = 0; u < LS_K; ++u)
-        if (u >= j) cn = fma(col[u], col[u], cn);
-      double bv = (lane >= j && lane < k) ? cn : -1.0;
-      int bl = lane;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int ol = __shfl_xor_sync(0xffffffffu, bl, o);
-        if (ov > bv || (ov == bv && ol < bl)) {
-          bv = ov;
-          bl = ol;
-        }
+        for (int u = 0; u < LS_K; ++u)
+          if (u >= j) cn = fma(col[u], col[u], cn);
+        cref = cn;
+        anew = false;
       }
-      const int p = bl;
+      // the first lane of the largest norm, on the bits (norms are >= 0)
+      const bool in = lane >= j && lane < k;
+      const unsigned long long bits = in ? (unsigned long long)__double_as_longlong(cn) : 0ull;
+      const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(bits >> 32));
+      const bool top = in && (unsigned)(bits >> 32) == hi;
+      const unsigned lo = __reduce_max_sync(0xffffffffu, top ? (unsigned)bits : 0u);
+      const int p = __ffs(__ballot_sync(0xffffffffu, top && (unsigned)bits == lo)) - 1;
       if (p != j) {  // swap columns j and p (and their permutation entries)
         const int src = lane == j ? p : (lane == p ? j : lane);
 #pragma unroll
         for (int u = 0; u < LS_K; ++u) col[u] = __shfl_sync(0xffffffffu, col[u], src);
         perm = __shfl_sync(0xffffffffu, perm, src);
+        cn = __shfl_sync(0xffffffffu, cn, src);
+        cref = __shfl_sync(0xffffffffu, cref, src);
       }
-      const double nrm = sqrt(bv);
-      if (j == 0) r00 = nrm;
-      if (nrm <= 1e-13 * r00 || nrm == 0.0) {
-        rank = j;
-        break;
-      }
-      // Householder vector of column j (rows j..k-1): v = x - alpha e_j
+      // column j (rows j..k-1) = x: |x|^2 and x.e in one reduction, the lower
+      // half of the lanes adding up the one, the upper half the other
       if (lane == j) {
 #pragma unroll
         for (int u = 0; u < LS_K; ++u) v[u] = u >= j ? col[u] : 0.0;
       }
       __syncwarp();
-      const double x0 = v[j];
+      const double xl = v[lane], x0 = v[j];
+      double q = xl * xl, xe = xl * eu;
+      const double give = lane < 16 ? xe : q;
+      double part = (lane < 16 ? q : xe) + __shfl_xor_sync(0xffffffffu, give, 16);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      q = __shfl_sync(0xffffffffu, part, 0);
+      xe = __shfl_sync(0xffffffffu, part, 16);
+      const bool plain = !(q > 1e-30 && q < 1e30);  // outside the FP32 seeds' range
+      const double rs = plain ? 0.0 : rsqrt64(q);
+      const double nrm = plain ? sqrt(q) : fma(0.5 * rs, fma(-(q * rs), q * rs, q), q * rs);
+      if (j == 0) r00 = nrm;
+      if (nrm <= 1e-13 * r00 || nrm == 0.0) {
+        rank = j;
+        break;
+      }
+      // Householder vector v = x - alpha e_j; 2 / |v|^2 = 1 / (|x| (|x| + |x0|))
       const double alpha = x0 > 0 ? -nrm : nrm;
+      const double den = nrm * (nrm + fabs(x0));
+      const double tau = plain ? 1.0 / den : rcp64(den);
       __syncwarp();
       if (lane == 0) v[j] = x0 - alpha;
       __syncwarp();
-      double vv = 0.0;
-#pragma unroll
-      for (int u = 0; u < LS_K; ++u)
-        if (u >= j) vv = fma(v[u], v[u], vv);
-      const double tau = vv > 0 ? 2.0 / vv : 0.0;
       // apply to the columns j+1..k-1 and to e
+      double rj = 0.0;  // the row of R this step leaves behind
       if (lane > j && lane < k) {
         double d = 0.0;
 #pragma unroll
@@ -406,11 +518,15 @@ template <int KIND> __global__ void __launch_bounds__(LS_LOCAL_T) k_spai_local(L
         const double f = tau * d;
 #pragma unroll
         for (int u = 0; u < LS_K; ++u)
-          if (u >= j) col[u] = fma(-f, v[u], col[u]);
+          if (u >= j) {
+            col[u] = fma(-f, v[u], col[u]);
+            if (u == j) rj = col[u];
+          }
+        cn = fmax(fma(-rj, rj, cn), 0.0);
+        anew = cn <= 1e-6 * cref;
       }
-      double se = lane >= j ? v[lane] * eu : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+      const double ej = __shfl_sync(0xffffffffu, eu, j);
+      const double se = fma(-alpha, ej, xe);
       if (lane >= j) eu = fma(-tau * se, v[lane], eu);
       if (lane == j) {
 #pragma unroll
@@ -420,20 +536,28 @@ template <int KIND> __global__ void __launch_bounds__(LS_LOCAL_T) k_spai_local(L
       __syncwarp();
     }
     // back substitution R w = (Q^T e) over the first `rank` columns: lane c
-    // holds R(0..c, c) in col[0..c], lane j holds (Q^T e)_j in eu
+    // holds R(0..c, c) in col[0..c], lane j holds (Q^T e)_j in eu; column j is
+    // taken out of the entries above it once w_j is known
+    double diag = 1.0;
+#pragma unroll
+    for (int u = 0; u < LS_K; ++u)
+      if (u == lane && lane < rank) diag = col[u];
+    const double inv = 1.0 / diag;
     double w = 0.0;
     for (int j = rank - 1; j >= 0; --j) {
-      double rjc = 0.0;
+      if (lane == j) {
+        w = eu * inv;
 #pragma unroll
-      for (int u = 0; u < LS_K; ++u)
-        if (u == j) rjc = col[u];
-      double t = (lane > j && lane < rank) ? rjc * w : 0.0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      const double ej = __shfl_sync(0xffffffffu, eu, j);
-      if (lane == j) w = (ej - t) / rjc;
+        for (int u = 0; u < LS_K; ++u)
+          if (u < j) v[u] = col[u];
+      }
+      __syncwarp();
+      const double wj = __shfl_sync(0xffffffffu, w, j);
+      if (lane < j) eu = fma(-wj, v[lane], eu);
+      __syncwarp();
     }
     if (lane < k) P.vals[i * k + perm] = lane < rank ? w : 0.0;
+    __syncwarp();
   }
 }
 
@@ -538,13 +662,30 @@ int spai_exact_rows(abx_operator *op, int k, int32_t *cols_out, double *vals_out
     return ABX_OK;
   };
   if (local) {
+    P.unit = fix_unit(op->k, op->radius);
+    P.fixc = fx::consts(P.unit, 1.0 / P.p0);
+    if (P.unit.ok)
+      for (int d = 0; d < 3; ++d) P.Lfix[d] = fx::to_fixed(P.L[d], P.unit.f, P.unit.k);
+    const bool fix = P.unit.ok;
     switch (P.kind) {
-    case ABX_K_CONST: ABX_TRY(launch_local(k_spai_local<ABX_K_CONST>)); break;
-    case ABX_K_GAUSSIAN: ABX_TRY(launch_local(k_spai_local<ABX_K_GAUSSIAN>)); break;
-    case ABX_K_WENDLAND_C2: ABX_TRY(launch_local(k_spai_local<ABX_K_WENDLAND_C2>)); break;
-    case ABX_K_COMPACT_GAUSSIAN: ABX_TRY(launch_local(k_spai_local<ABX_K_COMPACT_GAUSSIAN>)); break;
-    case ABX_K_LAPLACE: ABX_TRY(launch_local(k_spai_local<ABX_K_LAPLACE>)); break;
-    case ABX_K_MULTIQUADRIC: ABX_TRY(launch_local(k_spai_local<ABX_K_MULTIQUADRIC>)); break;
+    case ABX_K_CONST: ABX_TRY(launch_local(k_spai_local<ABX_K_CONST, false>)); break;
+    case ABX_K_GAUSSIAN:
+    case ABX_K_COMPACT_GAUSSIAN:
+      ABX_TRY(fix ? launch_local(k_spai_local<ABX_K_GAUSSIAN, true>)
+                  : launch_local(k_spai_local<ABX_K_GAUSSIAN, false>));
+      break;
+    case ABX_K_WENDLAND_C2:
+      ABX_TRY(fix ? launch_local(k_spai_local<ABX_K_WENDLAND_C2, true>)
+                  : launch_local(k_spai_local<ABX_K_WENDLAND_C2, false>));
+      break;
+    case ABX_K_LAPLACE:
+      ABX_TRY(fix ? launch_local(k_spai_local<ABX_K_LAPLACE, true>)
+                  : launch_local(k_spai_local<ABX_K_LAPLACE, false>));
+      break;
+    case ABX_K_MULTIQUADRIC:
+      ABX_TRY(fix ? launch_local(k_spai_local<ABX_K_MULTIQUADRIC, true>)
+                  : launch_local(k_spai_local<ABX_K_MULTIQUADRIC, false>));
+      break;
     }
   } else {
     switch (P.kind) {
