@@ -67,6 +67,28 @@ struct PointLayout {
   DevBuf<uint32_t> tmp;   // sort scratch
 };
 
+// Which units' queries k_pairs_thread walks instead of a unit kernel: units of
+// fewer than `queries` queries whose own row of the stencil holds at most `row`
+// columns (a unit of few queries beside a dense cluster still has a long
+// candidate list, which a warp stages faster than a lane walks it), and none
+// at all where they are less than 1 / `fold` of the set (the second launch).
+struct Split {
+  int queries, row, fold;
+  bool operator==(const Split &o) const {
+    return queries == o.queries && row == o.row && fold == o.fold;
+  }
+};
+// FP64: a unit kernel's lanes idle at ~100 instructions a pair.  N = 100,000 x 50
+// with units below 4, 7, 12 queries split: 423, 315, 246 us.  Counts: 698, 669,
+// 658 us, but 25.2, 25.4, 25.6 ms for the clustered 4M set.  Mixed products: the
+// pair itself is ~10 instructions, so that a unit pays at four queries already
+// (4M: 20.6, 20.9, 21.5 ms for the same three); sets of fewer than MIXED_MIN
+// rows keep to it altogether (2,000: 13 against 21 us; 12,000: 24 against 31;
+// 100,000 x 10: 118 against 78).
+constexpr Split SPLIT_FP64{12, 1 << 30, 16}, SPLIT_COUNT{7, 12, 4}, SPLIT_MIXED{4, 6, 3},
+    SPLIT_NONE{0, 0, 1};
+constexpr int64_t MIXED_MIN = 50000;
+
 // Written by k_tables into pinned host memory: seq last.
 struct HostCounts {
   int full, singles;
@@ -83,11 +105,11 @@ struct PairLayout {
   PointLayout *rows = nullptr;
   DevBuf<uint32_t> cell_start;  // fg.ncells + 1
   // Query units (first query in kernel order, count <= 32): full ones from the
-  // front of the array, those of fewer than `split` queries from its back, and
-  // the latter's queries once more as a list (k_units).
+  // front of the array, small ones (Split) from its back, and the latter's
+  // queries once more as a list (k_units).
   DevBuf<int2> units;
   DevBuf<int> singles;
-  int split = 0;
+  Split split = SPLIT_NONE;
   // full units, small units, their queries, stencil rows; work counters of a
   // count or product (4, 5) and of a list search (6, 7); small units and single
   // queries that a count or product works (8, 9)
@@ -129,13 +151,6 @@ namespace {
 constexpr int TPB = 256;
 constexpr int WARPS_PER_CTA = 4;
 constexpr int GROUP_E2 = 4;  // a unit spans at most this many fine cells along e2
-// Units of fewer queries are walked one query a thread.  Measured (N = 100,000
-// with 50 neighbours / the clustered 4M set): FP64 4: 423, 7: 315, 12: 246 us /
-// no difference; counts 4: 698, 7: 669, 12: 658 us / 25.2, 25.4, 25.6 ms; mixed
-// at 4M 4: 20.6, 7: 20.9, 12: 21.5 ms (its unit kernel spends little on a
-// query, so fewer make a unit worth while).
-constexpr int SPLIT_FP64 = 12, SPLIT_COUNT = 7, SPLIT_MIXED = 4;
-
 constexpr int COUNTS = 16;
 
 enum { POL_COUNT = 0, POL_LIST = 1, POL_MATVEC = 2 };
@@ -348,21 +363,20 @@ int build_cell_start(abx_context *ctx, PairLayout &L) {
 // cells share (e0, e1) and span fewer than GROUP_E2 cells along e2.  One warp
 // per (e0, e1) column walks its queries 32 at a time with the next 32 already
 // loaded; the unit that starts at query s is the run of lanes that continue
-// it.  A unit of at least `split` queries goes to the front of `units`; a smaller
-// one (low density, where a warp of 32 lanes would hold few queries) to the
-// back, and its queries to `singles`, which the one-query-a-thread kernels
-// walk.  Built on the host before, from a 16 B/point copy of the cells: 14 of
+// it.  A unit goes to the front of `units`, or, where `split` says so (low
+// density, where a warp of 32 lanes would hold few queries), to the back, and
+// its queries to `singles`, which k_pairs_thread walks.  Built on the host before, from a 16 B/point copy of the cells: 14 of
 // the 39 ms of a search at N = 4M.
 constexpr int UNIT_WARPS = 4;
 __global__ void __launch_bounds__(UNIT_WARPS * 32)
     k_units(const int4 *__restrict__ cell, const uint32_t *__restrict__ keys,
-            const uint32_t *__restrict__ cell_start, int64_t n, uint32_t ncol, int m2, int64_t cap,
-            int split, int2 *__restrict__ units, int *__restrict__ singles, int *__restrict__ counts) {
+            const uint32_t *__restrict__ cell_start, bool self, int64_t n, uint32_t ncol, int m2,
+            int K2, int64_t cap, Split split, int2 *__restrict__ units, int *__restrict__ singles, int *__restrict__ counts) {
   const int lane = threadIdx.x & 31;
   const uint32_t warps = gridDim.x * UNIT_WARPS;
   for (uint32_t col = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); col < ncol; col += warps) {
     int64_t s, end;
-    if (cell_start) {
+    if (self) {
       s = cell_start[(uint64_t)col * m2];
       end = cell_start[(uint64_t)(col + 1) * m2];
     } else {
@@ -374,6 +388,7 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
     int4 A = base + lane < end ? cell[base + lane] : none;
     int4 B = base + 32 + lane < end ? cell[base + 32 + lane] : none;
     int2 mine = make_int2(0, 0);  // lane i keeps the i-th unit not written out yet
+    int z_mine = 0;               // and its first cell along e2
     int held = 0;
     while (s < end || held > 0) {
       if (s < end) {
@@ -393,12 +408,22 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
         const bool go = s + lane < end && x == x0 && y == y0 && z >= z0 && z - z0 < GROUP_E2;
         const unsigned stop = ~__ballot_sync(0xffffffffu, go);
         const int count = stop ? __ffs(stop) - 1 : 32;
-        if (lane == held) mine = make_int2((int)s, count);
+        if (lane == held) {
+          mine = make_int2((int)s, count);
+          z_mine = z0;
+        }
         ++held;
         s += count;
       }
       if (held == 32 || s >= end) {
-        const bool full = lane < held && mine.y >= split, small = lane < held && mine.y < split;
+        bool small = lane < held && mine.y < split.queries;
+        if (small) {
+          const int z = min(max(z_mine, 0), m2 - 1);
+          const int za = max(z - K2, 0), zb = min(z + GROUP_E2 - 1 + K2, m2 - 1);
+          const uint32_t *row = cell_start + (uint64_t)col * m2;
+          small = row[zb + 1] - row[za] <= (uint32_t)split.row;
+        }
+        const bool full = lane < held && !small;
         const unsigned mf = __ballot_sync(0xffffffffu, full), ms = __ballot_sync(0xffffffffu, small);
         const unsigned lt = (1u << lane) - 1u;
         int tot = small ? mine.y : 0, incl = tot;
@@ -430,7 +455,7 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
   }
 }
 
-int build_units(abx_context *ctx, PairLayout &L, int split) {
+int build_units(abx_context *ctx, PairLayout &L, const Split &split) {
   PointLayout &Q = *L.rows;
   L.split = split;
   const int64_t n = Q.n;
@@ -443,8 +468,8 @@ int build_units(abx_context *ctx, PairLayout &L, int split) {
   const uint32_t ncol = (uint32_t)L.fg.m[0] * L.fg.m[1];
   const unsigned blocks = std::min(ceil_div(ncol, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
   k_units<<<blocks, UNIT_WARPS * 32, 0, ctx->stream>>>(
-      Q.cell.ptr, Q.keys.ptr, L.self ? L.cell_start.ptr : nullptr, n, ncol, L.fg.m[2], n,
-      split, L.units.ptr, L.singles.ptr, L.counts.ptr);
+      Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, ncol, L.fg.m[2], L.fg.K[2], n, split,
+      L.units.ptr, L.singles.ptr, L.counts.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
@@ -875,7 +900,6 @@ __device__ __forceinline__ TileBand tile_band(int span, const FineGrid &fg, doub
 // small units are worked by the unit kernel after all and tells the host which
 // of the two kernels have work.
 constexpr int TABLE_TPB = 256;
-constexpr int FOLD = 16;        // fewer than 1 / FOLD of the queries: no second kernel
 constexpr int ROWS_MAX = 1024;  // (2 K0 + 1)(2 K1 + 1), K <= 7 (make_fine_grid)
 __device__ __forceinline__ int row_reach(int a, int b, const FineGrid &fg, double prune2, int norm) {
   if (norm == -1) return fg.K[2];  // the chebyshev ball is the whole stencil box
@@ -888,7 +912,7 @@ __global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2
                                                       double thr, int norm, int *__restrict__ ext,
                                                       float4 *__restrict__ bands,
                                                       int4 *__restrict__ rows,
-                                                      int *__restrict__ counts, int nq,
+                                                      int *__restrict__ counts, int nq, int fold_at,
                                                       HostCounts *host, int seq) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x == 0) {
@@ -914,7 +938,7 @@ __global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2
     if (threadIdx.x == 0) {
       counts[3] = min(done, ROWS_MAX);
       // a second kernel is not worth its launch for few queries
-      const bool fold = (int64_t)counts[2] * FOLD < nq;
+      const bool fold = (int64_t)counts[2] * fold_at < nq;
       counts[8] = fold ? counts[1] : 0;
       counts[9] = fold ? 0 : counts[2];
       if (host) {
@@ -1668,13 +1692,13 @@ int build_tables(abx_context *ctx, PairLayout &L, int norm, double thr) {
   ABX_TRY(L.stencil.reserve(ROWS_MAX));
   k_tables<<<EXT_TAB * EXT_TAB / TABLE_TPB, TABLE_TPB, 0, ctx->stream>>>(
       L.fg, prune_distance2(L), L.r, thr, norm, L.ext.ptr, L.bands.ptr, L.stencil.ptr,
-      L.counts.ptr, (int)L.rows->n, L.host, ++L.host_seq);
+      L.counts.ptr, (int)L.rows->n, L.split.fold, L.host, ++L.host_seq);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
 
 // The units anew for another split, in the same buffers.
-int relist_units(abx_context *ctx, PairLayout &L, int split) {
+int relist_units(abx_context *ctx, PairLayout &L, const Split &split) {
   ABX_TRY(build_units(ctx, L, split));
   return build_tables(ctx, L, 2, L.r * L.r);
 }
@@ -1815,7 +1839,7 @@ int fill_fixed(abx_context *ctx, PointLayout &P, const fx::Unit &U) {
 // SoA FP64 (qsrc, nq, stride) -- or the column set itself when qsrc == null.
 // All on the context's stream, nothing waited for; norm and thr as KParams'.
 int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *qsrc, int64_t nq,
-                 int64_t qstride, PairLayout &L, int split, int norm = 2) {
+                 int64_t qstride, PairLayout &L, const Split &split, int norm = 2) {
   GridDesc g;
   ABX_TRY(particles_grid_desc(cols, &g));
   L.r = r;
@@ -1849,8 +1873,10 @@ fx::Unit fix_unit(const abx_kernel &k, double reach) {
   }
 }
 
-static int matvec_split(const abx_operator *op) {
-  return op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM ? SPLIT_MIXED : SPLIT_FP64;
+static Split matvec_split(const abx_operator *op) {
+  if (op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM)
+    return op->rows->n < MIXED_MIN ? SPLIT_NONE : SPLIT_MIXED;
+  return SPLIT_FP64;
 }
 
 int pair_layout_build(abx_operator *op) {
@@ -1899,7 +1925,7 @@ int sparse_matvec_device(abx_operator *op, const double *b, double *c) {
   PairLayout &L = *op->pairs;
   const int64_t nr = L.rows->n, nc = L.cols.n;
   if (nr == 0) return ABX_OK;
-  if (L.split != matvec_split(op)) ABX_TRY(relist_units(ctx, L, matvec_split(op)));
+  if (!(L.split == matvec_split(op))) ABX_TRY(relist_units(ctx, L, matvec_split(op)));
   const bool mixed = op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM;
   if (nc > 0)
     k_gather_b<<<ceil_div(nc, TPB), TPB, 0, ctx->stream>>>(
@@ -2610,7 +2636,7 @@ extern "C" int abx_operator_matvec_noalloc(abx_operator *op, const double *b, do
   cudaStream_t s = ctx->stream;
   PairLayout &L = *op->pairs;
   // (precision changed since: the units are listed anew, in the same buffers)
-  if (L.split != matvec_split(op)) ABX_TRY(relist_units(ctx, L, matvec_split(op)));
+  if (!(L.split == matvec_split(op))) ABX_TRY(relist_units(ctx, L, matvec_split(op)));
   if (nc == 0) {
     ABX_CHECK_CUDA(cudaMemsetAsync(c, 0, nr * sizeof(double), s));
     return ABX_OK;
