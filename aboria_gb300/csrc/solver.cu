@@ -245,37 +245,35 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 }
 
 // ------------------------------------------- LU with an integer update ---
-// The same factorisation (partial pivoting, panels of PW columns, LAPACK's
-// pivot convention) for blocks of kernel values of one size (Gaussian,
-// Wendland: at most 1, 1 on the diagonal), where the trailing update, n^3 / 3
-// multiply-adds, need not run at 2 FP64 operations a clock and SM: the panel's
-// rows and the block row's columns are scaled by powers of two to 56-bit
-// integers, x = (h 2^28 + l) 2^(e - 56) with signed halves, and a product sum
-// over the panel's 32 columns is two exact 64-bit sums, hi += h h and mid +=
-// h l + l h: three 32x32+64 multiply-adds (58 a clock and SM) for one FP64
-// multiply-add (1.8).  l l is below the scaled values' own 2^-57.  A row of L is
-// scaled by its largest entry in the panel and a column of U likewise, so the
-// error of a product is 2^-56 of the largest product of its row and column, where
-// FP64's partial sums round at 2^-53 of themselves.
+// The same factorisation (partial pivoting, LAPACK's pivot convention) for
+// blocks of kernel values of one size (Gaussian, Wendland: at most 1, 1 on the
+// diagonal), where the trailing update, n^3 / 3 multiply-adds, need not run at 2
+// FP64 operations a clock and SM: the rows of L21 and the columns of U12 are
+// scaled by powers of two to 56-bit integers, x = (h 2^28 + l) 2^(e - 56) with
+// signed halves, and a product sum over up to 64 columns is two exact 64-bit
+// sums, hi += h h and mid += h l + l h: three 32x32+64 multiply-adds (58 a clock
+// and SM) for one FP64 multiply-add (1.8).  l l is below the scaled values' own
+// 2^-57.  The scale is the largest entry of the row (column), so a product's
+// error is 2^-56 of the largest product of its row and column, where FP64's
+// partial sums round at 2^-53 of themselves.
 //
-// One CTA a domain.  The panel is factorised in shared memory (rows below the
-// diagonal block x 32 columns), row swaps of the other columns are deferred to
-// its end, the block row is solved a column a thread, and the update takes
-// UTR x UTC tiles, a 4 x 4 piece a thread.  Blocks of more rows than the shared
-// panel holds keep k_lu_fp64.  256 domains of 703 rows on average: @LU_OLD@ ->
-// @LU_NEW@ ms.
-constexpr int FL_T = 512;              // threads
-constexpr int UTR = 64, UTC = 128;     // update tile: rows, columns (4 x 4 a thread)
-constexpr int PLD = PW + 1;            // panel row stride
-constexpr int FL_MAX = 832;            // rows of a block: 832 * 33 * 8 B = 220 KB
-static_assert((UTR / 4) * (UTC / 4) == FL_T, "one 4 x 4 piece a thread");
-struct LuTiles {
-  int2 L[PW][UTR];  // (h, l) of the panel's rows, of the block row's columns
-  int2 U[PW][UTC];
-};
-static_assert(sizeof(LuTiles) <= (size_t)FL_MAX * PLD * 8, "tiles fit the panel's memory");
+// One CTA a domain, two to an SM.  What is left to the FP64 pipe sets the
+// blocking: panels of 16 columns are factorised in shared memory (the FP64 work
+// in a panel grows with its width); an update converts its sums and subtracts
+// them, two FP64 operations an entry, so the trailing matrix is updated for 64
+// columns at a time and only the rows and columns of those 64 panel by panel.
+// Pivots are compared as integers.  Blocks of more rows than the shared panel
+// holds keep k_lu_fp64.  256 domains of 703 rows on average (set-up and one
+// apply): 98 -> @LU_NEW@ ms.
+constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
+constexpr int FW = 16;         // panel width
+constexpr int FB = 64;         // columns of a trailing update
+constexpr int PLD = FW + 1;    // panel row stride
+constexpr int FL_MAX = 1600;   // rows of a block: 1600 * 17 * 8 B = 213 KB
+constexpr size_t FL_TILES = (size_t)FB * (64 + 64) * sizeof(int2);  // FB = 64 columns, 64 x 64
+static_assert(FL_TILES >= (size_t)FW * (256 + 16) * sizeof(int2), "tiles of one panel fit too");
 
-// x 2^(56 - e) as h 2^28 + l, |l| <= 2^27; |x| <= 2^e, e in scale_exp's range
+// x 2^(56 - e) as h 2^28 + l, |l| <= 2^27; |x| <= 2^e
 __device__ __forceinline__ int2 split56(double x, int e) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const int ex = (int)((u >> 52) & 0x7ff);
@@ -287,25 +285,115 @@ __device__ __forceinline__ int2 split56(double x, int e) {
   const int l = (int)((unsigned)f << 4) >> 4;  // the low 28 bits, signed
   return make_int2((int)((f - l) >> 28), l);
 }
-// smallest e with |x| <= 2^e from the bits of the largest |x| (0: any)
-__device__ __forceinline__ int scale_exp(unsigned long long maxbits) {
-  const int ex = (int)((maxbits >> 52) & 0x7ff);
-  return ex - 1022;
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+// e with |x| <= 2^e from the bits of the largest |x|
+__device__ __forceinline__ short scale_exp(unsigned long long maxbits) {
+  return (short)((int)(maxbits >> 52) - 1022);
 }
 
-__global__ void __launch_bounds__(FL_T) k_lu_fix(double *__restrict__ mat,
-                                                 const int64_t *__restrict__ dom_mat,
-                                                 const int *__restrict__ dom_size,
-                                                 const int *__restrict__ dom_off,
-                                                 int *__restrict__ piv, int *__restrict__ info) {
+// A[r0.., c0..] -= L[r0.., k0..k0+kw) U[k0.., c0..) for rows below r1 and
+// columns below c1, tiles of TR x TC, kw <= FB; le, ue: the exponents of L's rows
+// and U's columns.  Whole CTA; barriers at the start of every tile.
+template <int TR, int TC>
+__device__ __noinline__ void update_fix(double *A, int n, int r0, int r1, int c0, int c1, int k0,
+                                           int kw, const short *le, const short *ue, int2 *tiles) {
+  static_assert((TR / 4) * (TC / 4) == FL_T, "one 4 x 4 piece a thread");
+  const int tid = threadIdx.x;
+  int2 *L = tiles, *U = tiles + kw * TR;  // [k][row], [k][column]
+  const int tr = (tid % (TR / 4)) * 4, tc = (tid / (TR / 4)) * 4;
+  for (int ti = r0; ti < r1; ti += TR) {
+    for (int tj = c0; tj < c1; tj += TC) {
+      __syncthreads();
+      if (tj == c0)
+        for (int e = tid; e < kw * TR; e += FL_T) {
+          const int r = e % TR, k = e / TR;
+          L[k * TR + r] = ti + r < r1 ? split56(M(A, n, ti + r, k0 + k), le[ti + r]) : make_int2(0, 0);
+        }
+      for (int e = tid; e < kw * TC; e += FL_T) {
+        const int k = e % kw, j = e / kw;
+        U[k * TC + j] = tj + j < c1 ? split56(M(A, n, k0 + k, tj + j), ue[tj + j]) : make_int2(0, 0);
+      }
+      __syncthreads();
+      if (ti + tr >= r1 || tj + tc >= c1) continue;
+      long long hi[4][4] = {}, mid[4][4] = {};
+#pragma unroll 2
+      for (int k = 0; k < kw; ++k) {
+        int2 a[4], b[4];
+        *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&L[k * TR + tr]);
+        *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&L[k * TR + tr + 2]);
+        *reinterpret_cast<int4 *>(&b[0]) = *reinterpret_cast<const int4 *>(&U[k * TC + tc]);
+        *reinterpret_cast<int4 *>(&b[2]) = *reinterpret_cast<const int4 *>(&U[k * TC + tc + 2]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            hi[i][j] += (long long)a[i].x * b[j].x;
+            mid[i][j] += (long long)a[i].x * b[j].y;
+            mid[i][j] += (long long)a[i].y * b[j].x;
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int cj = tj + tc + j;
+        if (cj >= c1) continue;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int ri = ti + tr + i;
+          if (ri >= r1) continue;
+          // (hi 2^56 + mid 2^28) 2^(le - 56) 2^(ue - 56)
+          const long long t = hi[i][j] + ((mid[i][j] + (1ll << 27)) >> 28);
+          const int ex = max((int)le[ri] + (int)ue[cj] - 56 + 1023, 1);
+          const double sc = __longlong_as_double((long long)ex << 52);
+          M(A, n, ri, cj) = fma(-(double)t, sc, M(A, n, ri, cj));
+        }
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Rows k0 + c and sw[c] of one column swapped, c = 0, 1, ...
+__device__ __forceinline__ void swap_rows(double *col, int k0, int kw, const int *sw) {
+  for (int c = 0; c < kw; ++c) {
+    const int p = sw[c];
+    if (p != k0 + c) {
+      const double t = col[k0 + c];
+      col[k0 + c] = col[p];
+      col[p] = t;
+    }
+  }
+}
+// x := L^{-1} x for FW entries of a column, L unit lower; the exponent of the result.
+__device__ __noinline__ short solve_unit_lower(double *col, const double (*L)[FW + 1]) {
+  double x[FW];
+#pragma unroll
+  for (int c = 0; c < FW; ++c) x[c] = col[c];
+  unsigned long long mx = 0;
+#pragma unroll
+  for (int c = 0; c < FW; ++c) {
+    mx = max(mx, abs_bits(x[c]));
+#pragma unroll
+    for (int q = c + 1; q < FW; ++q) x[q] = fma(-L[q][c], x[c], x[q]);
+    col[c] = x[c];
+  }
+  return scale_exp(mx);
+}
+
+__global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
+                                                    const int64_t *__restrict__ dom_mat,
+                                                    const int *__restrict__ dom_size,
+                                                    const int *__restrict__ dom_off,
+                                                    int *__restrict__ piv, int *__restrict__ info) {
   extern __shared__ __align__(16) unsigned char lu_raw[];
-  double *Pn = reinterpret_cast<double *>(lu_raw);  // panel: rows k0..n-1 x PW, stride PLD
-  LuTiles &T = *reinterpret_cast<LuTiles *>(lu_raw);
-  __shared__ double red_v[FL_T / 32];
+  double *Pn = reinterpret_cast<double *>(lu_raw);  // panel: rows k0..n-1 x FW, stride PLD
+  int2 *tiles = reinterpret_cast<int2 *>(lu_raw);
+  __shared__ unsigned long long red_v[FL_T / 32];
   __shared__ int red_i[FL_T / 32];
-  __shared__ double L11[PW][PW + 1];
-  __shared__ int swaps[PW];
-  __shared__ short le[FL_MAX], ue[FL_MAX];  // exponents of the panel's rows, the block row's columns
+  __shared__ double L11[FB / FW][FW][FW + 1];
+  __shared__ int swaps[FB];
+  __shared__ short le[FL_MAX], ue[FL_MAX];  // exponents of L's rows, of U's columns
   const int d = blockIdx.x;
   const int n = dom_size[d];
   if (n > FL_MAX) return;  // k_lu_fp64's
@@ -313,146 +401,118 @@ __global__ void __launch_bounds__(FL_T) k_lu_fix(double *__restrict__ mat,
   int *pv = piv + dom_off[d];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int status = 0;
-  for (int k0 = 0; k0 < n; k0 += PW) {
-    const int kw = min(PW, n - k0), k1 = k0 + kw, rows = n - k0;
-    // ---- the panel, in shared memory
-    for (int c = warp; c < kw; c += FL_T / 32)
-      for (int r = lane; r < rows; r += 32) Pn[r * PLD + c] = M(A, n, k0 + r, k0 + c);
-    __syncthreads();
-    for (int c = 0; c < kw; ++c) {
-      // pivot: the first row of largest |entry| at or below the diagonal
-      double best = -1.0;
-      int bi = c;
-      for (int r = c + tid; r < rows; r += FL_T) {
-        const double v = fabs(Pn[r * PLD + c]);
-        if (v > best) { best = v; bi = r; }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-      }
-      if (lane == 0) { red_v[warp] = best; red_i[warp] = bi; }
+  for (int B0 = 0; B0 < n; B0 += FB) {
+    const int B1 = min(B0 + FB, n);
+    for (int k0 = B0; k0 < B1; k0 += FW) {
+      const int kw = min(FW, n - k0), k1 = k0 + kw, rows = n - k0;
+      // ---- the panel, in shared memory
+      for (int c = warp; c < kw; c += FL_T / 32)
+        for (int r = lane; r < rows; r += 32) Pn[r * PLD + c] = M(A, n, k0 + r, k0 + c);
       __syncthreads();
-      best = red_v[0];
-      bi = red_i[0];
-      for (int w = 1; w < FL_T / 32; ++w)
-        if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) { best = red_v[w]; bi = red_i[w]; }
-      if (tid == 0) {
-        swaps[c] = k0 + bi;
-        pv[k0 + c] = k0 + bi;
-        if (best == 0.0 && status == 0) status = k0 + c + 1;
-      }
-      if (bi != c && tid < kw) {
-        const double t = Pn[c * PLD + tid];
-        Pn[c * PLD + tid] = Pn[bi * PLD + tid];
-        Pn[bi * PLD + tid] = t;
-      }
-      __syncthreads();
-      const double dpiv = Pn[c * PLD + c];
-      const double inv = dpiv != 0.0 ? 1.0 / dpiv : 0.0;
-      for (int r = c + 1 + tid; r < rows; r += FL_T) {
-        const double l = Pn[r * PLD + c] * inv;
-        Pn[r * PLD + c] = l;
-        for (int cc = c + 1; cc < kw; ++cc)
-          Pn[r * PLD + cc] = fma(-l, Pn[c * PLD + cc], Pn[r * PLD + cc]);
-      }
-      __syncthreads();
-    }
-    for (int e = tid; e < kw * kw; e += FL_T) L11[e / kw][e % kw] = Pn[(e / kw) * PLD + e % kw];
-    // scale of every row below the diagonal block; the panel back to the matrix
-    for (int r = kw + tid; r < rows; r += FL_T) {
-      unsigned long long mx = 0;
-      for (int c = 0; c < kw; ++c)
-        mx = max(mx, (unsigned long long)__double_as_longlong(Pn[r * PLD + c]) & 0x7fffffffffffffffull);
-      le[r] = (short)scale_exp(mx);
-    }
-    for (int c = warp; c < kw; c += FL_T / 32)
-      for (int r = lane; r < rows; r += 32) M(A, n, k0 + r, k0 + c) = Pn[r * PLD + c];
-    __syncthreads();
-    // ---- the other columns: row swaps; right of the panel U12 = L11^{-1} A12
-    for (int j = tid; j < n; j += FL_T) {
-      if (j >= k0 && j < k1) continue;
-      double *col = A + (int64_t)j * n;
       for (int c = 0; c < kw; ++c) {
-        const int p = swaps[c];
-        if (p != k0 + c) {
-          const double t = col[k0 + c];
-          col[k0 + c] = col[p];
-          col[p] = t;
+        // pivot: the first row of largest |entry| at or below the diagonal
+        unsigned long long best = 0;
+        int bi = 0x7fffffff;
+        for (int r = c + tid; r < rows; r += FL_T) {
+          const unsigned long long v = abs_bits(Pn[r * PLD + c]);
+          if (v > best || bi == 0x7fffffff) { best = v; bi = r; }
         }
-      }
-      if (j < k1) continue;
-      // (a panel with columns to its right has all its PW columns)
-      double x[PW];
-#pragma unroll
-      for (int c = 0; c < PW; ++c) x[c] = col[k0 + c];
-      unsigned long long mx = 0;
-#pragma unroll
-      for (int c = 0; c < PW; ++c) {
-        mx = max(mx, (unsigned long long)__double_as_longlong(x[c]) & 0x7fffffffffffffffull);
-#pragma unroll
-        for (int q = c + 1; q < PW; ++q) x[q] = fma(-L11[q][c], x[c], x[q]);
-        col[k0 + c] = x[c];
-      }
-      ue[j] = (short)scale_exp(mx);
-    }
-    __syncthreads();
-    if (k1 >= n) break;
-    // ---- A22 -= L21 U12
-    for (int ti = k1; ti < n; ti += UTR) {
-      __syncthreads();
-      for (int e = tid; e < PW * UTR; e += FL_T) {
-        const int r = e % UTR, c = e / UTR;
-        T.L[c][r] = ti + r < n ? split56(M(A, n, ti + r, k0 + c), le[ti + r - k0])
-                                         : make_int2(0, 0);
-      }
-      for (int tj = k1; tj < n; tj += UTC) {
-        __syncthreads();
-        for (int e = tid; e < PW * UTC; e += FL_T) {
-          const int c = e % PW, j = e / PW;
-          T.U[c][j] = tj + j < n ? split56(M(A, n, k0 + c, tj + j), ue[tj + j])
-                                           : make_int2(0, 0);
-        }
-        __syncthreads();
-        const int tr = (tid % (UTR / 4)) * 4, tc = (tid / (UTR / 4)) * 4;
-        if (ti + tr >= n || tj + tc >= n) continue;
-        long long hi[4][4] = {}, mid[4][4] = {};
-#pragma unroll 2
-        for (int c = 0; c < PW; ++c) {
-          int2 a[4], b[4];
-          *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&T.L[c][tr]);
-          *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&T.L[c][tr + 2]);
-          *reinterpret_cast<int4 *>(&b[0]) = *reinterpret_cast<const int4 *>(&T.U[c][tc]);
-          *reinterpret_cast<int4 *>(&b[2]) = *reinterpret_cast<const int4 *>(&T.U[c][tc + 2]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              hi[i][j] += (long long)a[i].x * b[j].x;
-              mid[i][j] += (long long)a[i].x * b[j].y;
-              mid[i][j] += (long long)a[i].y * b[j].x;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int cj = tj + tc + j;
-          if (cj >= n) continue;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int ri = ti + tr + i;
-            if (ri >= n) continue;
-            // (hi 2^56 + mid 2^28) 2^(le - 56) 2^(ue - 56)
-            const long long t = hi[i][j] + ((mid[i][j] + (1ll << 27)) >> 28);
-            const int ex = max(le[ri - k0] + ue[cj] - 56 + 1023, 1);
-            const double sc = __longlong_as_double((long long)ex << 52);
-            M(A, n, ri, cj) = fma(-(double)t, sc, M(A, n, ri, cj));
+        {
+          const unsigned h = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+          const bool top = (unsigned)(best >> 32) == h;
+          const unsigned l = __reduce_max_sync(0xffffffffu, top ? (unsigned)best : 0u);
+          const unsigned i = __reduce_min_sync(
+              0xffffffffu, top && (unsigned)best == l ? (unsigned)bi : 0x7fffffffu);
+          if (lane == 0) {
+            red_v[warp] = ((unsigned long long)h << 32) | l;
+            red_i[warp] = (int)i;
           }
         }
+        __syncthreads();
+        best = red_v[0];
+        bi = red_i[0];
+        for (int w = 1; w < FL_T / 32; ++w)
+          if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) { best = red_v[w]; bi = red_i[w]; }
+        if (tid == 0) {
+          swaps[k0 - B0 + c] = k0 + bi;
+          pv[k0 + c] = k0 + bi;
+          if (best == 0 && status == 0) status = k0 + c + 1;
+        }
+        if (bi != c && tid < kw) {
+          const double t = Pn[c * PLD + tid];
+          Pn[c * PLD + tid] = Pn[bi * PLD + tid];
+          Pn[bi * PLD + tid] = t;
+        }
+        __syncthreads();
+        const double dpiv = Pn[c * PLD + c];
+        // 1 / pivot: Newton steps from the FP32 reciprocal (4 FP64 operations)
+        double inv;
+        if (fabs(dpiv) > 1e-30 && fabs(dpiv) < 1e30) {
+          inv = (double)fx::rcp32((float)dpiv);
+          inv = fma(fma(-dpiv, inv, 1.0), inv, inv);
+          inv = fma(fma(-dpiv, inv, 1.0), inv, inv);
+        } else {
+          inv = dpiv != 0.0 ? 1.0 / dpiv : 0.0;
+        }
+        for (int r = c + 1 + tid; r < rows; r += FL_T) {
+          const double l = Pn[r * PLD + c] * inv;
+          Pn[r * PLD + c] = l;
+          for (int cc = c + 1; cc < kw; ++cc)
+            Pn[r * PLD + cc] = fma(-l, Pn[c * PLD + cc], Pn[r * PLD + cc]);
+        }
+        __syncthreads();
       }
+      const int s = (k0 - B0) / FW;
+      for (int e = tid; e < kw * kw; e += FL_T)
+        L11[s][e / kw][e % kw] = Pn[(e / kw) * PLD + e % kw];
+      // scale of every row below the diagonal block; the panel back to the matrix
+      for (int r = kw + tid; r < rows; r += FL_T) {
+        unsigned long long mx = 0;
+        for (int c = 0; c < kw; ++c) mx = max(mx, abs_bits(Pn[r * PLD + c]));
+        le[k0 + r] = scale_exp(mx);
+      }
+      for (int c = warp; c < kw; c += FL_T / 32)
+        for (int r = lane; r < rows; r += 32) M(A, n, k0 + r, k0 + c) = Pn[r * PLD + c];
+      __syncthreads();
+      // ---- the other columns up to B1: row swaps; right of the panel U12 =
+      // L11^{-1} A12 (a panel with columns to its right has all its FW columns),
+      // and the rows below.  Columns beyond B1 wait: a later panel's pivot may
+      // bring up a row that has not had this panel's update.
+      for (int j = tid; j < B1; j += FL_T) {
+        if (j >= k0 && j < k1) continue;
+        double *col = A + (int64_t)j * n;
+        swap_rows(col, k0, kw, swaps + (k0 - B0));
+        if (j >= k1) ue[j] = solve_unit_lower(col + k0, L11[s]);
+      }
+      __syncthreads();
+      if (k1 < B1) update_fix<256, 16>(A, n, k1, n, k1, B1, k0, kw, le, ue, tiles);
     }
-    __syncthreads();
+    if (B1 >= n) break;
+    // ---- the block row right of B1, panel by panel
+    for (int j = B1 + tid; j < n; j += FL_T) swap_rows(A + (int64_t)j * n, B0, FB, swaps);
+    for (int k0 = B0; k0 < B1; k0 += FW) {
+      const int k1 = k0 + FW;
+      for (int j = B1 + tid; j < n; j += FL_T)
+        ue[j] = solve_unit_lower(A + (int64_t)j * n + k0, L11[(k0 - B0) / FW]);
+      for (int r = k1 + tid; r < B1; r += FL_T) {
+        unsigned long long mx = 0;
+        for (int k = k0; k < k1; ++k) mx = max(mx, abs_bits(M(A, n, r, k)));
+        le[r] = scale_exp(mx);
+      }
+      __syncthreads();
+      if (k1 < B1) update_fix<16, 256>(A, n, k1, B1, B1, n, k0, FW, le, ue, tiles);
+    }
+    // ---- the trailing matrix, for all FB columns
+    for (int r = B1 + tid; r < n; r += FL_T) {
+      unsigned long long ml = 0, mu = 0;
+      for (int k = B0; k < B1; ++k) {
+        ml = max(ml, abs_bits(M(A, n, r, k)));
+        mu = max(mu, abs_bits(M(A, n, k, r)));
+      }
+      le[r] = scale_exp(ml);
+      ue[r] = scale_exp(mu);
+    }
+    update_fix<64, 64>(A, n, B1, n, B1, n, B0, FB, le, ue, tiles);
   }
   if (tid == 0) info[d] = status;
 }
@@ -726,7 +786,7 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
     const bool flat = op->k.kind == ABX_K_GAUSSIAN || op->k.kind == ABX_K_COMPACT_GAUSSIAN ||
                       op->k.kind == ABX_K_WENDLAND_C2;
     if (flat) {
-      const size_t smem = std::max(sizeof(LuTiles), (size_t)std::min(S->max_size, FL_MAX) * PLD * 8);
+      const size_t smem = std::max(FL_TILES, (size_t)std::min(S->max_size, FL_MAX) * PLD * 8);
       if (cudaFuncSetAttribute(k_lu_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess) {
         set_error("LU: %zu bytes of shared memory refused", smem);
