@@ -213,6 +213,20 @@ FX_HD u64 sqrt60(u64 u) {
   return (((u64)(u32)q0) << 32) + (u64)low;
 }
 
+// m 2^-s as a double for m in [2^61, 2^62], rounded to nearest.
+FX_HD double make_double61(u64 m, int s) {
+  const u64 r = (m + 256) >> 9;  // 53 bits; 2^53 carries into the exponent
+  return from_bits(r + ((u64)(u32)(1083 - s) << 52));
+}
+FX_HD u32 funnel_l(u32 lo, u32 hi, int k) {  // upper word of (hi : lo) << k, 0 <= k < 32
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, k);
+#else
+  return k ? (hi << k) | (lo >> (32 - k)) : hi;
+#endif
+}
+FX_HD u64 join(u32 hi, u32 lo) { return ((u64)hi << 32) | lo; }
+
 // m * 2^-s as a double, rounded to nearest; m != 0, the result normal.
 FX_HD double make_double(u64 m, int s) {
   const u32 h = hi32(m);
@@ -301,36 +315,29 @@ FX_HD double wendland(u64 q2) {
   return make_double(mulhi63(t4, p), 59 + 4 * z);
 }
 
-// |dx|^2 of a split sum with its low part U = sum l^2, normalised: the value
-// is n 2^-62 2^-z R^2 with n in [2^62, 2^64), z even; n = 0 when d < 2^-30 R.
-FX_HD u64 norm_d2(i64 S, i64 T, u64 U, int &z) {
-  const u64 lo = U + ((u64)T << 33);
-  const u64 hi = (u64)S + (u64)(T >> 31) + (lo < U ? 1u : 0u);  // units of 2^-60
-  const int k = (hi32(hi) ? clz32(hi32(hi)) : 32 + clz32((u32)hi)) & ~1;
-  z = k - 2;
-  return k < 64 ? (hi << k) | ((lo >> 1) >> (63 - k)) : 0;
-}
-
 // d >= 2^-7 R: the coordinates' rounding to 2^-62 R is below 2^-54 of d.  Closer
 // pairs are left to the FP64 formula on the double coordinates.
 FX_HD bool laplace_far(i64 S) { return S >= (i64)1 << 46; }
-// 1 / (d + p0) for laplace_far pairs: n, z as norm_d2 gives them (n != 0), p0 / R = pm 2^-62 2^-pe
-// with pm in [2^62, 2^63) (or 0) and pe >= 0, R = 2^r.
-FX_HD double laplace(u64 n, int z, u64 pm, int pe, int r) {
-  const u64 q = sqrt60(n >> 4);  // d = q 2^-62 2^(1 - z/2) R, q in [2^61, 2^62)
-  // a = d + p0 at the scale of the larger, a 2^-62 2^E R
-  const int sh = pe + 1 - (z >> 1);
-  u64 a;
-  int E;
-  if (sh >= 0) {
-    a = q + (sh < 64 ? pm >> sh : 0);
-    E = 1 - (z >> 1);
-  } else {
-    a = pm + (sh > -64 ? q >> -sh : 0);
-    E = -pe;
-  }
-  const int y = clz32(hi32(a)) - 1;  // a in [2^61, 2^64)
-  const u64 A = y < 0 ? a >> 1 : a << y;
+
+// |dx|^2 of a split sum with its low part U = sum l^2, normalised, for
+// laplace_far pairs: the value is n 2^-62 2^-z R^2 with n in [2^62, 2^64) and z
+// even, 0 <= z <= 14.
+FX_HD u64 norm_d2(i64 S, i64 T, u64 U, int &z) {
+  const u32 t0 = (u32)T << 1, low = hi32(U) + t0;  // the word below S's
+  const u64 s = (u64)S + (u64)(T >> 31) + (low < t0 ? 1u : 0u);  // units of 2^-60
+  const int k = clz32(hi32(s)) & ~1;  // at most 16
+  z = k - 2;
+  return join(funnel_l((u32)s, hi32(s), k), funnel_l(low, (u32)s, k));
+}
+
+// 1 / (d + p0) for laplace_far pairs: n, z as norm_d2 gives them, P0 = p0 / R in
+// units of 2^-61 (p0 < R), R = 2^r.
+FX_HD double laplace(u64 n, int z, u64 P0, int r) {
+  // d = q 2^-62 2^(1 - z/2) R, q in [2^61, 2^62); a = d + p0 in units of 2^-61
+  // (below 2^-55 of d), normalised to [2^62, 2^63)
+  const u64 a = (sqrt60(n >> 4) >> (z >> 1)) + P0;
+  const int y = clz32(hi32(a)) - 1;  // 2^54 <= a < 2^63
+  const u64 A = join(funnel_l((u32)a, hi32(a), y), (u32)a << y);
   // reciprocal of A 2^-62 in [1, 2): FP32 seed, then 1 + e + e^2
   const u32 Y0 = (u32)f2i(rcp32((float)hi32(A) * 9.3132257461547852e-10f) * 1073741824.0f);
   const u64 w = (u64)(u32)A * Y0;
@@ -338,19 +345,49 @@ FX_HD double laplace(u64 n, int z, u64 pm, int pe, int r) {
   const i64 es = er >> 20;
   const i64 e2 = er + ((es * es) >> 20);
   const i64 add = ((i64)Y0 * (int32_t)(e2 >> 8) + (i64)(((u64)Y0 * (u32)(e2 & 255)) >> 8)) >> 20;
-  return make_double(((u64)Y0 << 32) + (u64)add, 62 + E - y + r);
+  // 1 / (A 2^-62) = Y 2^-62; a 2^-61 = A 2^-62 2^(1 - y)
+  return make_double61(join(Y0, 0) + (u64)add, 63 - y + r);
 }
 
 // sqrt(d^2 + c): v = (d^2 + c) / R^2 in units of 2^-63, 2^-8 <= v 2^-63 < 1;
 // R = 2^r.
 FX_HD double multiquadric(u64 v, int r) {
   const int k = (clz32(hi32(v)) - 1) | 1;
-  return make_double(sqrt60((v << k) >> 4), 62 + (k >> 1) - r);
+  return make_double61(sqrt60((v << k) >> 4), 62 + (k >> 1) - r);
+}
+
+// ------------------------------------------------- scaled 56-bit numbers ---
+// Operands of integer products of matrices: x 2^(56 - e) = h 2^28 + l with
+// signed halves, |l| <= 2^27, for |x| <= 2^e.  A sum of up to 64 products x y is
+// (hi 2^56 + mid 2^28) 2^(ex + ey - 112) with hi = sum h h and mid = sum (h l + l
+// h), both exact in 64 bits; l l is below the numbers' own 2^-57.
+FX_HD u64 abs_bits(double x) { return bits_of(x) & 0x7fffffffffffffffull; }
+// e with |x| <= 2^e from the bits of the largest |x|
+FX_HD int scale_exp(u64 maxbits) { return (int)(maxbits >> 52) - 1022; }
+struct Half2 {
+  int h, l;
+};
+FX_HD Half2 split56(double x, int e) {
+  const u64 u = bits_of(x);
+  const int ex = (int)((u >> 52) & 0x7ff);
+  const u64 m = (u & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
+  const int sh = (ex ? ex : 1) - 1075 + 56 - e;  // |x| 2^(56 - e) = m 2^sh, sh <= 4
+  i64 f = sh >= 0 ? (i64)(m << sh) : (sh > -63 ? (i64)(((m >> (-sh - 1)) + 1) >> 1) : 0);
+  if (u >> 63) f = -f;
+  const int l = (int)((u32)f << 4) >> 4;  // the low 28 bits, signed
+  return {(int)((f - l) >> 28), l};
+}
+// hi 2^56 + mid 2^28 in units of 2^56
+FX_HD i64 sum56(i64 hi, i64 mid) { return hi + ((mid + (1ll << 27)) >> 28); }
+// 2^(e - 56) (2^-1022 at least)
+FX_HD double scale56(int e) {
+  const int b = e - 56 + 1023;
+  return from_bits((u64)(b > 1 ? b : 1) << 52);
 }
 
 // ------------------------------------------------------------------- units ---
 // The fixed point of one kernel for pairs up to `reach` apart: coordinates
-// X = x f 2^k, and the kernel's constant (c, pe).  ok false: the kernel's
+// X = x f 2^k, and the kernel's constant.  ok false: the kernel's
 // parameter or the reach is outside what the value functions cover --
 //   Gaussian      t = p0 d^2 log2(e) must stay below 255 (at 16 and above the
 //                 coordinates' 63 bits overflow);
@@ -359,7 +396,7 @@ FX_HD double multiquadric(u64 v, int r) {
 //   Laplace       0 <= p0 < R.
 // R = 2^r: the power of two above the reach (above sqrt(reach^2 + p0)).
 struct Unit {
-  int ok, k, r, pe;
+  int ok, k, r;
   u64 c;
   Factor f;
 };
@@ -368,7 +405,7 @@ enum { GAUSSIAN = 1, WENDLAND = 2, LAPLACE = 4, MULTIQUADRIC = 5 };  // as abx.h
 template <int KIND> FX_HD Unit make_unit(double p0, double reach) {
   Unit U;
   U.ok = 0;
-  U.k = U.r = U.pe = 0;
+  U.k = U.r = 0;
   U.c = 0;
   U.f = make_factor(1.0, 0.0);
   double reach2 = reach * reach;
@@ -397,12 +434,7 @@ template <int KIND> FX_HD Unit make_unit(double p0, double reach) {
       U.c = (u64)ldexp(p0, 63 - 2 * e);
     } else if (KIND == LAPLACE) {
       if (p0 >= ldexp(1.0, e)) return U;
-      if (p0 > 0.0) {  // p0 / R = c 2^-62 2^-pe, c in [2^62, 2^63)
-        int g;
-        const double fr = frexp(p0, &g);
-        U.pe = e + 1 - g;
-        U.c = (u64)ldexp(fr, 63);
-      }
+      U.c = (u64)to_fixed(p0, U.f, 61 - e);
     } else
       return U;
   }
@@ -414,10 +446,10 @@ template <int KIND> FX_HD i64 fixed(double x, const Unit &U) { return to_fixed(x
 // What a kernel needs of the unit.
 struct Consts {
   u64 c;
-  int pe, r;
+  int r;
   double k0;  // value at distance 0 (Laplace)
 };
-FX_HD Consts consts(const Unit &U, double k0) { return {U.c, U.pe, U.r, k0}; }
+FX_HD Consts consts(const Unit &U, double k0) { return {U.c, U.r, k0}; }
 
 // Kernel value of one pair from its differences (diff(); the first dims of
 // them).  near: a Laplace pair closer than R / 128, left to the FP64 formula on
@@ -437,7 +469,7 @@ FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 
     near = !laplace_far(S);
     int z;
     const u64 n = norm_d2(S, T, U, z);
-    return laplace(n, z, C.c, C.pe, C.r);
+    return laplace(n, z, C.c, C.r);
   }
   if (KIND == WENDLAND) return wendland(sq_sum(S, T));
   if (KIND == MULTIQUADRIC) return multiquadric(sq_sum8(S, T) + C.c, C.r);

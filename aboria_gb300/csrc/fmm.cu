@@ -67,12 +67,16 @@ struct FmmPlan {
   DevBuf<int> links;                          // all levels, octant-major within a level
   DevBuf<int2> batches;                       // (first link, count <= NBL) of one octant
   std::vector<int> batch_off, batch_cnt;      // per level
-  // M2L: pairs (target, source, matrix id), grouped by level
-  DevBuf<int> m2l;
   int n_m2l = 0;
   DevBuf<double> Km;      // nmat x ncheb x ncheb
   DevBuf<float> Kmh, Kml; // split-TF32 hi/lo parts of the FP32 copy (mma.sync M2L, ncheb <= 64)
   DevBuf<float> Kp;       // the same packed as tcgen05 stage images (ncheb > 64, k_pack_tf32)
+  // FP64 M2L on the integer units: K and W as scaled 56-bit numbers, their
+  // exponents (per row of K, per node), tiles of 64 pairs
+  DevBuf<int2> Kq, Wq;
+  DevBuf<short> ke, we;
+  DevBuf<int> mf_mat, mf_first;
+  int mf_tiles = 0;
   DevBuf<float> W32l;     // lo part of W (the tcgen05 M2L reads W32 as the hi part)
   int nmat = 0;
   // M2L grouped by matrix (for the tensor-core GEMM): per matrix a list of
@@ -368,23 +372,125 @@ __global__ void k_transpose_tc(const double *__restrict__ in, int nchild, int nc
 }
 
 // --------------------------------------------------------------- M2L ---
-// FP64, one CTA per M2L pair: G[t] += K[m] W[s] (atomic: several sources per
-// target run concurrently).
-__global__ void __launch_bounds__(FT) k_m2l64(int ncheb, const int *__restrict__ pairs, int npairs,
-                                              const double *__restrict__ Km,
-                                              const double *__restrict__ W,
-                                              double *__restrict__ G) {
-  const int q = blockIdx.x;
-  if (q >= npairs) return;
-  const int t = pairs[3 * q], s = pairs[3 * q + 1], m = pairs[3 * q + 2];
-  __shared__ double ws[MAXC];
-  for (int j = threadIdx.x; j < ncheb; j += FT) ws[j] = W[(size_t)s * ncheb + j];
-  __syncthreads();
-  const double *K = Km + (size_t)m * ncheb * ncheb;
-  for (int i = threadIdx.x; i < ncheb; i += FT) {
-    double a = 0.0;
-    for (int j = 0; j < ncheb; ++j) a += K[(size_t)i * ncheb + j] * ws[j];
-    atomicAdd(&G[(size_t)t * ncheb + i], a);
+// FP64 M2L as integer products of matrices (scaled 56-bit numbers, fix64.cuh):
+// for one matrix K and 64 (target, source) pairs sharing it, a tile of TR rows
+// of K W[:, sources], each multiply-add three 32x32+64 ones (25 a clock and SM)
+// instead of an FP64 one (1.8, which bounded one CTA per pair).  K is split once
+// per plan with a scale per row (Kq, transposed), W per product with a scale per
+// node (Wq); both scales and 57 bits make a term's rounding smaller than the FP64
+// sum's own.  Sums are turned into FP64 every 64 terms, which the 64-bit sums
+// hold.  N = 1,048,576, 6.0e6 pairs: order 3 (27 nodes) 8.5 -> @M3@ ms, order 5
+// (125) @M5A@ -> @M5B@ ms.
+__global__ void k_split_k(const double *__restrict__ K, int64_t nrows, int ncheb, int ldr,
+                          int2 *__restrict__ Kq, short *__restrict__ ke) {
+  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= nrows) return;
+  const int64_t m = row / ncheb;
+  const int i = (int)(row % ncheb);
+  const double *k = K + row * ncheb;
+  fx::u64 mx = 0;
+  for (int j = 0; j < ncheb; ++j) mx = max(mx, fx::abs_bits(k[j]));
+  const int e = fx::scale_exp(mx);
+  ke[m * ldr + i] = (short)e;
+  for (int j = 0; j < ncheb; ++j) {
+    const fx::Half2 q = fx::split56(k[j], e);
+    Kq[(m * ncheb + j) * ldr + i] = make_int2(q.h, q.l);
+  }
+}
+__global__ void k_split_w(const double *__restrict__ W, int nnodes, int ncheb,
+                          int2 *__restrict__ Wq, short *__restrict__ we) {
+  const int node = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (node >= nnodes) return;
+  const double *w = W + (size_t)node * ncheb;
+  fx::u64 mx = 0;
+  for (int j = lane; j < ncheb; j += 32) mx = max(mx, fx::abs_bits(w[j]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const int e = fx::scale_exp(mx);
+  if (lane == 0) we[node] = (short)e;
+  for (int j = lane; j < ncheb; j += 32) {
+    const fx::Half2 q = fx::split56(w[j], e);
+    Wq[(size_t)node * ncheb + j] = make_int2(q.h, q.l);
+  }
+}
+constexpr int MF_P = 64;    // pairs per tile
+constexpr int MF_K = 32;    // columns staged at a time
+constexpr int MF_LD = MF_P + 2;
+template <int TR, bool MULTI>
+__global__ void __launch_bounds__(TR / 4 * (MF_P / 4), 512 / (TR / 4 * (MF_P / 4))) k_m2l_fix(
+    int ncheb, int ldr, const int2 *__restrict__ Kq, const short *__restrict__ ke,
+    const int2 *__restrict__ Wq, const short *__restrict__ we, const int2 *__restrict__ by_mat,
+    const int *__restrict__ mat_off, const int *__restrict__ tile_mat,
+    const int *__restrict__ tile_first, double *__restrict__ G) {
+  constexpr int T = TR / 4 * (MF_P / 4);
+  __shared__ __align__(16) int2 sA[MF_K][TR];
+  __shared__ __align__(16) int2 sB[MF_K][MF_LD];
+  __shared__ int tgt[MF_P], src[MF_P], sexp[MF_P];
+  const int tid = threadIdx.x, m = tile_mat[blockIdx.x], first = tile_first[blockIdx.x];
+  const int np = min(MF_P, mat_off[m + 1] - first), r0 = blockIdx.y * TR;
+  for (int p = tid; p < MF_P; p += T) {
+    const int2 ts = by_mat[first + min(p, np - 1)];
+    tgt[p] = ts.x;
+    src[p] = ts.y;
+    sexp[p] = we[ts.y];
+  }
+  const int tr = (tid % (TR / 4)) * 4, tc = (tid / (TR / 4)) * 4;
+  long long hi[4][4] = {}, mid[4][4] = {};
+  double sum[4][4] = {};
+  const int2 *Km = Kq + (size_t)m * ncheb * ldr + r0;
+  for (int k0 = 0; k0 < ncheb; k0 += MF_K) {
+    const int kc = min(MF_K, ncheb - k0);
+    __syncthreads();
+    for (int e = tid; e < kc * (TR / 2); e += T) {  // two entries at a time (ldr is even)
+      const int r = (e % (TR / 2)) * 2, k = e / (TR / 2);
+      int4 v = make_int4(0, 0, 0, 0);
+      if (r0 + r < ldr) v = *reinterpret_cast<const int4 *>(Km + (size_t)(k0 + k) * ldr + r);
+      *reinterpret_cast<int4 *>(&sA[k][r]) = v;
+    }
+    for (int e = tid; e < MF_K * MF_P; e += T) {
+      const int k = e % MF_K, p = e / MF_K;
+      if (k < kc) sB[k][p] = Wq[(size_t)src[p] * ncheb + k0 + k];
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int k = 0; k < kc; ++k) {
+      int2 a[4], b[4];
+      *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&sA[k][tr]);
+      *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&sA[k][tr + 2]);
+      *reinterpret_cast<int4 *>(&b[0]) = *reinterpret_cast<const int4 *>(&sB[k][tc]);
+      *reinterpret_cast<int4 *>(&b[2]) = *reinterpret_cast<const int4 *>(&sB[k][tc + 2]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          hi[i][j] += (long long)a[i].x * b[j].x;
+          mid[i][j] += (long long)a[i].x * b[j].y;
+          mid[i][j] += (long long)a[i].y * b[j].x;
+        }
+    }
+    if (MULTI && ((k0 / MF_K) & 1)) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sum[i][j] += (double)fx::sum56(hi[i][j], mid[i][j]);
+          hi[i][j] = mid[i][j] = 0;
+        }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int p = tc + j;
+    if (p >= np) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + tr + i;
+      if (r >= ncheb) continue;
+      double t = (double)fx::sum56(hi[i][j], mid[i][j]);
+      if (MULTI) t += sum[i][j];
+      atomicAdd(&G[(size_t)tgt[p] * ncheb + r], t * fx::scale56((int)ke[(size_t)m * ldr + r] + sexp[p]));
+    }
   }
 }
 
@@ -1488,11 +1594,10 @@ int fmm_plan_build(abx_operator *op, int order, FmmPlan *&out, double eta = 1.0)
     std::swap(dst.ptr, src.ptr);
     std::swap(dst.cap, src.cap);
   };
-  take(P->m2l, lists.m2l_trip);
   take(P->m2l_by_mat, lists.m2l_by_mat);
   take(P->p2p_rowptr, lists.p2p_rowptr);
   take(P->p2p_src, lists.p2p_src);
-  if ((st = P->m2l.reserve(1)) || (st = P->m2l_by_mat.reserve(1)) ||
+  if ((st = P->m2l_by_mat.reserve(1)) ||
       (st = P->p2p_rowptr.reserve(1)) || (st = P->p2p_src.reserve(1)))
     return fail(st);
   if (NN <= 1) {
@@ -1587,6 +1692,52 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
     k_l2p_p2p<KIND, false><<<P->nleaves, FT, 0, s>>>(
         P->D, P->n, P->ncheb, P->leaf_ids.ptr, P->node_begin.ptr, P->node_end.ptr, P->box.ptr, pos,
         npos, b, P->mi_d.ptr, P->G.ptr, P->p2p_rowptr.ptr, P->p2p_src.ptr, P->p0, P->tab, c);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  return ABX_OK;
+}
+}  // namespace
+
+namespace {
+// The FP64 M2L: G += K W.  The split matrices and the tiles of 64 pairs are made
+// by the plan's first FP64 product.
+int m2l_fix(FmmPlan *P, cudaStream_t s) {
+  const int nc = P->ncheb, ldr = (nc + 1) / 2 * 2;
+  if (!P->Kq.ptr) {
+    std::vector<int> mat, first;
+    for (int m = 0; m < P->nmat; ++m)
+      for (int q = P->mat_off[m]; q < P->mat_off[m + 1]; q += MF_P) {
+        mat.push_back(m);
+        first.push_back(q);
+      }
+    P->mf_tiles = (int)mat.size();
+    ABX_TRY(P->mf_mat.reserve(mat.size() + 1));
+    ABX_TRY(P->mf_first.reserve(first.size() + 1));
+    ABX_TRY(P->ke.reserve((size_t)P->nmat * ldr));
+    ABX_CHECK_CUDA(cudaMemcpyAsync(P->mf_mat.ptr, mat.data(), mat.size() * 4, cudaMemcpyHostToDevice, s));
+    ABX_CHECK_CUDA(cudaMemcpyAsync(P->mf_first.ptr, first.data(), first.size() * 4,
+                                   cudaMemcpyHostToDevice, s));
+    ABX_TRY(P->Kq.reserve((size_t)P->nmat * nc * ldr));
+    if (ldr != nc)
+      ABX_CHECK_CUDA(cudaMemsetAsync(P->Kq.ptr, 0, (size_t)P->nmat * nc * ldr * sizeof(int2), s));
+    const int64_t rows = (int64_t)P->nmat * nc;
+    k_split_k<<<ceil_div((size_t)rows, 128), 128, 0, s>>>(P->Km.ptr, rows, nc, ldr, P->Kq.ptr,
+                                                          P->ke.ptr);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    ABX_CHECK_CUDA(cudaStreamSynchronize(s));  // the host lists end here
+  }
+  ABX_TRY(P->Wq.reserve((size_t)P->nnodes * nc));
+  ABX_TRY(P->we.reserve((size_t)P->nnodes));
+  k_split_w<<<ceil_div((size_t)P->nnodes * 32, 256), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, P->Wq.ptr,
+                                                                  P->we.ptr);
+  auto run = [&](auto kern, int tr) {
+    const dim3 grid(P->mf_tiles, (nc + tr - 1) / tr);
+    kern<<<grid, tr / 4 * (MF_P / 4), 0, s>>>(nc, ldr, P->Kq.ptr, P->ke.ptr, P->Wq.ptr, P->we.ptr,
+                                              P->m2l_by_mat.ptr, P->mat_off_d.ptr, P->mf_mat.ptr,
+                                              P->mf_first.ptr, P->G.ptr);
+  };
+  if (nc <= 32) run(k_m2l_fix<32, false>, 32);
+  else if (nc <= 64) run(k_m2l_fix<64, false>, 64);
+  else run(k_m2l_fix<64, true>, 64);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
@@ -1707,7 +1858,7 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
       }
       k_add_g32<<<ceil_div(tot, 256), 256, 0, s>>>(P->G32.ptr, P->nnodes, nc, ldg, P->G.ptr);
     } else {
-      k_m2l64<<<P->n_m2l, FT, 0, s>>>(nc, P->m2l.ptr, P->n_m2l, P->Km.ptr, P->W.ptr, P->G.ptr);
+      ABX_TRY(m2l_fix(P, s));
     }
     ABX_CHECK_CUDA(cudaGetLastError());
   }

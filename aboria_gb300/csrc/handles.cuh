@@ -62,7 +62,6 @@ struct OctDev {
 // matrix key (level, integer box offset), and the leaves' P2P sources.
 struct FmmLists {
   DevBuf<int2> m2l_by_mat;          // (target, source), grouped by matrix
-  DevBuf<int> m2l_trip;             // (target, source, matrix) in the same order
   DevBuf<int> p2p_rowptr, p2p_src;  // CSR over the leaves (creation order)
   std::vector<int> mat_off;         // nmat + 1
   std::vector<std::array<int, 4>> mat_key;  // level, offset (in boxes) per dimension

@@ -284,16 +284,13 @@ __global__ void k_code_to_mat(const uint32_t *__restrict__ code, int64_t npairs,
 
 __global__ void k_group_pairs(const int2 *__restrict__ pairs, const uint32_t *__restrict__ mat,
                               const uint32_t *__restrict__ order, int64_t npairs,
-                              int2 *__restrict__ bymat, int *__restrict__ trip,
+                              int2 *__restrict__ bymat,
                               uint32_t *__restrict__ mat_count) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= npairs) return;
   const int2 pr = pairs[order[k]];
   const uint32_t m = mat[k];
   bymat[k] = pr;
-  trip[3 * k] = pr.x;
-  trip[3 * k + 1] = pr.y;
-  trip[3 * k + 2] = (int)m;
   atomicAdd(&mat_count[m], 1u);
 }
 
@@ -543,12 +540,10 @@ int fmm_traverse_device(abx_particles *p, const double *boxes, double eta, FmmLi
     while (bits < 32 && ((nmat - 1) >> bits) != 0) ++bits;
     ABX_TRY(radix_sort_pairs(mat.ptr, iota.ptr, nm2l, bits, mat_alt.ptr, iota_alt.ptr, rtmp.ptr, s));
     ABX_TRY(out.m2l_by_mat.reserve(nm2l));
-    ABX_TRY(out.m2l_trip.reserve(3 * nm2l));
     ABX_TRY(cnt.reserve(nmat + 1));
     ABX_CHECK_CUDA(cudaMemsetAsync(cnt.ptr, 0, (size_t)(nmat + 1) * 4, s));
     k_group_pairs<<<ceil_div(nm2l, OT_TPB), OT_TPB, 0, s>>>(mpairs.ptr, mat.ptr, iota.ptr, nm2l,
-                                                           out.m2l_by_mat.ptr, out.m2l_trip.ptr,
-                                                           cnt.ptr);
+                                                           out.m2l_by_mat.ptr, cnt.ptr);
     ABX_CHECK_CUDA(cudaGetLastError());
     std::vector<uint32_t> hc(nmat);
     ABX_CHECK_CUDA(cudaMemcpyAsync(hc.data(), cnt.ptr, (size_t)nmat * 4, cudaMemcpyDeviceToHost, s));

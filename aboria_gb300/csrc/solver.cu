@@ -29,8 +29,12 @@
 #include <cmath>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "handles.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace abx {
 
@@ -248,78 +252,97 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // The same factorisation (partial pivoting, LAPACK's pivot convention) for
 // blocks of kernel values of one size (Gaussian, Wendland: at most 1, 1 on the
 // diagonal), where the trailing update, n^3 / 3 multiply-adds, need not run at 2
-// FP64 operations a clock and SM: the rows of L21 and the columns of U12 are
-// scaled by powers of two to 56-bit integers, x = (h 2^28 + l) 2^(e - 56) with
-// signed halves, and a product sum over up to 64 columns is two exact 64-bit
-// sums, hi += h h and mid += h l + l h: three 32x32+64 multiply-adds (58 a clock
-// and SM) for one FP64 multiply-add (1.8).  l l is below the scaled values' own
-// 2^-57.  The scale is the largest entry of the row (column), so a product's
-// error is 2^-56 of the largest product of its row and column, where FP64's
-// partial sums round at 2^-53 of themselves.
+// FP64 operations a clock and SM: the rows of L21 and the columns of U12 become
+// scaled 56-bit integers (fix64.cuh), and a multiply-add three 32x32+64 ones (25
+// a clock and SM with all operands in registers) instead of an FP64 one (1.8).
+// The scale is the largest entry of the row (column), so a product's error is
+// 2^-56 of the largest product of its row and column, where FP64's partial sums
+// round at 2^-53 of themselves.
 //
-// One CTA a domain, two to an SM.  What is left to the FP64 pipe sets the
+// A cluster of CTAs a domain (more, the fewer domains there are: the largest
+// domain's time is the kernel's), two to an SM.  The first factorises the panels;
+// columns and tiles are dealt to all.  What is left to the FP64 pipe sets the
 // blocking: panels of 16 columns are factorised in shared memory (the FP64 work
 // in a panel grows with its width); an update converts its sums and subtracts
 // them, two FP64 operations an entry, so the trailing matrix is updated for 64
 // columns at a time and only the rows and columns of those 64 panel by panel.
-// Pivots are compared as integers.  Blocks of more rows than the shared panel
-// holds keep k_lu_fp64.  256 domains of 703 rows on average (set-up and one
+// Pivots are compared as integers.  Blocks of more than FL_MAX rows keep k_lu_fp64.  256 domains of 703 rows on average (set-up and one
 // apply): 98 -> @LU_NEW@ ms.
 constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
 constexpr int FW = 16;         // panel width
 constexpr int FB = 64;         // columns of a trailing update
 constexpr int PLD = FW + 1;    // panel row stride
-constexpr int FL_MAX = 1600;   // rows of a block: 1600 * 17 * 8 B = 213 KB
+constexpr int FL_MAX = 1600;   // rows of a block (le, ue)
+// rows of a panel in shared memory, so that two CTAs share an SM (one leaves the
+// integer pipe waiting: 40 ms); the few rows of larger blocks stay in L2
+constexpr int FL_ROWS = 712;
 constexpr size_t FL_TILES = (size_t)FB * (64 + 64) * sizeof(int2);  // FB = 64 columns, 64 x 64
 static_assert(FL_TILES >= (size_t)FW * (256 + 16) * sizeof(int2), "tiles of one panel fit too");
 
-// x 2^(56 - e) as h 2^28 + l, |l| <= 2^27; |x| <= 2^e
 __device__ __forceinline__ int2 split56(double x, int e) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const int ex = (int)((u >> 52) & 0x7ff);
-  const unsigned long long m = (u & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
-  const int sh = (ex ? ex : 1) - 1075 + 56 - e;  // |x| 2^(56 - e) = m 2^sh, sh <= 4
-  long long f = sh >= 0 ? (long long)(m << sh)
-                        : (sh > -63 ? (long long)(((m >> (-sh - 1)) + 1) >> 1) : 0ll);
-  if (u >> 63) f = -f;
-  const int l = (int)((unsigned)f << 4) >> 4;  // the low 28 bits, signed
-  return make_int2((int)((f - l) >> 28), l);
+  const fx::Half2 q = fx::split56(x, e);
+  return make_int2(q.h, q.l);
 }
-__device__ __forceinline__ unsigned long long abs_bits(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
-}
-// e with |x| <= 2^e from the bits of the largest |x|
-__device__ __forceinline__ short scale_exp(unsigned long long maxbits) {
-  return (short)((int)(maxbits >> 52) - 1022);
+using fx::abs_bits;
+using fx::scale_exp;
+
+// COUNT values per thread of a tile, read in one go (the reads' latency, not
+// their number, is what they cost) and split into (h, l).
+template <int COUNT, class Read, class Write>
+__device__ __forceinline__ void stage_split(Read read, Write write) {
+  constexpr int U = COUNT < 8 ? COUNT : 8;
+  for (int q0 = 0; q0 < COUNT; q0 += U) {
+    double v[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) v[q] = read(q0 + q);
+#pragma unroll
+    for (int q = 0; q < U; ++q) write(q0 + q, v[q]);
+  }
 }
 
-// A[r0.., c0..] -= L[r0.., k0..k0+kw) U[k0.., c0..) for rows below r1 and
-// columns below c1, tiles of TR x TC, kw <= FB; le, ue: the exponents of L's rows
-// and U's columns.  Whole CTA; barriers at the start of every tile.
-template <int TR, int TC>
+// A[r0.., c0..] -= L[r0.., k0..k0+KW) U[k0.., c0..) for rows below r1 and
+// columns below c1, tiles of TR x TC dealt to the cluster's CTAs; le, ue: the
+// exponents of L's rows and U's columns.  Whole CTA; barriers at the start of
+// every tile.
+template <int TR, int TC, int KW>
 __device__ __noinline__ void update_fix(double *A, int n, int r0, int r1, int c0, int c1, int k0,
-                                           int kw, const short *le, const short *ue, int2 *tiles) {
+                                        const short *le, const short *ue, int2 *tiles, int rank,
+                                        int ranks) {
   static_assert((TR / 4) * (TC / 4) == FL_T, "one 4 x 4 piece a thread");
   const int tid = threadIdx.x;
-  int2 *L = tiles, *U = tiles + kw * TR;  // [k][row], [k][column]
+  int2 *L = tiles, *U = tiles + KW * TR;  // [k][row], [k][column]
   const int tr = (tid % (TR / 4)) * 4, tc = (tid / (TR / 4)) * 4;
-  for (int ti = r0; ti < r1; ti += TR) {
-    for (int tj = c0; tj < c1; tj += TC) {
+  const int nti = (r1 - r0 + TR - 1) / TR, ntj = (c1 - c0 + TC - 1) / TC;
+  int have = -1;  // row tile in L
+  {
+    for (int t = rank; t < nti * ntj; t += ranks) {
+      const int ti = r0 + (t / ntj) * TR, tj = c0 + (t % ntj) * TC;
       __syncthreads();
-      if (tj == c0)
-        for (int e = tid; e < kw * TR; e += FL_T) {
-          const int r = e % TR, k = e / TR;
-          L[k * TR + r] = ti + r < r1 ? split56(M(A, n, ti + r, k0 + k), le[ti + r]) : make_int2(0, 0);
-        }
-      for (int e = tid; e < kw * TC; e += FL_T) {
-        const int k = e % kw, j = e / kw;
-        U[k * TC + j] = tj + j < c1 ? split56(M(A, n, k0 + k, tj + j), ue[tj + j]) : make_int2(0, 0);
-      }
+      if (ti != have)
+        stage_split<KW * TR / FL_T>(
+            [&](int q) {
+              const int e = tid + q * FL_T, r = e % TR, k = e / TR;
+              return ti + r < r1 ? M(A, n, ti + r, k0 + k) : 0.0;
+            },
+            [&](int q, double v) {
+              const int e = tid + q * FL_T, r = e % TR, k = e / TR;
+              L[k * TR + r] = split56(v, ti + r < r1 ? le[ti + r] : 0);
+            });
+      stage_split<KW * TC / FL_T>(
+          [&](int q) {
+            const int e = tid + q * FL_T, k = e % KW, j = e / KW;
+            return tj + j < c1 ? M(A, n, k0 + k, tj + j) : 0.0;
+          },
+          [&](int q, double v) {
+            const int e = tid + q * FL_T, k = e % KW, j = e / KW;
+            U[k * TC + j] = split56(v, tj + j < c1 ? ue[tj + j] : 0);
+          });
+      have = ti;
       __syncthreads();
       if (ti + tr >= r1 || tj + tc >= c1) continue;
       long long hi[4][4] = {}, mid[4][4] = {};
 #pragma unroll 2
-      for (int k = 0; k < kw; ++k) {
+      for (int k = 0; k < KW; ++k) {
         int2 a[4], b[4];
         *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&L[k * TR + tr]);
         *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&L[k * TR + tr + 2]);
@@ -328,25 +351,31 @@ __device__ __noinline__ void update_fix(double *A, int n, int r0, int r1, int c0
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            hi[i][j] += (long long)a[i].x * b[j].x;
-            mid[i][j] += (long long)a[i].x * b[j].y;
-            mid[i][j] += (long long)a[i].y * b[j].x;
-          }
+          for (int j = 0; j < 4; ++j) mid[i][j] += (long long)a[i].x * b[j].y;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) hi[i][j] += (long long)a[i].x * b[j].x;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) mid[i][j] += (long long)a[i].y * b[j].x;
       }
+      double v[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          v[i][j] = ti + tr + i < r1 && tj + tc + j < c1 ? M(A, n, ti + tr + i, tj + tc + j) : 0.0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int cj = tj + tc + j;
-        if (cj >= c1) continue;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int ri = ti + tr + i;
-          if (ri >= r1) continue;
-          // (hi 2^56 + mid 2^28) 2^(le - 56) 2^(ue - 56)
-          const long long t = hi[i][j] + ((mid[i][j] + (1ll << 27)) >> 28);
-          const int ex = max((int)le[ri] + (int)ue[cj] - 56 + 1023, 1);
-          const double sc = __longlong_as_double((long long)ex << 52);
-          M(A, n, ri, cj) = fma(-(double)t, sc, M(A, n, ri, cj));
+          if (ri >= r1 || cj >= c1) continue;
+          const double sc = fx::scale56((int)le[ri] + (int)ue[cj]);
+          M(A, n, ri, cj) = fma(-(double)fx::sum56(hi[i][j], mid[i][j]), sc, v[i][j]);
         }
       }
     }
@@ -370,7 +399,7 @@ __device__ __noinline__ short solve_unit_lower(double *col, const double (*L)[FW
   double x[FW];
 #pragma unroll
   for (int c = 0; c < FW; ++c) x[c] = col[c];
-  unsigned long long mx = 0;
+  fx::u64 mx = 0;
 #pragma unroll
   for (int c = 0; c < FW; ++c) {
     mx = max(mx, abs_bits(x[c]));
@@ -378,143 +407,169 @@ __device__ __noinline__ short solve_unit_lower(double *col, const double (*L)[FW
     for (int q = c + 1; q < FW; ++q) x[q] = fma(-L[q][c], x[c], x[q]);
     col[c] = x[c];
   }
-  return scale_exp(mx);
+  return (short)scale_exp(mx);
 }
 
 __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
                                                     const int64_t *__restrict__ dom_mat,
                                                     const int *__restrict__ dom_size,
                                                     const int *__restrict__ dom_off,
-                                                    int *__restrict__ piv, int *__restrict__ info) {
+                                                    int *__restrict__ piv, int *__restrict__ info,
+                                                    short *__restrict__ exps, int64_t nexp) {
   extern __shared__ __align__(16) unsigned char lu_raw[];
   double *Pn = reinterpret_cast<double *>(lu_raw);  // panel: rows k0..n-1 x FW, stride PLD
   int2 *tiles = reinterpret_cast<int2 *>(lu_raw);
-  __shared__ unsigned long long red_v[FL_T / 32];
+  __shared__ fx::u64 red_v[FL_T / 32];
   __shared__ int red_i[FL_T / 32];
   __shared__ double L11[FB / FW][FW][FW + 1];
   __shared__ int swaps[FB];
-  __shared__ short le[FL_MAX], ue[FL_MAX];  // exponents of L's rows, of U's columns
-  const int d = blockIdx.x;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), ranks = (int)cl.num_blocks();
+  const int d = blockIdx.x / ranks;
   const int n = dom_size[d];
   if (n > FL_MAX) return;  // k_lu_fp64's
   double *A = mat + dom_mat[d];
   int *pv = piv + dom_off[d];
+  short *le = exps + dom_off[d], *ue = le + nexp;  // exponents of L's rows, of U's columns
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int status = 0;
   for (int B0 = 0; B0 < n; B0 += FB) {
     const int B1 = min(B0 + FB, n);
     for (int k0 = B0; k0 < B1; k0 += FW) {
       const int kw = min(FW, n - k0), k1 = k0 + kw, rows = n - k0;
-      // ---- the panel, in shared memory
-      for (int c = warp; c < kw; c += FL_T / 32)
-        for (int r = lane; r < rows; r += 32) Pn[r * PLD + c] = M(A, n, k0 + r, k0 + c);
-      __syncthreads();
-      for (int c = 0; c < kw; ++c) {
-        // pivot: the first row of largest |entry| at or below the diagonal
-        unsigned long long best = 0;
-        int bi = 0x7fffffff;
-        for (int r = c + tid; r < rows; r += FL_T) {
-          const unsigned long long v = abs_bits(Pn[r * PLD + c]);
-          if (v > best || bi == 0x7fffffff) { best = v; bi = r; }
-        }
-        {
-          const unsigned h = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
-          const bool top = (unsigned)(best >> 32) == h;
-          const unsigned l = __reduce_max_sync(0xffffffffu, top ? (unsigned)best : 0u);
-          const unsigned i = __reduce_min_sync(
-              0xffffffffu, top && (unsigned)best == l ? (unsigned)bi : 0x7fffffffu);
-          if (lane == 0) {
-            red_v[warp] = ((unsigned long long)h << 32) | l;
-            red_i[warp] = (int)i;
+      if (rank == 0) {
+        // ---- the panel: its rows in shared memory, or where they are
+        auto row = [&](int r, int &step) -> double * {
+          step = r < FL_ROWS ? 1 : n;
+          return r < FL_ROWS ? Pn + r * PLD : A + (int64_t)k0 * n + k0 + r;
+        };
+        int st;
+        for (int c = warp; c < kw; c += FL_T / 32)
+          for (int r = lane; r < min(rows, FL_ROWS); r += 32)
+            Pn[r * PLD + c] = M(A, n, k0 + r, k0 + c);
+        __syncthreads();
+        for (int c = 0; c < kw; ++c) {
+          // pivot: the first row of largest |entry| at or below the diagonal
+          fx::u64 best = 0;
+          int bi = 0x7fffffff;
+          for (int r = c + tid; r < rows; r += FL_T) {
+            const double *pr = row(r, st);
+            const fx::u64 v = abs_bits(pr[(int64_t)c * st]);
+            if (v > best || bi == 0x7fffffff) { best = v; bi = r; }
           }
+          {
+            const unsigned h = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+            const bool top = (unsigned)(best >> 32) == h;
+            const unsigned l = __reduce_max_sync(0xffffffffu, top ? (unsigned)best : 0u);
+            const unsigned i = __reduce_min_sync(
+                0xffffffffu, top && (unsigned)best == l ? (unsigned)bi : 0x7fffffffu);
+            if (lane == 0) {
+              red_v[warp] = fx::join(h, l);
+              red_i[warp] = (int)i;
+            }
+          }
+          __syncthreads();
+          best = red_v[0];
+          bi = red_i[0];
+          for (int w = 1; w < FL_T / 32; ++w)
+            if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) { best = red_v[w]; bi = red_i[w]; }
+          if (tid == 0) {
+            pv[k0 + c] = k0 + bi;
+            if (best == 0 && status == 0) status = k0 + c + 1;
+          }
+          if (bi != c && tid < kw) {
+            double *pr = row(bi, st);
+            const double t = Pn[c * PLD + tid];
+            Pn[c * PLD + tid] = pr[(int64_t)tid * st];
+            pr[(int64_t)tid * st] = t;
+          }
+          __syncthreads();
+          const double dpiv = Pn[c * PLD + c];
+          // 1 / pivot: Newton steps from the FP32 reciprocal (4 FP64 operations)
+          double inv;
+          if (fabs(dpiv) > 1e-30 && fabs(dpiv) < 1e30) {
+            inv = (double)fx::rcp32((float)dpiv);
+            inv = fma(fma(-dpiv, inv, 1.0), inv, inv);
+            inv = fma(fma(-dpiv, inv, 1.0), inv, inv);
+          } else {
+            inv = dpiv != 0.0 ? 1.0 / dpiv : 0.0;
+          }
+          for (int r = c + 1 + tid; r < rows; r += FL_T) {
+            double *pr = row(r, st);
+            const double l = pr[(int64_t)c * st] * inv;
+            pr[(int64_t)c * st] = l;
+            for (int cc = c + 1; cc < kw; ++cc)
+              pr[(int64_t)cc * st] = fma(-l, Pn[c * PLD + cc], pr[(int64_t)cc * st]);
+          }
+          __syncthreads();
         }
-        __syncthreads();
-        best = red_v[0];
-        bi = red_i[0];
-        for (int w = 1; w < FL_T / 32; ++w)
-          if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) { best = red_v[w]; bi = red_i[w]; }
-        if (tid == 0) {
-          swaps[k0 - B0 + c] = k0 + bi;
-          pv[k0 + c] = k0 + bi;
-          if (best == 0 && status == 0) status = k0 + c + 1;
+        // scale of every row below the diagonal block; the panel back to the matrix
+        for (int r = kw + tid; r < rows; r += FL_T) {
+          fx::u64 mx = 0;
+          const double *pr = row(r, st);
+          for (int c = 0; c < kw; ++c) mx = max(mx, abs_bits(pr[(int64_t)c * st]));
+          le[k0 + r] = (short)scale_exp(mx);
         }
-        if (bi != c && tid < kw) {
-          const double t = Pn[c * PLD + tid];
-          Pn[c * PLD + tid] = Pn[bi * PLD + tid];
-          Pn[bi * PLD + tid] = t;
-        }
-        __syncthreads();
-        const double dpiv = Pn[c * PLD + c];
-        // 1 / pivot: Newton steps from the FP32 reciprocal (4 FP64 operations)
-        double inv;
-        if (fabs(dpiv) > 1e-30 && fabs(dpiv) < 1e30) {
-          inv = (double)fx::rcp32((float)dpiv);
-          inv = fma(fma(-dpiv, inv, 1.0), inv, inv);
-          inv = fma(fma(-dpiv, inv, 1.0), inv, inv);
-        } else {
-          inv = dpiv != 0.0 ? 1.0 / dpiv : 0.0;
-        }
-        for (int r = c + 1 + tid; r < rows; r += FL_T) {
-          const double l = Pn[r * PLD + c] * inv;
-          Pn[r * PLD + c] = l;
-          for (int cc = c + 1; cc < kw; ++cc)
-            Pn[r * PLD + cc] = fma(-l, Pn[c * PLD + cc], Pn[r * PLD + cc]);
-        }
-        __syncthreads();
+        for (int c = warp; c < kw; c += FL_T / 32)
+          for (int r = lane; r < min(rows, FL_ROWS); r += 32)
+            M(A, n, k0 + r, k0 + c) = Pn[r * PLD + c];
       }
+      cl.sync();
       const int s = (k0 - B0) / FW;
       for (int e = tid; e < kw * kw; e += FL_T)
-        L11[s][e / kw][e % kw] = Pn[(e / kw) * PLD + e % kw];
-      // scale of every row below the diagonal block; the panel back to the matrix
-      for (int r = kw + tid; r < rows; r += FL_T) {
-        unsigned long long mx = 0;
-        for (int c = 0; c < kw; ++c) mx = max(mx, abs_bits(Pn[r * PLD + c]));
-        le[k0 + r] = scale_exp(mx);
-      }
-      for (int c = warp; c < kw; c += FL_T / 32)
-        for (int r = lane; r < rows; r += 32) M(A, n, k0 + r, k0 + c) = Pn[r * PLD + c];
+        L11[s][e / kw][e % kw] = M(A, n, k0 + e / kw, k0 + e % kw);
+      for (int c = tid; c < kw; c += FL_T) swaps[k0 - B0 + c] = pv[k0 + c];
       __syncthreads();
       // ---- the other columns up to B1: row swaps; right of the panel U12 =
       // L11^{-1} A12 (a panel with columns to its right has all its FW columns),
       // and the rows below.  Columns beyond B1 wait: a later panel's pivot may
       // bring up a row that has not had this panel's update.
-      for (int j = tid; j < B1; j += FL_T) {
+      for (int j = rank * FL_T + tid; j < B1; j += ranks * FL_T) {
         if (j >= k0 && j < k1) continue;
         double *col = A + (int64_t)j * n;
         swap_rows(col, k0, kw, swaps + (k0 - B0));
         if (j >= k1) ue[j] = solve_unit_lower(col + k0, L11[s]);
       }
-      __syncthreads();
-      if (k1 < B1) update_fix<256, 16>(A, n, k1, n, k1, B1, k0, kw, le, ue, tiles);
+      cl.sync();
+      if (k1 < B1) {
+        update_fix<256, 16, FW>(A, n, k1, n, k1, B1, k0, le, ue, tiles, rank, ranks);
+        cl.sync();
+      }
     }
     if (B1 >= n) break;
     // ---- the block row right of B1, panel by panel
-    for (int j = B1 + tid; j < n; j += FL_T) swap_rows(A + (int64_t)j * n, B0, FB, swaps);
+    for (int j = B1 + rank * FL_T + tid; j < n; j += ranks * FL_T)
+      swap_rows(A + (int64_t)j * n, B0, FB, swaps);
     for (int k0 = B0; k0 < B1; k0 += FW) {
       const int k1 = k0 + FW;
-      for (int j = B1 + tid; j < n; j += FL_T)
+      for (int j = B1 + rank * FL_T + tid; j < n; j += ranks * FL_T)
         ue[j] = solve_unit_lower(A + (int64_t)j * n + k0, L11[(k0 - B0) / FW]);
-      for (int r = k1 + tid; r < B1; r += FL_T) {
-        unsigned long long mx = 0;
+      for (int r = k1 + rank * FL_T + tid; r < B1; r += ranks * FL_T) {
+        fx::u64 mx = 0;
         for (int k = k0; k < k1; ++k) mx = max(mx, abs_bits(M(A, n, r, k)));
-        le[r] = scale_exp(mx);
+        le[r] = (short)scale_exp(mx);
       }
-      __syncthreads();
-      if (k1 < B1) update_fix<16, 256>(A, n, k1, B1, B1, n, k0, FW, le, ue, tiles);
+      cl.sync();
+      if (k1 < B1) {
+        update_fix<16, 256, FW>(A, n, k1, B1, B1, n, k0, le, ue, tiles, rank, ranks);
+        cl.sync();
+      }
     }
     // ---- the trailing matrix, for all FB columns
-    for (int r = B1 + tid; r < n; r += FL_T) {
-      unsigned long long ml = 0, mu = 0;
+    for (int r = B1 + rank * FL_T + tid; r < n; r += ranks * FL_T) {
+      fx::u64 ml = 0, mu = 0;
       for (int k = B0; k < B1; ++k) {
         ml = max(ml, abs_bits(M(A, n, r, k)));
         mu = max(mu, abs_bits(M(A, n, k, r)));
       }
-      le[r] = scale_exp(ml);
-      ue[r] = scale_exp(mu);
+      le[r] = (short)scale_exp(ml);
+      ue[r] = (short)scale_exp(mu);
     }
-    update_fix<64, 64>(A, n, B1, n, B1, n, B0, FB, le, ue, tiles);
+    cl.sync();
+    update_fix<64, 64, FB>(A, n, B1, n, B1, n, B0, le, ue, tiles, rank, ranks);
+    cl.sync();
   }
-  if (tid == 0) info[d] = status;
+  if (rank == 0 && tid == 0) info[d] = status;
 }
 
 __global__ void k_to_f32(const double *__restrict__ a, int64_t n, float *__restrict__ b) {
@@ -786,14 +841,33 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
     const bool flat = op->k.kind == ABX_K_GAUSSIAN || op->k.kind == ABX_K_COMPACT_GAUSSIAN ||
                       op->k.kind == ABX_K_WENDLAND_C2;
     if (flat) {
-      const size_t smem = std::max(FL_TILES, (size_t)std::min(S->max_size, FL_MAX) * PLD * 8);
-      if (cudaFuncSetAttribute(k_lu_fix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess) {
-        set_error("LU: %zu bytes of shared memory refused", smem);
+      const size_t smem = std::max(FL_TILES, (size_t)std::min(S->max_size, FL_ROWS) * PLD * 8);
+      // CTAs a domain: enough for two on every SM, 8 at most
+      int ranks = 1;
+      while (ranks < 8 && S->ndom * ranks * 2 <= 4 * ctx->num_sms) ranks *= 2;
+      DevBuf<short> exps;
+      if ((st = exps.reserve(2 * (idx.size() + 1)))) return fail(st);
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim = {(unsigned)ranks, 1, 1};
+      cfg.gridDim = dim3((unsigned)(S->ndom * ranks));
+      cfg.blockDim = dim3(FL_T);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = s;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      cudaError_t le = cudaFuncSetAttribute(k_lu_fix, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)smem);
+      if (le == cudaSuccess)
+        le = cudaLaunchKernelEx(&cfg, k_lu_fix, S->mat.ptr, (const int64_t *)S->dom_mat.ptr,
+                                (const int *)S->dom_size.ptr, (const int *)S->dom_off.ptr, S->piv.ptr,
+                                S->info.ptr, exps.ptr, (int64_t)(idx.size() + 1));
+      if (le != cudaSuccess) {
+        set_error("LU launch: %s", cudaGetErrorString(le));
         return fail(ABX_ERR_CUDA);
       }
-      k_lu_fix<<<S->ndom, FL_T, smem, s>>>(S->mat.ptr, S->dom_mat.ptr, S->dom_size.ptr,
-                                           S->dom_off.ptr, S->piv.ptr, S->info.ptr);
+      // (exps is freed once the kernel is done: cudaFree waits)
     }
     if (!flat || S->max_size > FL_MAX)
       k_lu_fp64<<<S->ndom, LU_T, 0, s>>>(S->mat.ptr, S->dom_mat.ptr, S->dom_size.ptr,
