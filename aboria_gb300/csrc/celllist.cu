@@ -61,11 +61,12 @@ constexpr uint64_t ST_AGG = 1ull << 32, ST_INCL = 2ull << 32;
 constexpr int CL_HIST_COPIES = 32;  // spread of the keys kernel's histogram atomics
 
 struct ClHeader {
-  uint32_t hist[CL_MAX_PASSES][CL_RADIX];
-  uint32_t tile_counter[CL_MAX_PASSES];
   uint32_t dead;
   uint32_t error;  // 1: a look-back wait gave up; 2: a periodic wrap did not end
   uint32_t blocks_done;
+  uint32_t tile_counter[CL_MAX_PASSES];
+  // the few-launch sort of small sets uses nothing below
+  uint32_t hist[CL_MAX_PASSES][CL_RADIX];
   // per-block histograms land in one of CL_HIST_COPIES copies (few blocks
   // share a counter), the last block to finish sums them into hist
   uint32_t part[CL_HIST_COPIES][CL_MAX_PASSES][CL_RADIX];
@@ -120,7 +121,8 @@ __device__ __forceinline__ uint32_t cell_coord(uint64_t u, int d, const ClParams
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(CL_TPB) k_cl_keys(double *__restrict__ pos, int64_t n, ClParams P,
+__global__ void __launch_bounds__(CL_TPB) k_cl_keys(double *__restrict__ pos, int64_t n, int tile,
+                                                    ClParams P,
                                                     uint32_t *__restrict__ keys,
                                                     ClHeader *__restrict__ H) {
   __shared__ uint32_t h[CL_MAX_PASSES][CL_RADIX];
@@ -134,11 +136,10 @@ __global__ void __launch_bounds__(CL_TPB) k_cl_keys(double *__restrict__ pos, in
   __syncthreads();
   const uint64_t *tab = shared_tab ? sbnd : P.bnd_all;
   uint32_t dead = 0, err = 0;
-  for (int64_t base = (int64_t)blockIdx.x * CL_KEYS_TILE; base < n;
-       base += (int64_t)gridDim.x * CL_KEYS_TILE) {
+  for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
     constexpr int U = 4;  // particles per thread with their loads in flight together
 #pragma unroll 1
-    for (int it0 = 0; it0 < CL_KEYS_TILE / CL_TPB; it0 += U) {
+    for (int it0 = 0; it0 < tile / CL_TPB; it0 += U) {
       double rr[U][DIM];
 #pragma unroll
       for (int j = 0; j < U; ++j) {
@@ -219,8 +220,7 @@ __global__ void __launch_bounds__(CL_TPB) k_cl_keys(double *__restrict__ pos, in
             ++dead;
           }
           keys[i] = key;
-          atomicAdd(&h[0][key & (CL_RADIX - 1)], 1u);
-          for (int p = 1; p < P.npasses; ++p) atomicAdd(&h[p][(key >> (CL_RB * p)) & (CL_RADIX - 1)], 1u);
+          for (int p = 0; p < P.npasses; ++p) atomicAdd(&h[p][(key >> (CL_RB * p)) & (CL_RADIX - 1)], 1u);
         }
       }
     }
@@ -230,6 +230,10 @@ __global__ void __launch_bounds__(CL_TPB) k_cl_keys(double *__restrict__ pos, in
   for (int o = 16; o > 0; o >>= 1) dead += __shfl_xor_sync(0xffffffffu, dead, o);
   if ((threadIdx.x & 31) == 0 && dead) atomicAdd(&sdead, dead);
   __syncthreads();
+  if (P.npasses == 0) {  // no digit counts wanted
+    if (threadIdx.x == 0 && sdead) atomicAdd(&H->dead, sdead);
+    return;
+  }
   uint32_t *part = &H->part[blockIdx.x % CL_HIST_COPIES][0][0];
   for (int i = threadIdx.x; i < P.npasses * CL_RADIX; i += CL_TPB) {
     const uint32_t c = (&h[0][0])[i];
@@ -533,6 +537,13 @@ int run_build(abx_particles *p, const GridDesc &g, uint32_t *dead_out) {
   while (bits < 32 && ((uint64_t)P.dead_key >> bits) != 0) ++bits;
   P.npasses = (bits + CL_RB - 1) / CL_RB;
   if (P.npasses < 1) P.npasses = 1;
+  // Small sets: the sort of primitives.cu, with tiles of 2,048 to 4,096 keys (one
+  // launch up to 4,096 keys, two a pass beyond).  The look-back sort's tiles of
+  // 16,384 keys pay off once they fill the SMs; with 7 of them (N = 100,000)
+  // its passes took 65 us, and the digit counts of the keys kernel 15 more.
+  // Both sorts are stable: the same order.
+  const bool few = radix_few_tiles((size_t)n);
+  if (few) P.npasses = 0;
   for (int d = 0; d < 3; ++d) {
     P.size[d] = g.size[d];
     P.lo[d] = g.lo[d];
@@ -573,6 +584,8 @@ int run_build(abx_particles *p, const GridDesc &g, uint32_t *dead_out) {
   carve_size<uint32_t>(o, n);
   carve_size<uint32_t>(o, n);
   carve_size<uint32_t>(o, n);
+  const size_t sort_tmp = few ? radix_temp_u32((size_t)n) : 0;
+  carve_size<uint32_t>(o, sort_tmp);
   ABX_TRY(ctx->scratch.reserve(o + 256));
   unsigned char *sb = ctx->scratch.ptr;
   o = 0;
@@ -580,25 +593,34 @@ int run_build(abx_particles *p, const GridDesc &g, uint32_t *dead_out) {
   uint32_t *vals = carve<uint32_t>(sb, o, n);
   uint32_t *keys_alt = carve<uint32_t>(sb, o, n);
   uint32_t *vals_alt = carve<uint32_t>(sb, o, n);
+  uint32_t *tmp = carve<uint32_t>(sb, o, sort_tmp);
   ABX_TRY(p->keys.reserve(n));
-  const size_t nstatus = (size_t)ntiles * CL_RADIX;
+  const size_t nstatus = few ? 0 : (size_t)ntiles * CL_RADIX;
   if (p->cl_status.cap < nstatus) {
     ABX_TRY(p->cl_status.reserve(nstatus));
     ABX_CHECK_CUDA(cudaMemsetAsync(p->cl_status.ptr, 0, nstatus * 8, s));
   }
-  ABX_CHECK_CUDA(cudaMemsetAsync(H, 0, sizeof(ClHeader), s));
+  ABX_CHECK_CUDA(cudaMemsetAsync(H, 0, few ? offsetof(ClHeader, hist) : sizeof(ClHeader), s));
   ABX_CHECK_CUDA(cudaFuncSetAttribute(k_cl_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)sizeof(SweepSmem)));
-  const int kblocks = (int)std::min<int64_t>((n + CL_KEYS_TILE - 1) / CL_KEYS_TILE,
-                                             (int64_t)ctx->num_sms * 4);
+  const int tile = few ? CL_KEYS_TILE / 4 : CL_KEYS_TILE;
+  const int kblocks = (int)std::min<int64_t>((n + tile - 1) / tile, (int64_t)ctx->num_sms * 4);
   if (D == 1)
-    k_cl_keys<1><<<kblocks, CL_TPB, keys_smem, s>>>(p->pos.ptr, n, P, p->keys.ptr, H);
+    k_cl_keys<1><<<kblocks, CL_TPB, keys_smem, s>>>(p->pos.ptr, n, tile, P, p->keys.ptr, H);
   else if (D == 2)
-    k_cl_keys<2><<<kblocks, CL_TPB, keys_smem, s>>>(p->pos.ptr, n, P, p->keys.ptr, H);
+    k_cl_keys<2><<<kblocks, CL_TPB, keys_smem, s>>>(p->pos.ptr, n, tile, P, p->keys.ptr, H);
   else
-    k_cl_keys<3><<<kblocks, CL_TPB, keys_smem, s>>>(p->pos.ptr, n, P, p->keys.ptr, H);
+    k_cl_keys<3><<<kblocks, CL_TPB, keys_smem, s>>>(p->pos.ptr, n, tile, P, p->keys.ptr, H);
   ABX_CHECK_CUDA(cudaGetLastError());
   uint32_t *ki = p->keys.ptr, *vi = nullptr, *ko = keys_alt, *vo = vals;
+  if (few) {
+    SortSides S{};
+    S.sides = 1;
+    S.iota = true;
+    S.s[0] = SortSide{p->keys.ptr, vals, keys_alt, vals_alt, tmp, (size_t)n};
+    ABX_TRY(radix_sort_sides(S, bits, s));
+    vi = vals;
+  }
   for (int pass = 0; pass < P.npasses; ++pass) {
     p->cl_epoch = (p->cl_epoch + 1) & 0x3fffffffu;
     if (p->cl_epoch == 0) p->cl_epoch = 1;

@@ -151,5 +151,19 @@ size_t radix_temp_u32(size_t n);
 int radix_sort_pairs(uint32_t *keys, uint32_t *vals, size_t n, int bits,
                      uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *temp,
                      cudaStream_t s);
+// The same sort of up to two independent sets in the same launches (while they
+// are small); iota: the values are the input positions, `vals` need not be set.
+struct SortSide {
+  uint32_t *keys, *vals, *keys_alt, *vals_alt, *temp;
+  size_t n;
+};
+struct SortSides {
+  SortSide s[2];
+  int sides;
+  bool iota;
+};
+int radix_sort_sides(SortSides S, int bits, cudaStream_t s);
+// radix_sort_sides takes its few-launch path for n items (262,144 x 2 at most).
+bool radix_few_tiles(size_t n);
 
 }  // namespace abx

@@ -214,8 +214,24 @@ __device__ __forceinline__ int fine_coord(double x, double lo, double inv) {
 // Sort key of a point: clamped fine cell (row-major, e2 fastest) times 8 plus
 // its octant within the cell, so that consecutive points of a dense cell are
 // also close together (tighter query tiles).
-__global__ void k_fine_keys(const double *__restrict__ src, int64_t n, int64_t stride, FineGrid fg,
-                            uint32_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+// blockIdx.y: the set (particles, queries).
+struct PointSet {
+  const double *src;  // SoA
+  int64_t n, stride;
+  int clamp;  // anchor cells clamped to the grid (k_fill_layout)
+  uint32_t *keys;
+  const uint32_t *perm;
+  int4 *cell;
+  float4 *loc;
+  D4 *posk;
+};
+struct PointSets {
+  PointSet s[2];
+};
+__global__ void k_fine_keys(PointSets sets, FineGrid fg) {
+  const PointSet &S = sets.s[blockIdx.y];
+  const double *__restrict__ src = S.src;
+  const int64_t n = S.n, stride = S.stride;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int c[3];
@@ -232,8 +248,7 @@ __global__ void k_fine_keys(const double *__restrict__ src, int64_t n, int64_t s
     const double f = x - (fg.lo[e] + (double)c[e] * fg.h[e]);
     sub |= (f >= 0.5 * fg.h[e] ? 1u : 0u) << (2 - e);
   }
-  keys[i] = ((((uint32_t)c[0] * fg.m[1] + c[1]) * fg.m[2] + c[2]) << 3) | sub;
-  vals[i] = (uint32_t)i;
+  S.keys[i] = ((((uint32_t)c[0] * fg.m[1] + c[1]) * fg.m[2] + c[2]) << 3) | sub;
 }
 
 // Anchor cell of a point: the clamped cell for column particles (their range
@@ -241,13 +256,13 @@ __global__ void k_fine_keys(const double *__restrict__ src, int64_t n, int64_t s
 // the domain and must keep their true periodic image).  loc holds the FP32
 // offset from the anchor cell's corner and, in .w, the anchor's e2 index as
 // an (exact) float.
-__global__ void k_fill_layout(const double *__restrict__ src, int64_t stride, FineGrid fg,
-                              const uint32_t *__restrict__ perm, int64_t n, int clamp_anchor,
-                              int4 *__restrict__ cell, float4 *__restrict__ loc,
-                              D4 *__restrict__ posk) {
+__global__ void k_fill_layout(PointSets sets, FineGrid fg) {
+  const PointSet &S = sets.s[blockIdx.y];
+  const double *__restrict__ src = S.src;
+  const int64_t stride = S.stride;
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const uint32_t i = perm[k];
+  if (k >= S.n) return;
+  const uint32_t i = S.perm[k];
   double x[3];
   int u[3], c[3];
   float f[3];
@@ -262,13 +277,13 @@ __global__ void k_fill_layout(const double *__restrict__ src, int64_t stride, Fi
     }
     x[e] = src[(int64_t)d * stride + i];
     u[e] = fine_coord(x[e], fg.lo[e], fg.inv[e]);
-    c[e] = clamp_anchor ? min(max(u[e], 0), fg.m[e] - 1) : u[e];
+    c[e] = S.clamp ? min(max(u[e], 0), fg.m[e] - 1) : u[e];
     const double corner = fg.lo[e] + (double)c[e] * fg.h[e];
     f[e] = (float)(x[e] - corner);
   }
-  cell[k] = make_int4(c[0], c[1], c[2], 0);
-  loc[k] = make_float4(f[0], f[1], f[2], (float)c[2]);  // exact: c[2] < 2^24
-  posk[k] = D4{x[0], x[1], x[2], 0.0};
+  S.cell[k] = make_int4(c[0], c[1], c[2], 0);
+  S.loc[k] = make_float4(f[0], f[1], f[2], (float)c[2]);  // exact: c[2] < 2^24
+  S.posk[k] = D4{x[0], x[1], x[2], 0.0};
 }
 
 // First index of keys[0, n) whose value is >= key, by a 32-way search (whole
@@ -325,27 +340,42 @@ __global__ void k_fill_fixed(const D4 *__restrict__ posk, int64_t n, fx::Unit U,
   fz[k] = fx::to_fixed(x.z, U.f, U.k);
 }
 
-int build_points(abx_context *ctx, const double *src_soa, int64_t n, int64_t stride,
-                 const FineGrid &fg, bool clamp_anchor, PointLayout &P) {
-  cudaStream_t s = ctx->stream;
+int reserve_points(int64_t n, const double *src_soa, int64_t stride, bool clamp_anchor,
+                   PointLayout &P, PointSet &S) {
   P.n = n;
   ABX_TRY(P.perm.reserve(n ? n : 1));
   ABX_TRY(P.keys.reserve(n ? n : 1));
   ABX_TRY(P.cell.reserve(n ? n : 1));
   ABX_TRY(P.loc.reserve(n ? n : 1));
   ABX_TRY(P.posk.reserve(n ? n : 1));
-  if (n == 0) return ABX_OK;
-  const size_t rt = radix_temp_u32(n);
-  ABX_TRY(P.tmp.reserve(2 * (size_t)n + rt + 64));
-  k_fine_keys<<<ceil_div(n, TPB), TPB, 0, s>>>(src_soa, n, stride, fg, P.keys.ptr, P.perm.ptr);
+  if (n) ABX_TRY(P.tmp.reserve(2 * (size_t)n + radix_temp_u32(n) + 64));
+  S = PointSet{src_soa,    n,          stride,    clamp_anchor ? 1 : 0, P.keys.ptr,
+               P.perm.ptr, P.cell.ptr, P.loc.ptr, P.posk.ptr};
+  return ABX_OK;
+}
+
+// Kernel order of the particles and (rows) of the queries, which go through
+// each launch together: at 100,000 each, separately, every launch left two
+// thirds of the SMs idle.
+int build_points(abx_context *ctx, PointSets &sets, PointLayout &cols, PointLayout *rows,
+                 const FineGrid &fg) {
+  cudaStream_t s = ctx->stream;
+  const int64_t most = std::max(cols.n, rows ? rows->n : 0);
+  if (most == 0) return ABX_OK;
+  const dim3 grid(ceil_div(most, TPB), rows ? 2 : 1);
+  k_fine_keys<<<grid, TPB, 0, s>>>(sets, fg);
   ABX_CHECK_CUDA(cudaGetLastError());
   int bits = 0;
   while (bits < 32 && (((uint64_t)fg.ncells * 8 - 1) >> bits) != 0) ++bits;
-  ABX_TRY(radix_sort_pairs(P.keys.ptr, P.perm.ptr, n, bits, P.tmp.ptr, P.tmp.ptr + n,
-                           P.tmp.ptr + 2 * n, s));
-  k_fill_layout<<<ceil_div(n, TPB), TPB, 0, s>>>(src_soa, stride, fg, P.perm.ptr, n,
-                                                 clamp_anchor ? 1 : 0, P.cell.ptr, P.loc.ptr,
-                                                 P.posk.ptr);
+  SortSides S{};
+  S.sides = rows ? 2 : 1;
+  S.iota = true;
+  for (int i = 0; i < S.sides; ++i) {
+    PointLayout &P = i ? *rows : cols;
+    S.s[i] = SortSide{P.keys.ptr, P.perm.ptr, P.tmp.ptr, P.tmp.ptr + P.n, P.tmp.ptr + 2 * P.n, (size_t)P.n};
+  }
+  ABX_TRY(radix_sort_sides(S, bits, s));
+  k_fill_layout<<<grid, TPB, 0, s>>>(sets, fg);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
@@ -1844,16 +1874,13 @@ int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *
   ABX_TRY(particles_grid_desc(cols, &g));
   L.r = r;
   L.fg = make_fine_grid(g, r, std::max<int64_t>(cols->n, 1), 3);
-  ABX_TRY(build_points(ctx, cols->pos.ptr, cols->n, cols->n, L.fg, true, L.cols));
+  PointSets sets{};
+  ABX_TRY(reserve_points(cols->n, cols->pos.ptr, cols->n, true, L.cols, sets.s[0]));
+  L.self = !qsrc;
+  L.rows = L.self ? &L.cols : &L.rows_own;
+  if (!L.self) ABX_TRY(reserve_points(nq, qsrc, qstride, false, L.rows_own, sets.s[1]));
+  ABX_TRY(build_points(ctx, sets, L.cols, L.self ? nullptr : &L.rows_own, L.fg));
   ABX_TRY(build_cell_start(ctx, L));
-  if (!qsrc) {
-    L.self = true;
-    L.rows = &L.cols;
-  } else {
-    L.self = false;
-    ABX_TRY(build_points(ctx, qsrc, nq, qstride, L.fg, false, L.rows_own));
-    L.rows = &L.rows_own;
-  }
   ABX_TRY(build_units(ctx, L, split));
   ABX_TRY(build_tables(ctx, L, norm, norm == 2 ? r * r : std::fabs(r)));
   return ABX_OK;

@@ -194,28 +194,36 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(
 
 // ---- few tiles: the digit offsets without scan launches
 //
-// Up to RF_TILES tiles (524,288 items) a pass is two launches, counts per tile
+// Up to RF_MAX items a pass is two launches: counts per tile,
 // and the scatter, whose CTAs each add up the whole (tile, digit) table from L2
-// (at most 1 MB) instead of three scan launches between them; with so few
-// tiles an 11-bit digit costs little, so that 22-bit keys take two passes.  N =
-// 100,000, 21-bit keys: 3 x (hist, 3 scan kernels, scatter) + 2 copies -> 2 x 2
-// launches, @RS_OLD@ -> @RS_NEW@ us.
+// (16-bit counts, 512 KB at most: 2,048 items a tile, 4,096 above 128 tiles, 16 bytes a load: loads of one count each, 49
+// tiles in a row, were two thirds of the scatter's time).  With so few tiles an
+// 11-bit digit costs little, so that 22-bit keys take two passes.  Two
+// independent sets (a search's queries and its particles) go through every
+// launch together, blockIdx.y choosing the set: a pass over 100,000 items
+// occupies a third of the SMs.  N = 100,000, 21-bit keys: 3 x (hist, 3 scan
+// kernels, scatter) + 2 copies -> 2 x 2 launches, @RS_OLD@ -> @RS_NEW@ us.
 constexpr int RF_TILES = 128;
-template <int RB>
-__global__ void __launch_bounds__(RS_THREADS) k_rf_hist(const uint32_t *__restrict__ keys, size_t n,
-                                                        int shift, uint32_t *__restrict__ hist) {
+constexpr size_t RF_MAX = (size_t)RF_TILES * RS_TILE;
+static_assert(RS_TILE < 65536, "16-bit counts per tile");
+template <int RB, int ITEMS>
+__global__ void __launch_bounds__(RS_THREADS) k_rf_hist(SortSides S, bool alt, int shift) {
   constexpr int RADIX = 1 << RB;
   __shared__ uint32_t h[RADIX];
+  const SortSide &T = S.s[blockIdx.y];
+  const size_t n = T.n, base = (size_t)blockIdx.x * (RS_THREADS * ITEMS);
+  if (base >= n) return;
+  const uint32_t *__restrict__ keys = alt ? T.keys_alt : T.keys;
   for (int i = threadIdx.x; i < RADIX; i += RS_THREADS) h[i] = 0;
   __syncthreads();
-  const size_t base = (size_t)blockIdx.x * RS_TILE;
 #pragma unroll
-  for (int i = 0; i < RS_ITEMS; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const size_t g = base + i * RS_THREADS + threadIdx.x;
     if (g < n) atomicAdd(&h[(keys[g] >> shift) & (RADIX - 1)], 1u);
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < RADIX; d += RS_THREADS) hist[(size_t)blockIdx.x * RADIX + d] = h[d];
+  uint32_t *row = T.temp + (size_t)blockIdx.x * (RADIX / 2);
+  for (int d = threadIdx.x; d < RADIX / 2; d += RS_THREADS) row[d] = h[2 * d] | (h[2 * d + 1] << 16);
 }
 
 // Stable rank of every item of a tile among the items of its digit: warps own
@@ -237,18 +245,40 @@ __device__ __forceinline__ void rank_items(const int (&dig)[ITEMS], C *wc, uint3
   }
 }
 
-// Exclusive scan of RADIX values in shared memory by the CTA, THREADS at least
-// 32 and a power of two.
-template <int RADIX, int THREADS>
-__device__ __forceinline__ void scan_digits(uint32_t *v, uint32_t *warp_tot) {
-  constexpr int PER = RADIX / THREADS > 0 ? RADIX / THREADS : 1;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t loc[PER], sum = 0;
-#pragma unroll
-  for (int k = 0; k < PER; ++k) {
-    loc[k] = tid * PER + k < RADIX ? v[tid * PER + k] : 0u;
-    sum += loc[k];
+// Zeroes the warps' digit counts.
+template <int WARPS, int ROW, int THREADS>
+__device__ __forceinline__ void clear_counts(uint16_t (*wc)[ROW]) {
+  uint32_t *w = reinterpret_cast<uint32_t *>(&wc[0][0]);
+  for (int i = threadIdx.x; i < WARPS * ROW / 2; i += THREADS) w[i] = 0;
+}
+
+// The warps' counts to the counts of the warps before, two digits a word (a
+// tile's counts stay below 2^16); the totals to `total` if it is given.
+template <int WARPS, int ROW, int THREADS, int RADIX>
+__device__ __forceinline__ void scan_counts(uint16_t (*wc)[ROW], uint32_t *total) {
+  for (int d = threadIdx.x; d < RADIX / 2; d += THREADS) {
+    uint32_t run = 0;
+#pragma unroll 8
+    for (int w = 0; w < WARPS; ++w) {
+      uint32_t *p = reinterpret_cast<uint32_t *>(&wc[w][0]) + d;
+      const uint32_t c = *p;
+      *p = run;
+      run += c;
+    }
+    if (total) {
+      total[2 * d] = run & 0xffffu;
+      total[2 * d + 1] = run >> 16;
+    }
   }
+}
+
+// Exclusive scan over the CTA of PER values a thread.
+template <int PER>
+__device__ __forceinline__ void scan_values(uint32_t (&v)[PER], uint32_t *warp_tot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) sum += v[k];
   const uint32_t incl = warp_incl_scan(sum);
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
@@ -256,71 +286,85 @@ __device__ __forceinline__ void scan_digits(uint32_t *v, uint32_t *warp_tot) {
   for (int w = 0; w < warp; ++w) run += warp_tot[w];
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
-    if (tid * PER + k < RADIX) v[tid * PER + k] = run;
-    run += loc[k];
+    const uint32_t c = v[k];
+    v[k] = run;
+    run += c;
   }
-  __syncthreads();
 }
 
-template <int RB>
-__global__ void __launch_bounds__(RS_THREADS) k_rf_scatter(
-    const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
-    uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, size_t n, int shift,
-    const uint32_t *__restrict__ hist) {
+template <int RB, int ITEMS>
+__global__ void __launch_bounds__(RS_THREADS) k_rf_scatter(SortSides S, bool alt, int shift) {
   constexpr int RADIX = 1 << RB;
-  __shared__ uint16_t wcount[RS_WARPS][RADIX + 2];
+  constexpr int PER = RADIX / RS_THREADS;  // digits a thread adds up, consecutive
+  constexpr int TILE = RS_THREADS * ITEMS;
+  static_assert(PER == 1 || PER == 4 || PER == 8, "whole loads of 16-bit counts");
+  __shared__ __align__(16) uint16_t wcount[RS_WARPS][RADIX + 2];
   __shared__ uint32_t first[RADIX];
   __shared__ uint32_t warp_tot[RS_WARPS];
+  const SortSide &T = S.s[blockIdx.y];
+  const size_t n = T.n;
+  if ((size_t)blockIdx.x * TILE >= n) return;
+  const uint32_t *__restrict__ keys_in = alt ? T.keys_alt : T.keys;
+  const uint32_t *__restrict__ vals_in = alt ? T.vals_alt : T.vals;
+  uint32_t *__restrict__ keys_out = alt ? T.keys : T.keys_alt;
+  uint32_t *__restrict__ vals_out = alt ? T.vals : T.vals_alt;
+  const bool iota = S.iota && shift == 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < RS_WARPS * (RADIX + 2); i += RS_THREADS) (&wcount[0][0])[i] = 0;
-  const size_t base = (size_t)blockIdx.x * RS_TILE + (size_t)warp * (32 * RS_ITEMS);
-  uint32_t key[RS_ITEMS], val[RS_ITEMS], rank[RS_ITEMS];
-  int dig[RS_ITEMS];
+  const size_t base = (size_t)blockIdx.x * TILE + (size_t)warp * (32 * ITEMS);
+  uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
+  int dig[ITEMS];
 #pragma unroll
-  for (int i = 0; i < RS_ITEMS; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const size_t g = base + (size_t)i * 32 + lane;
     key[i] = g < n ? keys_in[g] : 0u;
-    val[i] = g < n ? vals_in[g] : 0u;
+    val[i] = g < n ? (iota ? (uint32_t)g : vals_in[g]) : 0u;
     dig[i] = g < n ? (int)((key[i] >> shift) & (RADIX - 1)) : RADIX;  // RADIX: never written out
   }
-  // this tile's and all tiles' counts of every digit
-  uint32_t before[RADIX / RS_THREADS > 0 ? RADIX / RS_THREADS : 1];
+  clear_counts<RS_WARPS, RADIX + 2, RS_THREADS>(wcount);
+  // all tiles' counts of every digit, and those of the tiles before
+  uint32_t tot[PER], pre[PER];
 #pragma unroll
-  for (int q = 0; q * RS_THREADS < RADIX; ++q) {
-    const int d = tid + q * RS_THREADS;
-    uint32_t pre = 0, tot = 0;
-    if (d < RADIX) {
+  for (int k = 0; k < PER; ++k) tot[k] = pre[k] = 0;
+  const unsigned tiles = (unsigned)((n + TILE - 1) / TILE);
+  const uint16_t *hist = reinterpret_cast<const uint16_t *>(T.temp) + tid * PER;
 #pragma unroll 8
-      for (unsigned t = 0; t < gridDim.x; ++t) {
-        const uint32_t c = hist[(size_t)t * RADIX + d];
-        tot += c;
-        pre += t < blockIdx.x ? c : 0u;
+  for (unsigned t = 0; t < tiles; ++t) {
+    const bool lower = t < blockIdx.x;
+    if (PER == 1) {
+      const uint32_t c = hist[(size_t)t * RADIX];
+      tot[0] += c;
+      pre[0] += lower ? c : 0u;
+    } else {
+      uint32_t w[PER / 2 ? PER / 2 : 1];
+      if (PER == 8) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(hist + (size_t)t * RADIX);
+        w[0] = v.x;
+        w[1 % (PER / 2 ? PER / 2 : 1)] = v.y;
+        w[2 % (PER / 2 ? PER / 2 : 1)] = v.z;
+        w[3 % (PER / 2 ? PER / 2 : 1)] = v.w;
+      } else {
+        const uint2 v = *reinterpret_cast<const uint2 *>(hist + (size_t)t * RADIX);
+        w[0] = v.x;
+        w[1 % (PER / 2 ? PER / 2 : 1)] = v.y;
       }
-      first[d] = tot;
-    }
-    before[q] = pre;
-  }
-  __syncthreads();
-  scan_digits<RADIX, RS_THREADS>(first, warp_tot);
-  rank_items<RADIX, RS_ITEMS>(dig, wcount[warp], rank);
-  __syncthreads();
 #pragma unroll
-  for (int q = 0; q * RS_THREADS < RADIX; ++q) {
-    const int d = tid + q * RS_THREADS;
-    if (d < RADIX) {
-      first[d] += before[q];
-      uint32_t run = 0;
-#pragma unroll
-      for (int w = 0; w < RS_WARPS; ++w) {
-        const uint32_t c = wcount[w][d];
-        wcount[w][d] = (uint16_t)run;
-        run += c;
+      for (int k = 0; k < PER; ++k) {
+        const uint32_t c = (k & 1) ? w[k / 2] >> 16 : w[k / 2] & 0xffffu;
+        tot[k] += c;
+        pre[k] += lower ? c : 0u;
       }
     }
   }
+  scan_values<PER>(tot, warp_tot);
+#pragma unroll
+  for (int k = 0; k < PER; ++k) first[tid * PER + k] = tot[k] + pre[k];
+  __syncthreads();
+  rank_items<RADIX, ITEMS>(dig, wcount[warp], rank);
+  __syncthreads();
+  scan_counts<RS_WARPS, RADIX + 2, RS_THREADS, RADIX>(wcount, nullptr);
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < RS_ITEMS; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     if (dig[i] < RADIX) {
       const uint32_t dst = first[dig[i]] + wcount[warp][dig[i]] + rank[i];
       keys_out[dst] = key[i];
@@ -329,48 +373,46 @@ __global__ void __launch_bounds__(RS_THREADS) k_rf_scatter(
   }
 }
 
-// ---- one tile: all passes in one launch, the items in shared memory between
-// them.
+// ---- one tile: all passes in one launch, a CTA a set, the items in shared
+// memory between them.
 constexpr int R1_THREADS = 512, R1_ITEMS = 8, R1_TILE = R1_THREADS * R1_ITEMS, R1_RB = 8;
-__global__ void __launch_bounds__(R1_THREADS) k_r1_sort(uint32_t *__restrict__ keys,
-                                                        uint32_t *__restrict__ vals, int n,
-                                                        int bits) {
+template <int ITEMS>
+__global__ void __launch_bounds__(R1_THREADS) k_r1_sort(SortSides S, int bits) {
   constexpr int RADIX = 1 << R1_RB, WARPS = R1_THREADS / 32;
-  __shared__ uint32_t sk[R1_TILE], sv[R1_TILE];
-  __shared__ uint16_t wcount[WARPS][RADIX + 2];
+  __shared__ uint32_t sk[R1_THREADS * ITEMS], sv[R1_THREADS * ITEMS];
+  __shared__ __align__(16) uint16_t wcount[WARPS][RADIX + 2];
   __shared__ uint32_t first[RADIX], warp_tot[WARPS];
+  const SortSide &T = S.s[blockIdx.x];
+  const int n = (int)T.n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < n; i += R1_THREADS) {
-    sk[i] = keys[i];
-    sv[i] = vals[i];
-  }
+  uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
+  int dig[ITEMS];
   for (int shift = 0; shift < bits; shift += R1_RB) {
-    for (int i = tid; i < WARPS * (RADIX + 2); i += R1_THREADS) (&wcount[0][0])[i] = 0;
-    __syncthreads();
-    uint32_t key[R1_ITEMS], val[R1_ITEMS], rank[R1_ITEMS];
-    int dig[R1_ITEMS];
+    clear_counts<WARPS, RADIX + 2, R1_THREADS>(wcount);
 #pragma unroll
-    for (int i = 0; i < R1_ITEMS; ++i) {
-      const int g = warp * (32 * R1_ITEMS) + i * 32 + lane;
-      key[i] = g < n ? sk[g] : 0u;
-      val[i] = g < n ? sv[g] : 0u;
-      dig[i] = g < n ? (int)((key[i] >> shift) & (RADIX - 1)) : RADIX;
-    }
-    rank_items<RADIX, R1_ITEMS>(dig, wcount[warp], rank);
-    __syncthreads();
-    if (tid < RADIX) {
-      uint32_t run = 0;
-      for (int w = 0; w < WARPS; ++w) {
-        const uint32_t c = wcount[w][tid];
-        wcount[w][tid] = (uint16_t)run;
-        run += c;
+    for (int i = 0; i < ITEMS; ++i) {
+      const int g = warp * (32 * ITEMS) + i * 32 + lane;
+      const bool in = g < n;
+      if (shift == 0) {
+        key[i] = in ? T.keys[g] : 0u;
+        val[i] = in ? (S.iota ? (uint32_t)g : T.vals[g]) : 0u;
+      } else {
+        key[i] = in ? sk[g] : 0u;
+        val[i] = in ? sv[g] : 0u;
       }
-      first[tid] = run;
+      dig[i] = in ? (int)((key[i] >> shift) & (RADIX - 1)) : RADIX;
     }
     __syncthreads();
-    scan_digits<RADIX, R1_THREADS>(first, warp_tot);
+    rank_items<RADIX, ITEMS>(dig, wcount[warp], rank);
+    __syncthreads();
+    scan_counts<WARPS, RADIX + 2, R1_THREADS, RADIX>(wcount, first);
+    __syncthreads();
+    uint32_t c[1] = {tid < RADIX ? first[tid] : 0u};
+    scan_values<1>(c, warp_tot);
+    if (tid < RADIX) first[tid] = c[0];
+    __syncthreads();
 #pragma unroll
-    for (int i = 0; i < R1_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
       if (dig[i] < RADIX) {
         const uint32_t dst = first[dig[i]] + wcount[warp][dig[i]] + rank[i];
         sk[dst] = key[i];
@@ -380,18 +422,25 @@ __global__ void __launch_bounds__(R1_THREADS) k_r1_sort(uint32_t *__restrict__ k
     __syncthreads();
   }
   for (int i = tid; i < n; i += R1_THREADS) {
-    keys[i] = sk[i];
-    vals[i] = sv[i];
+    T.keys[i] = sk[i];
+    T.vals[i] = sv[i];
   }
 }
 
 template <int RB>
-int rf_pass(const uint32_t *ki, const uint32_t *vi, uint32_t *ko, uint32_t *vo, size_t n, int shift,
-            uint32_t *hist, int ntiles, cudaStream_t s) {
-  k_rf_hist<RB><<<ntiles, RS_THREADS, 0, s>>>(ki, n, shift, hist);
-  k_rf_scatter<RB><<<ntiles, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n, shift, hist);
-  ABX_CHECK_CUDA(cudaGetLastError());
-  return ABX_OK;
+void rf_pass(const SortSides &S, dim3 grid, bool small, bool alt, int shift, cudaStream_t s) {
+  if (small) {
+    k_rf_hist<RB, RS_ITEMS / 2><<<grid, RS_THREADS, 0, s>>>(S, alt, shift);
+    k_rf_scatter<RB, RS_ITEMS / 2><<<grid, RS_THREADS, 0, s>>>(S, alt, shift);
+  } else {
+    k_rf_hist<RB, RS_ITEMS><<<grid, RS_THREADS, 0, s>>>(S, alt, shift);
+    k_rf_scatter<RB, RS_ITEMS><<<grid, RS_THREADS, 0, s>>>(S, alt, shift);
+  }
+}
+
+__global__ void k_sort_iota(uint32_t *v, size_t n) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) v[i] = (uint32_t)i;
 }
 
 }  // namespace
@@ -427,36 +476,68 @@ size_t radix_temp_u32(size_t n) {
   const size_t ntiles = (n + RS_TILE - 1) / RS_TILE;
   const size_t hist = ntiles * RADIX_MAX;
   // (the passes over few tiles: 2048 digits)
-  return std::max(hist + 64 + scan_temp_elems(hist), std::min<size_t>(ntiles, RF_TILES) * 2048);
+  return std::max(hist + 64 + scan_temp_elems(hist), std::min<size_t>(2 * ntiles, RF_TILES) * 1024 + 4);
+}
+
+bool radix_few_tiles(size_t n) { return n <= RF_MAX; }
+
+int radix_sort_sides(SortSides S, int bits, cudaStream_t s) {
+  size_t most = 0;
+  for (int i = 0; i < S.sides; ++i) most = std::max(most, S.s[i].n);
+  const int passes = (bits + 10) / 11;
+  if (most == 0) return ABX_OK;
+  if (!radix_few_tiles(most) || bits <= 0) {
+    for (int i = 0; i < S.sides; ++i) {
+      const SortSide &T = S.s[i];
+      if (S.iota && T.n) k_sort_iota<<<(unsigned)((T.n + 255) / 256), 256, 0, s>>>(T.vals, T.n);
+      ABX_TRY(radix_sort_pairs(T.keys, T.vals, T.n, bits, T.keys_alt, T.vals_alt, T.temp, s));
+    }
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
+  if (most <= (size_t)R1_TILE) {
+    if (most <= R1_TILE / 4)
+      k_r1_sort<R1_ITEMS / 4><<<S.sides, R1_THREADS, 0, s>>>(S, bits);
+    else if (most <= R1_TILE / 2)
+      k_r1_sort<R1_ITEMS / 2><<<S.sides, R1_THREADS, 0, s>>>(S, bits);
+    else
+      k_r1_sort<R1_ITEMS><<<S.sides, R1_THREADS, 0, s>>>(S, bits);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
+  const bool small = most <= RF_MAX / 2;
+  const int tile = small ? RS_TILE / 2 : RS_TILE;
+  const dim3 grid((unsigned)((most + tile - 1) / tile), S.sides);
+  for (int i = 0; i < S.sides; ++i)  // whole 16-byte loads (radix_temp_u32 has the room)
+    S.s[i].temp = reinterpret_cast<uint32_t *>((reinterpret_cast<uintptr_t>(S.s[i].temp) + 15) & ~(uintptr_t)15);
+  const int rb = (bits + passes - 1) / passes;
+  bool alt = false;
+  for (int shift = 0; shift < bits; shift += rb, alt = !alt) {
+    if (rb <= 8)
+      rf_pass<8>(S, grid, small, alt, shift, s);
+    else if (rb <= 10)
+      rf_pass<10>(S, grid, small, alt, shift, s);
+    else
+      rf_pass<11>(S, grid, small, alt, shift, s);
+  }
+  ABX_CHECK_CUDA(cudaGetLastError());
+  for (int i = 0; alt && i < S.sides; ++i) {
+    const SortSide &T = S.s[i];
+    ABX_CHECK_CUDA(cudaMemcpyAsync(T.keys, T.keys_alt, T.n * 4, cudaMemcpyDeviceToDevice, s));
+    ABX_CHECK_CUDA(cudaMemcpyAsync(T.vals, T.vals_alt, T.n * 4, cudaMemcpyDeviceToDevice, s));
+  }
+  return ABX_OK;
 }
 
 int radix_sort_pairs(uint32_t *keys, uint32_t *vals, size_t n, int bits, uint32_t *keys_alt,
                      uint32_t *vals_alt, uint32_t *temp, cudaStream_t s) {
   if (n <= 1 || bits <= 0) return ABX_OK;
   const int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
-  if (n <= (size_t)R1_TILE) {
-    k_r1_sort<<<1, R1_THREADS, 0, s>>>(keys, vals, (int)n, bits);
-    ABX_CHECK_CUDA(cudaGetLastError());
-    return ABX_OK;
-  }
-  if (ntiles <= RF_TILES) {
-    uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
-    const int passes = (bits + 10) / 11, rb = (bits + passes - 1) / passes;
-    for (int shift = 0; shift < bits; shift += rb) {
-      if (rb <= 8)
-        ABX_TRY(rf_pass<8>(ki, vi, ko, vo, n, shift, temp, ntiles, s));
-      else if (rb <= 10)
-        ABX_TRY(rf_pass<10>(ki, vi, ko, vo, n, shift, temp, ntiles, s));
-      else
-        ABX_TRY(rf_pass<11>(ki, vi, ko, vo, n, shift, temp, ntiles, s));
-      std::swap(ki, ko);
-      std::swap(vi, vo);
-    }
-    if (ki != keys) {
-      ABX_CHECK_CUDA(cudaMemcpyAsync(keys, ki, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-      ABX_CHECK_CUDA(cudaMemcpyAsync(vals, vi, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    }
-    return ABX_OK;
+  if (radix_few_tiles(n)) {
+    SortSides S{};
+    S.sides = 1;
+    S.s[0] = SortSide{keys, vals, keys_alt, vals_alt, temp, n};
+    return radix_sort_sides(S, bits, s);
   }
   // digit width: 9 or 10 bits where that saves a pass (17..20- and 25..27-bit keys)
   const int rb = (bits > 16 && bits <= 20) ? 10 : (bits > 24 && bits <= 27) ? 9 : 8;
