@@ -244,20 +244,30 @@ def radius_query_csr(p: Particles, q, r: float, lnorm: int = 2, with_dx: bool = 
     nq = int(q.shape[0])
     q = np.ascontiguousarray(q, dtype=np.float64)
     rowptr = np.empty(nq + 1, dtype=np.int64)
-    _check(lib().abx_radius_query_csr_lnorm(p._h, nq, _ptr(q), float(r), int(lnorm), _ptr(rowptr),
-                                            None, 0), "abx_radius_query_csr")
-    nnz = int(rowptr[-1])
-    cols = np.empty(max(nnz, 1), dtype=np.int32)
+    if with_dx and lnorm != 2:
+        raise ValueError("dx is returned by the euclidean search only")
+    nnz, cols, dx = C.c_int64(), C.c_void_p(), C.c_void_p()
+    _check(lib().abx_radius_query_csr_new(p._h, nq, _ptr(q), float(r), int(lnorm), _ptr(rowptr),
+                                          C.byref(nnz), C.byref(cols),
+                                          C.byref(dx) if with_dx else None),
+           "abx_radius_query_csr_new")
+    m = nnz.value
+    cols = np.asarray(_HostBlock(cols.value, (m,), "<i4"))
     if with_dx:
-        if lnorm != 2:
-            raise ValueError("dx is returned by the euclidean search only")
-        dx = np.empty((max(nnz, 1), p.dim), dtype=np.float64)
-        _check(lib().abx_radius_query_csr_dx(p._h, nq, _ptr(q), float(r), _ptr(rowptr), _ptr(cols),
-                                             _ptr(dx), nnz), "abx_radius_query_csr_dx")
-        return rowptr, cols[:nnz], dx[:nnz]
-    _check(lib().abx_radius_query_csr_lnorm(p._h, nq, _ptr(q), float(r), int(lnorm), _ptr(rowptr),
-                                            _ptr(cols), nnz), "abx_radius_query_csr")
-    return rowptr, cols[:nnz]
+        return rowptr, cols, np.asarray(_HostBlock(dx.value, (m, p.dim), "<f8"))
+    return rowptr, cols
+
+
+class _HostBlock:
+    """Host memory from the library as an array, given back with the last view."""
+
+    def __init__(self, ptr: int, shape, typestr: str):
+        self._ptr = ptr
+        self.__array_interface__ = dict(shape=shape, typestr=typestr, data=(ptr, False), version=3)
+
+    def __del__(self):
+        if not closing():
+            lib().abx_host_free(self._ptr)
 
 
 def radius_pairs(p: Particles, r: float):

@@ -27,7 +27,9 @@
 //    pair evaluates the reference's formula exactly (no FMA contraction).
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -1019,6 +1021,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
   const FineGrid &fg = P.fg;
   const unsigned lt = (1u << lane) - 1u;
   constexpr bool WCUT = KIND == K_WEND_CUT;
+  constexpr bool PCOUNT = POL == POL_COUNT && NORM == 2;  // counts two candidates at a time
   const float sc = WCUT ? P.p0f : 1.f;  // staging scale (d^2 = q^2 for WCUT)
   const int nfull = P.counts[0], nunits = nfull + P.counts[P.all_units ? 1 : 8];
   for (;;) {
@@ -1101,6 +1104,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
           if (kk[sub] >= 0) {
             cls[sub] = __ldg(&P.cloc[kk[sub]]);
             if (POL == POL_MATVEC) bws[sub] = __ldg(&P.b32[kk[sub]]);
+            if (POL == POL_LIST) bws[sub] = __uint_as_float(__ldg(&P.cperm[kk[sub]]));
           }
         }
 #pragma unroll
@@ -1151,6 +1155,15 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
             const float4 c1 = 2 * h + 1 < nt ? sm.p[2 * h + 1] : make_float4(1e4f, 1e4f, 1e4f, 0.f);
             sm.pp[2 * h] = make_float4(c0.x, c1.x, c0.y, c1.y);
             sm.pp[2 * h + 1] = make_float4(c0.z, c1.z, c0.w, c1.w);
+          }
+        }
+        if (PCOUNT) {
+          for (int h = lane; 2 * h < nt; h += 32) {
+            const float4 c0 = sm.p[2 * h];
+            const float far = __int_as_float(0x7f800000);  // an odd tail: never counted
+            const float4 c1 = 2 * h + 1 < nt ? sm.p[2 * h + 1] : make_float4(far, far, far, 0.f);
+            sm.pp[2 * h] = make_float4(c0.x, c1.x, c0.y, c1.y);
+            sm.pp[2 * h + 1] = make_float4(c0.z, c1.z, 0.f, 0.f);
           }
         }
         if (!WCUT && POL == POL_MATVEC && lane == 0 && (nt & 1)) {
@@ -1225,8 +1238,35 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
           }
           acc32 = acc2.x + acc2.y;
         }
+        if (PCOUNT) {
+          // d^2 - mid for two candidates per packed instruction: the sign counts
+          // (one LEA.HI), the smallest magnitude says whether any lies in the band
+          const float2 nqx = make_float2(-pq0, -pq0), nqy = make_float2(-pq1, -pq1),
+                       nqz = make_float2(-pq2, -pq2);
+          const float2 nmid = make_float2(-r2mid, -r2mid);
+          const int npair = (nt + 1) >> 1;
+          float least = r2half + r2half;
+          unsigned hits = 0;
+#pragma unroll 8
+          for (int h = 0; h < npair; ++h) {
+            const float4 A = sm.pp[2 * h];
+            const float2 B = *reinterpret_cast<const float2 *>(&sm.pp[2 * h + 1]);
+            const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nqx);
+            const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nqy);
+            const float2 dz = __fadd2_rn(B, nqz);
+            float2 dd = __fmul2_rn(dx, dx);
+            dd = __ffma2_rn(dy, dy, dd);
+            dd = __ffma2_rn(dz, dz, dd);
+            const float2 off = __fadd2_rn(dd, nmid);
+            hits += __float_as_uint(off.x) >> 31;
+            hits += __float_as_uint(off.y) >> 31;
+            least = fminf(least, fminf(fabsf(off.x), fabsf(off.y)));
+          }
+          count += (int)hits;
+          need = least <= r2half;
+        }
 #pragma unroll 4
-        for (int j = 0; j < nt && POL != POL_MATVEC; ++j) {
+        for (int j = 0; j < nt && POL != POL_MATVEC && !PCOUNT; ++j) {
           const float4 c = sm.p[j];
           const float dd = norm32<NORM>(c.x - pq0, c.y - pq1, c.z - pq2);
           const bool in = dd <= r2lo;
@@ -1239,7 +1279,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
           if (POL == POL_LIST && in && active) {
             const int2 mt = sm.meta[j];
             if (P.dx_out) write_dx(P, out_off, xq, mt.x, ws.seg[mt.y].z);
-            P.cols_out[out_off++] = (int32_t)P.cperm[mt.x];
+            P.cols_out[out_off++] = __float_as_int(c.w);
           }
         }
         if (!WCUT && __any_sync(0xffffffffu, need)) {
@@ -1253,8 +1293,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
               const float4 c = sm.p[j];
               const float dd = norm32<NORM>(c.x - pq0, c.y - pq1, c.z - pq2);
               const bool wend = POL == POL_MATVEC && KIND == ABX_K_WENDLAND_C2;
-              const bool flagged = wend ? fabsf(__fadd_rn(dd, -r2mid)) <= r2half
-                                        : (dd > r2lo && dd <= r2hi);
+              const bool mid = (wend || PCOUNT) && fabsf(__fadd_rn(dd, -r2mid)) <= r2half;
+              const bool flagged = mid || (!wend && dd > r2lo && dd <= r2hi);
               if (flagged) {
                 const int2 mt = sm.meta[j];
                 int img[3], du0, du1;
@@ -1264,6 +1304,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
                   // the packed loop added the clamped value: take it back out
                   // for pairs the FP64 test rejects
                   if (!inside) acc32 -= kern32x2_wendland_clamped(make_float2(dd, dd), P).x * c.w;
+                } else if (PCOUNT) {
+                  count += (inside ? 1 : 0) - (__fadd_rn(dd, -r2mid) < 0.f ? 1 : 0);
                 } else if (inside) {
                   if (POL == POL_MATVEC) acc32 = fmaf(kern32<KIND>(dd, P), c.w, acc32);
                   if (POL == POL_COUNT) ++count;
@@ -2077,10 +2119,28 @@ int rowptr_device(abx_context *ctx, SearchSpace &W, int64_t n, int64_t &nnz) {
 }
 }  // namespace
 
+// Host memory for lists whose length is known once they are counted.
+struct OwnedLists {
+  bool want_dx = false;
+  int64_t nnz = 0;
+  void *cols = nullptr, *dx = nullptr;
+  ~OwnedLists() {
+    std::free(cols);
+    std::free(dx);
+  }
+  int allocate(int64_t n, int dim) {
+    nnz = n;
+    cols = std::malloc((size_t)std::max<int64_t>(n, 1) * sizeof(int32_t));
+    if (want_dx) dx = std::malloc((size_t)std::max<int64_t>(n, 1) * dim * sizeof(double));
+    ABX_REQUIRE(cols && (dx || !want_dx), ABX_ERR_ALLOC, "no host memory for %lld neighbours", (long long)n);
+    return ABX_OK;
+  }
+};
+
 // Radius queries for arbitrary points (C ABI helpers).
 int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, double r,
                  int32_t *counts_user, int64_t *rowptr_user, int32_t *cols_user, int64_t cap,
-                 int lnorm, double *dx_user = nullptr) {
+                 int lnorm, double *dx_user = nullptr, OwnedLists *own = nullptr) {
   abx_context *ctx = p->ctx;
   cudaStream_t s = ctx->stream;
   ABX_REQUIRE(p->searchable, ABX_ERR_STATE, "init_neighbour_search not called on this particle set");
@@ -2103,6 +2163,7 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
       int64_t z = 0;
       ABX_CHECK_CUDA(cudaMemcpy(rowptr_user, &z, sizeof(int64_t), cudaMemcpyDefault));
     }
+    if (own) ABX_TRY(own->allocate(0, D));
     return ABX_OK;
   }
   // counts go by row, straight to the caller's device memory where it is that
@@ -2127,6 +2188,12 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
     int64_t nnz = 0;
     ABX_TRY(rowptr_device(ctx, W, nq, nnz));
     ABX_CHECK_CUDA(cudaMemcpyAsync(rowptr_user, W.rowptr.ptr, (nq + 1) * 8, cudaMemcpyDefault, s));
+    if (own) {
+      ABX_TRY(own->allocate(nnz, D));
+      cols_user = static_cast<int32_t *>(own->cols);
+      dx_user = static_cast<double *>(own->dx);
+      cap = nnz;
+    }
     if (cols_user) {
       ABX_REQUIRE(cap >= nnz, ABX_ERR_CAPACITY, "cols capacity %lld < nnz %lld", (long long)cap,
                   (long long)nnz);
@@ -2309,6 +2376,22 @@ int abx_radius_count_lnorm(abx_particles *p, int64_t nq, const double *q, double
   ABX_TRY(ctx_activate(p->ctx));
   return radius_query(p, nq, q, r, counts, nullptr, nullptr, 0, lnorm);
 }
+
+int abx_radius_query_csr_new(abx_particles *p, int64_t nq, const double *q, double r, int lnorm,
+                             int64_t *rowptr, int64_t *nnz, void **cols, void **dx) {
+  ABX_REQUIRE(p && (q || nq == 0) && rowptr && nnz && cols, ABX_ERR_INVALID, "null argument");
+  ABX_REQUIRE(!dx || lnorm == 2, ABX_ERR_INVALID, "dx is returned by the euclidean search only");
+  ABX_TRY(ctx_activate(p->ctx));
+  OwnedLists own;
+  own.want_dx = dx != nullptr;
+  ABX_TRY(radius_query(p, nq, q, r, nullptr, rowptr, nullptr, 0, lnorm, nullptr, &own));
+  *nnz = own.nnz;
+  *cols = std::exchange(own.cols, nullptr);
+  if (dx) *dx = std::exchange(own.dx, nullptr);
+  return ABX_OK;
+}
+
+void abx_host_free(void *ptr) { std::free(ptr); }
 
 int abx_radius_query_csr_lnorm(abx_particles *p, int64_t nq, const double *q, double r, int lnorm,
                                int64_t *rowptr, int32_t *cols, int64_t cap) {

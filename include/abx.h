@@ -39,7 +39,7 @@ extern "C" {
 #define ABX_OK 0
 #define ABX_ERR_INVALID 1   /* bad argument */
 #define ABX_ERR_CUDA 2      /* CUDA runtime error */
-#define ABX_ERR_ALLOC 3     /* device allocation failed */
+#define ABX_ERR_ALLOC 3     /* allocation failed */
 #define ABX_ERR_STATE 4     /* e.g. neighbour search not initialised */
 #define ABX_ERR_TIMEOUT 5   /* a bounded device-side wait gave up */
 #define ABX_ERR_CAPACITY 6  /* caller-provided output too small */
@@ -192,6 +192,14 @@ ABX_API int abx_radius_count_lnorm(abx_particles *p, int64_t nq, const double *q
                                    int lnorm, int32_t *counts);
 ABX_API int abx_radius_query_csr_lnorm(abx_particles *p, int64_t nq, const double *q, double r,
                                        int lnorm, int64_t *rowptr, int32_t *cols, int64_t cap);
+/* The lists in one call: rowptr (host or device), and *cols (and *dx, where dx
+ * is not NULL: euclidean only) host memory that the call allocates and
+ * abx_host_free gives back.  With abx_radius_query_csr the length has to be
+ * asked for first, and the search runs twice. */
+ABX_API int abx_radius_query_csr_new(abx_particles *p, int64_t nq, const double *q, double r,
+                                     int lnorm, int64_t *rowptr, int64_t *nnz, void **cols,
+                                     void **dx);
+ABX_API void abx_host_free(void *ptr);
 /* euclidean_search in a linearly transformed coordinate system
  * (LinearTransform / ScaleTransform, src/Transform.h; the search iterator's
  * m_dx = transform(p - x), src/Search.h:438-445): T is the row-major dim x dim
