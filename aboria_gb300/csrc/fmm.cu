@@ -30,6 +30,8 @@
 #include <map>
 #include <vector>
 
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 #include "fix64.cuh"
 #include "handles.cuh"
@@ -70,14 +72,17 @@ struct FmmPlan {
   int n_m2l = 0;
   DevBuf<double> Km;      // nmat x ncheb x ncheb
   DevBuf<float> Kmh, Kml; // split-TF32 hi/lo parts of the FP32 copy (mma.sync M2L, ncheb <= 64)
-  DevBuf<float> Kp;       // the same packed as tcgen05 stage images (ncheb > 64, k_pack_tf32)
+  DevBuf<__half> Kp;      // the same packed as tcgen05 stage images (ncheb > 64, k_pack_f16)
+  DevBuf<float> Kp_scale;  // power of two of each matrix' packed values
   // FP64 M2L on the integer units: K and W as scaled 56-bit numbers, their
   // exponents (per row of K, per node), tiles of 64 pairs
   DevBuf<int2> Kq, Wq;
   DevBuf<short> ke, we;
   DevBuf<int> mf_mat, mf_first;
   int mf_tiles = 0;
-  DevBuf<float> W32l;     // lo part of W (the tcgen05 M2L reads W32 as the hi part)
+  // W as scaled FP16, hi and lo, and each node's power of two (tcgen05 M2L)
+  DevBuf<__half> W16h, W16l;
+  DevBuf<float> W16_scale;
   int nmat = 0;
   // M2L grouped by matrix (for the tensor-core GEMM): per matrix a list of
   // (target, source)
@@ -667,10 +672,16 @@ __global__ void __launch_bounds__(64 * WM) k_m2l_tc2(int ncheb, int ldk, int ldg
 // per (M2L matrix, N-pair tile) computes all NRB = ceil(ncheb/128) row
 // blocks, so the gathered source expansions of the tile are read once:
 //   G[targets][rb*128 + r] += sum_k K[rb*128 + r][k] * W[sources][k]
-// as split TF32 (K = Kh + Kl, W = Wh + Wl; Kl Wh + Kh Wl + Kh Wh) on
-// tcgen05.mma kind::tf32 into NRB accumulators of 128 x N FP32 in TMEM.
+// as split FP16 (K = Kh + Kl, W = Wh + Wl; Kl Wh + Kh Wl + Kh Wh) on
+// tcgen05.mma kind::f16 into NRB accumulators of 128 x N FP32 in TMEM.  Every K
+// matrix and every node's W has its own power of two, which brings its largest
+// value to [2^14, 2^15): hi and lo then have the 11 + 11 bits that TF32 parts
+// have, down to 2^-24 of those units (2^-38 of the largest), and a 16-byte
+// chunk, a stage and an MMA hold twice the columns; the tensor pipe's FP16 rate
+// is twice TF32's, and the operands' shared-memory traffic, which bounds
+// 64-pair tiles, is half.  Order 7, N = 1M: @M7A@ -> @M7B@ ms.
 // The K matrices are packed once per plan into the shared-memory image of a
-// pipeline stage (k_pack_tf32), so a stage's A operand is one bulk copy on the
+// pipeline stage (k_pack_f16), so a stage's A operand is one bulk copy on the
 // TMA engine (cp.async.bulk, completion counted on the stage's `fullA`
 // mbarrier) and bypasses the load/store pipeline; the W rows of the tile's
 // sources are gathered 16 bytes per lane with cp.async.  Operands use the
@@ -689,8 +700,8 @@ __global__ void __launch_bounds__(64 * WM) k_m2l_tc2(int ncheb, int ldk, int ldg
 // its copies and MMAs in flight and still releases its TMEM.  The ring depth
 // keeps the CTAs resident on an SM (by shared memory) within the SM's 512
 // TMEM columns.
-constexpr int T5_KB = 8;
-constexpr int T5_PART = 128 * T5_KB * 4;  // bytes of one K operand part: 128 rows x 8 columns
+constexpr int T5_KB = 16;
+constexpr int T5_PART = 128 * T5_KB * 2;  // bytes of one K operand part: 128 rows x 16 columns
 constexpr uint32_t T5_POLL_CAP = 1u << 30;  // second bound on the polls of one wait
 // Per row-block count: N pairs per tile, ring depth S, producer lag LAG and
 // TMEM columns.  Three or four row blocks use 64-pair tiles so that two CTAs
@@ -703,7 +714,7 @@ template <int NRB> struct T5Cfg {
   // for a block the producer has not signalled)
   static constexpr int LAG = NRB == 2 ? 2 : 1;
   static constexpr int A_BYTES = NRB * 2 * T5_PART;       // K hi, lo of every row block
-  static constexpr int B_PART = N * T5_KB * 4;            // W of the N pairs, one part
+  static constexpr int B_PART = N * T5_KB * 2;            // W of the N pairs, one part
   static constexpr int STAGE = A_BYTES + 2 * B_PART;
   static constexpr size_t SMEM = (size_t)S * STAGE + 1024 + 2048;  // + alignment, barriers, indices
   static constexpr uint32_t TCOLS = NRB * N <= 128 ? 128u : (NRB * N <= 256 ? 256u : 512u);
@@ -719,28 +730,86 @@ static_assert(T5Cfg<1>::LAG < T5Cfg<1>::S && T5Cfg<2>::LAG < T5Cfg<2>::S &&
                   T5Cfg<3>::LAG < T5Cfg<3>::S && T5Cfg<4>::LAG < T5Cfg<4>::S,
               "producer lag below the ring depth");
 
-// Packed split-TF32 M2L matrices: per (matrix, 8-column block kb, 128-row
+// Power of two that brings values up to `big` to [2^14, 2^15) (in FP32's range;
+// 1 for zero), as the factor that takes them back.
+__device__ __forceinline__ float f16_unit(float big) {
+  if (!(big > 0.f && big <= 3.4e38f)) return 1.f;
+  int e;
+  frexpf(big, &e);
+  return ldexpf(1.f, min(max(e - 15, -126), 113));
+}
+
+// Power of two of each M2L matrix: a CTA a matrix.
+constexpr int KS_TPB = 256;
+__global__ void __launch_bounds__(KS_TPB) k_mat_scale(const double *__restrict__ K, int64_t len,
+                                                      float *__restrict__ scale) {
+  __shared__ float part[KS_TPB / 32];
+  float big = 0.f;
+  for (int64_t i = threadIdx.x; i < len; i += KS_TPB)
+    big = fmaxf(big, fabsf((float)K[blockIdx.x * len + i]));
+  for (int d = 16; d > 0; d >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, d));
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = big;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < KS_TPB / 32; ++w) big = fmaxf(big, part[w]);
+    scale[blockIdx.x] = f16_unit(big);
+  }
+}
+
+// Packed split-FP16 M2L matrices: per (matrix, 16-column block kb, 128-row
 // block rb, part hi/lo) the 4 KB shared-memory image of the operand tile,
-// element (r, k) at ((k/4) * 16 + r/8) * 128 + (r%8) * 16 + (k%4) * 4 bytes;
-// zero beyond ncheb.  hi = tf32(K), lo = tf32(K - hi).
-__global__ void k_pack_tf32(const double *__restrict__ K, int64_t nmat, int ncheb, int nkb,
-                            int nrb, float *__restrict__ out) {
+// element (r, k) at ((k/8) * 16 + r/8) * 128 + (r%8) * 16 + (k%8) * 2 bytes;
+// zero beyond ncheb.  hi = fp16(K / scale), lo = fp16(K / scale - hi).
+__global__ void k_pack_f16(const double *__restrict__ K, const float *__restrict__ scale,
+                           int64_t nmat, int ncheb, int nkb, int nrb, __half *__restrict__ out) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nmat * nkb * nrb * 2 * (T5_PART / 4)) return;
+  if (e >= nmat * nkb * nrb * 2 * (T5_PART / 2)) return;
   int64_t t = e;
-  const int w = (int)(t % (T5_PART / 4));
-  t /= T5_PART / 4;
+  const int w = (int)(t % (T5_PART / 2));
+  t /= T5_PART / 2;
   const int part = (int)(t % 2);
   t /= 2;
   const int rb = (int)(t % nrb);
   t /= nrb;
   const int kb = (int)(t % nkb);
   const int64_t m = t / nkb;
-  const int kk = w & 3, rl = (w >> 2) & 7, rh = (w >> 5) & 15, kq = w >> 9;
-  const int i = rb * 128 + rh * 8 + rl, k = kb * T5_KB + kq * 4 + kk;
-  const float f = (i < ncheb && k < ncheb) ? (float)K[(m * ncheb + i) * ncheb + k] : 0.f;
-  const uint32_t h = f2tf32(f);
-  out[e] = part == 0 ? __uint_as_float(h) : __uint_as_float(f2tf32(f - __uint_as_float(h)));
+  const int kk = w & 7, rl = (w >> 3) & 7, rh = (w >> 6) & 15, kq = w >> 10;
+  const int i = rb * 128 + rh * 8 + rl, k = kb * T5_KB + kq * 8 + kk;
+  // (scale: a power of two down to 2^-126, whose reciprocal is a float)
+  const float f =
+      (i < ncheb && k < ncheb) ? (float)K[(m * ncheb + i) * ncheb + k] * (1.f / scale[m]) : 0.f;
+  const __half h = __float2half_rn(f);
+  out[e] = part == 0 ? h : __float2half_rn(f - __half2float(h));
+}
+
+// W as scaled split FP16 (rows of ldk values, zero beyond ncheb): a warp a node.
+__global__ void __launch_bounds__(256) k_split_f16(const double *__restrict__ W, int64_t nnodes,
+                                                   int ncheb, int ldk, __half *__restrict__ hi,
+                                                   __half *__restrict__ lo,
+                                                   float *__restrict__ scale) {
+  const int64_t node = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (node >= nnodes) return;
+  float v[16];  // ncheb <= 512
+  float big = 0.f;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int k = q * 32 + lane;
+    v[q] = k < ncheb ? (float)W[node * ncheb + k] : 0.f;
+    big = fmaxf(big, fabsf(v[q]));
+  }
+  for (int d = 16; d > 0; d >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, d));
+  const float unit = f16_unit(big), inv = 1.f / unit;
+  if (lane == 0) scale[node] = unit;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int k = q * 32 + lane;
+    if (k >= ldk) break;
+    const float f = v[q] * inv;
+    const __half h = __float2half_rn(f);
+    hi[node * ldk + k] = h;
+    lo[node * ldk + k] = __float2half_rn(f - __half2float(h));
+  }
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
@@ -753,10 +822,9 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
 }
 
-// Instruction descriptor, kind::tf32: D F32, A and B TF32, both K-major.
-__host__ __device__ constexpr uint32_t umma_idesc_tf32(int m, int n) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(m >> 4) << 24);
+// Instruction descriptor, kind::f16: D F32, A and B FP16, both K-major.
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 __device__ __forceinline__ uint64_t globaltimer_ns() {
@@ -798,13 +866,15 @@ __device__ __forceinline__ void cp16(uint32_t dst, const void *src, int nbytes) 
 
 template <int NRB>
 __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, int ldg,
-                                                 const float *__restrict__ Ap,
+                                                 const __half *__restrict__ Ap,
+                                                 const float *__restrict__ Ap_scale,
                                                  const int2 *__restrict__ pairs,
                                                  const int *__restrict__ mat_off,
                                                  const int *__restrict__ tile_mat,
                                                  const int *__restrict__ tile_first,
-                                                 const float *__restrict__ Wh,
-                                                 const float *__restrict__ Wl,
+                                                 const __half *__restrict__ Wh,
+                                                 const __half *__restrict__ Wl,
+                                                 const float *__restrict__ W_scale,
                                                  float *__restrict__ G32, int *__restrict__ status,
                                                  uint64_t limit_ns, int drop_arrive) {
   using C = T5Cfg<NRB>;
@@ -815,6 +885,7 @@ __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, in
   uint64_t *fullB = fullA + S, *empty = fullB + S, *accb = empty + S;
   uint32_t *tslot = (uint32_t *)(accb + 1);
   int *sSrc = (int *)(tslot + 4), *sTgt = sSrc + T5_N, *sInfo = sTgt + T5_N;
+  float *sScale = (float *)(sInfo + 4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tile = blockIdx.x;
   const int m = tile_mat[tile], p0 = tile_first[tile];
@@ -823,7 +894,9 @@ __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, in
     const int2 pr = tid < np ? pairs[p0 + tid] : make_int2(-1, -1);
     sTgt[tid] = pr.x;
     sSrc[tid] = pr.y;
+    sScale[tid] = pr.y >= 0 ? W_scale[pr.y] : 0.f;
   }
+  const float mat_scale = Ap_scale[m];
   if (tid == 0) {
     for (int q = 0; q < S; ++q) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&fullA[q])));
@@ -873,11 +946,11 @@ __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, in
             : "memory");
       }
 #pragma unroll
-      for (int e = lane; e < T5_N * (T5_KB / 4); e += 32) {
+      for (int e = lane; e < T5_N * (T5_KB / 8); e += 32) {
         const int rl = e & 7, kq = (e >> 3) & 1, rh = e >> 4;
         const int src = sSrc[rh * 8 + rl];
         const uint32_t off = (uint32_t)((kq * (T5_N / 8) + rh) * 128 + rl * 16);
-        const size_t g = (size_t)(src >= 0 ? src : 0) * ldk + p * T5_KB + kq * 4;
+        const size_t g = (size_t)(src >= 0 ? src : 0) * ldk + p * T5_KB + kq * 8;
         cp16(sb + C::A_BYTES + off, Wh + g, src >= 0 ? 16 : 0);
         cp16(sb + C::A_BYTES + C::B_PART + off, Wl + g, src >= 0 ? 16 : 0);
       }
@@ -910,7 +983,7 @@ __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, in
     }
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer
-    constexpr uint32_t idesc = umma_idesc_tf32(128, T5_N);
+    constexpr uint32_t idesc = umma_idesc_f16(128, T5_N);
     constexpr uint32_t ks = (128 / 8) * 128;    // core-matrix stride along K (K rows)
     constexpr uint32_t bks = (T5_N / 8) * 128;  // the same for the T5_N pair rows
     bool ok = true;
@@ -937,7 +1010,7 @@ __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, in
           const uint32_t acc = (c > 0 || t > 0) ? 1u : 0u;
           asm volatile(
               "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(
                   tmem + (uint32_t)(rb * T5_N)),
               "l"(ad[t]), "l"(bd[t]), "r"(idesc), "r"(acc));
         }
@@ -997,9 +1070,11 @@ __global__ void __launch_bounds__(128) k_m2l_tc5(int ncheb, int nkb, int ldk, in
           const int tgt = sTgt[c0 + q];
           if (tgt >= 0 && i0 + g < ncheb) {
             const float4 a = *reinterpret_cast<const float4 *>(&tt[q * 32 + g]);
+            const float sc = sScale[c0 + q];
             float *dst = G32 + (size_t)tgt * ldg + i0 + g;
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(a.x),
-                         "f"(a.y), "f"(a.z), "f"(a.w)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst),
+                         "f"(a.x * mat_scale * sc), "f"(a.y * mat_scale * sc),
+                         "f"(a.z * mat_scale * sc), "f"(a.w * mat_scale * sc)
                          : "memory");
           }
         }
@@ -1793,7 +1868,6 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
       const size_t tot = (size_t)P->nnodes * nc;
       const int ldg = (nc + 3) / 4 * 4;
       const int ldk = (nc + 31) / 32 * 32;
-      ABX_TRY(P->W32.reserve((size_t)P->nnodes * ldk));
       ABX_TRY(P->G32.reserve((size_t)P->nnodes * ldg));
       ABX_CHECK_CUDA(cudaMemsetAsync(P->G32.ptr, 0, (size_t)P->nnodes * ldg * 4, s));
       if (nc <= 64) {
@@ -1805,6 +1879,7 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
           k_split_tf32<<<ceil_div(nk, 256), 256, 0, s>>>(P->Km.ptr, (int64_t)P->nmat * nc, nc,
                                                          ldk, P->Kmh.ptr, P->Kml.ptr);
         }
+        ABX_TRY(P->W32.reserve((size_t)P->nnodes * ldk));
         k_to_f32_padded<<<ceil_div((size_t)P->nnodes * ldk, 256), 256, 0, s>>>(
             P->W.ptr, P->nnodes, nc, ldk, P->W32.ptr);
         auto launch_m2l = [&](auto kern, int mt, int threads, size_t smem) -> int {
@@ -1825,22 +1900,26 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
         const int nkb = (nc + T5_KB - 1) / T5_KB;
         const int nrb = (nc + 127) / 128;  // 1..4 for orders 5..8
         if (!P->Kp.ptr) {
-          const size_t nk = (size_t)P->nmat * nkb * nrb * 2 * (T5_PART / 4);
+          const size_t nk = (size_t)P->nmat * nkb * nrb * 2 * (T5_PART / 2);
           ABX_TRY(P->Kp.reserve(nk));
-          k_pack_tf32<<<ceil_div(nk, 256), 256, 0, s>>>(P->Km.ptr, P->nmat, nc, nkb, nrb,
-                                                        P->Kp.ptr);
+          ABX_TRY(P->Kp_scale.reserve(P->nmat));
+          k_mat_scale<<<P->nmat, KS_TPB, 0, s>>>(P->Km.ptr, (int64_t)nc * nc, P->Kp_scale.ptr);
+          k_pack_f16<<<ceil_div(nk, 256), 256, 0, s>>>(P->Km.ptr, P->Kp_scale.ptr, P->nmat, nc, nkb,
+                                                       nrb, P->Kp.ptr);
         }
-        ABX_TRY(P->W32l.reserve((size_t)P->nnodes * ldk));
-        k_split_tf32<<<ceil_div((size_t)P->nnodes * ldk, 256), 256, 0, s>>>(
-            P->W.ptr, P->nnodes, nc, ldk, P->W32.ptr, P->W32l.ptr);
+        ABX_TRY(P->W16h.reserve((size_t)P->nnodes * ldk));
+        ABX_TRY(P->W16l.reserve((size_t)P->nnodes * ldk));
+        ABX_TRY(P->W16_scale.reserve(P->nnodes));
+        k_split_f16<<<ceil_div(P->nnodes, 8), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, ldk, P->W16h.ptr,
+                                                           P->W16l.ptr, P->W16_scale.ptr);
         int *status = p->ctx->dev_flag.ptr + 8;
         ABX_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int), s));
         auto launch_tc5 = [&](auto kern, size_t smem) -> int {
           ABX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)smem));
-          kern<<<P->ntiles, 128, smem, s>>>(nc, nkb, ldk, ldg, P->Kp.ptr, P->m2l_by_mat.ptr,
+          kern<<<P->ntiles, 128, smem, s>>>(nc, nkb, ldk, ldg, P->Kp.ptr, P->Kp_scale.ptr, P->m2l_by_mat.ptr,
                                             P->mat_off_d.ptr, P->tile_mat.ptr, P->tile_first.ptr,
-                                            P->W32.ptr, P->W32l.ptr, P->G32.ptr, status,
+                                            P->W16h.ptr, P->W16l.ptr, P->W16_scale.ptr, P->G32.ptr, status,
                                             (uint64_t)(P->wait_limit_s * 1e9), P->drop_arrive);
           return ABX_OK;
         };
