@@ -1334,12 +1334,18 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
 // bounding-box test, as FP32 offsets (for the prefilter) and as FP64
 // positions shifted by their periodic image (x_j - image*L, for the kernel
 // value), with their weights and (column index, segment) for the exact test.
-struct WarpTile64 {
-  float4 pf[STAGE];
+// Two tiles in turn: a lane's neighbours left over from one are evaluated beside
+// the next one's.
+template <int KIND> struct WarpTile64 {
+  // FP32 offsets as pairs of candidates: (x_a, x_b, y_a, y_b), (z_a, z_b)
+  float4 pxy[STAGE / 2];
+  float2 pz[STAGE / 2];
   // (bits of) the position: double, or fixed point (FIX)
-  long long ux[STAGE], uy[STAGE], uz[STAGE];
-  double b[STAGE], s[STAGE];
-  int2 meta[STAGE];
+  long long ux[2 * STAGE], uy[2 * STAGE], uz[2 * STAGE];
+  double b[2 * STAGE], s[KIND == ABX_K_SCALAR_SUM ? 2 * STAGE : 1];
+  // column and segment: of the last tile, of both where a value may want them
+  static constexpr int METAS = KIND == ABX_K_LAPLACE ? 2 : 1;
+  int2 meta[METAS * STAGE];
 };
 
 // FP64-accurate kernel value of one accepted pair from its fixed-point
@@ -1362,28 +1368,34 @@ __device__ __forceinline__ double pair64(const D4 &xq, const D4 &xj, const int *
 
 // FP64 sparse matvec: the reference's arithmetic for every accepted pair,
 // FP64 work only for accepted pairs.  Per staged tile of <= 64 candidates:
-//  (1) every lane classifies all candidates with the FP32 offsets into
-//      accepted (d2 <= r2lo), rejected (d2 > r2hi) and the rounding band,
-//      where the reference's exact FP64 test decides (rare); the result is a
-//      64-bit mask of this lane's neighbours among the candidates;
+//  (1) every lane classifies all candidates, two per packed FP32x2 instruction:
+//      the sign of d2 - r2mid goes into a 64-bit mask of this lane's neighbours,
+//      the least magnitude says whether any lies in the rounding band, where the
+//      reference's exact FP64 test decides (rare);
 //  (2) every lane walks its own mask and evaluates the FP64 distance, kernel
-//      and product for those pairs only.
-// The warp then pays for max over lanes of its neighbour count, not for every
-// (query, candidate) combination.  With FIX the values come from the integer
+//      and product for those pairs only, until fewer than CARRY of the lanes
+//      have any left; those are carried into the next tile's walk.
+// A walk to the end of every tile costs the largest of 32 neighbour counts, of
+// which 56 % of the lanes are busy on average (candidates of a tile lie
+// together, the queries do not); two tiles at a time 74 %: @W_OLD@ -> @W_NEW@ ms
+// for the set below.  With FIX the values come from the integer
 // units (fix64.cuh) and the FP64 pipe is left with one multiply-add a pair: N =
 // 1,048,576 clustered, 1,250 neighbours a row, Wendland: @U_OLD@ -> @U_NEW@ ms.  The distance for the kernel
 // value is |(x_j - image*L) - x_i|, which differs from the reference's
 // x_j - (x_i + image*L) by at most an ulp of the box length (the acceptance
 // decision itself is exact); the row sum order differs from the reference's.
+constexpr int CARRY = 20;  // of 32 lanes: with fewer at work the rest of a tile waits for the next
+
 template <int POL, int KIND, bool FIX>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
     k_pairs_fp64(KParams P) {
   __shared__ WarpSeg seg_all[WARPS_PER_CTA];
-  __shared__ WarpTile64 tile_all[WARPS_PER_CTA];
+  using Tile = WarpTile64<KIND>;
+  __shared__ Tile tile_all[WARPS_PER_CTA];
   static_assert(POL == POL_MATVEC, "the FP64 pair kernel computes matvecs only");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   WarpSeg &ws = seg_all[wid];
-  WarpTile64 &sm = tile_all[wid];
+  Tile &sm = tile_all[wid];
   const FineGrid &fg = P.fg;
   const unsigned lt = (1u << lane) - 1u;
   const int nfull = P.counts[0], nunits = nfull + P.counts[P.all_units ? 1 : 8];
@@ -1417,9 +1429,9 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
     int span = 0;
 #pragma unroll
     for (int e = 0; e < 3; ++e) span = max(span, hi[e] - lo[e] + 2 * fg.K[e] + 2);
-    const float4 bd = span < BAND_TAB ? P.bands[2 * span]
-                                      : tile_band(span, fg, P.r, P.r2, P.r2, 2).a;
-    const float r2lo = bd.x, r2hi = bd.y, r2box = bd.z;
+    const TileBand bd = span < BAND_TAB ? TileBand{P.bands[2 * span], P.bands[2 * span + 1]}
+                                        : tile_band(span, fg, P.r, P.r2, P.r2, 2);
+    const float r2lo = bd.a.x, r2hi = bd.a.y, r2box = bd.a.z, r2mid = bd.b.x, r2half = bd.b.y;
     const D4 xq = P.qpos[qi];
     longlong2 fq = make_longlong2(0, 0);
     long long fqz = 0;
@@ -1430,6 +1442,30 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
     }
     const double si = (KIND == ABX_K_SCALAR_SUM) ? P.s_row[qi] : 0.0;
     double acc = 0.0;
+    const int few = U.y * CARRY / 32;
+    unsigned long long left = 0;  // this lane's neighbours in the tile before
+    int half = 0;                 // 0 or STAGE: the slots of the tile being staged
+    auto evaluate = [&](int j) {  // distance, kernel and product of the pair in slot j
+      double v;
+      if (FIX) {
+        bool near;
+        v = fix_value<KIND>(fx::diff(sm.ux[j], fq.x), fx::diff(sm.uy[j], fq.y),
+                            fx::diff(sm.uz[j], fqz), P, tab, near);
+        if (KIND == ABX_K_LAPLACE && near) {
+          const int2 mt = sm.meta[j & (Tile::METAS * STAGE - 1)];
+          int img[3], du0, du1;
+          unpack_seg(mt.y, img, du0, du1);
+          v = pair64<KIND>(xq, P.cpos[mt.x], img, P, 0.0, 0.0);
+        }
+      } else {
+        const double dx = __longlong_as_double(sm.ux[j]) - xq.x,
+                     dy = __longlong_as_double(sm.uy[j]) - xq.y,
+                     dz = __longlong_as_double(sm.uz[j]) - xq.z;
+        v = kern64<KIND>(fma(dz, dz, fma(dy, dy, dx * dx)), P, si,
+                         KIND == ABX_K_SCALAR_SUM ? sm.s[j] : 0.0);
+      }
+      acc = fma(v, sm.b[j], acc);
+    };
 
     for (int row0 = 0; row0 < nrows; row0 += 32) {
       const int nseg = build_segments(P, lo, hi, a0, a1, R1, nrows, row0, ws, lane);
@@ -1478,80 +1514,110 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
             const int slot = nt + __popc(km & lt);
             int img[3], du0, du1;
             unpack_seg(ws.seg[sx[sub]].z, img, du0, du1);
-            sm.pf[slot] = st;
+            float *xy = reinterpret_cast<float *>(&sm.pxy[slot >> 1]) + (slot & 1);
+            xy[0] = st.x;
+            xy[2] = st.y;
+            reinterpret_cast<float *>(sm.pz)[slot] = st.z;
+            const int at = half + slot;
             if (FIX) {
               const longlong2 f = P.fxy[k];
-              sm.ux[slot] = fx::diff(f.x, img[0] * P.Lfix[0]);
-              sm.uy[slot] = fx::diff(f.y, img[1] * P.Lfix[1]);
-              sm.uz[slot] = fx::diff(P.fz[k], img[2] * P.Lfix[2]);
+              sm.ux[at] = fx::diff(f.x, img[0] * P.Lfix[0]);
+              sm.uy[at] = fx::diff(f.y, img[1] * P.Lfix[1]);
+              sm.uz[at] = fx::diff(P.fz[k], img[2] * P.Lfix[2]);
             } else {
               const D4 pj = P.cpos[k];
-              sm.ux[slot] = __double_as_longlong(__dsub_rn(pj.x, (double)img[0] * fg.L[0]));
-              sm.uy[slot] = __double_as_longlong(__dsub_rn(pj.y, (double)img[1] * fg.L[1]));
-              sm.uz[slot] = __double_as_longlong(__dsub_rn(pj.z, (double)img[2] * fg.L[2]));
+              sm.ux[at] = __double_as_longlong(__dsub_rn(pj.x, (double)img[0] * fg.L[0]));
+              sm.uy[at] = __double_as_longlong(__dsub_rn(pj.y, (double)img[1] * fg.L[1]));
+              sm.uz[at] = __double_as_longlong(__dsub_rn(pj.z, (double)img[2] * fg.L[2]));
             }
-            sm.b[slot] = P.b64[k];
-            if (KIND == ABX_K_SCALAR_SUM) sm.s[slot] = P.s_col[k];
-            sm.meta[slot] = make_int2(k, sx[sub]);
+            sm.b[at] = P.b64[k];
+            if (KIND == ABX_K_SCALAR_SUM) sm.s[at] = P.s_col[k];
+            sm.meta[at & (Tile::METAS * STAGE - 1)] = make_int2(k, ws.seg[sx[sub]].z);
           }
           nt += __popc(km);
         }
         __syncwarp();
+        if (lane == 0 && (nt & 1)) {  // an odd tail is paired with a candidate at infinity
+          float *xy = reinterpret_cast<float *>(&sm.pxy[nt >> 1]);
+          xy[1] = xy[3] = __int_as_float(0x7f800000);
+          reinterpret_cast<float *>(sm.pz)[nt] = __int_as_float(0x7f800000);
+        }
+        __syncwarp();
         // (1) this lane's neighbours among the nt staged candidates
-        unsigned m0 = 0u, m1 = 0u, band0 = 0u, band1 = 0u;
+        unsigned long long mask = 0;
         if (active) {
-          for (int j = 0; j < nt; ++j) {
-            const float4 c = sm.pf[j];
-            const float d0 = c.x - pq0, d1 = c.y - pq1, d2v = c.z - pq2;
-            const float dd = fmaf(d2v, d2v, fmaf(d1, d1, d0 * d0));
-            const unsigned in = dd <= r2lo ? 1u : 0u;
-            const unsigned bd = (dd > r2lo && dd <= r2hi) ? 1u : 0u;
-            if (j < 32) {
-              m0 |= in << j;
-              band0 |= bd << j;
-            } else {
-              m1 |= in << (j - 32);
-              band1 |= bd << (j - 32);
+          const float2 nqx = make_float2(-pq0, -pq0), nqy = make_float2(-pq1, -pq1),
+                       nqz = make_float2(-pq2, -pq2), nmid = make_float2(-r2mid, -r2mid);
+          float least = r2half + r2half;
+          unsigned word[2] = {0u, 0u};
+          const int npair = (nt + 1) >> 1;
+#pragma unroll
+          for (int w = 0; w < 2; ++w) {
+            const int n16 = min(max(npair - 16 * w, 0), 16);
+#pragma unroll 4
+            for (int h = 0; h < n16; ++h) {
+              const float4 A = sm.pxy[16 * w + h];
+              const float2 B = sm.pz[16 * w + h];
+              const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nqx);
+              const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nqy);
+              const float2 dz = __fadd2_rn(B, nqz);
+              float2 dd = __fmul2_rn(dx, dx);
+              dd = __ffma2_rn(dy, dy, dd);
+              dd = __ffma2_rn(dz, dz, dd);
+              const float2 off = __fadd2_rn(dd, nmid);
+              word[w] = __funnelshift_l(__float_as_uint(off.x), word[w], 1);
+              word[w] = __funnelshift_l(__float_as_uint(off.y), word[w], 1);
+              least = fminf(least, fminf(fabsf(off.x), fabsf(off.y)));
             }
+            // the first candidate's sign to bit 0
+            if (n16) word[w] = __brev(word[w] << (32 - 2 * n16));
           }
-        }
-        // rare: the reference's exact FP64 test for pairs in the band
-        while (band0 | band1) {
-          const int j = band0 ? __ffs(band0) - 1 : 32 + __ffs(band1) - 1;
-          if (j < 32) band0 &= band0 - 1u; else band1 &= band1 - 1u;
-          const int2 mt = sm.meta[j];
-          int img[3], du0, du1;
-          unpack_seg(ws.seg[mt.y].z, img, du0, du1);
-          if (!(exact_d2(xq, P.cpos[mt.x], img, fg) > P.r2)) {
-            if (j < 32) m0 |= 1u << j; else m1 |= 1u << (j - 32);
-          }
-        }
-        // (2) distance, kernel and product for this lane's neighbours
-        while (m0 | m1) {
-          const int j = m0 ? __ffs(m0) - 1 : 32 + __ffs(m1) - 1;
-          if (j < 32) m0 &= m0 - 1u; else m1 &= m1 - 1u;
-          double v;
-          if (FIX) {
-            bool near;
-            v = fix_value<KIND>(fx::diff(sm.ux[j], fq.x), fx::diff(sm.uy[j], fq.y),
-                                fx::diff(sm.uz[j], fqz), P, tab, near);
-            if (KIND == ABX_K_LAPLACE && near) {
-              const int2 mt = sm.meta[j];
+          mask = word[0] | (unsigned long long)word[1] << 32;
+          if (least <= r2half) {  // rare: the reference's exact FP64 test for pairs in the band
+            for (int j = 0; j < nt; ++j) {
+              const float *xy = reinterpret_cast<const float *>(&sm.pxy[j >> 1]) + (j & 1);
+              const float d0 = xy[0] - pq0, d1 = xy[2] - pq1,
+                          d2v = reinterpret_cast<const float *>(sm.pz)[j] - pq2;
+              const float dd = fmaf(d2v, d2v, fmaf(d1, d1, d0 * d0));
+              if (!(fabsf(dd - r2mid) <= r2half) && !(dd > r2lo && dd <= r2hi)) continue;
+              const int2 mt = sm.meta[(half + j) & (Tile::METAS * STAGE - 1)];
               int img[3], du0, du1;
-              unpack_seg(ws.seg[mt.y].z, img, du0, du1);
-              v = pair64<KIND>(xq, P.cpos[mt.x], img, P, 0.0, 0.0);
+              unpack_seg(mt.y, img, du0, du1);
+              const bool in = !(exact_d2(xq, P.cpos[mt.x], img, fg) > P.r2);
+              mask = in ? mask | 1ull << j : mask & ~(1ull << j);
             }
-          } else {
-            const double dx = __longlong_as_double(sm.ux[j]) - xq.x,
-                         dy = __longlong_as_double(sm.uy[j]) - xq.y,
-                         dz = __longlong_as_double(sm.uz[j]) - xq.z;
-            v = kern64<KIND>(fma(dz, dz, fma(dy, dy, dx * dx)), P, si, sm.s[j]);
           }
-          acc = fma(v, sm.b[j], acc);
         }
+        // (2) what is left of the tile before, together with this one's
+        while (__any_sync(0xffffffffu, left != 0)) {
+          const bool old = left != 0;
+          unsigned long long &from = old ? left : mask;
+          if (from != 0) {
+            const int j = __ffsll((long long)from) - 1;
+            from &= from - 1;
+            evaluate((old ? half ^ STAGE : half) + j);
+          }
+        }
+        while (__popc(__ballot_sync(0xffffffffu, mask != 0)) > few) {
+          if (mask != 0) {
+            const int j = __ffsll((long long)mask) - 1;
+            mask &= mask - 1;
+            evaluate(half + j);
+          }
+        }
+        left = mask;
+        half ^= STAGE;
         __syncwarp();
       }
     }
+    while (__any_sync(0xffffffffu, left != 0)) {
+      if (left != 0) {
+        const int j = __ffsll((long long)left) - 1;
+        left &= left - 1;
+        evaluate((half ^ STAGE) + j);
+      }
+    }
+    __syncwarp();
     if (active) P.c[P.qperm[qi]] = acc;
   }
 }
