@@ -132,11 +132,9 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
                                                   const int64_t *__restrict__ dom_mat,
                                                   const int *__restrict__ dom_size,
                                                   const int *__restrict__ dom_off,
-                                                  int *__restrict__ piv, int *__restrict__ info,
-                                                  int above) {
+                                                  int *__restrict__ piv, int *__restrict__ info) {
   const int d = blockIdx.x;
   const int n = dom_size[d];
-  if (n <= above) return;  // k_lu_fix's
   double *A = mat + dom_mat[d];
   int *pv = piv + dom_off[d];
   __shared__ double red_v[LU_T / 32];
@@ -266,13 +264,12 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // in a panel grows with its width); an update converts its sums and subtracts
 // them, two FP64 operations an entry, so the trailing matrix is updated for 64
 // columns at a time and only the rows and columns of those 64 panel by panel.
-// Pivots are compared as integers.  Blocks of more than FL_MAX rows keep k_lu_fp64.  256 domains of 703 rows on average (set-up and one
+// Pivots are compared as integers. 256 domains of 703 rows on average (set-up and one
 // apply): 98 -> @LU_NEW@ ms.
 constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
 constexpr int FW = 16;         // panel width
 constexpr int FB = 64;         // columns of a trailing update
 constexpr int PLD = FW + 1;    // panel row stride
-constexpr int FL_MAX = 1600;   // rows of a block (le, ue)
 // rows of a panel in shared memory, so that two CTAs share an SM (one leaves the
 // integer pipe waiting: 40 ms); the few rows of larger blocks stay in L2
 constexpr int FL_ROWS = 712;
@@ -427,7 +424,6 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
   const int rank = (int)cl.block_rank(), ranks = (int)cl.num_blocks();
   const int d = blockIdx.x / ranks;
   const int n = dom_size[d];
-  if (n > FL_MAX) return;  // k_lu_fp64's
   double *A = mat + dom_mat[d];
   int *pv = piv + dom_off[d];
   short *le = exps + dom_off[d], *ue = le + nexp;  // exponents of L's rows, of U's columns
@@ -837,7 +833,7 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
     cudaMemcpyAsync(S->idx.ptr, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, s);
     if ((st = launch_assemble(ctx, *S, p, op->k, op->radius, size))) return fail(st);
     // blocks of kernel values of one size: integer update (k_lu_fix); kernels
-    // whose values span many magnitudes, and blocks beyond its panel: FP64
+    // whose values span many magnitudes: FP64
     const bool flat = op->k.kind == ABX_K_GAUSSIAN || op->k.kind == ABX_K_COMPACT_GAUSSIAN ||
                       op->k.kind == ABX_K_WENDLAND_C2;
     if (flat) {
@@ -869,10 +865,9 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
       }
       // (exps is freed once the kernel is done: cudaFree waits)
     }
-    if (!flat || S->max_size > FL_MAX)
+    if (!flat)
       k_lu_fp64<<<S->ndom, LU_T, 0, s>>>(S->mat.ptr, S->dom_mat.ptr, S->dom_size.ptr,
-                                          S->dom_off.ptr, S->piv.ptr, S->info.ptr,
-                                          flat ? FL_MAX : 0);
+                                          S->dom_off.ptr, S->piv.ptr, S->info.ptr);
     if (cudaGetLastError() != cudaSuccess) {
       set_error("LU launch failed");
       return fail(ABX_ERR_CUDA);
