@@ -150,8 +150,11 @@ FX_HD u64 sq_low(i64 d) {
 }
 // The sum in units of u^2 2^64 for coordinates in units of u ...
 FX_HD u64 sq_sum(i64 S, i64 T) { return (u64)S + (u64)(T >> 31); }
-// ... and with three bits more (a sum below 2^60 of those units).
-FX_HD u64 sq_sum8(i64 S, i64 T) { return ((u64)S << 3) + (u64)(T >> 28); }
+// ... and with three bits more (a sum below 2^60 of those units), for which the
+// low parts' squares L (sq_low) count too.
+FX_HD u64 sq_sum8(i64 S, i64 T, u64 L) {
+  return ((u64)S << 3) + (u64)((T + (i64)(L >> 31)) >> 28);
+}
 
 FX_HD float rsqrt32(float x) {
 #ifdef __CUDA_ARCH__
@@ -349,7 +352,7 @@ FX_HD double laplace(u64 n, int z, u64 P0, int r) {
   return make_double61(join(Y0, 0) + (u64)add, 63 - y + r);
 }
 
-// sqrt(d^2 + c): v = (d^2 + c) / R^2 in units of 2^-63, 2^-8 <= v 2^-63 < 1;
+// sqrt(d^2 + c): v = (d^2 + c) / R^2 in units of 2^-63, 2^-10 <= v 2^-63 < 1;
 // R = 2^r.
 FX_HD double multiquadric(u64 v, int r) {
   const int k = (clz32(hi32(v)) - 1) | 1;
@@ -392,7 +395,8 @@ FX_HD double scale56(int e) {
 //   Gaussian      t = p0 d^2 log2(e) must stay below 255 (at 16 and above the
 //                 coordinates' 63 bits overflow);
 //   Wendland      q must stay below 1.99 (the same);
-//   multiquadric  p0 >= R^2 / 256: sqrt60 loses relative accuracy below;
+//   multiquadric  p0 >= R^2 / 1024: the sum's units show at distance 0 below (at
+//                 the limit 2^-52.4 at most and 2^-53.6 rms, as in FP64);
 //   Laplace       0 <= p0 < R.
 // R = 2^r: the power of two above the reach (above sqrt(reach^2 + p0)).
 struct Unit {
@@ -430,7 +434,7 @@ template <int KIND> FX_HD Unit make_unit(double p0, double reach) {
   } else {
     U.k = 62 - e;
     if (KIND == MULTIQUADRIC) {
-      if (p0 < ldexp(1.0, 2 * e - 8)) return U;
+      if (p0 < ldexp(1.0, 2 * e - 10)) return U;
       U.c = (u64)ldexp(p0, 63 - 2 * e);
     } else if (KIND == LAPLACE) {
       if (p0 >= ldexp(1.0, e)) return U;
@@ -461,10 +465,13 @@ FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 
   if (dims > 1) sq_acc(dy, S, T);
   if (dims > 2) sq_acc(dz, S, T);
   near = false;
-  if (KIND == LAPLACE) {
-    u64 U = sq_low(dx);
+  u64 U = 0;
+  if (KIND == LAPLACE || KIND == MULTIQUADRIC) {
+    U = sq_low(dx);
     if (dims > 1) U += sq_low(dy);
     if (dims > 2) U += sq_low(dz);
+  }
+  if (KIND == LAPLACE) {
     if ((S | T) == 0 && U == 0) return C.k0;
     near = !laplace_far(S);
     int z;
@@ -472,7 +479,7 @@ FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 
     return laplace(n, z, C.c, C.r);
   }
   if (KIND == WENDLAND) return wendland(sq_sum(S, T));
-  if (KIND == MULTIQUADRIC) return multiquadric(sq_sum8(S, T) + C.c, C.r);
+  if (KIND == MULTIQUADRIC) return multiquadric(sq_sum8(S, T, U) + C.c, C.r);
   return exp2_neg(sq_sum(S, T), tab);
 }
 
