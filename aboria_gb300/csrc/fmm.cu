@@ -111,6 +111,7 @@ struct FmmPlan {
   DevBuf<int> mi_d;                 // ncheb x 3 multi-indices
   DevBuf<int> tile_mat, tile_first; // tensor-core M2L tiles
   int ntiles = 0;
+  int sms = 1;  // of the plan's GPU
 };
 
 void fmm_plan_free(FmmPlan *P) { delete P; }
@@ -320,47 +321,69 @@ __global__ void __launch_bounds__(FT) k_p2m32(int D, int n, int ncheb, const int
 // L2L: G[c][i] += sum_j Tc[o][j][i] G[p][j]   (each child once).
 // T is the compute type: double in FP64 mode; float in mixed mode (FP32
 // copies of the matrices, FP32 sums of ncheb terms, FP64 storage).
+// JS threads a row share its ncheb terms, and a term's NBL inputs are one or two
+// vector reads: a row's walk of 343 loads from L2 is what a level with few links
+// takes (8 batches of order 7: @J_OLD@ -> @J_NEW@ us), the reads of single inputs
+// what one with many does (4,096 batches: @K_OLD@ -> @K_NEW@ us).
 constexpr int NBL = 8;  // links per M2M / L2L batch
+constexpr int JS = 4;
 template <typename T, bool M2M>
-__global__ void __launch_bounds__(FT) k_m2m_l2l(int ncheb, const int *__restrict__ links,
-                                                const int2 *__restrict__ batches,
-                                                const T *__restrict__ Tm_all,
-                                                double *__restrict__ V) {
+__global__ void __launch_bounds__(FT * JS) k_m2m_l2l(int ncheb, const int *__restrict__ links,
+                                                     const int2 *__restrict__ batches,
+                                                     const T *__restrict__ Tm_all,
+                                                     double *__restrict__ V) {
   const int2 bt = batches[blockIdx.x];
-  __shared__ T vin[NBL][MAXC];
+  // inputs [j][link]; then the partial sums of all threads of a row but the first
+  __shared__ __align__(16) T vin[MAXC][NBL];
+  static_assert(MAXC >= (JS - 1) * FT, "the partial sums fit into the inputs' place");
   __shared__ int sout[NBL];
   const int o = links[3 * bt.x + 2];
   // M2M reads the children and writes the parents; L2L the other way round
-  for (int e = threadIdx.x; e < NBL * ncheb; e += FT) {
+  for (int e = threadIdx.x; e < NBL * ncheb; e += FT * JS) {
     const int b = e / ncheb, j = e - b * ncheb;
     T v = 0;
     if (b < bt.y) {
       const int nd = links[3 * (bt.x + b) + (M2M ? 1 : 0)];
       v = (T)V[(size_t)nd * ncheb + j];
     }
-    vin[b][j] = v;
+    vin[j][b] = v;
   }
   if (threadIdx.x < bt.y) sout[threadIdx.x] = links[3 * (bt.x + threadIdx.x) + (M2M ? 0 : 1)];
   __syncthreads();
   const T *Tm = Tm_all + (size_t)o * ncheb * ncheb;  // [j][i]
-  const int i = blockIdx.y * FT + threadIdx.x;
+  const int it = threadIdx.x % FT, js = threadIdx.x / FT, i = blockIdx.y * FT + it;
+  T a[NBL];
+#pragma unroll
+  for (int b = 0; b < NBL; ++b) a[b] = 0;
   if (i < ncheb) {
-    T a[NBL];
-#pragma unroll
-    for (int b = 0; b < NBL; ++b) a[b] = 0;
-#pragma unroll 4
-    for (int j = 0; j < ncheb; ++j) {
+#pragma unroll 8
+    for (int j = js; j < ncheb; j += JS) {
       const T t = Tm[(size_t)j * ncheb + i];
+      T in[NBL];
+      constexpr int V16 = 16 / sizeof(T);
 #pragma unroll
-      for (int b = 0; b < NBL; ++b) a[b] += t * vin[b][j];
-    }
+      for (int q = 0; q < NBL / V16; ++q)
+        *reinterpret_cast<int4 *>(&in[q * V16]) = *reinterpret_cast<const int4 *>(&vin[j][q * V16]);
 #pragma unroll
-    for (int b = 0; b < NBL; ++b) {
-      if (b >= bt.y) break;
-      double *dst = &V[(size_t)sout[b] * ncheb + i];
-      if (M2M) atomicAdd(dst, (double)a[b]);
-      else *dst += (double)a[b];
+      for (int b = 0; b < NBL; ++b) a[b] += t * in[b];
     }
+  }
+  __syncthreads();
+  T(*part)[NBL] = vin;
+  if (js > 0)
+#pragma unroll
+    for (int b = 0; b < NBL; ++b) part[(js - 1) * FT + it][b] = a[b];
+  __syncthreads();
+  if (js > 0 || i >= ncheb) return;
+  for (int q = 0; q < JS - 1; ++q)
+#pragma unroll
+    for (int b = 0; b < NBL; ++b) a[b] += part[q * FT + it][b];
+#pragma unroll
+  for (int b = 0; b < NBL; ++b) {
+    if (b >= bt.y) break;
+    double *dst = &V[(size_t)sout[b] * ncheb + i];
+    if (M2M) atomicAdd(dst, (double)a[b]);
+    else *dst += (double)a[b];
   }
 }
 
@@ -1394,28 +1417,36 @@ __global__ void __launch_bounds__(PT * PW) k_l2p64(
   }
 }
 
-// P2P in FP64 accuracy on the integer units, added to the L2P result: one warp
-// per target leaf, one lane per target.  Leaves hold 32 targets on average and
+// Leaves an SM from which 4 warps work a leaf, below 16: 512 leaves (20,000 points
+// in 3-D) 618 us the whole product with 4, 505 with 16; 1,024 (30,000 in 2-D) 303
+// with 4, 374 with 16.
+constexpr int64_t P2P_LEAVES4 = 5;
+// P2P in FP64 accuracy on the integer units, added to the L2P result: WPL warps,
+// a CTA, per target leaf, each taking every WPL-th tile of its sources; one lane
+// per target.  Leaves hold 32 targets on average and
 // a third of them a few more than 32: a last tile of r <= 16 targets is worked
 // by 32 / p lanes a target (p the power of two above r), each taking every
 // (32 / p)-th source, and the lanes' sums are added.  N = 1,048,576 uniform,
 // Laplace, order 3: the whole product @F_OLD@ -> @F_NEW@ ms.
-template <int KIND>
-__global__ void __launch_bounds__(PT * PW) k_p2p_fix(
-    int D, int nleaves, const int *__restrict__ leaves, const int *__restrict__ nb,
+// With a warp a leaf few leaves left most of the GPU idle while a warp walked 400
+// sources (12,934 points in 2-D, 581 -> 308 us the whole product), and many a
+// last wave of long leaves (1,048,576 in 3-D, 10.9 -> 10.5 ms).
+template <int KIND, int WPL>
+__global__ void __launch_bounds__(PT * WPL) k_p2p_fix(
+    int D, const int *__restrict__ leaves, const int *__restrict__ nb,
     const int *__restrict__ ne, const double *__restrict__ pos, int64_t npos,
     const longlong2 *__restrict__ fxy, const long long *__restrict__ fz,
     const double *__restrict__ b, const int *__restrict__ rp, const int *__restrict__ src, double p0,
     const fx::Consts C, double *__restrict__ c) {
-  __shared__ longlong2 sxy_all[PW][PT], szb_all[PW][PT];
+  __shared__ longlong2 sxy_all[WPL][PT], szb_all[WPL][PT];
+  __shared__ double part[WPL][PT];
   __shared__ fx::u64 tab[KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
   if (KIND == ABX_K_GAUSSIAN) {
-    for (int i = threadIdx.x; i < fx::EXP_TAB; i += PT * PW) tab[i] = fx::exp_table.v[i];
+    for (int i = threadIdx.x; i < fx::EXP_TAB; i += PT * WPL) tab[i] = fx::exp_table.v[i];
     __syncthreads();
   }
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-  const int li = blockIdx.x * PW + wl;
-  if (li >= nleaves) return;  // whole warps: only warp-level synchronisation below
+  const int li = blockIdx.x;
   longlong2 *sxy = sxy_all[wl], *szb = szb_all[wl];
   const int leaf = leaves[li];
   for (int i0 = nb[leaf]; i0 < ne[leaf]; i0 += PT) {
@@ -1431,9 +1462,11 @@ __global__ void __launch_bounds__(PT * PW) k_p2p_fix(
       z = fx::biased(fz[i]);
     }
     double acc = 0.0;
+    int tile = 0;
     for (int e = rp[li]; e < rp[li + 1]; ++e) {
       const int sl = src[e];
       for (int j0 = nb[sl]; j0 < ne[sl]; j0 += PT) {
+        if (tile++ % WPL != wl) continue;
         const int cnt = min(PT, ne[sl] - j0);
         __syncwarp();
         if (lane < cnt) {
@@ -1461,6 +1494,11 @@ __global__ void __launch_bounds__(PT * PW) k_p2p_fix(
       }
     }
     for (int o = p; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    __syncthreads();
+    part[wl][lane] = acc;
+    __syncthreads();
+    if (wl != 0) continue;
+    for (int w = 1; w < WPL; ++w) acc += part[w][lane];
     if (act && grp == 0) c[i] += acc;
   }
 }
@@ -1734,6 +1772,7 @@ int fmm_plan_build(abx_operator *op, int order, FmmPlan *&out, double eta = 1.0)
     return fail(ABX_ERR_CUDA);
   }
   P->max_level.assign(1, maxlev);
+  P->sms = std::max(ctx->num_sms, 1);
   P->build_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   out = P;
   return ABX_OK;
@@ -1759,10 +1798,16 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
     k_l2p64<<<lb, PT * PW, 0, s>>>(P->D, P->n, P->ncheb, P->nleaves, P->leaf_ids.ptr,
                                    P->node_begin.ptr, P->node_end.ptr, P->box.ptr, pos, npos,
                                    P->G.ptr, P->tab, c);
-    k_p2p_fix<FK><<<lb, PT * PW, 0, s>>>(P->D, P->nleaves, P->leaf_ids.ptr, P->node_begin.ptr,
-                                         P->node_end.ptr, pos, npos, P->fxy.ptr, P->fz.ptr, b,
-                                         P->p2p_rowptr.ptr, P->p2p_src.ptr, P->p0,
-                                         fx::consts(P->unit, 1.0 / P->p0), c);
+    auto p2p = [&](auto kernel, int threads) {
+      kernel<<<P->nleaves, threads, 0, s>>>(P->D, P->leaf_ids.ptr, P->node_begin.ptr,
+                                        P->node_end.ptr, pos, npos, P->fxy.ptr, P->fz.ptr, b,
+                                        P->p2p_rowptr.ptr, P->p2p_src.ptr, P->p0,
+                                        fx::consts(P->unit, 1.0 / P->p0), c);
+    };
+    if (P->nleaves >= P->sms * P2P_LEAVES4)
+      p2p(k_p2p_fix<FK, 4>, PT * 4);
+    else
+      p2p(k_p2p_fix<FK, 16>, PT * 16);
   } else
     k_l2p_p2p<KIND, false><<<P->nleaves, FT, 0, s>>>(
         P->D, P->n, P->ncheb, P->leaf_ids.ptr, P->node_begin.ptr, P->node_end.ptr, P->box.ptr, pos,
@@ -1856,10 +1901,10 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
     if (P->batch_cnt[lev] > 0) {
       const int2 *bt = P->batches.ptr + P->batch_off[lev];
       if (mixed)
-        k_m2m_l2l<float, true><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT, 0, s>>>(nc, P->links.ptr, bt,
+        k_m2m_l2l<float, true><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
                                                               P->Tc32T.ptr, P->W.ptr);
       else
-        k_m2m_l2l<double, true><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT, 0, s>>>(nc, P->links.ptr, bt,
+        k_m2m_l2l<double, true><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
                                                                P->TcT.ptr, P->W.ptr);
     }
   ABX_CHECK_CUDA(cudaGetLastError());
@@ -1945,10 +1990,10 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
     if (P->batch_cnt[lev] > 0) {
       const int2 *bt = P->batches.ptr + P->batch_off[lev];
       if (mixed)
-        k_m2m_l2l<float, false><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT, 0, s>>>(nc, P->links.ptr, bt,
+        k_m2m_l2l<float, false><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
                                                                P->Tc32.ptr, P->G.ptr);
       else
-        k_m2m_l2l<double, false><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT, 0, s>>>(nc, P->links.ptr, bt,
+        k_m2m_l2l<double, false><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
                                                                 P->Tc.ptr, P->G.ptr);
     }
   ABX_CHECK_CUDA(cudaGetLastError());
