@@ -321,13 +321,12 @@ __global__ void __launch_bounds__(FT) k_p2m32(int D, int n, int ncheb, const int
 // L2L: G[c][i] += sum_j Tc[o][j][i] G[p][j]   (each child once).
 // T is the compute type: double in FP64 mode; float in mixed mode (FP32
 // copies of the matrices, FP32 sums of ncheb terms, FP64 storage).
-// JS threads a row share its ncheb terms, and a term's NBL inputs are one or two
-// vector reads: a row's walk of 343 loads from L2 is what a level with few links
-// takes (8 batches of order 7: @J_OLD@ -> @J_NEW@ us), the reads of single inputs
-// what one with many does (4,096 batches: @K_OLD@ -> @K_NEW@ us).
+// JS threads a row share its ncheb terms, and a term's NBL inputs are vector
+// reads.  A row's walk of 343 loads from L2 is what a level with few links takes:
+// four threads a row there (8 batches of order 7: 91 -> 40 us); with links enough
+// the shared sums only cost (4,096 batches: @K1@ us with one, 936 with four).
 constexpr int NBL = 8;  // links per M2M / L2L batch
-constexpr int JS = 4;
-template <typename T, bool M2M>
+template <typename T, bool M2M, int JS>
 __global__ void __launch_bounds__(FT * JS) k_m2m_l2l(int ncheb, const int *__restrict__ links,
                                                      const int2 *__restrict__ batches,
                                                      const T *__restrict__ Tm_all,
@@ -370,7 +369,7 @@ __global__ void __launch_bounds__(FT * JS) k_m2m_l2l(int ncheb, const int *__res
   }
   __syncthreads();
   T(*part)[NBL] = vin;
-  if (js > 0)
+  if (JS > 1 && js > 0)
 #pragma unroll
     for (int b = 0; b < NBL; ++b) part[(js - 1) * FT + it][b] = a[b];
   __syncthreads();
@@ -1817,6 +1816,19 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
 }
 }  // namespace
 
+// One level's M2M or L2L.  Threads a row: see k_m2m_l2l; the line at 32 CTAs an SM
+// lies between 1,536 CTAs (order 7: four threads 110 us M2M, one 159) and 12,288.
+template <typename T, bool M2M>
+void launch_links(const FmmPlan *P, int lev, const T *mats, double *V, cudaStream_t s) {
+  if (P->batch_cnt[lev] == 0) return;
+  const dim3 grid(P->batch_cnt[lev], ceil_div(P->ncheb, FT));
+  const int2 *bt = P->batches.ptr + P->batch_off[lev];
+  if ((int64_t)grid.x * grid.y < 8 * (int64_t)P->sms)
+    k_m2m_l2l<T, M2M, 4><<<grid, 4 * FT, 0, s>>>(P->ncheb, P->links.ptr, bt, mats, V);
+  else
+    k_m2m_l2l<T, M2M, 1><<<grid, FT, 0, s>>>(P->ncheb, P->links.ptr, bt, mats, V);
+}
+
 namespace {
 // The FP64 M2L: G += K W.  The split matrices and the tiles of 64 pairs are made
 // by the plan's first FP64 product.
@@ -1897,16 +1909,10 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
                                       P->mi_d.ptr, P->tab, P->W.ptr);
   }
   const int maxlev = P->max_level.empty() ? 0 : P->max_level[0];
-  for (int lev = maxlev; lev >= 1; --lev)
-    if (P->batch_cnt[lev] > 0) {
-      const int2 *bt = P->batches.ptr + P->batch_off[lev];
-      if (mixed)
-        k_m2m_l2l<float, true><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
-                                                              P->Tc32T.ptr, P->W.ptr);
-      else
-        k_m2m_l2l<double, true><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
-                                                               P->TcT.ptr, P->W.ptr);
-    }
+  for (int lev = maxlev; lev >= 1; --lev) {
+    if (mixed) launch_links<float, true>(P, lev, P->Tc32T.ptr, P->W.ptr, s);
+    else launch_links<double, true>(P, lev, P->TcT.ptr, P->W.ptr, s);
+  }
   ABX_CHECK_CUDA(cudaGetLastError());
   if (P->n_m2l > 0) {
     if (mixed) {
@@ -1986,16 +1992,10 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
     }
     ABX_CHECK_CUDA(cudaGetLastError());
   }
-  for (int lev = 1; lev <= maxlev; ++lev)
-    if (P->batch_cnt[lev] > 0) {
-      const int2 *bt = P->batches.ptr + P->batch_off[lev];
-      if (mixed)
-        k_m2m_l2l<float, false><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
-                                                               P->Tc32.ptr, P->G.ptr);
-      else
-        k_m2m_l2l<double, false><<<dim3(P->batch_cnt[lev], ceil_div(nc, FT)), FT * JS, 0, s>>>(nc, P->links.ptr, bt,
-                                                                P->Tc.ptr, P->G.ptr);
-    }
+  for (int lev = 1; lev <= maxlev; ++lev) {
+    if (mixed) launch_links<float, false>(P, lev, P->Tc32.ptr, P->G.ptr, s);
+    else launch_links<double, false>(P, lev, P->Tc.ptr, P->G.ptr, s);
+  }
   ABX_CHECK_CUDA(cudaGetLastError());
   if (P->nleaves == 0) return ABX_OK;
   switch (P->kind) {

