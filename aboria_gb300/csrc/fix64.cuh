@@ -153,7 +153,7 @@ FX_HD u64 sq_sum(i64 S, i64 T) { return (u64)S + (u64)(T >> 31); }
 // ... and with three bits more (a sum below 2^60 of those units), for which the
 // low parts' squares L (sq_low) count too.
 FX_HD u64 sq_sum8(i64 S, i64 T, u64 L) {
-  return ((u64)S << 3) + (u64)((T + (i64)(L >> 31)) >> 28);
+  return ((u64)S << 3) + (u64)((T + (i64)(L >> 33)) >> 28);
 }
 
 FX_HD float rsqrt32(float x) {

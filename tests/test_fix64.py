@@ -35,6 +35,22 @@ double v_wend(const double *x, const double *y, int dim, double reach, double p0
 double v_lap(const double *x, const double *y, int dim, double reach, double p0) {
   return run<LAPLACE>(x, y, dim, reach, p0);
 }
+// sum of n products of scaled 56-bit numbers
+double dot56(const double *x, const double *y, int n) {
+  u64 mx = 0, my = 0;
+  for (int i = 0; i < n; ++i) {
+    mx = abs_bits(x[i]) > mx ? abs_bits(x[i]) : mx;
+    my = abs_bits(y[i]) > my ? abs_bits(y[i]) : my;
+  }
+  const int ex = scale_exp(mx), ey = scale_exp(my);
+  i64 hi = 0, mid = 0;
+  for (int i = 0; i < n; ++i) {
+    const Half2 a = split56(x[i], ex), b = split56(y[i], ey);
+    hi += (i64)a.h * b.h;
+    mid += (i64)a.h * b.l + (i64)a.l * b.h;
+  }
+  return (double)sum56(hi, mid) * scale56(ex + ey);
+}
 double v_mq(const double *x, const double *y, int dim, double reach, double p0) {
   return run<MULTIQUADRIC>(x, y, dim, reach, p0);
 }
@@ -51,7 +67,7 @@ def lib(tmp_path_factory):
                     str(ROOT / "aboria_gb300" / "csrc"), str(d / "fix64_host.cpp"), "-o", str(so)],
                    check=True)
     lib = C.CDLL(str(so))
-    for f in ("v_gauss", "v_wend", "v_lap", "v_mq"):
+    for f in ("v_gauss", "v_wend", "v_lap", "v_mq", "dot56"):
         getattr(lib, f).restype = C.c_double
     return lib
 
@@ -73,7 +89,7 @@ def _exact(kind, x, y, p0):
 
 @pytest.mark.parametrize("kind,p0r2", [("gauss", 4.0), ("gauss", 21.0), ("wend", 1.0),
                                        ("lap", 0.0), ("lap", 1e-11), ("lap", 0.02), ("lap", 0.4),
-                                       ("mq", 0.02), ("mq", 0.7)])
+                                       ("mq", 0.005), ("mq", 0.02), ("mq", 0.7)])
 @pytest.mark.parametrize("dim", [1, 2, 3])
 def test_values_within_an_ulp(lib, kind, p0r2, dim):
     rng = random.Random(7 * dim + len(kind))
@@ -109,3 +125,20 @@ def test_limits(lib):
     assert lib.v_wend(x, far, 1, C.c_double(0.5), C.c_double(2.0)) == 0.0     # q = 1
     assert lib.v_mq(x, x, 1, C.c_double(0.5), C.c_double(0.25)) == 0.5
     assert lib.v_lap(x, x, 1, C.c_double(0.5), C.c_double(0.125)) == 8.0
+
+
+@pytest.mark.parametrize("n", [1, 2, 16, 63, 64])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -300, 2.0 ** 300])
+def test_scaled_products(lib, n, scale):
+    """n products: each operand good to 2^-57 of the largest, the low parts'
+    products (2^-58) left out, one rounding of the sum."""
+    rng = random.Random(n)
+    for _ in range(200):
+        x = [rng.choice([-1, 1]) * rng.random() * scale * 2.0 ** -rng.randrange(40) for _ in range(n)]
+        y = [rng.choice([-1, 1]) * rng.random() for _ in range(n)]
+        got = lib.dot56((C.c_double * n)(*x), (C.c_double * n)(*y), n)
+        want = sum(Decimal(a) * Decimal(b) for a, b in zip(x, y))
+        big = Decimal(max(map(abs, x))) * Decimal(max(map(abs, y)))
+        # (largest within a factor of two of the unit: 2 x 2 for both)
+        slack = big * 4 * (n * (Decimal(2) ** -57 * 2 + Decimal(2) ** -58) + Decimal(2) ** -56)
+        assert abs(Decimal(got) - want) <= slack + abs(want) * Decimal(2) ** -52
