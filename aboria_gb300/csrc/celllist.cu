@@ -12,7 +12,8 @@
 //  2. k_cl_onesweep  one launch per 10-bit digit of a stable LSD radix sort:
 //                    tiles claimed in order, per-tile digit counts published
 //                    and prefixed by decoupled look-back (no histogram scan
-//                    launches).
+//                    launches).  Up to 524,288 particles the sort of
+//                    primitives.cu instead, and no histograms in 1.
 //  3. k_cl_ranges    bucket_begin/bucket_end of every cell straight from the
 //                    sorted keys (each boundary between two keys writes the
 //                    cells in its gap; no memset, no scan).

@@ -150,10 +150,10 @@ FX_HD u64 sq_low(i64 d) {
 }
 // The sum in units of u^2 2^64 for coordinates in units of u ...
 FX_HD u64 sq_sum(i64 S, i64 T) { return (u64)S + (u64)(T >> 31); }
-// ... and with three bits more (a sum below 2^60 of those units), for which the
-// low parts' squares L (sq_low) count too.
-FX_HD u64 sq_sum8(i64 S, i64 T, u64 L) {
-  return ((u64)S << 3) + (u64)((T + (i64)(L >> 33)) >> 28);
+// ... and with BITS bits more (a sum below 2^(63 - BITS) of those units), for which
+// the low parts' squares L (sq_low) count too.
+template <int BITS> FX_HD u64 sq_sum_low(i64 S, i64 T, u64 L) {
+  return ((u64)S << BITS) + (u64)((T + (i64)(L >> 33)) >> (31 - BITS));
 }
 
 FX_HD float rsqrt32(float x) {
@@ -392,8 +392,9 @@ FX_HD double scale56(int e) {
 // The fixed point of one kernel for pairs up to `reach` apart: coordinates
 // X = x f 2^k, and the kernel's constant.  ok false: the kernel's
 // parameter or the reach is outside what the value functions cover --
-//   Gaussian      t = p0 d^2 log2(e) must stay below 255 (at 16 and above the
-//                 coordinates' 63 bits overflow);
+//   Gaussian      t = p0 d^2 log2(e) must stay below 1020, where the value is
+//                 normal; from 255 on, where 63 bits hold no difference in
+//                 units of 2^-59, units of 2^-58 (r = 1);
 //   Wendland      q must stay below 1.99 (the same);
 //   multiquadric  p0 >= R^2 / 1024: the sum's units show at distance 0 below (at
 //                 the limit 2^-52.4 at most and 2^-53.6 rms, as in FP64);
@@ -419,14 +420,16 @@ template <int KIND> FX_HD Unit make_unit(double p0, double reach) {
   frexp(sqrt(reach2) * (1.0 + 1e-12), &e);
   U.r = e;
   if (KIND == GAUSSIAN) {
-    if (!(p0 > 1e-200) || p0 * reach2 * 1.4426950408889634 >= 255.0) return U;
+    const double most = p0 * reach2 * 1.4426950408889634;
+    if (!(p0 > 1e-200) || !(most < 1020.0)) return U;
     // sqrt(p0 log2(e)) as hi + lo: log2(e) as a sum of two doubles, one
     // Newton step on the square root
     const double l = 1.4426950408889634, m = 2.0355273740931033e-17;
     const double ah = p0 * l, al = fma(p0, l, -ah) + p0 * m;
     const double s = sqrt(ah), lo = (fma(-s, s, ah) + al) / (2.0 * s);
     U.f = make_factor(s + lo, lo - ((s + lo) - s));
-    U.k = 59;  // t = sum X^2 in units of 2^-54
+    U.r = most < 255.0 ? 0 : 1;
+    U.k = U.r ? 58 : 59;  // t = sum X^2 in units of 2^-52 or 2^-54
   } else if (KIND == WENDLAND) {
     if (!(p0 > 1e-100) || p0 * p0 * reach2 >= 3.96) return U;
     U.f = make_factor(p0, 0.0);
@@ -479,8 +482,13 @@ FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 
     return laplace(n, z, C.c, C.r);
   }
   if (KIND == WENDLAND) return wendland(sq_sum(S, T));
-  if (KIND == MULTIQUADRIC) return multiquadric(sq_sum8(S, T, U) + C.c, C.r);
-  return exp2_neg(sq_sum(S, T), tab);
+  if (KIND == MULTIQUADRIC) return multiquadric(sq_sum_low<3>(S, T, U) + C.c, C.r);
+  if (C.r == 0) return exp2_neg(sq_sum(S, T), tab);
+  // wide (make_unit): t = sum X^2 in units of 2^-52
+  U = sq_low(dx);
+  if (dims > 1) U += sq_low(dy);
+  if (dims > 2) U += sq_low(dz);
+  return exp2_neg(sq_sum_low<2>(S, T, U), tab);
 }
 
 }  // namespace fx

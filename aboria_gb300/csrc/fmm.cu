@@ -10,8 +10,8 @@
 //    (src/detail/FastMultipoleMethod.h:1249-1279), P2P at target leaves over
 //    the connected list (leaf or whole subtree).
 //
-// GB300 design: the traversal runs once per operator on the host and is
-// flattened into per-level lists (M2L pairs, P2P leaf pairs, parent/child
+// GB300 design: the traversal runs once per operator (octree.cu, on the device)
+// and is flattened into per-level lists (M2L pairs, P2P leaf pairs, parent/child
 // links); translation operators are precomputed instead of re-evaluating the
 // kernel at node pairs on every call: one M2M/L2L matrix per child octant
 // (the Chebyshev interpolation is scale invariant) and one M2L matrix per
@@ -19,10 +19,13 @@
 // offset in [-3, 3]^D.  Each matvec is five passes of device kernels: P2M,
 // M2M (bottom-up), M2L, L2L (top-down), then L2P+P2P per target leaf.
 //
-// M2L in the mixed-precision mode runs as a GEMM per (level, offset) on the
-// tensor cores (3xTF32 split with FP32 accumulation, mma.sync m16n8k8):
-//   G[:, targets] += K_o * W[:, sources]  (one CTA per 16-row x 64-target tile)
-// and P2P in FP32; the FP64 mode keeps every pass in FP64.
+// M2L runs as a GEMM per (level, offset):
+//   G[:, targets] += K_o * W[:, sources]
+// in the mixed-precision mode on the tensor cores with FP32 accumulation (split
+// FP16 on tcgen05 above 64 nodes, 3xTF32 on mma.sync below) and P2P in FP32; in
+// the FP64 mode M2L is a product of scaled 56-bit integers and P2P takes its
+// kernel values from the integer units (fix64.cuh), both with errors no larger
+// than FP64's own.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(FT) k_p2m32(int D, int n, int ncheb, const int
 // JS threads a row share its ncheb terms, and a term's NBL inputs are vector
 // reads.  A row's walk of 343 loads from L2 is what a level with few links takes:
 // four threads a row there (8 batches of order 7: 91 -> 40 us); with links enough
-// the shared sums only cost (4,096 batches: @K1@ us with one, 936 with four).
+// the shared sums only cost (4,096 batches: 364 us with one, 936 with four).
 constexpr int NBL = 8;  // links per M2M / L2L batch
 template <typename T, bool M2M, int JS>
 __global__ void __launch_bounds__(FT * JS) k_m2m_l2l(int ncheb, const int *__restrict__ links,
@@ -406,8 +409,8 @@ __global__ void k_transpose_tc(const double *__restrict__ in, int nchild, int nc
 // per plan with a scale per row (Kq, transposed), W per product with a scale per
 // node (Wq); both scales and 57 bits make a term's rounding smaller than the FP64
 // sum's own.  Sums are turned into FP64 every 64 terms, which the 64-bit sums
-// hold.  N = 1,048,576, 6.0e6 pairs: order 3 (27 nodes) 8.5 -> @M3@ ms, order 5
-// (125) @M5A@ -> @M5B@ ms.
+// hold.  N = 1,048,576, 6.0e6 pairs: order 3 (27 nodes) 8.5 -> 2.3 ms; 100,000
+// points, order 5 (125), the whole product 20.8 -> 5.7 ms.
 __global__ void k_split_k(const double *__restrict__ K, int64_t nrows, int ncheb, int ldr,
                           int2 *__restrict__ Kq, short *__restrict__ ke) {
   const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -701,7 +704,8 @@ __global__ void __launch_bounds__(64 * WM) k_m2l_tc2(int ncheb, int ldk, int ldg
 // have, down to 2^-24 of those units (2^-38 of the largest), and a 16-byte
 // chunk, a stage and an MMA hold twice the columns; the tensor pipe's FP16 rate
 // is twice TF32's, and the operands' shared-memory traffic, which bounds
-// 64-pair tiles, is half.  Order 7, N = 1M: @M7A@ -> @M7B@ ms.
+// 64-pair tiles, is half.  Order 7, N = 1M: 10.4 -> 6.2 ms (the loads
+// and the reductions into G alone, without an MMA, take 6.5).
 // The K matrices are packed once per plan into the shared-memory image of a
 // pipeline stage (k_pack_f16), so a stage's A operand is one bulk copy on the
 // TMA engine (cp.async.bulk, completion counted on the stage's `fullA`
@@ -1426,7 +1430,7 @@ constexpr int64_t P2P_LEAVES4 = 5;
 // a third of them a few more than 32: a last tile of r <= 16 targets is worked
 // by 32 / p lanes a target (p the power of two above r), each taking every
 // (32 / p)-th source, and the lanes' sums are added.  N = 1,048,576 uniform,
-// Laplace, order 3: the whole product @F_OLD@ -> @F_NEW@ ms.
+// Laplace, order 3: the whole product 57.2 -> 19.3 ms with this alone.
 // With a warp a leaf few leaves left most of the GPU idle while a warp walked 400
 // sources (12,934 points in 2-D, 581 -> 308 us the whole product), and many a
 // last wave of long leaves (1,048,576 in 3-D, 10.9 -> 10.5 ms).
@@ -1832,7 +1836,8 @@ void launch_links(const FmmPlan *P, int lev, const T *mats, double *V, cudaStrea
 namespace {
 // The FP64 M2L: G += K W.  The split matrices and the tiles of 64 pairs are made
 // by the plan's first FP64 product.
-int m2l_fix(FmmPlan *P, cudaStream_t s) {
+// The split matrices and buffers of the FP64 M2L, once per plan.
+int m2l_fix_prepare(FmmPlan *P, cudaStream_t s) {
   const int nc = P->ncheb, ldr = (nc + 1) / 2 * 2;
   if (!P->Kq.ptr) {
     std::vector<int> mat, first;
@@ -1858,7 +1863,12 @@ int m2l_fix(FmmPlan *P, cudaStream_t s) {
     ABX_CHECK_CUDA(cudaStreamSynchronize(s));  // the host lists end here
   }
   ABX_TRY(P->Wq.reserve((size_t)P->nnodes * nc));
-  ABX_TRY(P->we.reserve((size_t)P->nnodes));
+  return P->we.reserve((size_t)P->nnodes);
+}
+
+int m2l_fix(FmmPlan *P, cudaStream_t s) {
+  const int nc = P->ncheb, ldr = (nc + 1) / 2 * 2;
+  ABX_TRY(m2l_fix_prepare(P, s));
   k_split_w<<<ceil_div((size_t)P->nnodes * 32, 256), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, P->Wq.ptr,
                                                                   P->we.ptr);
   auto run = [&](auto kern, int tr) {
@@ -1874,6 +1884,12 @@ int m2l_fix(FmmPlan *P, cudaStream_t s) {
   return ABX_OK;
 }
 }  // namespace
+
+// What a plan's FP64 products keep: a first product then allocates nothing and
+// waits for nothing.
+int fmm_plan_prepare(FmmPlan *P, cudaStream_t s) {
+  return P->n_m2l > 0 ? m2l_fix_prepare(P, s) : ABX_OK;
+}
 
 // c = K b through the five FMM passes (storage order of the octree set).
 int fmm_matvec_device(abx_operator *op, const double *b, double *c) {

@@ -131,7 +131,7 @@ struct abx_operator {
   abx::PairLayout *pairs = nullptr;
   abx::FmmPlan *fmm = nullptr;
   abx::HostStage stage_b, stage_c;
-  abx::DevBuf<double> partial;  // dense mixed matvec: row sums per column chunk
+  abx::DevBuf<double> partial;  // dense matvec: row sums per column chunk; FP64: the columns
   int64_t last_candidates = 0, last_pairs = 0;
 };
 
@@ -176,4 +176,5 @@ int dense_matvec_device(abx_operator *op, const double *b, double *c);
 // fmm.cu
 int fmm_matvec_device(abx_operator *op, const double *b, double *c);
 void fmm_plan_free(FmmPlan *P);
+int fmm_plan_prepare(FmmPlan *P, cudaStream_t s);
 }  // namespace abx

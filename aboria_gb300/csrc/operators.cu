@@ -75,7 +75,8 @@ template <int KIND> __device__ __forceinline__ float dk32(float d2, float p0f, f
 
 // `F` (may be null): leave at once where k_dense_fix has done the product.  Column
 // chunks (blockIdx.y) as in k_dense_fix: with one CTA per 256 rows, 460 x 1484
-// took 2.0 ms, the latency of 1,484 values one after the other; @DC@ us.
+// took 2.0 ms, the latency of 1,484 values one after the other; with
+// chunks 124 us.
 struct DenseFix;
 __device__ bool dense_fix_done(const DenseFix *F);
 template <int KIND>
@@ -368,6 +369,14 @@ int dense_chunks(abx_context *ctx, int64_t nc, unsigned blocks, int per_sm, int6
   return tiles > 0 ? (int)((nc + chunk_cols - 1) / chunk_cols) : 1;
 }
 
+// Room for an FP64 product of nr x nc.
+int dense_reserve(abx_context *ctx, int64_t nr, int64_t nc, abx_operator *op) {
+  int64_t chunk_cols;
+  const int used = dense_chunks(ctx, nc, ceil_div(nr, DT), 16, chunk_cols);
+  return op->partial.reserve(sizeof(DenseFix) / 8 + 4 + (sizeof(FixCol) / 8) * (size_t)nc +
+                             (used > 1 ? (size_t)used * nr : 0));
+}
+
 template <int KIND>
 int launch_dense_fix(abx_context *ctx, const DenseParams &P, abx_operator *op) {
   cudaStream_t s = ctx->stream;
@@ -376,7 +385,7 @@ int launch_dense_fix(abx_context *ctx, const DenseParams &P, abx_operator *op) {
   const int used = dense_chunks(ctx, P.nc, blocks, 16, chunk_cols);
   // one buffer: the unit, the columns, the chunks' row sums
   const size_t nf = sizeof(DenseFix) / 8 + 4, nb = (sizeof(FixCol) / 8) * (size_t)P.nc;
-  ABX_TRY(op->partial.reserve(nf + nb + (used > 1 ? (size_t)used * P.nr : 0)));
+  ABX_TRY(dense_reserve(ctx, P.nr, P.nc, op));
   DenseFix *F = reinterpret_cast<DenseFix *>(op->partial.ptr);
   FixCol *cols = reinterpret_cast<FixCol *>(op->partial.ptr + (nf / 4) * 4);
   double *partial = used > 1 ? op->partial.ptr + (nf / 4) * 4 + nb : nullptr;
@@ -422,7 +431,7 @@ int launch_dense(abx_context *ctx, const DenseParams &P, bool mixed, abx_operato
   }
   int64_t chunk_cols;
   const int used = dense_chunks(ctx, P.nc, blocks, 16, chunk_cols);
-  if (used > 1) ABX_TRY(op->partial.reserve((size_t)used * P.nr));
+  ABX_TRY(dense_reserve(ctx, P.nr, P.nc, op));
   double *partial = used > 1 ? op->partial.ptr : nullptr;
   k_dense_fp64<KIND><<<dim3(blocks, used), DT, 0, ctx->stream>>>(P, nullptr, chunk_cols, partial);
   if (partial)
@@ -550,6 +559,15 @@ int abx_operator_set_precision(abx_operator *op, int mode) {
   ABX_REQUIRE(mode == ABX_PREC_FP64 || mode == ABX_PREC_MIXED, ABX_ERR_INVALID,
               "unknown precision mode %d", mode);
   op->precision = mode;
+  // the buffers of an FP64 product, so that the first one allocates nothing
+  if (mode == ABX_PREC_FP64 && op->kind == 1 && op->rows->n > 0) {
+    ABX_TRY(ctx_activate(op->rows->ctx));
+    ABX_TRY(dense_reserve(op->rows->ctx, op->rows->n, op->cols->n, op));
+  }
+  if (mode == ABX_PREC_FP64 && op->fmm) {
+    ABX_TRY(ctx_activate(op->rows->ctx));
+    ABX_TRY(fmm_plan_prepare(op->fmm, op->rows->ctx->stream));
+  }
   return ABX_OK;
 }
 

@@ -397,8 +397,8 @@ int build_cell_start(abx_context *ctx, PairLayout &L) {
 // loaded; the unit that starts at query s is the run of lanes that continue
 // it.  A unit goes to the front of `units`, or, where `split` says so (low
 // density, where a warp of 32 lanes would hold few queries), to the back, and
-// its queries to `singles`, which k_pairs_thread walks.  Built on the host before, from a 16 B/point copy of the cells: 14 of
-// the 39 ms of a search at N = 4M.
+// its queries to `singles`, which k_pairs_thread walks.  Built on the host before,
+// from a 16 B/point copy of the cells: 14 of the 39 ms of a search at N = 4M.
 constexpr int UNIT_WARPS = 4;
 __global__ void __launch_bounds__(UNIT_WARPS * 32)
     k_units(const int4 *__restrict__ cell, const uint32_t *__restrict__ keys,
@@ -1377,11 +1377,11 @@ __device__ __forceinline__ double pair64(const D4 &xq, const D4 &xj, const int *
 //      have any left; those are carried into the next tile's walk.
 // A walk to the end of every tile costs the largest of 32 neighbour counts, of
 // which 56 % of the lanes are busy on average (candidates of a tile lie
-// together, the queries do not); two tiles at a time 74 %: @W_OLD@ -> @W_NEW@ ms
-// for the set below.  With FIX the values come from the integer
-// units (fix64.cuh) and the FP64 pipe is left with one multiply-add a pair: N =
-// 1,048,576 clustered, 1,250 neighbours a row, Wendland: @U_OLD@ -> @U_NEW@ ms.  The distance for the kernel
-// value is |(x_j - image*L) - x_i|, which differs from the reference's
+// together, the queries do not); two tiles at a time 74 %.  With FIX the values
+// come from the integer units (fix64.cuh) and the FP64 pipe is left with one
+// multiply-add a pair.  N = 1,048,576 clustered, 1,250 neighbours a row, Wendland:
+// 103 -> 21.0 ms, with the packed test and the carried lanes 19.2 (issue slots 68 %
+// busy, ALU 54 %, 21.7 lanes of 32).  The distance for the kernel value is |(x_j - image*L) - x_i|, which differs from the reference's
 // x_j - (x_i + image*L) by at most an ulp of the box length (the acceptance
 // decision itself is exact); the row sum order differs from the reference's.
 constexpr int CARRY = 20;  // of 32 lanes: with fewer at work the rest of a tile waits for the next
@@ -1631,8 +1631,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
 // The FP32 test is as cheap as the loads; FP64 values (~100 instructions) are
 // not evaluated where they are found but queued per lane in shared memory and
 // evaluated when a queue is full, as long as DRAIN lanes have one.  N = 100,000,
-// 50 neighbours a row: counts @C_OLD@ -> @C_NEW@, FP64 Gaussian product @S_OLD@
-// -> @S_NEW@ us.
+// 50 neighbours a row: a count of 100,000 moved points 2,060 -> 474 us (330 with
+// the sorts of primitives.cu), FP64 Gaussian product 3,229 -> 197 us.
 enum { VAL_FP64 = 0, VAL_MIXED = 1, VAL_FIX = 2 };
 constexpr int QCAP = 16;   // queued pairs per lane
 constexpr int DRAIN = 22;  // lanes that make an evaluation worth its issue

@@ -194,15 +194,16 @@ __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(
 
 // ---- few tiles: the digit offsets without scan launches
 //
-// Up to RF_MAX items a pass is two launches: counts per tile,
-// and the scatter, whose CTAs each add up the whole (tile, digit) table from L2
-// (16-bit counts, 512 KB at most: 2,048 items a tile, 4,096 above 128 tiles, 16 bytes a load: loads of one count each, 49
-// tiles in a row, were two thirds of the scatter's time).  With so few tiles an
-// 11-bit digit costs little, so that 22-bit keys take two passes.  Two
-// independent sets (a search's queries and its particles) go through every
-// launch together, blockIdx.y choosing the set: a pass over 100,000 items
-// occupies a third of the SMs.  N = 100,000, 21-bit keys: 3 x (hist, 3 scan
-// kernels, scatter) + 2 copies -> 2 x 2 launches, @RS_OLD@ -> @RS_NEW@ us.
+// Up to RF_MAX items a pass is two launches: counts per tile, and the scatter,
+// whose CTAs each add up the whole (tile, digit) table from L2 (16-bit counts,
+// 512 KB at most: 2,048 items a tile, 4,096 above 128 tiles; 16 bytes a load:
+// loads of one count each, 49 tiles in a row, were two thirds of the scatter's
+// time).  With so few tiles an 11-bit digit costs little, so that 22-bit keys take
+// two passes.  Two independent sets (a search's queries and its particles) go
+// through every launch together, blockIdx.y choosing the set: a pass over 100,000
+// items occupies a third of the SMs.  N = 100,000, 21-bit keys: 3 x (hist, 3 scan
+// kernels, scatter) + 2 copies -> 2 x 2 launches, 29 us a pass for two such sets
+// (77 one after the other with single counts).
 constexpr int RF_TILES = 128;
 constexpr size_t RF_MAX = (size_t)RF_TILES * RS_TILE;
 static_assert(RS_TILE < 65536, "16-bit counts per tile");

@@ -265,8 +265,9 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // in a panel grows with its width); an update converts its sums and subtracts
 // them, two FP64 operations an entry, so the trailing matrix is updated for 64
 // columns at a time and only the rows and columns of those 64 panel by panel.
-// Pivots are compared as integers. 256 domains of 703 rows on average (set-up and one
-// apply): 98 -> @LU_NEW@ ms.
+// Pivots are compared as integers.  256 domains of 703 rows on average (set-up and
+// one apply): 98 -> 36 ms, 31.9 with the largest domains first; blocks of 1,700
+// rows (4,003 points): 592 -> 50 ms.
 constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
 constexpr int FW = 16;         // panel width
 constexpr int FB = 64;         // columns of a trailing update

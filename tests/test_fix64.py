@@ -76,7 +76,10 @@ def _exact(kind, x, y, p0):
     d2 = sum((Decimal(b) - Decimal(a)) ** 2 for a, b in zip(x, y))
     p = Decimal(p0)
     if kind == "gauss":
-        return (-d2 * p).exp(), Decimal(0)
+        # beyond p0 d^2 = 177 coordinates are in units of 2^-58: the value's slope,
+        # ln 2 2 sqrt(3 t), times a difference's error of up to one unit
+        k, t = (-d2 * p).exp(), d2 * p * Decimal("1.443")
+        return k, k * t.sqrt() * Decimal(2) ** -55
     if kind == "lap":
         return 1 / (d2.sqrt() + p), Decimal(0)
     if kind == "mq":
@@ -87,7 +90,7 @@ def _exact(kind, x, y, p0):
     return (t ** 4 * (4 * q + 1), 20 * q * abs(t) ** 3 * Decimal(2) ** -59) if t > 0 else (Decimal(0), Decimal(0))
 
 
-@pytest.mark.parametrize("kind,p0r2", [("gauss", 4.0), ("gauss", 21.0), ("wend", 1.0),
+@pytest.mark.parametrize("kind,p0r2", [("gauss", 4.0), ("gauss", 21.0), ("gauss", 170.0), ("gauss", 180.0), ("gauss", 600.0), ("wend", 1.0),
                                        ("lap", 0.0), ("lap", 1e-11), ("lap", 0.02), ("lap", 0.4),
                                        ("mq", 0.005), ("mq", 0.02), ("mq", 0.7)])
 @pytest.mark.parametrize("dim", [1, 2, 3])
