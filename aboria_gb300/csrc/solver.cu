@@ -31,6 +31,7 @@
 #include <vector>
 
 #include <cooperative_groups.h>
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "handles.cuh"
@@ -252,8 +253,9 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // blocks of kernel values of one size (Gaussian, Wendland: at most 1, 1 on the
 // diagonal), where the trailing update, n^3 / 3 multiply-adds, need not run at 2
 // FP64 operations a clock and SM: the rows of L21 and the columns of U12 become
-// scaled 56-bit integers (fix64.cuh), and a multiply-add three 32x32+64 ones (25
-// a clock and SM with all operands in registers) instead of an FP64 one (1.8).
+// scaled 56-bit integers (fix64.cuh), and an FP64 multiply-add (1.8 a clock and SM)
+// becomes three 32x32+64 ones (25 a clock and SM with all operands in registers)
+// within a block of columns, 28 FP16 ones on the tensor cores beyond (update_mma).
 // The scale is the largest entry of the row (column), so a product's error is
 // 2^-56 of the largest product of its row and column, where FP64's partial sums
 // round at 2^-53 of themselves.
@@ -266,8 +268,8 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // them, two FP64 operations an entry, so the trailing matrix is updated for 64
 // columns at a time and only the rows and columns of those 64 panel by panel.
 // Pivots are compared as integers.  256 domains of 703 rows on average (set-up and
-// one apply): 98 -> 36 ms, 31.9 with the largest domains first; blocks of 1,700
-// rows (4,003 points): 592 -> 50 ms.
+// one apply): 98 -> 36 ms, 31.9 with the largest domains first, 24.5 with tensor
+// cores; blocks of 1,700 rows (4,003 points): 592 -> 35 ms.
 constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
 constexpr int FW = 16;         // panel width
 constexpr int FB = 64;         // columns of a trailing update
@@ -275,8 +277,6 @@ constexpr int PLD = FW + 1;    // panel row stride
 // rows of a panel in shared memory, so that two CTAs share an SM (one leaves the
 // integer pipe waiting: 40 ms); the few rows of larger blocks stay in L2
 constexpr int FL_ROWS = 712;
-constexpr size_t FL_TILES = (size_t)FB * (64 + 64) * sizeof(int2);  // FB = 64 columns, 64 x 64
-static_assert(FL_TILES >= (size_t)FW * (256 + 16) * sizeof(int2), "tiles of one panel fit too");
 
 __device__ __forceinline__ int2 split56(double x, int e) {
   const fx::Half2 q = fx::split56(x, e);
@@ -382,6 +382,148 @@ __device__ __noinline__ void update_fix(double *A, int n, int r0, int r1, int c0
   __syncthreads();
 }
 
+// ---- the trailing update on the tensor cores
+// The same scaled 56-bit integers as seven signed 8-bit digits each, exact in
+// FP16, and of their 49 products of digits those 28 with i + j >= 6, what the
+// three multiply-adds of update_fix keep: products and sums of one weight i + j
+// stay below 2^24, so that FP32 accumulators hold them exactly.  A tile is 64 x
+// 32 with all FB terms: L's digits (56 KB) stay for a row of tiles, U's are 28 KB,
+// two CTAs an SM; a warp has 16 x 16 entries, 56 accumulators a thread.  With 32-bit
+// multiply-adds (25 a clock and SM) this took 14.3 of the 31.8 ms (set-up and one
+// apply) of 256 domains of 703 rows, now 7.1 of 24.5.
+constexpr int MD = 7;                     // digits
+constexpr int MT_R = 64, MT_C = 32;       // tile
+static_assert(FB == 64, "rows of digits are 128 bytes");
+constexpr size_t MD_BYTES = (size_t)MD * (MT_R + MT_C) * FB * 2;
+static_assert(MD_BYTES >= (size_t)FW * (256 + 16) * sizeof(int2), "the tiles of one panel fit too");
+
+// Byte offset of digit d, row r (of a tile's R), k: 128-byte rows whose 16-byte
+// chunks are permuted by r, so that ldmatrix reads 8 rows without conflicts.
+template <int R> __device__ __forceinline__ uint32_t digit_at(int d, int r, int k) {
+  return (uint32_t)((d * R + r) * 128 + (((k >> 3) ^ (r & 7)) << 4) + (k & 7) * 2);
+}
+
+// Digits of the values of (r, k) and (r, k + 1), as pairs of FP16.
+template <int R>
+__device__ __forceinline__ void put_digits(unsigned char *base, int r, int k, double v0, double v1,
+                                           int e) {
+  const int2 p0 = split56(v0, e), p1 = split56(v1, e);
+  long long q0 = ((long long)p0.x << 28) + p0.y, q1 = ((long long)p1.x << 28) + p1.y;
+#pragma unroll
+  for (int d = 0; d < MD; ++d) {
+    // the top digit is what is left (at most 256)
+    const int a = d < MD - 1 ? (int)(signed char)(q0 & 255) : (int)q0;
+    const int b = d < MD - 1 ? (int)(signed char)(q1 & 255) : (int)q1;
+    q0 = (q0 - a) >> 8;
+    q1 = (q1 - b) >> 8;
+    // 1536 + a as FP16 bits, less 1536
+    const uint32_t bits = (uint32_t)(0x6600 + a) | (uint32_t)(0x6600 + b) << 16;
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&bits), __half2half2(__float2half(1536.f)));
+    *reinterpret_cast<__half2 *>(base + digit_at<R>(d, r, k)) = h;
+  }
+}
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// A[r0.., r0..] -= L[r0.., k0..k0+FB) U[k0.., r0..) to the end of the matrix.
+__device__ __noinline__ void update_mma(double *A, int n, int r0, int k0, const short *le,
+                                        const short *ue, unsigned char *sm, int rank, int ranks) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned char *L = sm, *U = sm + (size_t)MD * MT_R * 128;
+  const uint32_t sL = (uint32_t)__cvta_generic_to_shared(L), sU = (uint32_t)__cvta_generic_to_shared(U);
+  const int wr = (warp & 3) * 16, wc = (warp >> 2) * 16;  // the warp's 16 x 16 entries
+  const int nti = (n - r0 + MT_R - 1) / MT_R, ntj = (n - r0 + MT_C - 1) / MT_C;
+  int have = -1;  // row tile in L
+  for (int t = rank; t < nti * ntj; t += ranks) {
+    const int ti = r0 + (t / ntj) * MT_R, tj = r0 + (t % ntj) * MT_C;
+    __syncthreads();
+    if (ti != have) {
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {  // 4 pairs a thread at a time
+        double v[8];
+        const int r = tid % MT_R;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int k = 2 * (tid / MT_R + 4 * (h * 4 + q / 2)) + (q & 1);
+          v[q] = ti + r < n ? M(A, n, ti + r, k0 + k) : 0.0;
+        }
+        const int e = ti + r < n ? le[ti + r] : 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          put_digits<MT_R>(L, r, 2 * (tid / MT_R + 4 * (h * 4 + q)), v[2 * q], v[2 * q + 1], e);
+      }
+      have = ti;
+    }
+    {
+      double v[8];
+      const int k = 2 * (tid % 32);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int j = tid / 32 + 8 * (q / 2);
+        v[q] = tj + j < n ? M(A, n, k0 + k + (q & 1), tj + j) : 0.0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = tid / 32 + 8 * q;
+        put_digits<MT_C>(U, j, k, v[2 * q], v[2 * q + 1], tj + j < n ? ue[tj + j] : 0);
+      }
+    }
+    __syncthreads();
+    if (ti + wr >= n || tj + wc >= n) continue;
+    float acc[MD][2][4] = {};  // sums of weight MD - 1 + w
+#pragma unroll 1
+    for (int kk = 0; kk < FB; kk += 16) {
+      uint32_t a[MD][4];
+#pragma unroll
+      for (int d = 0; d < MD; ++d)
+        ldmatrix4(a[d], sL + digit_at<MT_R>(d, wr + (lane & 15), kk + (lane >> 4) * 8));
+#pragma unroll
+      for (int d = 0; d < MD; ++d) {
+        uint32_t b[4];
+        ldmatrix4(b, sU + digit_at<MT_C>(d, wc + (lane & 7) + (lane >> 4) * 8, kk + ((lane >> 3) & 1) * 8));
+#pragma unroll
+        for (int i = MD - 1 - d; i < MD; ++i) {
+          mma_f16(acc[i + d - (MD - 1)][0], a[i], b[0], b[1]);
+          mma_f16(acc[i + d - (MD - 1)][1], a[i], b[2], b[3]);
+        }
+      }
+    }
+    double v[2][4];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int ri = ti + wr + (lane >> 2) + 8 * (q >> 1), cj = tj + wc + 8 * c + 2 * (lane & 3) + (q & 1);
+        v[c][q] = ri < n && cj < n ? M(A, n, ri, cj) : 0.0;
+      }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int ri = ti + wr + (lane >> 2) + 8 * (q >> 1), cj = tj + wc + 8 * c + 2 * (lane & 3) + (q & 1);
+        if (ri >= n || cj >= n) continue;
+        // in units of 2^56: weights 7 to 12, and 6 rounded
+        long long s = (long long)__float2int_rn(acc[MD - 1][c][q]);
+#pragma unroll
+        for (int w = MD - 2; w > 0; --w) s = s * 256 + __float2int_rn(acc[w][c][q]);
+        s += (__float2int_rn(acc[0][c][q]) + 128) >> 8;
+        M(A, n, ri, cj) = fma(-(double)s, fx::scale56((int)le[ri] + (int)ue[cj]), v[c][q]);
+      }
+  }
+  __syncthreads();
+}
+
 // Rows k0 + c and sw[c] of one column swapped, c = 0, 1, ...
 __device__ __forceinline__ void swap_rows(double *col, int k0, int kw, const int *sw) {
   for (int c = 0; c < kw; ++c) {
@@ -415,7 +557,7 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
                                                     const int *__restrict__ dom_off,
                                                     int *__restrict__ piv, int *__restrict__ info,
                                                     short *__restrict__ exps, int64_t nexp) {
-  extern __shared__ __align__(16) unsigned char lu_raw[];
+  extern __shared__ __align__(128) unsigned char lu_raw[];
   double *Pn = reinterpret_cast<double *>(lu_raw);  // panel: rows k0..n-1 x FW, stride PLD
   int2 *tiles = reinterpret_cast<int2 *>(lu_raw);
   __shared__ fx::u64 red_v[FL_T / 32];
@@ -564,7 +706,7 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
       ue[r] = (short)scale_exp(mu);
     }
     cl.sync();
-    update_fix<64, 64, FB>(A, n, B1, n, B1, n, B0, le, ue, tiles, rank, ranks);
+    update_mma(A, n, B1, B0, le, ue, lu_raw, rank, ranks);
     cl.sync();
   }
   if (rank == 0 && tid == 0) info[d] = status;
@@ -856,7 +998,7 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
     const bool flat = op->k.kind == ABX_K_GAUSSIAN || op->k.kind == ABX_K_COMPACT_GAUSSIAN ||
                       op->k.kind == ABX_K_WENDLAND_C2;
     if (flat) {
-      const size_t smem = std::max(FL_TILES, (size_t)std::min(S->max_size, FL_ROWS) * PLD * 8);
+      const size_t smem = std::max(MD_BYTES, (size_t)std::min(S->max_size, FL_ROWS) * PLD * 8);
       // CTAs a domain: enough for two on every SM, 8 at most
       int ranks = 1;
       while (ranks < 8 && S->ndom * ranks * 2 <= 4 * ctx->num_sms) ranks *= 2;
