@@ -23,8 +23,8 @@
 //   G[:, targets] += K_o * W[:, sources]
 // in the mixed-precision mode on the tensor cores with FP32 accumulation (split
 // FP16 on tcgen05 above 64 nodes, 3xTF32 on mma.sync below) and P2P in FP32; in
-// the FP64 mode M2L is a product of scaled 56-bit integers and P2P takes its
-// kernel values from the integer units (fix64.cuh), both with errors no larger
+// the FP64 mode M2L is a product of scaled 56-bit integers, by their digits on the
+// tensor cores, and P2P takes its kernel values from the integer units (fix64.cuh), both with errors no larger
 // than FP64's own.
 #include <algorithm>
 #include <chrono>
@@ -36,6 +36,7 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "digits.cuh"
 #include "fix64.cuh"
 #include "handles.cuh"
 
@@ -77,9 +78,8 @@ struct FmmPlan {
   DevBuf<float> Kmh, Kml; // split-TF32 hi/lo parts of the FP32 copy (mma.sync M2L, ncheb <= 64)
   DevBuf<__half> Kp;      // the same packed as tcgen05 stage images (ncheb > 64, k_pack_f16)
   DevBuf<float> Kp_scale;  // power of two of each matrix' packed values
-  // FP64 M2L on the integer units: K and W as scaled 56-bit numbers, their
-  // exponents (per row of K, per node), tiles of 64 pairs
-  DevBuf<int2> Kq, Wq;
+  // FP64 M2L: digits of K and W, their exponents (per row of K, per node), tiles
+  DevBuf<__half> Kd, Wd;
   DevBuf<short> ke, we;
   DevBuf<int> mf_mat, mf_first;
   int mf_tiles = 0;
@@ -402,126 +402,154 @@ __global__ void k_transpose_tc(const double *__restrict__ in, int nchild, int nc
 }
 
 // --------------------------------------------------------------- M2L ---
-// FP64 M2L as integer products of matrices (scaled 56-bit numbers, fix64.cuh):
-// for one matrix K and 64 (target, source) pairs sharing it, a tile of TR rows
-// of K W[:, sources], each multiply-add three 32x32+64 ones (25 a clock and SM)
-// instead of an FP64 one (1.8, which bounded one CTA per pair).  K is split once
-// per plan with a scale per row (Kq, transposed), W per product with a scale per
-// node (Wq); both scales and 57 bits make a term's rounding smaller than the FP64
-// sum's own.  Sums are turned into FP64 every 64 terms, which the 64-bit sums
-// hold.  N = 1,048,576, 6.0e6 pairs: order 3 (27 nodes) 8.5 -> 2.3 ms; 100,000
-// points, order 5 (125), the whole product 20.8 -> 5.7 ms.
-__global__ void k_split_k(const double *__restrict__ K, int64_t nrows, int ncheb, int ldr,
-                          int2 *__restrict__ Kq, short *__restrict__ ke) {
-  const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= nrows) return;
-  const int64_t m = row / ncheb;
-  const int i = (int)(row % ncheb);
-  const double *k = K + row * ncheb;
-  fx::u64 mx = 0;
-  for (int j = 0; j < ncheb; ++j) mx = max(mx, fx::abs_bits(k[j]));
-  const int e = fx::scale_exp(mx);
-  ke[m * ldr + i] = (short)e;
-  for (int j = 0; j < ncheb; ++j) {
-    const fx::Half2 q = fx::split56(k[j], e);
-    Kq[(m * ncheb + j) * ldr + i] = make_int2(q.h, q.l);
-  }
-}
-__global__ void k_split_w(const double *__restrict__ W, int nnodes, int ncheb,
-                          int2 *__restrict__ Wq, short *__restrict__ we) {
-  const int node = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+// FP64 M2L as products of matrices of scaled 56-bit integers on the tensor cores
+// (digits.cuh): for one matrix K and a tile of TC (target, source) pairs sharing
+// it, TR rows of K W[:, sources], a warp 16 x 16 of them.  Digits are made once, of
+// K per plan with a scale per row (Kd), of W per product with a scale per node
+// (Wd); both scales and 57 bits make a term's rounding smaller than the FP64 sum's
+// own.  32 terms are staged at a time, the next while the last are multiplied.
+// With FP64 one CTA a pair was bound by the pipe's 1.8 multiply-adds a clock and
+// SM, with three 32x32+64-bit ones by their 25.  N = 1,048,576, 6.0e6 pairs: order 3
+// (27 nodes) 8.5 -> 2.3 -> 1.8 ms; 100,000 points, order 5 (125), the whole
+// product 20.8 -> 5.7 -> 3.6 ms.
+using dg::MD;
+constexpr int MF_K = 32;                // terms staged at a time
+constexpr int MF_ROW = MD * MF_K;       // FP16 values of a row's 32 terms: [digit][term]
+constexpr int MF_T = 256;
+constexpr int mf_pairs(int nc) { return nc <= 32 ? 64 : 32; }  // pairs per tile
+// Digits of `rows` rows of nc values, a warp a row; row r's 32 terms c go to
+// ((r / per * chunks + c) * per + r % per) * MF_ROW (rows of one matrix together).
+__global__ void __launch_bounds__(256) k_split_digits(const double *__restrict__ V, int64_t rows,
+                                                      int nc, int per, __half *__restrict__ out,
+                                                      short *__restrict__ exps) {
+  const int64_t row = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (node >= nnodes) return;
-  const double *w = W + (size_t)node * ncheb;
+  if (row >= rows) return;
+  const double *v = V + row * nc;
   fx::u64 mx = 0;
-  for (int j = lane; j < ncheb; j += 32) mx = max(mx, fx::abs_bits(w[j]));
+  for (int j = lane; j < nc; j += 32) mx = max(mx, fx::abs_bits(v[j]));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const int e = fx::scale_exp(mx);
-  if (lane == 0) we[node] = (short)e;
-  for (int j = lane; j < ncheb; j += 32) {
-    const fx::Half2 q = fx::split56(w[j], e);
-    Wq[(size_t)node * ncheb + j] = make_int2(q.h, q.l);
+  const int e = fx::scale_exp(mx), chunks = (nc + MF_K - 1) / MF_K;
+  if (lane == 0) exps[row] = (short)e;
+  for (int c = 0; c < chunks; ++c) {
+    const int j = c * MF_K + lane;
+    long long q = j < nc ? dg::whole(v[j], e) : 0;
+    __half *o = out + (((row / per) * chunks + c) * per + row % per) * MF_ROW + lane;
+#pragma unroll
+    for (int d = 0; d < MD; ++d) o[d * MF_K] = __low2half(dg::pair(dg::next(q, d), 0));
   }
 }
-constexpr int MF_P = 64;    // pairs per tile
-constexpr int MF_K = 32;    // columns staged at a time
-constexpr int MF_LD = MF_P + 2;
-template <int TR, bool MULTI>
-__global__ void __launch_bounds__(TR / 4 * (MF_P / 4), 512 / (TR / 4 * (MF_P / 4))) k_m2l_fix(
-    int ncheb, int ldr, const int2 *__restrict__ Kq, const short *__restrict__ ke,
-    const int2 *__restrict__ Wq, const short *__restrict__ we, const int2 *__restrict__ by_mat,
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// 16-byte asynchronous copy; nbytes = 0 writes zeros.
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, int nbytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(nbytes)
+               : "memory");
+}
+
+// Byte offset of digit d, row r (of a tile's R), 16-byte chunk c of 4: permuted, so
+// that ldmatrix reads 8 rows without conflicts.
+template <int R> __device__ __forceinline__ uint32_t mf_at(int d, int r, int c) {
+  return (uint32_t)((d * R + r) * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+}
+template <int TR, int TC> constexpr size_t mf_stage() { return (size_t)MD * (TR + TC) * MF_K * 2; }
+
+template <int TR, int TC, int STAGES>
+__global__ void __launch_bounds__(MF_T, 2) k_m2l_fix(
+    int nc, const __half *__restrict__ Kd, const short *__restrict__ ke,
+    const __half *__restrict__ Wd, const short *__restrict__ we, const int2 *__restrict__ by_mat,
     const int *__restrict__ mat_off, const int *__restrict__ tile_mat,
     const int *__restrict__ tile_first, double *__restrict__ G) {
-  constexpr int T = TR / 4 * (MF_P / 4);
-  __shared__ __align__(16) int2 sA[MF_K][TR];
-  __shared__ __align__(16) int2 sB[MF_K][MF_LD];
-  __shared__ int tgt[MF_P], src[MF_P], sexp[MF_P];
-  const int tid = threadIdx.x, m = tile_mat[blockIdx.x], first = tile_first[blockIdx.x];
-  const int np = min(MF_P, mat_off[m + 1] - first), r0 = blockIdx.y * TR;
-  for (int p = tid; p < MF_P; p += T) {
-    const int2 ts = by_mat[first + min(p, np - 1)];
-    tgt[p] = ts.x;
-    src[p] = ts.y;
-    sexp[p] = we[ts.y];
+  static_assert((TR / 16) * (TC / 16) == MF_T / 32, "16 x 16 a warp");
+  extern __shared__ __align__(128) unsigned char mf_raw[];
+  __shared__ int tgt[TC], src[TC], sexp[TC];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = tile_mat[blockIdx.x], first = tile_first[blockIdx.x];
+  const int np = min(TC, mat_off[m + 1] - first), r0 = blockIdx.y * TR;
+  if (tid < TC) {
+    const int2 ts = by_mat[first + min(tid, np - 1)];
+    tgt[tid] = ts.x;
+    src[tid] = ts.y;
+    sexp[tid] = we[ts.y];
   }
-  const int tr = (tid % (TR / 4)) * 4, tc = (tid / (TR / 4)) * 4;
-  long long hi[4][4] = {}, mid[4][4] = {};
-  double sum[4][4] = {};
-  const int2 *Km = Kq + (size_t)m * ncheb * ldr + r0;
-  for (int k0 = 0; k0 < ncheb; k0 += MF_K) {
-    const int kc = min(MF_K, ncheb - k0);
+  __syncthreads();
+  const uint32_t base = smem_addr(mf_raw);
+  const int chunks = (nc + MF_K - 1) / MF_K;
+  const int wr = (warp % (TR / 16)) * 16, wc = (warp / (TR / 16)) * 16;
+  auto load = [&](int c) {  // terms 32 c .. of the tile's rows and sources
+    const uint32_t st = base + (uint32_t)((c % STAGES) * mf_stage<TR, TC>());
+    constexpr int PIECES = MF_ROW * 2 / 16;
+    for (int e = tid; e < (TR + TC) * PIECES; e += MF_T) {
+      const int r = e / PIECES, q = e - r * PIECES, d = q >> 2, ch = q & 3;
+      if (r < TR) {
+        const bool in = r0 + r < nc;
+        cp16(st + mf_at<TR>(d, r, ch),
+             Kd + (((size_t)m * chunks + c) * nc + (in ? r0 + r : 0)) * MF_ROW + q * 8, in ? 16 : 0);
+      } else {
+        const int p = r - TR;
+        cp16(st + (uint32_t)(MD * TR * MF_K * 2) + mf_at<TC>(d, p, ch),
+             Wd + ((size_t)src[p] * chunks + c) * MF_ROW + q * 8, 16);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[MD][2][4] = {};
+  double total[2][4] = {};
+  load(0);
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    if (STAGES > 1 && c + 1 < chunks) {
+      load(c + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
     __syncthreads();
-    for (int e = tid; e < kc * (TR / 2); e += T) {  // two entries at a time (ldr is even)
-      const int r = (e % (TR / 2)) * 2, k = e / (TR / 2);
-      int4 v = make_int4(0, 0, 0, 0);
-      if (r0 + r < ldr) v = *reinterpret_cast<const int4 *>(Km + (size_t)(k0 + k) * ldr + r);
-      *reinterpret_cast<int4 *>(&sA[k][r]) = v;
-    }
-    for (int e = tid; e < MF_K * MF_P; e += T) {
-      const int k = e % MF_K, p = e / MF_K;
-      if (k < kc) sB[k][p] = Wq[(size_t)src[p] * ncheb + k0 + k];
+    const uint32_t sA = base + (uint32_t)((c % STAGES) * mf_stage<TR, TC>());
+    const uint32_t sB = sA + (uint32_t)(MD * TR * MF_K * 2);
+    if (r0 + wr < nc && wc < np) {
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        if (c * MF_K + h * 16 >= nc) break;
+        uint32_t a[MD][4];
+#pragma unroll
+        for (int d = 0; d < MD; ++d)
+          dg::ldmatrix4(a[d], sA + mf_at<TR>(d, wr + (lane & 15), 2 * h + (lane >> 4)));
+#pragma unroll
+        for (int d = 0; d < MD; ++d) {
+          uint32_t b[4];
+          dg::ldmatrix4(b, sB + mf_at<TC>(d, wc + (lane & 7) + (lane >> 4) * 8, 2 * h + ((lane >> 3) & 1)));
+          dg::multiply(acc, a, b, d);
+        }
+      }
+      if (STAGES > 1 && ((c + 1) * MF_K % dg::MAX_TERMS == 0 || c + 1 == chunks)) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) total[b][q] += (double)dg::sum(acc, b, q);
+#pragma unroll
+        for (int w = 0; w < MD; ++w)
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[w][b][q] = 0.f;
+      }
     }
     __syncthreads();
-#pragma unroll 2
-    for (int k = 0; k < kc; ++k) {
-      int2 a[4], b[4];
-      *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&sA[k][tr]);
-      *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&sA[k][tr + 2]);
-      *reinterpret_cast<int4 *>(&b[0]) = *reinterpret_cast<const int4 *>(&sB[k][tc]);
-      *reinterpret_cast<int4 *>(&b[2]) = *reinterpret_cast<const int4 *>(&sB[k][tc + 2]);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          hi[i][j] += (long long)a[i].x * b[j].x;
-          mid[i][j] += (long long)a[i].x * b[j].y;
-          mid[i][j] += (long long)a[i].y * b[j].x;
-        }
-    }
-    if (MULTI && ((k0 / MF_K) & 1)) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          sum[i][j] += (double)fx::sum56(hi[i][j], mid[i][j]);
-          hi[i][j] = mid[i][j] = 0;
-        }
-    }
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int p = tc + j;
-    if (p >= np) continue;
+  for (int b = 0; b < 2; ++b)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = r0 + tr + i;
-      if (r >= ncheb) continue;
-      double t = (double)fx::sum56(hi[i][j], mid[i][j]);
-      if (MULTI) t += sum[i][j];
-      atomicAdd(&G[(size_t)tgt[p] * ncheb + r], t * fx::scale56((int)ke[(size_t)m * ldr + r] + sexp[p]));
+    for (int q = 0; q < 4; ++q) {
+      const int r = r0 + wr + (lane >> 2) + 8 * (q >> 1), p = wc + 8 * b + 2 * (lane & 3) + (q & 1);
+      if (r >= nc || p >= np) continue;
+      const double t = STAGES > 1 ? total[b][q] : (double)dg::sum(acc, b, q);
+      atomicAdd(&G[(size_t)tgt[p] * nc + r], t * fx::scale56((int)ke[(size_t)m * nc + r] + sexp[p]));
     }
-  }
 }
 
 // Mixed precision M2L on the tensor cores: for one matrix K (ncheb x ncheb,
@@ -838,10 +866,6 @@ __global__ void __launch_bounds__(256) k_split_f16(const double *__restrict__ W,
   }
 }
 
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
 // Shared-memory matrix descriptor: no swizzle, K-major.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
@@ -882,12 +906,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_
     }
   }
   return false;
-}
-
-// 16-byte asynchronous copy; nbytes = 0 writes zeros.
-__device__ __forceinline__ void cp16(uint32_t dst, const void *src, int nbytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(nbytes)
-               : "memory");
 }
 
 template <int NRB>
@@ -1838,50 +1856,48 @@ namespace {
 // by the plan's first FP64 product.
 // The split matrices and buffers of the FP64 M2L, once per plan.
 int m2l_fix_prepare(FmmPlan *P, cudaStream_t s) {
-  const int nc = P->ncheb, ldr = (nc + 1) / 2 * 2;
-  if (!P->Kq.ptr) {
+  const int nc = P->ncheb, chunks = (nc + MF_K - 1) / MF_K;
+  if (!P->Kd.ptr) {
     std::vector<int> mat, first;
     for (int m = 0; m < P->nmat; ++m)
-      for (int q = P->mat_off[m]; q < P->mat_off[m + 1]; q += MF_P) {
+      for (int q = P->mat_off[m]; q < P->mat_off[m + 1]; q += mf_pairs(nc)) {
         mat.push_back(m);
         first.push_back(q);
       }
     P->mf_tiles = (int)mat.size();
+    const int64_t rows = (int64_t)P->nmat * nc;
     ABX_TRY(P->mf_mat.reserve(mat.size() + 1));
     ABX_TRY(P->mf_first.reserve(first.size() + 1));
-    ABX_TRY(P->ke.reserve((size_t)P->nmat * ldr));
+    ABX_TRY(P->ke.reserve((size_t)rows));
     ABX_CHECK_CUDA(cudaMemcpyAsync(P->mf_mat.ptr, mat.data(), mat.size() * 4, cudaMemcpyHostToDevice, s));
     ABX_CHECK_CUDA(cudaMemcpyAsync(P->mf_first.ptr, first.data(), first.size() * 4,
                                    cudaMemcpyHostToDevice, s));
-    ABX_TRY(P->Kq.reserve((size_t)P->nmat * nc * ldr));
-    if (ldr != nc)
-      ABX_CHECK_CUDA(cudaMemsetAsync(P->Kq.ptr, 0, (size_t)P->nmat * nc * ldr * sizeof(int2), s));
-    const int64_t rows = (int64_t)P->nmat * nc;
-    k_split_k<<<ceil_div((size_t)rows, 128), 128, 0, s>>>(P->Km.ptr, rows, nc, ldr, P->Kq.ptr,
-                                                          P->ke.ptr);
+    ABX_TRY(P->Kd.reserve((size_t)rows * chunks * MF_ROW));
+    k_split_digits<<<ceil_div((size_t)rows, 8), 256, 0, s>>>(P->Km.ptr, rows, nc, nc, P->Kd.ptr,
+                                                             P->ke.ptr);
     ABX_CHECK_CUDA(cudaGetLastError());
     ABX_CHECK_CUDA(cudaStreamSynchronize(s));  // the host lists end here
   }
-  ABX_TRY(P->Wq.reserve((size_t)P->nnodes * nc));
+  ABX_TRY(P->Wd.reserve((size_t)P->nnodes * chunks * MF_ROW));
   return P->we.reserve((size_t)P->nnodes);
 }
 
 int m2l_fix(FmmPlan *P, cudaStream_t s) {
-  const int nc = P->ncheb, ldr = (nc + 1) / 2 * 2;
+  const int nc = P->ncheb;
   ABX_TRY(m2l_fix_prepare(P, s));
-  k_split_w<<<ceil_div((size_t)P->nnodes * 32, 256), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, P->Wq.ptr,
-                                                                  P->we.ptr);
-  auto run = [&](auto kern, int tr) {
-    const dim3 grid(P->mf_tiles, (nc + tr - 1) / tr);
-    kern<<<grid, tr / 4 * (MF_P / 4), 0, s>>>(nc, ldr, P->Kq.ptr, P->ke.ptr, P->Wq.ptr, P->we.ptr,
-                                              P->m2l_by_mat.ptr, P->mat_off_d.ptr, P->mf_mat.ptr,
-                                              P->mf_first.ptr, P->G.ptr);
+  k_split_digits<<<ceil_div((size_t)P->nnodes, 8), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, 1, P->Wd.ptr,
+                                                                P->we.ptr);
+  auto run = [&](auto kern, int tr, size_t smem) -> int {
+    ABX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3(P->mf_tiles, (nc + tr - 1) / tr), MF_T, smem, s>>>(
+        nc, P->Kd.ptr, P->ke.ptr, P->Wd.ptr, P->we.ptr, P->m2l_by_mat.ptr, P->mat_off_d.ptr,
+        P->mf_mat.ptr, P->mf_first.ptr, P->G.ptr);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
   };
-  if (nc <= 32) run(k_m2l_fix<32, false>, 32);
-  else if (nc <= 64) run(k_m2l_fix<64, false>, 64);
-  else run(k_m2l_fix<64, true>, 64);
-  ABX_CHECK_CUDA(cudaGetLastError());
-  return ABX_OK;
+  // up to 32 nodes: one stage, 32 rows
+  return nc <= 32 ? run(k_m2l_fix<32, 64, 1>, 32, mf_stage<32, 64>())
+                  : run(k_m2l_fix<64, 32, 2>, 64, 2 * mf_stage<64, 32>());
 }
 }  // namespace
 

@@ -31,9 +31,9 @@
 #include <vector>
 
 #include <cooperative_groups.h>
-#include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "digits.cuh"
 #include "handles.cuh"
 
 namespace cg = cooperative_groups;
@@ -383,15 +383,12 @@ __device__ __noinline__ void update_fix(double *A, int n, int r0, int r1, int c0
 }
 
 // ---- the trailing update on the tensor cores
-// The same scaled 56-bit integers as seven signed 8-bit digits each, exact in
-// FP16, and of their 49 products of digits those 28 with i + j >= 6, what the
-// three multiply-adds of update_fix keep: products and sums of one weight i + j
-// stay below 2^24, so that FP32 accumulators hold them exactly.  A tile is 64 x
+// The same scaled 56-bit integers as digits (digits.cuh).  A tile is 64 x
 // 32 with all FB terms: L's digits (56 KB) stay for a row of tiles, U's are 28 KB,
 // two CTAs an SM; a warp has 16 x 16 entries, 56 accumulators a thread.  With 32-bit
 // multiply-adds (25 a clock and SM) this took 14.3 of the 31.8 ms (set-up and one
 // apply) of 256 domains of 703 rows, now 7.1 of 24.5.
-constexpr int MD = 7;                     // digits
+using dg::MD;
 constexpr int MT_R = 64, MT_C = 32;       // tile
 static_assert(FB == 64, "rows of digits are 128 bytes");
 constexpr size_t MD_BYTES = (size_t)MD * (MT_R + MT_C) * FB * 2;
@@ -407,33 +404,12 @@ template <int R> __device__ __forceinline__ uint32_t digit_at(int d, int r, int 
 template <int R>
 __device__ __forceinline__ void put_digits(unsigned char *base, int r, int k, double v0, double v1,
                                            int e) {
-  const int2 p0 = split56(v0, e), p1 = split56(v1, e);
-  long long q0 = ((long long)p0.x << 28) + p0.y, q1 = ((long long)p1.x << 28) + p1.y;
+  long long q0 = dg::whole(v0, e), q1 = dg::whole(v1, e);
 #pragma unroll
   for (int d = 0; d < MD; ++d) {
-    // the top digit is what is left (at most 256)
-    const int a = d < MD - 1 ? (int)(signed char)(q0 & 255) : (int)q0;
-    const int b = d < MD - 1 ? (int)(signed char)(q1 & 255) : (int)q1;
-    q0 = (q0 - a) >> 8;
-    q1 = (q1 - b) >> 8;
-    // 1536 + a as FP16 bits, less 1536
-    const uint32_t bits = (uint32_t)(0x6600 + a) | (uint32_t)(0x6600 + b) << 16;
-    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&bits), __half2half2(__float2half(1536.f)));
-    *reinterpret_cast<__half2 *>(base + digit_at<R>(d, r, k)) = h;
+    const int a = dg::next(q0, d), b = dg::next(q1, d);
+    *reinterpret_cast<__half2 *>(base + digit_at<R>(d, r, k)) = dg::pair(a, b);
   }
-}
-
-__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr));
-}
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // A[r0.., r0..] -= L[r0.., k0..k0+FB) U[k0.., r0..) to the end of the matrix.
@@ -487,16 +463,12 @@ __device__ __noinline__ void update_mma(double *A, int n, int r0, int k0, const 
       uint32_t a[MD][4];
 #pragma unroll
       for (int d = 0; d < MD; ++d)
-        ldmatrix4(a[d], sL + digit_at<MT_R>(d, wr + (lane & 15), kk + (lane >> 4) * 8));
+        dg::ldmatrix4(a[d], sL + digit_at<MT_R>(d, wr + (lane & 15), kk + (lane >> 4) * 8));
 #pragma unroll
       for (int d = 0; d < MD; ++d) {
         uint32_t b[4];
-        ldmatrix4(b, sU + digit_at<MT_C>(d, wc + (lane & 7) + (lane >> 4) * 8, kk + ((lane >> 3) & 1) * 8));
-#pragma unroll
-        for (int i = MD - 1 - d; i < MD; ++i) {
-          mma_f16(acc[i + d - (MD - 1)][0], a[i], b[0], b[1]);
-          mma_f16(acc[i + d - (MD - 1)][1], a[i], b[2], b[3]);
-        }
+        dg::ldmatrix4(b, sU + digit_at<MT_C>(d, wc + (lane & 7) + (lane >> 4) * 8, kk + ((lane >> 3) & 1) * 8));
+        dg::multiply(acc, a, b, d);
       }
     }
     double v[2][4];
@@ -513,12 +485,7 @@ __device__ __noinline__ void update_mma(double *A, int n, int r0, int k0, const 
       for (int q = 0; q < 4; ++q) {
         const int ri = ti + wr + (lane >> 2) + 8 * (q >> 1), cj = tj + wc + 8 * c + 2 * (lane & 3) + (q & 1);
         if (ri >= n || cj >= n) continue;
-        // in units of 2^56: weights 7 to 12, and 6 rounded
-        long long s = (long long)__float2int_rn(acc[MD - 1][c][q]);
-#pragma unroll
-        for (int w = MD - 2; w > 0; --w) s = s * 256 + __float2int_rn(acc[w][c][q]);
-        s += (__float2int_rn(acc[0][c][q]) + 128) >> 8;
-        M(A, n, ri, cj) = fma(-(double)s, fx::scale56((int)le[ri] + (int)ue[cj]), v[c][q]);
+        M(A, n, ri, cj) = fma(-(double)dg::sum(acc, c, q), fx::scale56((int)le[ri] + (int)ue[cj]), v[c][q]);
       }
   }
   __syncthreads();
