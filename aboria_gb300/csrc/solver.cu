@@ -254,8 +254,7 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // diagonal), where the trailing update, n^3 / 3 multiply-adds, need not run at 2
 // FP64 operations a clock and SM: the rows of L21 and the columns of U12 become
 // scaled 56-bit integers (fix64.cuh), and an FP64 multiply-add (1.8 a clock and SM)
-// becomes three 32x32+64 ones (25 a clock and SM with all operands in registers)
-// within a block of columns, 28 FP16 ones on the tensor cores beyond (update_mma).
+// becomes 28 exact FP16 ones on the tensor cores (update_mma).
 // The scale is the largest entry of the row (column), so a product's error is
 // 2^-56 of the largest product of its row and column, where FP64's partial sums
 // round at 2^-53 of themselves.
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // them, two FP64 operations an entry, so the trailing matrix is updated for 64
 // columns at a time and only the rows and columns of those 64 panel by panel.
 // Pivots are compared as integers.  256 domains of 703 rows on average (set-up and
-// one apply): 98 -> 36 ms, 31.9 with the largest domains first, 24.5 with tensor
+// one apply): 98 -> 36 ms, 31.9 with the largest domains first, 22.8 with tensor
 // cores; blocks of 1,700 rows (4,003 points): 592 -> 35 ms.
 constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
 constexpr int FW = 16;         // panel width
@@ -278,196 +277,112 @@ constexpr int PLD = FW + 1;    // panel row stride
 // integer pipe waiting: 40 ms); the few rows of larger blocks stay in L2
 constexpr int FL_ROWS = 712;
 
-__device__ __forceinline__ int2 split56(double x, int e) {
-  const fx::Half2 q = fx::split56(x, e);
-  return make_int2(q.h, q.l);
-}
 using fx::abs_bits;
 using fx::scale_exp;
 
-// COUNT values per thread of a tile, read in one go (the reads' latency, not
-// their number, is what they cost) and split into (h, l).
-template <int COUNT, class Read, class Write>
-__device__ __forceinline__ void stage_split(Read read, Write write) {
-  constexpr int U = COUNT < 8 ? COUNT : 8;
-  for (int q0 = 0; q0 < COUNT; q0 += U) {
-    double v[U];
-#pragma unroll
-    for (int q = 0; q < U; ++q) v[q] = read(q0 + q);
-#pragma unroll
-    for (int q = 0; q < U; ++q) write(q0 + q, v[q]);
-  }
+// ---- updates on the tensor cores
+// The same scaled 56-bit integers as digits (digits.cuh).  Tiles of the trailing
+// matrix are 64 x 32 with all FB terms: L's digits (56 KB) stay for a row of tiles,
+// U's are 28 KB, two CTAs an SM; those within a block of columns or rows are 128 x
+// 16 and 16 x 128 with the FW terms of a panel.  A warp has 16 x 16 entries, 56
+// accumulators a thread.  With 32-bit multiply-adds (25 a clock and SM) the
+// trailing matrix took 14.3 of the 31.8 ms (set-up and one apply) of 256 domains of
+// 703 rows, now 7.1 of 24.3; with the others' multiply-adds here as well 22.8.
+using dg::MD;
+template <int TR, int TC, int KW> constexpr size_t digit_bytes() { return (size_t)MD * (TR + TC) * KW * 2; }
+constexpr size_t MD_BYTES = digit_bytes<64, 32, FB>();
+static_assert(MD_BYTES >= digit_bytes<128, 16, FW>(), "the tiles of one panel fit too");
+
+// Byte offset of digit d, row r (of a tile's R), term k: rows of KW terms whose
+// 16-byte chunks are permuted by r, so that ldmatrix reads 8 rows without conflicts.
+template <int R, int KW> __device__ __forceinline__ uint32_t digit_at(int d, int r, int k) {
+  static_assert(KW == 64 || KW == 16, "128- or 32-byte rows");
+  const int swap = KW == 64 ? r & 7 : (r >> 2) & 1;
+  return (uint32_t)((d * R + r) * (KW * 2) + (((k >> 3) ^ swap) << 4) + (k & 7) * 2);
 }
 
-// A[r0.., c0..] -= L[r0.., k0..k0+KW) U[k0.., c0..) for rows below r1 and
-// columns below c1, tiles of TR x TC dealt to the cluster's CTAs; le, ue: the
-// exponents of L's rows and U's columns.  Whole CTA; barriers at the start of
-// every tile.
-template <int TR, int TC, int KW>
-__device__ __noinline__ void update_fix(double *A, int n, int r0, int r1, int c0, int c1, int k0,
-                                        const short *le, const short *ue, int2 *tiles, int rank,
-                                        int ranks) {
-  static_assert((TR / 4) * (TC / 4) == FL_T, "one 4 x 4 piece a thread");
-  const int tid = threadIdx.x;
-  int2 *L = tiles, *U = tiles + KW * TR;  // [k][row], [k][column]
-  const int tr = (tid % (TR / 4)) * 4, tc = (tid / (TR / 4)) * 4;
-  const int nti = (r1 - r0 + TR - 1) / TR, ntj = (c1 - c0 + TC - 1) / TC;
-  int have = -1;  // row tile in L
-  {
-    for (int t = rank; t < nti * ntj; t += ranks) {
-      const int ti = r0 + (t / ntj) * TR, tj = c0 + (t % ntj) * TC;
-      __syncthreads();
-      if (ti != have)
-        stage_split<KW * TR / FL_T>(
-            [&](int q) {
-              const int e = tid + q * FL_T, r = e % TR, k = e / TR;
-              return ti + r < r1 ? M(A, n, ti + r, k0 + k) : 0.0;
-            },
-            [&](int q, double v) {
-              const int e = tid + q * FL_T, r = e % TR, k = e / TR;
-              L[k * TR + r] = split56(v, ti + r < r1 ? le[ti + r] : 0);
-            });
-      stage_split<KW * TC / FL_T>(
-          [&](int q) {
-            const int e = tid + q * FL_T, k = e % KW, j = e / KW;
-            return tj + j < c1 ? M(A, n, k0 + k, tj + j) : 0.0;
-          },
-          [&](int q, double v) {
-            const int e = tid + q * FL_T, k = e % KW, j = e / KW;
-            U[k * TC + j] = split56(v, tj + j < c1 ? ue[tj + j] : 0);
-          });
-      have = ti;
-      __syncthreads();
-      if (ti + tr >= r1 || tj + tc >= c1) continue;
-      long long hi[4][4] = {}, mid[4][4] = {};
-#pragma unroll 2
-      for (int k = 0; k < KW; ++k) {
-        int2 a[4], b[4];
-        *reinterpret_cast<int4 *>(&a[0]) = *reinterpret_cast<const int4 *>(&L[k * TR + tr]);
-        *reinterpret_cast<int4 *>(&a[2]) = *reinterpret_cast<const int4 *>(&L[k * TR + tr + 2]);
-        *reinterpret_cast<int4 *>(&b[0]) = *reinterpret_cast<const int4 *>(&U[k * TC + tc]);
-        *reinterpret_cast<int4 *>(&b[2]) = *reinterpret_cast<const int4 *>(&U[k * TC + tc + 2]);
+// Digits of COUNT pairs of values, terms (k, k + 1) of row r, `at` giving the pair's
+// row and term; four pairs are read in one go (the reads' latency, not their
+// number, is what they cost).
+template <int R, int KW, int COUNT, class At, class Read, class Exp>
+__device__ __forceinline__ void stage_digits(unsigned char *base, At at, Read read, Exp exp) {
+  constexpr int U = COUNT < 4 ? COUNT : 4;
+#pragma unroll 1
+  for (int q0 = 0; q0 < COUNT; q0 += U) {
+    double v[U][2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+    for (int q = 0; q < U; ++q) {
+      const int2 rk = at(q0 + q);
+      v[q][0] = read(rk.x, rk.y);
+      v[q][1] = read(rk.x, rk.y + 1);
+    }
 #pragma unroll
-          for (int j = 0; j < 4; ++j) mid[i][j] += (long long)a[i].x * b[j].y;
+    for (int q = 0; q < U; ++q) {
+      const int2 rk = at(q0 + q);
+      const int e = exp(rk.x);
+      long long a = dg::whole(v[q][0], e), b = dg::whole(v[q][1], e);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) hi[i][j] += (long long)a[i].x * b[j].x;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) mid[i][j] += (long long)a[i].y * b[j].x;
-      }
-      double v[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          v[i][j] = ti + tr + i < r1 && tj + tc + j < c1 ? M(A, n, ti + tr + i, tj + tc + j) : 0.0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int cj = tj + tc + j;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int ri = ti + tr + i;
-          if (ri >= r1 || cj >= c1) continue;
-          const double sc = fx::scale56((int)le[ri] + (int)ue[cj]);
-          M(A, n, ri, cj) = fma(-(double)fx::sum56(hi[i][j], mid[i][j]), sc, v[i][j]);
-        }
+      for (int d = 0; d < MD; ++d) {
+        const int x = dg::next(a, d), y = dg::next(b, d);
+        *reinterpret_cast<__half2 *>(base + digit_at<R, KW>(d, rk.x, rk.y)) = dg::pair(x, y);
       }
     }
   }
-  __syncthreads();
 }
 
-// ---- the trailing update on the tensor cores
-// The same scaled 56-bit integers as digits (digits.cuh).  A tile is 64 x
-// 32 with all FB terms: L's digits (56 KB) stay for a row of tiles, U's are 28 KB,
-// two CTAs an SM; a warp has 16 x 16 entries, 56 accumulators a thread.  With 32-bit
-// multiply-adds (25 a clock and SM) this took 14.3 of the 31.8 ms (set-up and one
-// apply) of 256 domains of 703 rows, now 7.1 of 24.5.
-using dg::MD;
-constexpr int MT_R = 64, MT_C = 32;       // tile
-static_assert(FB == 64, "rows of digits are 128 bytes");
-constexpr size_t MD_BYTES = (size_t)MD * (MT_R + MT_C) * FB * 2;
-static_assert(MD_BYTES >= (size_t)FW * (256 + 16) * sizeof(int2), "the tiles of one panel fit too");
-
-// Byte offset of digit d, row r (of a tile's R), k: 128-byte rows whose 16-byte
-// chunks are permuted by r, so that ldmatrix reads 8 rows without conflicts.
-template <int R> __device__ __forceinline__ uint32_t digit_at(int d, int r, int k) {
-  return (uint32_t)((d * R + r) * 128 + (((k >> 3) ^ (r & 7)) << 4) + (k & 7) * 2);
-}
-
-// Digits of the values of (r, k) and (r, k + 1), as pairs of FP16.
-template <int R>
-__device__ __forceinline__ void put_digits(unsigned char *base, int r, int k, double v0, double v1,
-                                           int e) {
-  long long q0 = dg::whole(v0, e), q1 = dg::whole(v1, e);
-#pragma unroll
-  for (int d = 0; d < MD; ++d) {
-    const int a = dg::next(q0, d), b = dg::next(q1, d);
-    *reinterpret_cast<__half2 *>(base + digit_at<R>(d, r, k)) = dg::pair(a, b);
-  }
-}
-
-// A[r0.., r0..] -= L[r0.., k0..k0+FB) U[k0.., r0..) to the end of the matrix.
-__device__ __noinline__ void update_mma(double *A, int n, int r0, int k0, const short *le,
-                                        const short *ue, unsigned char *sm, int rank, int ranks) {
+// A[r0.., c0..] -= L[r0.., k0..k0+KW) U[k0.., c0..) for rows below r1 and columns
+// below c1, tiles dealt to the cluster's CTAs; le, ue: the exponents of L's rows and
+// U's columns.  Whole CTA; barriers at the start of every tile.
+template <int TR, int TC, int KW>
+__device__ __noinline__ void update_mma(double *A, int n, int r0, int r1, int c0, int c1, int k0,
+                                        const short *le, const short *ue, unsigned char *sm,
+                                        int rank, int ranks) {
+  static_assert((TR / 16) * (TC / 16) == FL_T / 32, "16 x 16 a warp");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned char *L = sm, *U = sm + (size_t)MD * MT_R * 128;
+  unsigned char *L = sm, *U = sm + (size_t)MD * TR * KW * 2;
   const uint32_t sL = (uint32_t)__cvta_generic_to_shared(L), sU = (uint32_t)__cvta_generic_to_shared(U);
-  const int wr = (warp & 3) * 16, wc = (warp >> 2) * 16;  // the warp's 16 x 16 entries
-  const int nti = (n - r0 + MT_R - 1) / MT_R, ntj = (n - r0 + MT_C - 1) / MT_C;
+  const int wr = (warp % (TR / 16)) * 16, wc = (warp / (TR / 16)) * 16;
+  const int nti = (r1 - r0 + TR - 1) / TR, ntj = (c1 - c0 + TC - 1) / TC;
+  // pairs of terms a thread stages; fewer pairs than threads: the first ones do
+  constexpr int NL = TR * KW / 2, NU = TC * KW / 2;
+  constexpr int CL = NL < FL_T ? 1 : NL / FL_T, CU = NU < FL_T ? 1 : NU / FL_T;
   int have = -1;  // row tile in L
   for (int t = rank; t < nti * ntj; t += ranks) {
-    const int ti = r0 + (t / ntj) * MT_R, tj = r0 + (t % ntj) * MT_C;
+    const int ti = r0 + (t / ntj) * TR, tj = c0 + (t % ntj) * TC;
     __syncthreads();
-    if (ti != have) {
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {  // 4 pairs a thread at a time
-        double v[8];
-        const int r = tid % MT_R;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int k = 2 * (tid / MT_R + 4 * (h * 4 + q / 2)) + (q & 1);
-          v[q] = ti + r < n ? M(A, n, ti + r, k0 + k) : 0.0;
-        }
-        const int e = ti + r < n ? le[ti + r] : 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          put_digits<MT_R>(L, r, 2 * (tid / MT_R + 4 * (h * 4 + q)), v[2 * q], v[2 * q + 1], e);
-      }
-      have = ti;
-    }
-    {
-      double v[8];
-      const int k = 2 * (tid % 32);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int j = tid / 32 + 8 * (q / 2);
-        v[q] = tj + j < n ? M(A, n, k0 + k + (q & 1), tj + j) : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = tid / 32 + 8 * q;
-        put_digits<MT_C>(U, j, k, v[2 * q], v[2 * q + 1], tj + j < n ? ue[tj + j] : 0);
-      }
-    }
+    if (ti != have && tid < NL)  // lanes along the rows, which are consecutive in A
+      stage_digits<TR, KW, CL>(
+          L,
+          [&](int q) {
+            const int e = tid + q * FL_T;
+            return make_int2(e % TR, 2 * (e / TR));
+          },
+          [&](int r, int k) { return ti + r < r1 ? M(A, n, ti + r, k0 + k) : 0.0; },
+          [&](int r) { return ti + r < r1 ? (int)le[ti + r] : 0; });
+    have = ti;
+    if (tid < NU)  // lanes along the terms
+      stage_digits<TC, KW, CU>(
+          U,
+          [&](int q) {
+            const int e = tid + q * FL_T;
+            return make_int2(e / (KW / 2), 2 * (e % (KW / 2)));
+          },
+          [&](int j, int k) { return tj + j < c1 ? M(A, n, k0 + k, tj + j) : 0.0; },
+          [&](int j) { return tj + j < c1 ? (int)ue[tj + j] : 0; });
     __syncthreads();
-    if (ti + wr >= n || tj + wc >= n) continue;
+    if (ti + wr >= r1 || tj + wc >= c1) continue;
     float acc[MD][2][4] = {};  // sums of weight MD - 1 + w
 #pragma unroll 1
-    for (int kk = 0; kk < FB; kk += 16) {
+    for (int kk = 0; kk < KW; kk += 16) {
       uint32_t a[MD][4];
 #pragma unroll
       for (int d = 0; d < MD; ++d)
-        dg::ldmatrix4(a[d], sL + digit_at<MT_R>(d, wr + (lane & 15), kk + (lane >> 4) * 8));
+        dg::ldmatrix4(a[d], sL + digit_at<TR, KW>(d, wr + (lane & 15), kk + (lane >> 4) * 8));
 #pragma unroll
       for (int d = 0; d < MD; ++d) {
         uint32_t b[4];
-        dg::ldmatrix4(b, sU + digit_at<MT_C>(d, wc + (lane & 7) + (lane >> 4) * 8, kk + ((lane >> 3) & 1) * 8));
+        dg::ldmatrix4(b, sU + digit_at<TC, KW>(d, wc + (lane & 7) + (lane >> 4) * 8,
+                                               kk + ((lane >> 3) & 1) * 8));
         dg::multiply(acc, a, b, d);
       }
     }
@@ -477,14 +392,14 @@ __device__ __noinline__ void update_mma(double *A, int n, int r0, int k0, const 
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int ri = ti + wr + (lane >> 2) + 8 * (q >> 1), cj = tj + wc + 8 * c + 2 * (lane & 3) + (q & 1);
-        v[c][q] = ri < n && cj < n ? M(A, n, ri, cj) : 0.0;
+        v[c][q] = ri < r1 && cj < c1 ? M(A, n, ri, cj) : 0.0;
       }
 #pragma unroll
     for (int c = 0; c < 2; ++c)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int ri = ti + wr + (lane >> 2) + 8 * (q >> 1), cj = tj + wc + 8 * c + 2 * (lane & 3) + (q & 1);
-        if (ri >= n || cj >= n) continue;
+        if (ri >= r1 || cj >= c1) continue;
         M(A, n, ri, cj) = fma(-(double)dg::sum(acc, c, q), fx::scale56((int)le[ri] + (int)ue[cj]), v[c][q]);
       }
   }
@@ -526,7 +441,6 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
                                                     short *__restrict__ exps, int64_t nexp) {
   extern __shared__ __align__(128) unsigned char lu_raw[];
   double *Pn = reinterpret_cast<double *>(lu_raw);  // panel: rows k0..n-1 x FW, stride PLD
-  int2 *tiles = reinterpret_cast<int2 *>(lu_raw);
   __shared__ fx::u64 red_v[FL_T / 32];
   __shared__ int red_i[FL_T / 32];
   __shared__ double L11[FB / FW][FW][FW + 1];
@@ -639,7 +553,7 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
       }
       cl.sync();
       if (k1 < B1) {
-        update_fix<256, 16, FW>(A, n, k1, n, k1, B1, k0, le, ue, tiles, rank, ranks);
+        update_mma<128, 16, FW>(A, n, k1, n, k1, B1, k0, le, ue, lu_raw, rank, ranks);
         cl.sync();
       }
     }
@@ -658,7 +572,7 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
       }
       cl.sync();
       if (k1 < B1) {
-        update_fix<16, 256, FW>(A, n, k1, B1, B1, n, k0, le, ue, tiles, rank, ranks);
+        update_mma<16, 128, FW>(A, n, k1, B1, B1, n, k0, le, ue, lu_raw, rank, ranks);
         cl.sync();
       }
     }
@@ -673,7 +587,7 @@ __global__ void __launch_bounds__(FL_T, 2) k_lu_fix(double *__restrict__ mat,
       ue[r] = (short)scale_exp(mu);
     }
     cl.sync();
-    update_mma(A, n, B1, B0, le, ue, lu_raw, rank, ranks);
+    update_mma<64, 32, FB>(A, n, B1, n, B1, n, B0, le, ue, lu_raw, rank, ranks);
     cl.sync();
   }
   if (rank == 0 && tid == 0) info[d] = status;
