@@ -1,7 +1,7 @@
-// Products of matrices of scaled 56-bit integers (fix64.cuh: split56) on the
+// Products of matrices of scaled 56-bit integers (fix64.cuh: whole56) on the
 // tensor cores: an integer is seven signed 8-bit digits, each exact in FP16, and of
-// the 49 products of digits those 28 with i + j >= 6 are formed, what the three
-// 32x32+64-bit multiply-adds of two 28-bit halves keep.  The products of one weight
+// the 49 products of digits those 28 with i + j >= 6 are formed, as much as three
+// 32x32+64-bit multiply-adds of two 28-bit halves give.  The products of one weight
 // i + j, summed over up to 128 terms, stay within 2^24: FP32 accumulators hold them
 // exactly, whatever the order.  28 FP16 multiply-adds take the place of three
 // integer ones at 25 a clock and SM.
@@ -15,20 +15,9 @@
 namespace abx {
 namespace dg {
 
-constexpr int MD = 7;         // digits
+constexpr int MD = fx::DIGITS;
 constexpr int MAX_TERMS = 128;  // terms of an exact sum
 
-// x 2^(56 - e) as an integer, |x| <= 2^e.
-__device__ __forceinline__ long long whole(double x, int e) {
-  const fx::Half2 q = fx::split56(x, e);
-  return ((long long)q.h << 28) + q.l;
-}
-// The digit d of q, d = 0, 1, ... in turn; the last is what is left (at most 256).
-__device__ __forceinline__ int next(long long &q, int d) {
-  const int a = d < MD - 1 ? (int)(signed char)(q & 255) : (int)q;
-  q = (q - a) >> 8;
-  return a;
-}
 // Two digits as FP16: 1536 + a as bits, less 1536.
 __device__ __forceinline__ __half2 pair(int a, int b) {
   const uint32_t bits = (uint32_t)(0x6600 + a) | (uint32_t)(0x6600 + b) << 16;

@@ -360,28 +360,28 @@ FX_HD double multiquadric(u64 v, int r) {
 }
 
 // ------------------------------------------------- scaled 56-bit numbers ---
-// Operands of integer products of matrices: x 2^(56 - e) = h 2^28 + l with
-// signed halves, |l| <= 2^27, for |x| <= 2^e.  A sum of up to 64 products x y is
-// (hi 2^56 + mid 2^28) 2^(ex + ey - 112) with hi = sum h h and mid = sum (h l + l
-// h), both exact in 64 bits; l l is below the numbers' own 2^-57.
+// Operands of integer products of matrices (digits.cuh): x 2^(56 - e) as an
+// integer for |x| <= 2^e, and its seven signed 8-bit digits, the lowest first.
+// Of a product x y the digits' products below 256^6 are left out, which are below
+// the numbers' own 2^-57.
 FX_HD u64 abs_bits(double x) { return bits_of(x) & 0x7fffffffffffffffull; }
 // e with |x| <= 2^e from the bits of the largest |x|
 FX_HD int scale_exp(u64 maxbits) { return (int)(maxbits >> 52) - 1022; }
-struct Half2 {
-  int h, l;
-};
-FX_HD Half2 split56(double x, int e) {
+FX_HD i64 whole56(double x, int e) {
   const u64 u = bits_of(x);
   const int ex = (int)((u >> 52) & 0x7ff);
   const u64 m = (u & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
   const int sh = (ex ? ex : 1) - 1075 + 56 - e;  // |x| 2^(56 - e) = m 2^sh, sh <= 4
   i64 f = sh >= 0 ? (i64)(m << sh) : (sh > -63 ? (i64)(((m >> (-sh - 1)) + 1) >> 1) : 0);
-  if (u >> 63) f = -f;
-  const int l = (int)((u32)f << 4) >> 4;  // the low 28 bits, signed
-  return {(int)((f - l) >> 28), l};
+  return (u >> 63) ? -f : f;
 }
-// hi 2^56 + mid 2^28 in units of 2^56
-FX_HD i64 sum56(i64 hi, i64 mid) { return hi + ((mid + (1ll << 27)) >> 28); }
+constexpr int DIGITS = 7;
+// The digit d of q, d = 0, 1, ... in turn; the last is what is left (at most 256).
+FX_HD int next_digit(i64 &q, int d) {
+  const int a = d < DIGITS - 1 ? (int)(signed char)(q & 255) : (int)q;
+  q = (q - a) >> 8;
+  return a;
+}
 // 2^(e - 56) (2^-1022 at least)
 FX_HD double scale56(int e) {
   const int b = e - 56 + 1023;

@@ -434,10 +434,10 @@ __global__ void __launch_bounds__(256) k_split_digits(const double *__restrict__
   if (lane == 0) exps[row] = (short)e;
   for (int c = 0; c < chunks; ++c) {
     const int j = c * MF_K + lane;
-    long long q = j < nc ? dg::whole(v[j], e) : 0;
+    fx::i64 q = j < nc ? fx::whole56(v[j], e) : 0;
     __half *o = out + (((row / per) * chunks + c) * per + row % per) * MF_ROW + lane;
 #pragma unroll
-    for (int d = 0; d < MD; ++d) o[d * MF_K] = __low2half(dg::pair(dg::next(q, d), 0));
+    for (int d = 0; d < MD; ++d) o[d * MF_K] = __low2half(dg::pair(fx::next_digit(q, d), 0));
   }
 }
 

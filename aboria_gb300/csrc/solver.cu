@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // Pivots are compared as integers.  256 domains of 703 rows on average (set-up and
 // one apply): 98 -> 36 ms, 31.9 with the largest domains first, 22.8 with tensor
 // cores; blocks of 1,700 rows (4,003 points): 592 -> 35 ms.
-constexpr int FL_T = 256;      // threads, a 4 x 4 piece of an update tile each
+constexpr int FL_T = 256;      // threads
 constexpr int FW = 16;         // panel width
 constexpr int FB = 64;         // columns of a trailing update
 constexpr int PLD = FW + 1;    // panel row stride
@@ -320,10 +320,10 @@ __device__ __forceinline__ void stage_digits(unsigned char *base, At at, Read re
     for (int q = 0; q < U; ++q) {
       const int2 rk = at(q0 + q);
       const int e = exp(rk.x);
-      long long a = dg::whole(v[q][0], e), b = dg::whole(v[q][1], e);
+      fx::i64 a = fx::whole56(v[q][0], e), b = fx::whole56(v[q][1], e);
 #pragma unroll
       for (int d = 0; d < MD; ++d) {
-        const int x = dg::next(a, d), y = dg::next(b, d);
+        const int x = fx::next_digit(a, d), y = fx::next_digit(b, d);
         *reinterpret_cast<__half2 *>(base + digit_at<R, KW>(d, rk.x, rk.y)) = dg::pair(x, y);
       }
     }

@@ -43,13 +43,20 @@ double dot56(const double *x, const double *y, int n) {
     my = abs_bits(y[i]) > my ? abs_bits(y[i]) : my;
   }
   const int ex = scale_exp(mx), ey = scale_exp(my);
-  i64 hi = 0, mid = 0;
+  i64 w[2 * DIGITS - 1] = {};  // sums by weight
   for (int i = 0; i < n; ++i) {
-    const Half2 a = split56(x[i], ex), b = split56(y[i], ey);
-    hi += (i64)a.h * b.h;
-    mid += (i64)a.h * b.l + (i64)a.l * b.h;
+    i64 a = whole56(x[i], ex), b = whole56(y[i], ey);
+    int p[DIGITS], q[DIGITS];
+    for (int d = 0; d < DIGITS; ++d) p[d] = next_digit(a, d), q[d] = next_digit(b, d);
+    for (int d = 0; d < DIGITS; ++d)
+      for (int c = DIGITS - 1 - d; c < DIGITS; ++c) w[c + d] += p[c] * q[d];
   }
-  return (double)sum56(hi, mid) * scale56(ex + ey);
+  i64 s = w[2 * DIGITS - 2];
+  for (int k = 2 * DIGITS - 3; k >= DIGITS; --k) s = s * 256 + w[k];
+  s += (w[DIGITS - 1] + 128) >> 8;
+  for (int k = DIGITS - 1; k < 2 * DIGITS - 1; ++k)
+    if (w[k] > (1 << 24) || -w[k] > (1 << 24)) return 1e300;  // not exact in FP32
+  return (double)s * scale56(ex + ey);
 }
 double v_mq(const double *x, const double *y, int dim, double reach, double p0) {
   return run<MULTIQUADRIC>(x, y, dim, reach, p0);
@@ -133,8 +140,8 @@ def test_limits(lib):
 @pytest.mark.parametrize("n", [1, 2, 16, 63, 64])
 @pytest.mark.parametrize("scale", [1.0, 2.0 ** -300, 2.0 ** 300])
 def test_scaled_products(lib, n, scale):
-    """n products: each operand good to 2^-57 of the largest, the low parts'
-    products (2^-58) left out, one rounding of the sum."""
+    """n products by digits: each operand good to 2^-57 of the largest, the low
+    digits' products (2^-58) left out, one rounding of the sum."""
     rng = random.Random(n)
     for _ in range(200):
         x = [rng.choice([-1, 1]) * rng.random() * scale * 2.0 ** -rng.randrange(40) for _ in range(n)]
