@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import aboria_gb300 as ab
+import oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,20 @@ def test_mixed_product_of_scaled_weights(order):
     for w in (b, b * 2.0 ** 60, b * 2.0 ** -60, b * 2.0 ** (60 * (p.positions[:, 0] - 0.5)), 0 * b):
         want = exact * w
         assert np.linalg.norm(mixed * w - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("dim,order", [(1, 8), (2, 5), (2, 6), (2, 8), (3, 3), (3, 4), (3, 6)])
+def test_fp64_m2l_by_digits(dim, order):
+    """Node counts around the M2L kernel's 16, 32, 64 and 128 terms (8, 25, 36, 64,
+    27, 64, 216), tiles that are not full, weights over many magnitudes."""
+    n = 3000 if dim < 3 else 1500
+    rng = np.random.default_rng(dim * 10 + order)
+    x = rng.uniform(0, 1, (n, dim))
+    p = ab.Particles(dim).set(x)
+    p.init_octree([0.0] * dim, [1.0] * dim, [False] * dim, 20)
+    b = rng.standard_normal(n) * 2.0 ** rng.integers(-20, 1, n)
+    got = ab.create_fmm_operator(p, ab.Kernel.make(ab.K_MULTIQUADRIC, 0.01), order) * b
+    want = oracle.fmm(p.positions, [0.0] * dim, [1.0] * dim, 20, order, ab.K_MULTIQUADRIC, [0.01], b)
+    # two sums of at most 216 terms, 189 pairs and 1,500 sources a target, with up to
+    # 50 times the result's size in the terms of signed weights
+    assert np.linalg.norm(got - want) <= 50 * 2000 * 2.0 ** -53 * np.linalg.norm(want)
