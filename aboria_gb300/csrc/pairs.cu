@@ -1765,7 +1765,10 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
               } else {
                 bool in = dd <= r2lo;
                 if (!in && dd <= r2hi) {  // rare: the reference's FP64 test
-                  const int img[3] = {i0 - 1, i1 - 1, i2};
+                  // (opaque: otherwise the image shifts' FP64 products are computed for
+                  // every row, ahead of this branch: 3 of 4 FP64 instructions)
+                  int img[3] = {i0 - 1, i1 - 1, i2};
+                  asm volatile("" : "+r"(img[0]), "+r"(img[1]), "+r"(img[2]));
                   in = !(exact_norm(P.qpos[qi], P.cpos[k], img, fg, NORM) > P.thr);
                 }
                 if (POL == POL_COUNT) count += in ? 1 : 0;
