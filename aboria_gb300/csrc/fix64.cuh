@@ -365,8 +365,12 @@ FX_HD double multiquadric(u64 v, int r) {
 // Of a product x y the digits' products below 256^6 are left out, which are below
 // the numbers' own 2^-57.
 FX_HD u64 abs_bits(double x) { return bits_of(x) & 0x7fffffffffffffffull; }
-// e with |x| <= 2^e from the bits of the largest |x|
-FX_HD int scale_exp(u64 maxbits) { return (int)(maxbits >> 52) - 1022; }
+// e with |x| <= 2^e from the bits of the largest |x|; NOT_FINITE, which makes
+// every integer 0 and every scale NaN, if that is infinite or NaN
+constexpr int NOT_FINITE = 16384;
+FX_HD int scale_exp(u64 maxbits) {
+  return maxbits >= 0x7ff0000000000000ull ? NOT_FINITE : (int)(maxbits >> 52) - 1022;
+}
 FX_HD i64 whole56(double x, int e) {
   const u64 u = bits_of(x);
   const int ex = (int)((u >> 52) & 0x7ff);
@@ -382,9 +386,10 @@ FX_HD int next_digit(i64 &q, int d) {
   q = (q - a) >> 8;
   return a;
 }
-// 2^(e - 56) (2^-1022 at least)
+// 2^(e - 56) (2^-1022 at least; infinite from 2^1024 on)
 FX_HD double scale56(int e) {
   const int b = e - 56 + 1023;
+  if (b > 2046) return from_bits(b > NOT_FINITE / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull);
   return from_bits((u64)(b > 1 ? b : 1) << 52);
 }
 

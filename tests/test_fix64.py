@@ -143,6 +143,10 @@ def test_scaled_products(lib, n, scale):
     """n products by digits: each operand good to 2^-57 of the largest, the low
     digits' products (2^-58) left out, one rounding of the sum."""
     rng = random.Random(n)
+    for bad in (float("inf"), float("nan")):
+        v = lib.dot56((C.c_double * n)(*[bad] * n), (C.c_double * n)(*[1.0] * n), n)
+        assert v != v
+    assert lib.dot56((C.c_double * n)(*[1e200] * n), (C.c_double * n)(*[1e200] * n), n) == float("inf")
     for _ in range(200):
         x = [rng.choice([-1, 1]) * rng.random() * scale * 2.0 ** -rng.randrange(40) for _ in range(n)]
         y = [rng.choice([-1, 1]) * rng.random() for _ in range(n)]

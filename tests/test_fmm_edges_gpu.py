@@ -56,3 +56,18 @@ def test_fp64_m2l_by_digits(dim, order):
     # two sums of at most 216 terms, 189 pairs and 1,500 sources a target, with up to
     # 50 times the result's size in the terms of signed weights
     assert np.linalg.norm(got - want) <= 50 * 2000 * 2.0 ** -53 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("order", [3, 5])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_weights_that_are_not_finite_reach_every_target(order, mixed, value):
+    rng = np.random.default_rng(order)
+    p = ab.Particles(3).set(rng.uniform(0, 1, (2000, 3)))
+    p.init_octree([0.0] * 3, [1.0] * 3, [False] * 3, 20)
+    b = rng.uniform(1, 2, 2000)
+    K = ab.create_fmm_operator(p, ab.Kernel.make(ab.K_MULTIQUADRIC, 0.01), order,
+                               ab.PREC_MIXED if mixed else ab.PREC_FP64)
+    assert np.all(np.isfinite(K * b))
+    b[7] = value
+    assert not np.any(np.isfinite(K * b))
