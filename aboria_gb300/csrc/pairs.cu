@@ -35,6 +35,7 @@
 #include "common.cuh"
 #include "fix64.cuh"
 #include "handles.cuh"
+#include "unit_work.cuh"
 
 namespace abx {
 
@@ -91,12 +92,6 @@ constexpr Split SPLIT_FP64{12, 1 << 30, 16}, SPLIT_COUNT{7, 12, 4}, SPLIT_MIXED{
     SPLIT_NONE{0, 0, 1};
 constexpr int64_t MIXED_MIN = 50000;
 
-// Written by k_tables into pinned host memory: seq last.
-struct HostCounts {
-  int full, singles;
-  int seq;
-};
-
 struct PairLayout {
   FineGrid fg;
   double r = 0;
@@ -116,12 +111,12 @@ struct PairLayout {
   // count or product (4, 5) and of a list search (6, 7); small units and single
   // queries that a count or product works (8, 9)
   DevBuf<int> counts;
-  // the first three on the host, once the device has written them: one of the
-  // two pair kernels has no work at uniform density, and is not launched then
-  HostCounts *host = nullptr;
-  int host_seq = 0;
+  // written by k_tables into pinned host memory: one of the two pair kernels has
+  // no work at uniform density, and is not launched then (unit_work.cuh)
+  uint64_t *work = nullptr;
+  uint32_t work_seq = 0;
   ~PairLayout() {
-    if (host) cudaFreeHost(host);
+    if (work) cudaFreeHost(work);
   }
   DevBuf<float> bk32;
   DevBuf<double> bk64;
@@ -541,7 +536,7 @@ struct KParams {
   const int *counts;     // full units, small units, singles
   int all_units;         // 1: the small units too (searches that write lists)
   int *counter;          // work counters: units, singles
-  int known_full, known_singles;  // work of the two kernels, -1: not known (yet)
+  UnitWork work;         // of the two kernels, as far as the host knows
   const float4 *bands;   // two entries a span: r2lo, r2hi, r2box, rbox_inf; r2mid, r2half
   const int4 *stencil;   // unpruned rows of a cell's stencil, counts[3] of them
   int lanes;             // lanes a query of the singles
@@ -945,7 +940,7 @@ __global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2
                                                       float4 *__restrict__ bands,
                                                       int4 *__restrict__ rows,
                                                       int *__restrict__ counts, int nq, int fold_at,
-                                                      HostCounts *host, int seq) {
+                                                      uint64_t *work, uint32_t seq) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x == 0) {
     __shared__ int wsum[TABLE_TPB / 32];
@@ -973,12 +968,8 @@ __global__ void __launch_bounds__(TABLE_TPB) k_tables(FineGrid fg, double prune2
       const bool fold = (int64_t)counts[2] * fold_at < nq;
       counts[8] = fold ? counts[1] : 0;
       counts[9] = fold ? 0 : counts[2];
-      if (host) {
-        host->full = counts[0] + counts[8];
-        host->singles = counts[9];
-        __threadfence_system();
-        *(volatile int *)&host->seq = seq;
-      }
+      if (work)
+        *(volatile uint64_t *)work = unit_work_word(seq, counts[0] + counts[8] > 0, counts[9] > 0);
     }
   }
   if (t < EXT_TAB * EXT_TAB) {
@@ -1833,7 +1824,7 @@ int build_tables(abx_context *ctx, PairLayout &L, int norm, double thr) {
   ABX_TRY(L.stencil.reserve(ROWS_MAX));
   k_tables<<<EXT_TAB * EXT_TAB / TABLE_TPB, TABLE_TPB, 0, ctx->stream>>>(
       L.fg, prune_distance2(L), L.r, thr, norm, L.ext.ptr, L.bands.ptr, L.stencil.ptr,
-      L.counts.ptr, (int)L.rows->n, L.split.fold, L.host, ++L.host_seq);
+      L.counts.ptr, (int)L.rows->n, L.split.fold, L.work, ++L.work_seq);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
@@ -1868,9 +1859,7 @@ KParams base_params(const PairLayout &L) {
   P.counts = L.counts.ptr;
   P.counter = L.counts.ptr + 4;
   P.qperm = L.rows->perm.ptr;
-  const bool known = L.host && *(volatile int *)&L.host->seq == L.host_seq;
-  P.known_full = known ? L.host->full : -1;
-  P.known_singles = known ? L.host->singles : -1;
+  P.work = L.work ? unit_work(L.work, L.work_seq) : UnitWork{true, true};
   P.fxy = L.cols.fxy.ptr;
   P.fz = L.cols.fz.ptr;
   P.qfxy = L.rows->fxy.ptr;
@@ -1906,7 +1895,7 @@ template <int KIND> int launch_matvec(abx_context *ctx, KParams P, bool mixed, b
   constexpr int FK = KIND == ABX_K_COMPACT_GAUSSIAN ? ABX_K_GAUSSIAN : KIND;
   constexpr bool CAN_FIX = FK == ABX_K_GAUSSIAN || FK == ABX_K_WENDLAND_C2 ||
                            FK == ABX_K_LAPLACE || FK == ABX_K_MULTIQUADRIC;
-  const bool units = P.known_full != 0, singles = P.known_singles != 0;
+  const bool units = P.work.full, singles = P.work.singles;
   if (mixed) {
     if (units) k_pairs_mixed<POL_MATVEC, FK><<<ub, T, 0, s>>>(P);
     if (singles) k_pairs_thread<POL_MATVEC, FK, VAL_MIXED><<<tb, T, 0, s>>>(P);
@@ -2021,9 +2010,9 @@ int pair_layout_build(abx_operator *op) {
   abx_context *ctx = op->rows->ctx;
   if (!op->pairs) op->pairs = new PairLayout();
   PairLayout &L = *op->pairs;  // a rebuild keeps the buffers
-  if (!L.host) {
-    ABX_CHECK_CUDA(cudaHostAlloc((void **)&L.host, sizeof(HostCounts), cudaHostAllocMapped));
-    *L.host = HostCounts{};
+  if (!L.work) {
+    ABX_CHECK_CUDA(cudaHostAlloc((void **)&L.work, sizeof(uint64_t), cudaHostAllocMapped));
+    *L.work = 0;
   }
   L.cols_version = ~uint64_t(0);  // valid once everything below has succeeded
   const bool self = op->rows == op->cols;
