@@ -21,8 +21,8 @@
 //    error).  A pair is accepted outright if d2 <= r2_lo, rejected if
 //    d2 > r2_hi, and only inside that rounding band is the reference's exact
 //    FP64 test evaluated, so neighbour decisions are identical to the FP64
-//    test.  Kernel values are FP32; each lane sums a staged block of <= 32
-//    terms in FP32 and adds the block into an FP64 accumulator.
+//    test.  Kernel values are FP32; each lane sums at most 64 terms in FP32 (32 in
+//    either half of a packed sum) before it adds them into an FP64 accumulator.
 //  * FP64 mode: candidates are staged as absolute FP64 positions and every
 //    pair evaluates the reference's formula exactly (no FMA contraction).
 #include <algorithm>
@@ -1627,6 +1627,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
 enum { VAL_FP64 = 0, VAL_MIXED = 1, VAL_FIX = 2 };
 constexpr int QCAP = 16;   // queued pairs per lane
 constexpr int DRAIN = 22;  // lanes that make an evaluation worth its issue
+constexpr int FLUSH32 = 32;  // terms of an FP32 sum, which then goes to the FP64 one
 
 template <int POL, int KIND, int VAL, int NORM = 2>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
@@ -1671,7 +1672,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
     const double si = (QUEUE && KIND == ABX_K_SCALAR_SUM) ? P.s_row[qi] : 0.0;
     double acc = 0.0;
     float acc32 = 0.f;
-    int count = 0, nq = 0, rows32 = 0;
+    int count = 0, nq = 0, steps = 0;
     auto evaluate = [&]() {  // one queued pair of every lane that has one
       if (nq > 0) {
         --nq;
@@ -1772,16 +1773,18 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
               }
               ++k;
             }
+            // every FLUSH32 candidates, however many a row of the stencil holds: a row
+            // may cross a cluster that the query is not in
+            if (VAL == VAL_MIXED && POL == POL_MATVEC && (++steps & (FLUSH32 - 1)) == 0) {
+              acc += (double)acc32;
+              acc32 = 0.f;
+            }
             if (QUEUE && __any_sync(0xffffffffu, nq == QCAP)) {
               do evaluate();
               while (__popc(__ballot_sync(0xffffffffu, nq > 0)) >= DRAIN);
             }
           }
         }
-      }
-      if (VAL == VAL_MIXED && POL == POL_MATVEC && (++rows32 & 3) == 0) {
-        acc += (double)acc32;
-        acc32 = 0.f;
       }
     }
     if (QUEUE)
