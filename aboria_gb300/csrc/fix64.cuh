@@ -371,6 +371,14 @@ constexpr int NOT_FINITE = 16384;
 FX_HD int scale_exp(u64 maxbits) {
   return maxbits >= 0x7ff0000000000000ull ? NOT_FINITE : (int)(maxbits >> 52) - 1022;
 }
+// The size of a number is its biased exponent.  Numbers that span ONE_SIZE powers of
+// two at most (within a factor of 8) keep FP64's precision in one scale: 56 bits for
+// the largest are 53 and more for the smallest.
+constexpr int ONE_SIZE = 2;
+FX_HD int size_of(double x) { return (int)(abs_bits(x) >> 52); }
+FX_HD int size_span(int smallest, int largest) {  // infinite and NaN: no size
+  return largest == 2047 ? largest : largest - smallest;
+}
 FX_HD i64 whole56(double x, int e) {
   const u64 u = bits_of(x);
   const int ex = (int)((u >> 52) & 0x7ff);

@@ -24,8 +24,9 @@
 // in the mixed-precision mode on the tensor cores with FP32 accumulation (split
 // FP16 on tcgen05 above 64 nodes, 3xTF32 on mma.sync below) and P2P in FP32; in
 // the FP64 mode M2L is a product of scaled 56-bit integers, by their digits on the
-// tensor cores, and P2P takes its kernel values from the integer units (fix64.cuh), both with errors no larger
-// than FP64's own.
+// tensor cores, for matrices whose rows hold values of one size, and in FP64 for the
+// others; P2P takes its kernel values from the integer units (fix64.cuh).  Both have
+// errors no larger than FP64's own.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -81,8 +82,10 @@ struct FmmPlan {
   // FP64 M2L: digits of K and W, their exponents (per row of K, per node), tiles
   DevBuf<__half> Kd, Wd;
   DevBuf<short> ke, we;
-  DevBuf<int> mf_mat, mf_first;
-  int mf_tiles = 0;
+  DevBuf<int> mf_mat, mf_first;  // tiles of the matrices that are multiplied by digits
+  DevBuf<int> mw_mat, mw_first;  // and of those with rows of many sizes (k_m2l64)
+  int mf_tiles = 0, mw_tiles = 0;
+  bool m2l64_ready = false;
   // W as scaled FP16, hi and lo, and each node's power of two (tcgen05 M2L)
   DevBuf<__half> W16h, W16l;
   DevBuf<float> W16_scale;
@@ -406,8 +409,12 @@ __global__ void k_transpose_tc(const double *__restrict__ in, int nchild, int nc
 // (digits.cuh): for one matrix K and a tile of TC (target, source) pairs sharing
 // it, TR rows of K W[:, sources], a warp 16 x 16 of them.  Digits are made once, of
 // K per plan with a scale per row (Kd), of W per product with a scale per node
-// (Wd); both scales and 57 bits make a term's rounding smaller than the FP64 sum's
-// own.  32 terms are staged at a time, the next while the last are multiplied.
+// (Wd).  A term is good to 2^-56 of the largest K of its row times the largest W of its
+// node, so matrices with a row that spans more than fx::ONE_SIZE powers of two (a
+// broad Gaussian's on coarse levels) are left to k_m2l64: their small entries would
+// have fewer than FP64's 53 bits.  1 / d and sqrt(d^2 + c) stay within two at box
+// distances of 1 to 2.45.  32 terms are staged at a time, the next while the last are
+// multiplied.
 // With FP64 one CTA a pair was bound by the pipe's 1.8 multiply-adds a clock and
 // SM, with three 32x32+64-bit ones by their 25.  N = 1,048,576, 6.0e6 pairs: order 3
 // (27 nodes) 8.5 -> 2.3 -> 1.8 ms; 100,000 points, order 5 (125), the whole
@@ -438,6 +445,67 @@ __global__ void __launch_bounds__(256) k_split_digits(const double *__restrict__
     __half *o = out + (((row / per) * chunks + c) * per + row % per) * MF_ROW + lane;
 #pragma unroll
     for (int d = 0; d < MD; ++d) o[d * MF_K] = __low2half(dg::pair(fx::next_digit(q, d), 0));
+  }
+}
+
+// Powers of two that the rows of each matrix span at most (fx::size_span): a CTA a
+// matrix.
+__global__ void __launch_bounds__(MF_T) k_row_span(const double *__restrict__ Km, int nc,
+                                                   int *__restrict__ span) {
+  __shared__ int most;
+  if (threadIdx.x == 0) most = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i < nc; i += MF_T / 32) {
+    const double *row = Km + ((size_t)blockIdx.x * nc + i) * nc;
+    int lo = 2047, hi = 0;
+    for (int j = lane; j < nc; j += 32) {
+      const int e = fx::size_of(row[j]);
+      lo = min(lo, e);
+      hi = max(hi, e);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) atomicMax(&most, fx::size_span(lo, hi));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) span[blockIdx.x] = most;
+}
+
+// The same product in FP64, MW_PAIRS pairs of one matrix a CTA, four of them with
+// every K that is read.  Bound by the FP64 pipe.
+constexpr int MW_PAIRS = 16;
+__global__ void __launch_bounds__(FT) k_m2l64(int ncheb, const double *__restrict__ Km,
+                                              const int2 *__restrict__ by_mat,
+                                              const int *__restrict__ mat_off,
+                                              const int *__restrict__ tile_mat,
+                                              const int *__restrict__ tile_first,
+                                              const double *__restrict__ W,
+                                              double *__restrict__ G) {
+  constexpr int U = 4;
+  __shared__ double ws[MAXC][U];
+  const int m = tile_mat[blockIdx.x], first = tile_first[blockIdx.x];
+  const int last = min(first + MW_PAIRS, mat_off[m + 1]);
+  const double *K = Km + (size_t)m * ncheb * ncheb;
+  for (int q = first; q < last; q += U) {
+    const int np = min(U, last - q);
+    __syncthreads();
+    for (int e = threadIdx.x; e < U * ncheb; e += FT) {
+      const int u = e / ncheb, j = e - u * ncheb;
+      ws[j][u] = u < np ? W[(size_t)by_mat[q + u].y * ncheb + j] : 0.0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ncheb; i += FT) {
+      double a[U] = {};
+      for (int j = 0; j < ncheb; ++j) {
+        const double k = K[(size_t)i * ncheb + j];
+#pragma unroll
+        for (int u = 0; u < U; ++u) a[u] += k * ws[j][u];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < np) atomicAdd(&G[(size_t)by_mat[q + u].x * ncheb + i], a[u]);
+    }
   }
 }
 
@@ -1852,39 +1920,60 @@ void launch_links(const FmmPlan *P, int lev, const T *mats, double *V, cudaStrea
 }
 
 namespace {
-// The FP64 M2L: G += K W.  The split matrices and the tiles of 64 pairs are made
-// by the plan's first FP64 product.
-// The split matrices and buffers of the FP64 M2L, once per plan.
-int m2l_fix_prepare(FmmPlan *P, cudaStream_t s) {
+// The FP64 M2L's tiles, split matrices and buffers, once per plan.
+int m2l64_prepare(FmmPlan *P, cudaStream_t s) {
   const int nc = P->ncheb, chunks = (nc + MF_K - 1) / MF_K;
-  if (!P->Kd.ptr) {
-    std::vector<int> mat, first;
-    for (int m = 0; m < P->nmat; ++m)
-      for (int q = P->mat_off[m]; q < P->mat_off[m + 1]; q += mf_pairs(nc)) {
-        mat.push_back(m);
-        first.push_back(q);
-      }
-    P->mf_tiles = (int)mat.size();
+  if (P->m2l64_ready) return ABX_OK;
+  DevBuf<int> span_d;
+  std::vector<int> span((size_t)P->nmat);
+  ABX_TRY(span_d.reserve(span.size()));
+  k_row_span<<<P->nmat, MF_T, 0, s>>>(P->Km.ptr, nc, span_d.ptr);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  ABX_CHECK_CUDA(cudaMemcpyAsync(span.data(), span_d.ptr, span.size() * 4, cudaMemcpyDeviceToHost, s));
+  ABX_CHECK_CUDA(cudaStreamSynchronize(s));
+  std::vector<int> mat[2], first[2];  // by digits, in FP64
+  for (int m = 0; m < P->nmat; ++m) {
+    const int wide = span[m] > fx::ONE_SIZE, tile = wide ? MW_PAIRS : mf_pairs(nc);
+    for (int q = P->mat_off[m]; q < P->mat_off[m + 1]; q += tile) {
+      mat[wide].push_back(m);
+      first[wide].push_back(q);
+    }
+  }
+  auto up = [&](DevBuf<int> &dst, const std::vector<int> &v) -> int {
+    ABX_TRY(dst.reserve(v.size() + 1));
+    ABX_CHECK_CUDA(cudaMemcpyAsync(dst.ptr, v.data(), v.size() * 4, cudaMemcpyHostToDevice, s));
+    return ABX_OK;
+  };
+  ABX_TRY(up(P->mf_mat, mat[0]));
+  ABX_TRY(up(P->mf_first, first[0]));
+  ABX_TRY(up(P->mw_mat, mat[1]));
+  ABX_TRY(up(P->mw_first, first[1]));
+  P->mf_tiles = (int)mat[0].size();
+  P->mw_tiles = (int)mat[1].size();
+  if (P->mf_tiles > 0) {
     const int64_t rows = (int64_t)P->nmat * nc;
-    ABX_TRY(P->mf_mat.reserve(mat.size() + 1));
-    ABX_TRY(P->mf_first.reserve(first.size() + 1));
     ABX_TRY(P->ke.reserve((size_t)rows));
-    ABX_CHECK_CUDA(cudaMemcpyAsync(P->mf_mat.ptr, mat.data(), mat.size() * 4, cudaMemcpyHostToDevice, s));
-    ABX_CHECK_CUDA(cudaMemcpyAsync(P->mf_first.ptr, first.data(), first.size() * 4,
-                                   cudaMemcpyHostToDevice, s));
     ABX_TRY(P->Kd.reserve((size_t)rows * chunks * MF_ROW));
     k_split_digits<<<ceil_div((size_t)rows, 8), 256, 0, s>>>(P->Km.ptr, rows, nc, nc, P->Kd.ptr,
                                                              P->ke.ptr);
     ABX_CHECK_CUDA(cudaGetLastError());
-    ABX_CHECK_CUDA(cudaStreamSynchronize(s));  // the host lists end here
+    ABX_TRY(P->Wd.reserve((size_t)P->nnodes * chunks * MF_ROW));
+    ABX_TRY(P->we.reserve((size_t)P->nnodes));
   }
-  ABX_TRY(P->Wd.reserve((size_t)P->nnodes * chunks * MF_ROW));
-  return P->we.reserve((size_t)P->nnodes);
+  ABX_CHECK_CUDA(cudaStreamSynchronize(s));  // the host lists end here
+  P->m2l64_ready = true;
+  return ABX_OK;
 }
 
-int m2l_fix(FmmPlan *P, cudaStream_t s) {
+// G += K W in FP64.
+int m2l64(FmmPlan *P, cudaStream_t s) {
   const int nc = P->ncheb;
-  ABX_TRY(m2l_fix_prepare(P, s));
+  ABX_TRY(m2l64_prepare(P, s));
+  if (P->mw_tiles > 0)
+    k_m2l64<<<P->mw_tiles, FT, 0, s>>>(nc, P->Km.ptr, P->m2l_by_mat.ptr, P->mat_off_d.ptr,
+                                       P->mw_mat.ptr, P->mw_first.ptr, P->W.ptr, P->G.ptr);
+  ABX_CHECK_CUDA(cudaGetLastError());
+  if (P->mf_tiles == 0) return ABX_OK;
   k_split_digits<<<ceil_div((size_t)P->nnodes, 8), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, 1, P->Wd.ptr,
                                                                 P->we.ptr);
   auto run = [&](auto kern, int tr, size_t smem) -> int {
@@ -1904,7 +1993,7 @@ int m2l_fix(FmmPlan *P, cudaStream_t s) {
 // What a plan's FP64 products keep: a first product then allocates nothing and
 // waits for nothing.
 int fmm_plan_prepare(FmmPlan *P, cudaStream_t s) {
-  return P->n_m2l > 0 ? m2l_fix_prepare(P, s) : ABX_OK;
+  return P->n_m2l > 0 ? m2l64_prepare(P, s) : ABX_OK;
 }
 
 // c = K b through the five FMM passes (storage order of the octree set).
@@ -2020,7 +2109,7 @@ int fmm_matvec_device(abx_operator *op, const double *b, double *c) {
       }
       k_add_g32<<<ceil_div(tot, 256), 256, 0, s>>>(P->G32.ptr, P->nnodes, nc, ldg, P->G.ptr);
     } else {
-      ABX_TRY(m2l_fix(P, s));
+      ABX_TRY(m2l64(P, s));
     }
     ABX_CHECK_CUDA(cudaGetLastError());
   }
