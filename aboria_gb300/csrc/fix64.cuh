@@ -400,6 +400,17 @@ FX_HD double scale56(int e) {
   if (b > 2046) return from_bits(b > NOT_FINITE / 2 ? 0x7ff8000000000000ull : 0x7ff0000000000000ull);
   return from_bits((u64)(b > 1 ? b : 1) << 52);
 }
+// 2^k for -1074 <= k <= 1023
+FX_HD double pow2(int k) { return from_bits(k >= -1022 ? (u64)(k + 1023) << 52 : 1ull << (k + 1074)); }
+// t 2^(e - 56) for a whole number t, rounded once, e the sum of two scales (-2044 at
+// least), also where 2^(e - 56) itself is beyond the doubles; NaN if one of the two
+// was NOT_FINITE.
+FX_HD double times56(double t, int e) {
+  const int k = e - 56;
+  if (k >= -1022 && k <= 1023) return t * pow2(k);
+  if (e > NOT_FINITE / 2) return from_bits(0x7ff8000000000000ull);
+  return t * pow2(k / 2) * pow2(k - k / 2);  // the first product is exact, or infinite as the second
+}
 
 // ------------------------------------------------------------------- units ---
 // The fixed point of one kernel for pairs up to `reach` apart: coordinates

@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(MF_T, 2) k_m2l_fix(
       const int r = r0 + wr + (lane >> 2) + 8 * (q >> 1), p = wc + 8 * b + 2 * (lane & 3) + (q & 1);
       if (r >= nc || p >= np) continue;
       const double t = STAGES > 1 ? total[b][q] : (double)dg::sum(acc, b, q);
-      atomicAdd(&G[(size_t)tgt[p] * nc + r], t * fx::scale56((int)ke[(size_t)m * nc + r] + sexp[p]));
+      atomicAdd(&G[(size_t)tgt[p] * nc + r], fx::times56(t, (int)ke[(size_t)m * nc + r] + sexp[p]));
     }
 }
 

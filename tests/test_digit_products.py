@@ -45,6 +45,7 @@ double dot56(const double *x, const double *y, int n) {
   for (int k = 2 * DIGITS - 3; k >= DIGITS; --k) s = s * 256 + w[k];
   return (double)(s + ((w[DIGITS - 1] + 128) >> 8)) * scale56(ex + ey);
 }
+double scaled(double t, int e) { return times56(t, e); }
 double dot64(const double *x, const double *y, int n) {
   double s = 0;
   for (int i = 0; i < n; ++i) s = __builtin_fma(x[i], y[i], s);
@@ -63,7 +64,7 @@ def lib(tmp_path_factory):
                     str(ROOT / "aboria_gb300" / "csrc"), str(d / "digits_host.cpp"), "-o", str(so)],
                    check=True)
     lib = C.CDLL(str(so))
-    lib.dot56.restype = lib.dot64.restype = C.c_double
+    lib.dot56.restype = lib.dot64.restype = lib.scaled.restype = C.c_double
     return lib
 
 
@@ -139,3 +140,15 @@ def test_extreme_digits(lib, digits, n):
     got = lib.dot56((C.c_double * n)(*[x] * n), (C.c_double * n)(*[x] * n), n)
     want = n * Fraction(x) ** 2
     assert abs(Fraction(got) - want) <= n * Fraction(1, 2 ** 55) + want / 2 ** 53
+
+
+@pytest.mark.parametrize("e", [-2044, -1500, -1140, -1100, -1074, -966, -965, 0, 1079, 1080, 1500, 2000])
+def test_scales_beyond_the_doubles(lib, e):
+    for t in (0, 1, 3, 2 ** 53 - 1, -(2 ** 62), 2 ** 66):
+        got = lib.scaled(C.c_double(float(t)), e)
+        want = Fraction(t) * Fraction(2) ** (e - 56)
+        if abs(want) >= Fraction(2) ** 1024:
+            assert got == math.copysign(float("inf"), t)
+        else:
+            assert got == float(want)  # (Fraction rounds once)
+    assert math.isnan(lib.scaled(C.c_double(1.0), 16384 + 5))
