@@ -482,9 +482,14 @@ struct Consts {
 };
 FX_HD Consts consts(const Unit &U, double k0) { return {U.c, U.r, k0}; }
 
+// Points within a unit of each other (2^-62 R) have no difference left.  Laplace:
+// from p0 = R / 256 on, 1 / p0 is their value to half an ulp; below, only a point
+// with itself has it for sure.
+constexpr u64 SAME_PLACE_P0 = 1ull << 53;  // in units of 2^-61 R
+
 // Kernel value of one pair from its differences (diff(); the first dims of
-// them).  near: a Laplace pair closer than R / 128, left to the FP64 formula on
-// the double coordinates (except coincident points, which are exact).
+// them).  near: a Laplace pair closer than R / 128 that is left to the FP64 formula on
+// the double coordinates, unless it is a point with itself (whose value this is).
 template <int KIND>
 FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 *tab, bool &near) {
   i64 S = 0, T = 0;
@@ -499,7 +504,10 @@ FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 
     if (dims > 2) U += sq_low(dz);
   }
   if (KIND == LAPLACE) {
-    if ((S | T) == 0 && U == 0) return C.k0;
+    if ((S | T) == 0 && U == 0) {
+      near = C.c < SAME_PLACE_P0;
+      return C.k0;
+    }
     near = !laplace_far(S);
     int z;
     const u64 n = norm_d2(S, T, U, z);

@@ -540,6 +540,7 @@ struct KParams {
   const float4 *bands;   // two entries a span: r2lo, r2hi, r2box, rbox_inf; r2mid, r2half
   const int4 *stencil;   // unpruned rows of a cell's stencil, counts[3] of them
   int lanes;             // lanes a query of the singles
+  int self;              // the queries are the columns, in the same order
   // fixed point (fix64.cuh): column and query positions, box lengths, constants
   const longlong2 *fxy, *qfxy;
   const long long *fz, *qfz;
@@ -645,6 +646,8 @@ __device__ __forceinline__ void unpack_seg(int z, int img[3], int &du0, int &du1
   du0 = ((z >> 6) & 0xfff) - 2048;
   du1 = ((z >> 18) & 0xfff) - 2048;
 }
+
+constexpr int CENTRE = 21;  // the image bits of a segment (and of `code`): 0 in every dimension
 
 // dx of an accepted pair as the reference's search iterator exposes it:
 // x_j - (x_i + image*L) over the real dimensions (src/Search.h:188-190, 443),
@@ -1444,9 +1447,11 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
                             fx::diff(sm.uz[j], fqz), P, tab, near);
         if (KIND == ABX_K_LAPLACE && near) {
           const int2 mt = sm.meta[j & (Tile::METAS * STAGE - 1)];
-          int img[3], du0, du1;
-          unpack_seg(mt.y, img, du0, du1);
-          v = pair64<KIND>(xq, P.cpos[mt.x], img, P, 0.0, 0.0);
+          if (!(P.self && mt.x == qi && (mt.y & 63) == CENTRE)) {
+            int img[3], du0, du1;
+            unpack_seg(mt.y, img, du0, du1);
+            v = pair64<KIND>(xq, P.cpos[mt.x], img, P, 0.0, 0.0);
+          }
         }
       } else {
         const double dx = __longlong_as_double(sm.ux[j]) - xq.x,
@@ -1684,14 +1689,14 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
         if (VAL == VAL_FIX) {
           const longlong2 f = P.fxy[k];
           long long dx = fx::diff(f.x, fq.x), dy = fx::diff(f.y, fq.y), dz = fx::diff(P.fz[k], fqz);
-          if (code != 21) {  // 21: the centre image in every dimension
+          if (code != CENTRE) {
             dx = fx::diff(dx, img[0] * P.Lfix[0]);
             dy = fx::diff(dy, img[1] * P.Lfix[1]);
             dz = fx::diff(dz, img[2] * P.Lfix[2]);
           }
           bool near;
           v = fix_value<KIND>(dx, dy, dz, P, tab, near);
-          if (KIND == ABX_K_LAPLACE && near)
+          if (KIND == ABX_K_LAPLACE && near && !(P.self && (int)k == qi && code == CENTRE))
             v = pair64<KIND>(P.qpos[qi], P.cpos[k], img, P, 0.0, 0.0);
         } else
           v = pair64<KIND>(xq, P.cpos[k], img, P, si, KIND == ABX_K_SCALAR_SUM ? P.s_col[k] : 0.0);
@@ -1862,6 +1867,7 @@ KParams base_params(const PairLayout &L) {
   P.counts = L.counts.ptr;
   P.counter = L.counts.ptr + 4;
   P.qperm = L.rows->perm.ptr;
+  P.self = L.self;
   P.work = L.work ? unit_work(L.work, L.work_seq) : UnitWork{true, true};
   P.fxy = L.cols.fxy.ptr;
   P.fz = L.cols.fz.ptr;

@@ -400,7 +400,7 @@ __device__ __forceinline__ void local_matrix(const LsParams &P, int64_t i, int s
         bool near;
         v = fx::value<KIND>(fx::diff(oxy.x, qx), fx::diff(oxy.y, qy), fx::diff(fz[u], qz), P.dim,
                             P.fixc, tab, near);
-        if (near || d2 >= lo) v = ls_coeff<KIND>(P, s, su);
+        if ((near && su != s) || d2 >= lo) v = ls_coeff<KIND>(P, s, su);
       }
       col[u] = v;
     }
