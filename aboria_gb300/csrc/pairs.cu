@@ -131,10 +131,12 @@ struct PairLayout {
 void pair_layout_free(PairLayout *L) { delete L; }
 
 // Workspace of a particle set's searches: a search builds its layout anew in
-// buffers that only grow and go with the set.  One search at a time holds it.
+// buffers that only grow and go with the set.  One search at a time holds it, from
+// the copy of host queries to the device on.
 struct SearchSpace {
   std::mutex m;
   PairLayout L;
+  HostStage queries;
   DevBuf<double> qsoa, dxd;
   DevBuf<int32_t> cnt, cols;
   DevBuf<int64_t> rowptr, rpk, sums;
@@ -2215,10 +2217,10 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
   ABX_REQUIRE(lnorm == 2 || lnorm == 1 || lnorm == -1, ABX_ERR_INVALID,
               "norm %d not supported (2 euclidean, 1 manhattan, -1 chebyshev)", lnorm);
   const int D = p->dim;
-  const void *qd;
-  ABX_TRY(p->stage_b.in(ctx, q_host_or_dev, (size_t)nq * D * sizeof(double), &qd));
   std::lock_guard<std::mutex> hold(p->search->m);
   SearchSpace &W = *p->search;
+  const void *qd;
+  ABX_TRY(W.queries.in(ctx, q_host_or_dev, (size_t)nq * D * sizeof(double), &qd));
   PairLayout &L = W.L;
   ABX_TRY(W.qsoa.reserve((size_t)D * (nq ? nq : 1)));
   if (nq)
