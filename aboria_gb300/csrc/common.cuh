@@ -138,6 +138,13 @@ struct VecArg {
   bool host = false;
 };
 
+// A stream that is being captured into a graph takes launches, but no allocation and
+// no wait.
+inline bool stream_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+}
+
 // ------------------------------------------------------------ kernels ---
 inline unsigned int ceil_div(size_t a, size_t b) { return (unsigned int)((a + b - 1) / b); }
 

@@ -116,7 +116,7 @@ struct FmmPlan {
   DevBuf<long long> fz;
   DevBuf<int> mi_d;                 // ncheb x 3 multi-indices
   DevBuf<int> tile_mat, tile_first; // tensor-core M2L tiles
-  int ntiles = 0;
+  int ntiles = 0, tile_pairs = 0;
   int sms = 1;  // of the plan's GPU
 };
 
@@ -472,20 +472,20 @@ __global__ void __launch_bounds__(MF_T) k_row_span(const double *__restrict__ Km
   if (threadIdx.x == 0) span[blockIdx.x] = most;
 }
 
-// The same product in FP64, MW_PAIRS pairs of one matrix a CTA, four of them with
-// every K that is read.  Bound by the FP64 pipe.
-constexpr int MW_PAIRS = 16;
+// The same product in FP64, tiles of `pairs` pairs of one matrix a CTA, four of them
+// with every K that is read.  Bound by the FP64 pipe.
+constexpr int MW_PAIRS = 16;  // (P->tile_mat, whatever its tiles, does as well)
 __global__ void __launch_bounds__(FT) k_m2l64(int ncheb, const double *__restrict__ Km,
                                               const int2 *__restrict__ by_mat,
                                               const int *__restrict__ mat_off,
                                               const int *__restrict__ tile_mat,
-                                              const int *__restrict__ tile_first,
+                                              const int *__restrict__ tile_first, int pairs,
                                               const double *__restrict__ W,
                                               double *__restrict__ G) {
   constexpr int U = 4;
   __shared__ double ws[MAXC][U];
   const int m = tile_mat[blockIdx.x], first = tile_first[blockIdx.x];
-  const int last = min(first + MW_PAIRS, mat_off[m + 1]);
+  const int last = min(first + pairs, mat_off[m + 1]);
   const double *K = Km + (size_t)m * ncheb * ncheb;
   for (int q = first; q < last; q += U) {
     const int np = min(U, last - q);
@@ -1811,7 +1811,7 @@ int fmm_plan_build(abx_operator *op, int order, FmmPlan *&out, double eta = 1.0)
   // tensor-core M2L tiles: 64 pairs for the mma.sync kernel (<= 64 nodes),
   // t5_pairs pairs for the tcgen05 kernel, of one matrix each
   std::vector<int> tmat, tfirst;
-  const int tile_pairs = nc <= 64 ? TC_PAIRS : t5_pairs((nc + 127) / 128);
+  const int tile_pairs = P->tile_pairs = nc <= 64 ? TC_PAIRS : t5_pairs((nc + 127) / 128);
   for (int m = 0; m < P->nmat; ++m)
     for (int q = P->mat_off[m]; q < P->mat_off[m + 1]; q += tile_pairs) {
       tmat.push_back(m);
@@ -1868,6 +1868,12 @@ int fmm_plan_build(abx_operator *op, int order, FmmPlan *&out, double eta = 1.0)
 }
 
 namespace {
+// The integer near field's positions.
+int p2p_fix_prepare(FmmPlan *P, int64_t npos) {
+  ABX_TRY(P->fz.reserve((size_t)npos));
+  return P->fxy.reserve((size_t)npos);
+}
+
 template <int KIND>
 int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, const double *b,
                    double *c, bool mixed) {
@@ -1877,10 +1883,10 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
         P->D, P->n, P->ncheb, P->nleaves, P->leaf_ids.ptr, P->node_begin.ptr, P->node_end.ptr,
         P->box.ptr, P->posf.ptr, P->b32.ptr, b, P->G.ptr, P->p2p_rowptr.ptr, P->p2p_src.ptr,
         P->p0, P->tab32, c);
-  } else if (KIND != ABX_K_CONST && P->unit.ok) {
+  } else if (KIND != ABX_K_CONST && P->unit.ok &&
+             (P->fxy.cap >= (size_t)npos || !stream_capturing(s))) {
     constexpr int FK = KIND == ABX_K_COMPACT_GAUSSIAN || KIND == ABX_K_CONST ? ABX_K_GAUSSIAN : KIND;
-    ABX_TRY(P->fxy.reserve((size_t)npos));
-    ABX_TRY(P->fz.reserve((size_t)npos));
+    ABX_TRY(p2p_fix_prepare(P, npos));
     const unsigned lb = ceil_div((size_t)P->nleaves, PW);
     k_fixed_pos<<<ceil_div((size_t)npos, 256), 256, 0, s>>>(P->D, pos, npos, P->unit, P->fxy.ptr,
                                                             P->fz.ptr);
@@ -1968,10 +1974,17 @@ int m2l64_prepare(FmmPlan *P, cudaStream_t s) {
 // G += K W in FP64.
 int m2l64(FmmPlan *P, cudaStream_t s) {
   const int nc = P->ncheb;
+  auto by_fp64 = [&](const int *mat, const int *first, int tiles, int pairs) {
+    k_m2l64<<<tiles, FT, 0, s>>>(nc, P->Km.ptr, P->m2l_by_mat.ptr, P->mat_off_d.ptr, mat, first,
+                                 pairs, P->W.ptr, P->G.ptr);
+  };
+  if (!P->m2l64_ready && stream_capturing(s)) {
+    by_fp64(P->tile_mat.ptr, P->tile_first.ptr, P->ntiles, P->tile_pairs);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
   ABX_TRY(m2l64_prepare(P, s));
-  if (P->mw_tiles > 0)
-    k_m2l64<<<P->mw_tiles, FT, 0, s>>>(nc, P->Km.ptr, P->m2l_by_mat.ptr, P->mat_off_d.ptr,
-                                       P->mw_mat.ptr, P->mw_first.ptr, P->W.ptr, P->G.ptr);
+  if (P->mw_tiles > 0) by_fp64(P->mw_mat.ptr, P->mw_first.ptr, P->mw_tiles, MW_PAIRS);
   ABX_CHECK_CUDA(cudaGetLastError());
   if (P->mf_tiles == 0) return ABX_OK;
   k_split_digits<<<ceil_div((size_t)P->nnodes, 8), 256, 0, s>>>(P->W.ptr, P->nnodes, nc, 1, P->Wd.ptr,
@@ -1991,8 +2004,9 @@ int m2l64(FmmPlan *P, cudaStream_t s) {
 }  // namespace
 
 // What a plan's FP64 products keep: a first product then allocates nothing and
-// waits for nothing.
-int fmm_plan_prepare(FmmPlan *P, cudaStream_t s) {
+// waits for nothing.  (Without it, one that is captured runs the FP64 kernels.)
+int fmm_plan_prepare(FmmPlan *P, int64_t npos, cudaStream_t s) {
+  if (P->unit.ok) ABX_TRY(p2p_fix_prepare(P, npos));
   return P->n_m2l > 0 ? m2l64_prepare(P, s) : ABX_OK;
 }
 

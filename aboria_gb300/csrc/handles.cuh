@@ -176,5 +176,5 @@ int dense_matvec_device(abx_operator *op, const double *b, double *c);
 // fmm.cu
 int fmm_matvec_device(abx_operator *op, const double *b, double *c);
 void fmm_plan_free(FmmPlan *P);
-int fmm_plan_prepare(FmmPlan *P, cudaStream_t s);
+int fmm_plan_prepare(FmmPlan *P, int64_t npos, cudaStream_t s);
 }  // namespace abx

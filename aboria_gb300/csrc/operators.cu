@@ -370,11 +370,14 @@ int dense_chunks(abx_context *ctx, int64_t nc, unsigned blocks, int per_sm, int6
 }
 
 // Room for an FP64 product of nr x nc.
-int dense_reserve(abx_context *ctx, int64_t nr, int64_t nc, abx_operator *op) {
+size_t dense_room(abx_context *ctx, int64_t nr, int64_t nc) {
   int64_t chunk_cols;
   const int used = dense_chunks(ctx, nc, ceil_div(nr, DT), 16, chunk_cols);
-  return op->partial.reserve(sizeof(DenseFix) / 8 + 4 + (sizeof(FixCol) / 8) * (size_t)nc +
-                             (used > 1 ? (size_t)used * nr : 0));
+  return sizeof(DenseFix) / 8 + 4 + (sizeof(FixCol) / 8) * (size_t)nc +
+         (used > 1 ? (size_t)used * nr : 0);
+}
+int dense_reserve(abx_context *ctx, int64_t nr, int64_t nc, abx_operator *op) {
+  return op->partial.reserve(dense_room(ctx, nr, nc));
 }
 
 template <int KIND>
@@ -421,6 +424,12 @@ int launch_dense(abx_context *ctx, const DenseParams &P, bool mixed, abx_operato
                                                                                partial);
     if (partial)
       k_dense_reduce<<<ceil_div(P.nr, 256), 256, 0, ctx->stream>>>(partial, P.nr, used, P.c);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
+  if (op->partial.cap < dense_room(ctx, P.nr, P.nc) && stream_capturing(ctx->stream)) {
+    // no room, and none to be had: one CTA walks all columns
+    k_dense_fp64<KIND><<<blocks, DT, 0, ctx->stream>>>(P, nullptr, P.nc, nullptr);
     ABX_CHECK_CUDA(cudaGetLastError());
     return ABX_OK;
   }
@@ -558,7 +567,6 @@ int abx_operator_set_precision(abx_operator *op, int mode) {
   ABX_REQUIRE(op, ABX_ERR_INVALID, "null operator");
   ABX_REQUIRE(mode == ABX_PREC_FP64 || mode == ABX_PREC_MIXED, ABX_ERR_INVALID,
               "unknown precision mode %d", mode);
-  op->precision = mode;
   // the buffers of an FP64 product, so that the first one allocates nothing
   if (mode == ABX_PREC_FP64 && op->kind == 1 && op->rows->n > 0) {
     ABX_TRY(ctx_activate(op->rows->ctx));
@@ -566,8 +574,9 @@ int abx_operator_set_precision(abx_operator *op, int mode) {
   }
   if (mode == ABX_PREC_FP64 && op->fmm) {
     ABX_TRY(ctx_activate(op->rows->ctx));
-    ABX_TRY(fmm_plan_prepare(op->fmm, op->rows->ctx->stream));
+    ABX_TRY(fmm_plan_prepare(op->fmm, op->rows->n, op->rows->ctx->stream));
   }
+  op->precision = mode;
   return ABX_OK;
 }
 
