@@ -68,6 +68,10 @@ struct PointLayout {
   DevBuf<longlong2> fxy;
   DevBuf<long long> fz;
   DevBuf<uint32_t> tmp;   // sort scratch
+  void release() {
+    perm.release(), cell.release(), loc.release(), posk.release();
+    keys.release(), fxy.release(), fz.release(), tmp.release();
+  }
 };
 
 // Which units' queries k_pairs_thread walks instead of a unit kernel: units of
@@ -140,8 +144,22 @@ struct SearchSpace {
   DevBuf<double> qsoa, dxd;
   DevBuf<int32_t> cnt, cols;
   DevBuf<int64_t> rowptr, rpk, sums;
+  // Between searches it keeps what is in proportion to the set (about 80 B a
+  // particle, and as much a query for no more queries than that) and lists up to
+  // KEEP_BYTES; the buffers of a search with more queries, or longer lists, go back.
+  void trim(int64_t nq, int64_t n) {
+    if (nq > std::max(n, KEEP_QUERIES)) {
+      L.rows_own.release();
+      L.units.release(), L.singles.release();
+      queries.buf.release(), qsoa.release(), cnt.release();
+      rowptr.release(), rpk.release(), sums.release();
+    }
+    if (cols.cap * sizeof(int32_t) > KEEP_BYTES) cols.release();
+    if (dxd.cap * sizeof(double) > KEEP_BYTES) dxd.release();
+  }
+  static constexpr int64_t KEEP_QUERIES = 1 << 20;
+  static constexpr size_t KEEP_BYTES = size_t(256) << 20;
 };
-constexpr size_t KEEP_BYTES = size_t(256) << 20;
 SearchSpace *search_space_new() { return new SearchSpace(); }
 void search_space_free(SearchSpace *w) { delete w; }
 
@@ -2284,9 +2302,7 @@ int radius_query(abx_particles *p, int64_t nq, const double *q_host_or_dev, doub
     }
   }
   ABX_CHECK_CUDA(cudaStreamSynchronize(s));
-  // lists can be larger than everything else: the large ones are not kept
-  if (W.cols.cap * sizeof(int32_t) > KEEP_BYTES) W.cols.release();
-  if (W.dxd.cap * sizeof(double) > KEEP_BYTES) W.dxd.release();
+  W.trim(nq, p->n);
   return ABX_OK;
 }
 
