@@ -1285,10 +1285,6 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
           const float dd = norm32<NORM>(c.x - pq0, c.y - pq1, c.z - pq2);
           const bool in = dd <= r2lo;
           need |= (dd > r2lo) & (dd <= r2hi);
-          if (POL == POL_MATVEC) {
-            const float w = kern32<KIND>(dd, P);
-            acc32 = fmaf(in ? w : 0.f, c.w, acc32);
-          }
           if (POL == POL_COUNT) count += in ? 1 : 0;
           if (POL == POL_LIST && in && active) {
             const int2 mt = sm.meta[j];
