@@ -828,20 +828,6 @@ __device__ __forceinline__ float sqrt_approx(float x) {
   return r;
 }
 
-// Wendland C2 of two pairs with the cut-off folded into the clamp
-// t = max(1 - q, 0): exactly zero for q >= 1.
-__device__ __forceinline__ float2 kern32x2_wendland_clamped(float2 dd, const KParams &P) {
-  const float2 r = make_float2(sqrt_approx(dd.x), sqrt_approx(dd.y));
-  const float2 q = __fmul2_rn(r, make_float2(P.p0f, P.p0f));
-  float2 t = __ffma2_rn(q, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
-  t.x = fmaxf(t.x, 0.f);
-  t.y = fmaxf(t.y, 0.f);
-  const float2 t2 = __fmul2_rn(t, t);
-  const float2 t4 = __fmul2_rn(t2, t2);
-  const float2 pw = __ffma2_rn(q, make_float2(4.f, 4.f), make_float2(1.f, 1.f));
-  return __fmul2_rn(t4, pw);
-}
-
 // Kernel values of two pairs at once on the packed FP32x2 pipe.
 template <int KIND> __device__ __forceinline__ float2 kern32x2(float2 dd, const KParams &P) {
   if (KIND == ABX_K_CONST) return make_float2(P.p0f, P.p0f);
@@ -1233,21 +1219,13 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
             float2 dd = __fmul2_rn(dx, dx);
             dd = __ffma2_rn(dy, dy, dd);
             dd = __ffma2_rn(dz, dz, dd);
-            float2 w;
-            if (KIND == ABX_K_WENDLAND_C2) {
-              // the kernel vanishes for q >= 1: the clamp is the cut-off for
-              // every pair outside the rounding band (d2 > r2hi means q > 1),
-              // and band pairs are flagged for the exact test below
-              const float2 off = __fadd2_rn(dd, make_float2(-r2mid, -r2mid));
-              need |= (fabsf(off.x) <= r2half) | (fabsf(off.y) <= r2half);
-              w = kern32x2_wendland_clamped(dd, P);
-            } else {
-              const bool ia = dd.x <= r2lo, ib = dd.y <= r2lo;
-              need |= ((dd.x > r2lo) & (dd.x <= r2hi)) | ((dd.y > r2lo) & (dd.y <= r2hi));
-              w = kern32x2<KIND>(dd, P);
-              w.x = ia ? w.x : 0.f;
-              w.y = ib ? w.y : 0.f;
-            }
+            // (a Wendland kernel here has a support wider than the radius: its value
+            // does not vanish at the cut-off, see K_WEND_CUT)
+            const bool ia = dd.x <= r2lo, ib = dd.y <= r2lo;
+            need |= ((dd.x > r2lo) & (dd.x <= r2hi)) | ((dd.y > r2lo) & (dd.y <= r2hi));
+            float2 w = kern32x2<KIND>(dd, P);
+            w.x = ia ? w.x : 0.f;
+            w.y = ib ? w.y : 0.f;
             acc2 = __ffma2_rn(w, make_float2(B.z, B.w), acc2);
           }
           acc32 = acc2.x + acc2.y;
@@ -1302,19 +1280,14 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
             for (int j = 0; j < nt; ++j) {
               const float4 c = sm.p[j];
               const float dd = norm32<NORM>(c.x - pq0, c.y - pq1, c.z - pq2);
-              const bool wend = POL == POL_MATVEC && KIND == ABX_K_WENDLAND_C2;
-              const bool mid = (wend || PCOUNT) && fabsf(__fadd_rn(dd, -r2mid)) <= r2half;
-              const bool flagged = mid || (!wend && dd > r2lo && dd <= r2hi);
+              const bool mid = PCOUNT && fabsf(__fadd_rn(dd, -r2mid)) <= r2half;
+              const bool flagged = mid || (dd > r2lo && dd <= r2hi);
               if (flagged) {
                 const int2 mt = sm.meta[j];
                 int img[3], du0, du1;
                 unpack_seg(ws.seg[mt.y].z, img, du0, du1);
                 const bool inside = !(exact_norm(xq, P.cpos[mt.x], img, fg, NORM) > P.thr);
-                if (wend) {
-                  // the packed loop added the clamped value: take it back out
-                  // for pairs the FP64 test rejects
-                  if (!inside) acc32 -= kern32x2_wendland_clamped(make_float2(dd, dd), P).x * c.w;
-                } else if (PCOUNT) {
+                if (PCOUNT) {
                   count += (inside ? 1 : 0) - (__fadd_rn(dd, -r2mid) < 0.f ? 1 : 0);
                 } else if (inside) {
                   if (POL == POL_MATVEC) acc32 = fmaf(kern32<KIND>(dd, P), c.w, acc32);
