@@ -561,6 +561,7 @@ struct KParams {
   const int4 *stencil;   // unpruned rows of a cell's stencil, counts[3] of them
   int lanes;             // lanes a query of the singles
   int self;              // the queries are the columns, in the same order
+  float near2;           // Laplace in fixed point: pairs closer than its root go by FP64
   // fixed point (fix64.cuh): column and query positions, box lengths, constants
   const longlong2 *fxy, *qfxy;
   const long long *fz, *qfz;
@@ -1339,14 +1340,25 @@ __device__ __forceinline__ double fix_value(long long dx, long long dy, long lon
   return fx::value<KIND>(dz, dy, dx, 3 - P.fg.eoff, P.fixc, tab, near);
 }
 
-// FP64 distance and kernel value of one accepted pair, dx = (x_j - image*L) - x_i.
+// FP64 distance and kernel value of one accepted pair, dx = (x_j - image*L) - x_i; the
+// image bits as in a segment (the centre one, whose shifts are 0, without them).
 template <int KIND>
-__device__ __forceinline__ double pair64(const D4 &xq, const D4 &xj, const int *img,
-                                         const KParams &P, double si, double sj) {
-  const double dx = __dsub_rn(xj.x, (double)img[0] * P.fg.L[0]) - xq.x;
-  const double dy = __dsub_rn(xj.y, (double)img[1] * P.fg.L[1]) - xq.y;
-  const double dz = __dsub_rn(xj.z, (double)img[2] * P.fg.L[2]) - xq.z;
+__device__ __forceinline__ double pair64(const D4 &xq, D4 xj, int code, const KParams &P, double si,
+                                         double sj) {
+  if ((code & 63) != CENTRE) {
+    xj.x = __dsub_rn(xj.x, (double)((code & 3) - 1) * P.fg.L[0]);
+    xj.y = __dsub_rn(xj.y, (double)(((code >> 2) & 3) - 1) * P.fg.L[1]);
+    xj.z = __dsub_rn(xj.z, (double)(((code >> 4) & 3) - 1) * P.fg.L[2]);
+  }
+  const double dx = xj.x - xq.x, dy = xj.y - xq.y, dz = xj.z - xq.z;
   return kern64<KIND>(fma(dz, dz, fma(dy, dy, dx * dx)), P, si, sj);
+}
+
+// The same for a Laplace pair that the fixed-point value leaves out (k0 for a point
+// with itself).
+__device__ __forceinline__ double near_pair64(const D4 &xq, int qi, int k, int code, const KParams &P) {
+  if (P.self && k == qi && (code & 63) == CENTRE) return P.fixc.k0;
+  return pair64<ABX_K_LAPLACE>(xq, P.cpos[k], code, P, 0.0, 0.0);
 }
 
 // FP64 sparse matvec: the reference's arithmetic for every accepted pair,
@@ -1376,6 +1388,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
   using Tile = WarpTile64<KIND>;
   __shared__ Tile tile_all[WARPS_PER_CTA];
   static_assert(POL == POL_MATVEC, "the FP64 pair kernel computes matvecs only");
+  constexpr bool NEAR = FIX && KIND == ABX_K_LAPLACE;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   WarpSeg &ws = seg_all[wid];
   Tile &sm = tile_all[wid];
@@ -1434,13 +1447,9 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
         bool near;
         v = fix_value<KIND>(fx::diff(sm.ux[j], fq.x), fx::diff(sm.uy[j], fq.y),
                             fx::diff(sm.uz[j], fqz), P, tab, near);
-        if (KIND == ABX_K_LAPLACE && near) {
+        if (NEAR && near) {
           const int2 mt = sm.meta[j & (Tile::METAS * STAGE - 1)];
-          if (!(P.self && mt.x == qi && (mt.y & 63) == CENTRE)) {
-            int img[3], du0, du1;
-            unpack_seg(mt.y, img, du0, du1);
-            v = pair64<KIND>(xq, P.cpos[mt.x], img, P, 0.0, 0.0);
-          }
+          v = near_pair64(xq, qi, mt.x, mt.y, P);
         }
       } else {
         const double dx = __longlong_as_double(sm.ux[j]) - xq.x,
@@ -1529,12 +1538,13 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
         }
         __syncwarp();
         // (1) this lane's neighbours among the nt staged candidates
-        unsigned long long mask = 0;
+        unsigned long long mask = 0, nmask = 0;  // nmask: those that go by FP64
         if (active) {
           const float2 nqx = make_float2(-pq0, -pq0), nqy = make_float2(-pq1, -pq1),
                        nqz = make_float2(-pq2, -pq2), nmid = make_float2(-r2mid, -r2mid);
+          const float2 nnear = make_float2(r2mid - P.near2, r2mid - P.near2);
           float least = r2half + r2half;
-          unsigned word[2] = {0u, 0u};
+          unsigned word[2] = {0u, 0u}, nword[2] = {0u, 0u};
           const int npair = (nt + 1) >> 1;
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
@@ -1553,11 +1563,18 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
               word[w] = __funnelshift_l(__float_as_uint(off.x), word[w], 1);
               word[w] = __funnelshift_l(__float_as_uint(off.y), word[w], 1);
               least = fminf(least, fminf(fabsf(off.x), fabsf(off.y)));
+              if (NEAR) {
+                const float2 no = __fadd2_rn(off, nnear);  // d^2 - near2
+                nword[w] = __funnelshift_l(__float_as_uint(no.x), nword[w], 1);
+                nword[w] = __funnelshift_l(__float_as_uint(no.y), nword[w], 1);
+              }
             }
             // the first candidate's sign to bit 0
             if (n16) word[w] = __brev(word[w] << (32 - 2 * n16));
+            if (NEAR && n16) nword[w] = __brev(nword[w] << (32 - 2 * n16));
           }
           mask = word[0] | (unsigned long long)word[1] << 32;
+          if (NEAR) nmask = nword[0] | (unsigned long long)nword[1] << 32;
           if (least <= r2half) {  // rare: the reference's exact FP64 test for pairs in the band
             for (int j = 0; j < nt; ++j) {
               const float *xy = reinterpret_cast<const float *>(&sm.pxy[j >> 1]) + (j & 1);
@@ -1570,6 +1587,18 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
               unpack_seg(mt.y, img, du0, du1);
               const bool in = !(exact_d2(xq, P.cpos[mt.x], img, fg) > P.r2);
               mask = in ? mask | 1ull << j : mask & ~(1ull << j);
+            }
+          }
+        }
+        if (NEAR) {  // together, so that a clump of near pairs is not a walk of both kinds
+          nmask &= mask;
+          mask &= ~nmask;
+          while (__any_sync(0xffffffffu, nmask != 0)) {
+            if (nmask != 0) {
+              const int j = half + __ffsll((long long)nmask) - 1;
+              nmask &= nmask - 1;
+              const int2 mt = sm.meta[j];
+              acc = fma(near_pair64(xq, qi, mt.x, mt.y, P), sm.b[j], acc);
             }
           }
         }
@@ -1628,6 +1657,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
     k_pairs_thread(KParams P) {
   constexpr bool QUEUE = POL == POL_MATVEC && VAL != VAL_MIXED;
   constexpr bool WCUT = KIND == K_WEND_CUT;
+  constexpr bool NEAR = VAL == VAL_FIX && KIND == ABX_K_LAPLACE;
+  constexpr int NEAR_CODE = 64;  // beside the image bits of a queued pair
   __shared__ unsigned long long queue[QUEUE ? WARPS_PER_CTA * QCAP * 32 : 1];
   __shared__ fx::u64 tab[VAL == VAL_FIX && KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1673,22 +1704,22 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
         const unsigned long long ent = qu[nq * 32];
         const unsigned k = (unsigned)ent;
         const int code = (int)(ent >> 32);
-        const int img[3] = {(code & 3) - 1, ((code >> 2) & 3) - 1, ((code >> 4) & 3) - 1};
         double v;
-        if (VAL == VAL_FIX) {
+        if (NEAR && (code & NEAR_CODE)) {
+          v = near_pair64(P.qpos[qi], qi, (int)k, code, P);
+        } else if (VAL == VAL_FIX) {
           const longlong2 f = P.fxy[k];
           long long dx = fx::diff(f.x, fq.x), dy = fx::diff(f.y, fq.y), dz = fx::diff(P.fz[k], fqz);
           if (code != CENTRE) {
-            dx = fx::diff(dx, img[0] * P.Lfix[0]);
-            dy = fx::diff(dy, img[1] * P.Lfix[1]);
-            dz = fx::diff(dz, img[2] * P.Lfix[2]);
+            dx = fx::diff(dx, ((code & 3) - 1) * P.Lfix[0]);
+            dy = fx::diff(dy, (((code >> 2) & 3) - 1) * P.Lfix[1]);
+            dz = fx::diff(dz, (((code >> 4) & 3) - 1) * P.Lfix[2]);
           }
           bool near;
           v = fix_value<KIND>(dx, dy, dz, P, tab, near);
-          if (KIND == ABX_K_LAPLACE && near && !(P.self && (int)k == qi && code == CENTRE))
-            v = pair64<KIND>(P.qpos[qi], P.cpos[k], img, P, 0.0, 0.0);
+          if (NEAR && near) v = near_pair64(P.qpos[qi], qi, (int)k, code, P);
         } else
-          v = pair64<KIND>(xq, P.cpos[k], img, P, si, KIND == ABX_K_SCALAR_SUM ? P.s_col[k] : 0.0);
+          v = pair64<KIND>(xq, P.cpos[k], code, P, si, KIND == ABX_K_SCALAR_SUM ? P.s_col[k] : 0.0);
         acc = fma(v, P.b64[k], acc);
       }
     };
@@ -1761,7 +1792,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
                 if (POL == POL_MATVEC && VAL == VAL_MIXED && in)
                   acc32 = fmaf(kern32<KIND>(dd, P), __ldg(&P.b32[k]), acc32);
                 if (QUEUE && in) {
-                  qu[nq * 32] = (unsigned long long)k | ((unsigned long long)code << 32);
+                  const int c = NEAR && dd < P.near2 ? code | NEAR_CODE : code;
+                  qu[nq * 32] = (unsigned long long)k | ((unsigned long long)c << 32);
                   ++nq;
                 }
               }
@@ -1857,6 +1889,9 @@ KParams base_params(const PairLayout &L) {
   P.counter = L.counts.ptr + 4;
   P.qperm = L.rows->perm.ptr;
   P.self = L.self;
+  // R / 128 (fx::laplace_far), with room for the FP32 distances: the value itself
+  // says what is left out
+  P.near2 = (float)std::ldexp(1.0 + 1e-3, 2 * (L.unit.r - 7));
   P.work = L.work ? unit_work(L.work, L.work_seq) : UnitWork{true, true};
   P.fxy = L.cols.fxy.ptr;
   P.fz = L.cols.fz.ptr;
