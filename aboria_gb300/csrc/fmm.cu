@@ -329,8 +329,8 @@ __global__ void __launch_bounds__(FT) k_p2m32(int D, int n, int ncheb, const int
 // copies of the matrices, FP32 sums of ncheb terms, FP64 storage).
 // JS threads a row share its ncheb terms, and a term's NBL inputs are vector
 // reads.  A row's walk of 343 loads from L2 is what a level with few links takes:
-// four threads a row there (8 batches of order 7: 91 -> 40 us); with links enough
-// the shared sums only cost (4,096 batches: 364 us with one, 936 with four).
+// four threads a row there; with links enough the shared sums only cost
+// (launch_links has both sides).
 constexpr int NBL = 8;  // links per M2M / L2L batch
 template <typename T, bool M2M, int JS>
 __global__ void __launch_bounds__(FT * JS) k_m2m_l2l(int ncheb, const int *__restrict__ links,
@@ -1912,14 +1912,20 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
 }
 }  // namespace
 
-// One level's M2M or L2L.  Threads a row: see k_m2m_l2l; the line at 32 CTAs an SM
-// lies between 1,536 CTAs (order 7: four threads 110 us M2M, one 159) and 12,288.
+// One level's M2M or L2L.  Threads a row (k_m2m_l2l): four below the line, one from it
+// on.  Measured in us, M2M / L2L, four against one, 152 SMs:
+//   FP32    64 CTAs   21 / 18 against 26 / 23       FP64    64   40 / 37 against 63 / 59
+//          240        44 / 40 against 58 / 54               192  161 / 158 against 174 / 169
+//          512        33 / 17 against 25 / 22             1,024  355 / 351 against 392 / 374
+//        1,024        75 / 49 against 38 / 34             1,536  855 / 849 against 875 / 869
+//        1,536       148 / 110 against 62 / 58            4,096  886 / 875 against 861 / 849
 template <typename T, bool M2M>
 void launch_links(const FmmPlan *P, int lev, const T *mats, double *V, cudaStream_t s) {
   if (P->batch_cnt[lev] == 0) return;
   const dim3 grid(P->batch_cnt[lev], ceil_div(P->ncheb, FT));
   const int2 *bt = P->batches.ptr + P->batch_off[lev];
-  if ((int64_t)grid.x * grid.y < 8 * (int64_t)P->sms)
+  constexpr int64_t LINE = sizeof(T) == 4 ? 2 : 16;  // CTAs an SM
+  if ((int64_t)grid.x * grid.y < LINE * P->sms)
     k_m2m_l2l<T, M2M, 4><<<grid, 4 * FT, 0, s>>>(P->ncheb, P->links.ptr, bt, mats, V);
   else
     k_m2m_l2l<T, M2M, 1><<<grid, FT, 0, s>>>(P->ncheb, P->links.ptr, bt, mats, V);
