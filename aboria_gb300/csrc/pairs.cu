@@ -1025,6 +1025,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 7)
   constexpr bool PCOUNT = POL == POL_COUNT && NORM == 2;  // counts two candidates at a time
   const float sc = WCUT ? P.p0f : 1.f;  // staging scale (d^2 = q^2 for WCUT)
   const int nfull = P.counts[0], nunits = nfull + P.counts[P.all_units ? 1 : 8];
+  if (blockIdx.x * WARPS_PER_CTA >= nunits) return;  // see grid_blocks
   for (;;) {
     int unit = 0;
     if (lane == 0) unit = atomicAdd(P.counter, 1);
@@ -1395,6 +1396,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
   const FineGrid &fg = P.fg;
   const unsigned lt = (1u << lane) - 1u;
   const int nfull = P.counts[0], nunits = nfull + P.counts[P.all_units ? 1 : 8];
+  if (blockIdx.x * WARPS_PER_CTA >= nunits) return;  // see grid_blocks
   __shared__ fx::u64 tab[FIX && KIND == ABX_K_GAUSSIAN ? fx::EXP_TAB : 1];
   if (FIX && KIND == ABX_K_GAUSSIAN) {
     for (int i = threadIdx.x; i < fx::EXP_TAB; i += WARPS_PER_CTA * 32) tab[i] = fx::exp_table.v[i];
@@ -1669,6 +1671,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
     __syncthreads();
   }
   const int nsing = P.counts[9], nrows = P.counts[3];
+  if ((int64_t)blockIdx.x * (WARPS_PER_CTA * 32) >= (int64_t)nsing * P.lanes) return;  // see grid_blocks
   const int sub = lane & (P.lanes - 1);
   const int span = 2 * max(max(fg.K[0], fg.K[1]), fg.K[2]) + 2;
   const float4 bd = span < BAND_TAB ? P.bands[2 * span]
@@ -1903,7 +1906,11 @@ KParams base_params(const PairLayout &L) {
 }
 
 // CTAs of the kernels that take their work from a counter: as many as there
-// can be work for, 8 an SM at most.
+// can be work for, 8 an SM at most.  How much there is only the device knows; CTAs
+// beyond it return at once, as the first ones, which are dealt evenly over the SMs,
+// would not get it all otherwise (300 clumps of 200 points, whose 2,200 units would
+// fill a quarter of the warps: busiest SM 1.69e6 cycles, 1.25e6 with as many CTAs as
+// units; average 1.03e6).
 int grid_blocks(abx_context *ctx, const KParams &P) {
   const int64_t need = (P.units_cap + WARPS_PER_CTA - 1) / WARPS_PER_CTA;
   return (int)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms * 8, need));
