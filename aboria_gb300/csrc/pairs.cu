@@ -77,12 +77,13 @@ struct PointLayout {
 // Which units' queries k_pairs_thread walks instead of a unit kernel: units of
 // fewer than `queries` queries whose own row of the stencil holds at most `row`
 // columns (a unit of few queries beside a dense cluster still has a long
-// candidate list, which a warp stages faster than a lane walks it), and none
+// candidate list, which a warp stages faster than a lane walks it) and, where
+// `around` is not 0, no row of the whole stencil holds more than that; and none
 // at all where they are less than 1 / `fold` of the set (the second launch).
 struct Split {
-  int queries, row, fold;
+  int queries, row, fold, around;
   bool operator==(const Split &o) const {
-    return queries == o.queries && row == o.row && fold == o.fold;
+    return queries == o.queries && row == o.row && fold == o.fold && around == o.around;
   }
 };
 // FP64: a unit kernel's lanes idle at ~100 instructions a pair.  N = 100,000 x 50
@@ -92,8 +93,13 @@ struct Split {
 // (4M: 20.6, 20.9, 21.5 ms for the same three); sets of fewer than MIXED_MIN
 // rows keep to it altogether (2,000: 13 against 21 us; 12,000: 24 against 31;
 // 100,000 x 10: 118 against 78).
-constexpr Split SPLIT_FP64{12, 1 << 30, 16}, SPLIT_COUNT{7, 12, 4}, SPLIT_MIXED{4, 6, 3},
-    SPLIT_NONE{0, 0, 1};
+// FP64 values outside make_unit's rules cost the unit kernel less (its lanes share
+// the FP64 pipe), a lane's long walk as much: only where no walk is long.  30,000
+// points in 16 clusters, constant kernel: 285 us without the split, 405 with
+// SPLIT_FP64's, 300 to 320 with this; 300,000 uniform 515, 195, 195.  In 1-D a stencil is one
+// row, which lanes cannot share: no split (3,000 points, constant 46 -> 31 us).
+constexpr Split SPLIT_FP64{12, 1 << 30, 16, 0}, SPLIT_VALUES{12, 1 << 30, 16, 48},
+    SPLIT_COUNT{7, 12, 4, 0}, SPLIT_MIXED{4, 6, 3, 0}, SPLIT_NONE{0, 0, 1, 0};
 constexpr int64_t MIXED_MIN = 50000;
 
 struct PairLayout {
@@ -417,9 +423,11 @@ int build_cell_start(abx_context *ctx, PairLayout &L) {
 constexpr int UNIT_WARPS = 4;
 __global__ void __launch_bounds__(UNIT_WARPS * 32)
     k_units(const int4 *__restrict__ cell, const uint32_t *__restrict__ keys,
-            const uint32_t *__restrict__ cell_start, bool self, int64_t n, uint32_t ncol, int m2,
-            int K2, int64_t cap, Split split, int2 *__restrict__ units, int *__restrict__ singles, int *__restrict__ counts) {
-  const int lane = threadIdx.x & 31;
+            const uint32_t *__restrict__ cell_start, bool self, int64_t n, FineGrid fg, int64_t cap,
+            Split split, int2 *__restrict__ units, int *__restrict__ singles,
+            int *__restrict__ counts) {
+  const int lane = threadIdx.x & 31, m2 = fg.m[2], K2 = fg.K[2];
+  const uint32_t ncol = (uint32_t)fg.m[0] * fg.m[1];
   const uint32_t warps = gridDim.x * UNIT_WARPS;
   for (uint32_t col = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); col < ncol; col += warps) {
     int64_t s, end;
@@ -469,6 +477,18 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
           const int za = max(z - K2, 0), zb = min(z + GROUP_E2 - 1 + K2, m2 - 1);
           const uint32_t *row = cell_start + (uint64_t)col * m2;
           small = row[zb + 1] - row[za] <= (uint32_t)split.row;
+          if (split.around) {
+            const int c0 = (int)(col / fg.m[1]), c1 = (int)(col % fg.m[1]);
+            for (int o0 = -fg.K[0]; small && o0 <= fg.K[0]; ++o0)
+              for (int o1 = -fg.K[1]; small && o1 <= fg.K[1]; ++o1) {
+                int w0 = c0 + o0, w1 = c1 + o1;
+                if (fg.periodic[0]) w0 += w0 < 0 ? fg.m[0] : w0 >= fg.m[0] ? -fg.m[0] : 0;
+                if (fg.periodic[1]) w1 += w1 < 0 ? fg.m[1] : w1 >= fg.m[1] ? -fg.m[1] : 0;
+                if (w0 < 0 || w0 >= fg.m[0] || w1 < 0 || w1 >= fg.m[1]) continue;
+                const uint32_t *r = cell_start + ((uint64_t)w0 * fg.m[1] + w1) * m2;
+                small = r[zb + 1] - r[za] <= (uint32_t)split.around;
+              }
+          }
         }
         const bool full = lane < held && !small;
         const unsigned mf = __ballot_sync(0xffffffffu, full), ms = __ballot_sync(0xffffffffu, small);
@@ -515,8 +535,8 @@ int build_units(abx_context *ctx, PairLayout &L, const Split &split) {
   const uint32_t ncol = (uint32_t)L.fg.m[0] * L.fg.m[1];
   const unsigned blocks = std::min(ceil_div(ncol, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
   k_units<<<blocks, UNIT_WARPS * 32, 0, ctx->stream>>>(
-      Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, ncol, L.fg.m[2], L.fg.K[2], n, split,
-      L.units.ptr, L.singles.ptr, L.counts.ptr);
+      Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, L.fg, n, split, L.units.ptr,
+      L.singles.ptr, L.counts.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
@@ -2043,7 +2063,8 @@ fx::Unit fix_unit(const abx_kernel &k, double reach) {
 static Split matvec_split(const abx_operator *op) {
   if (op->precision == ABX_PREC_MIXED && op->k.kind != ABX_K_SCALAR_SUM)
     return op->rows->n < MIXED_MIN ? SPLIT_NONE : SPLIT_MIXED;
-  return SPLIT_FP64;
+  if (op->cols->dim == 1) return SPLIT_NONE;
+  return fix_unit(op->k, op->radius).ok ? SPLIT_FP64 : SPLIT_VALUES;
 }
 
 int pair_layout_build(abx_operator *op) {
