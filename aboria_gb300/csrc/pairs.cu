@@ -420,23 +420,31 @@ int build_cell_start(abx_context *ctx, PairLayout &L) {
 // density, where a warp of 32 lanes would hold few queries), to the back, and
 // its queries to `singles`, which k_pairs_thread walks.  Built on the host before,
 // from a 16 B/point copy of the cells: 14 of the 39 ms of a search at N = 4M.
+// Few columns (1-D: one) are walked in `segs` segments of cells, where units end: one
+// warp took 620 us for 50,000 points, 64 take less than 10.
 constexpr int UNIT_WARPS = 4;
+constexpr uint32_t FEW_COLUMNS = 4;
+constexpr int SEG_CELLS = 16;  // at least
 __global__ void __launch_bounds__(UNIT_WARPS * 32)
     k_units(const int4 *__restrict__ cell, const uint32_t *__restrict__ keys,
             const uint32_t *__restrict__ cell_start, bool self, int64_t n, FineGrid fg, int64_t cap,
-            Split split, int2 *__restrict__ units, int *__restrict__ singles,
+            int segs, Split split, int2 *__restrict__ units, int *__restrict__ singles,
             int *__restrict__ counts) {
   const int lane = threadIdx.x & 31, m2 = fg.m[2], K2 = fg.K[2];
   const uint32_t ncol = (uint32_t)fg.m[0] * fg.m[1];
   const uint32_t warps = gridDim.x * UNIT_WARPS;
-  for (uint32_t col = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); col < ncol; col += warps) {
+  const int len = (m2 + segs - 1) / segs;
+  for (uint32_t item = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); item < ncol * segs; item += warps) {
+    const uint32_t col = item / segs;
+    const int z_from = min((int)(item % segs) * len, m2), z_to = min(z_from + len, m2);
+    const uint64_t from = (uint64_t)col * m2 + z_from, to = (uint64_t)col * m2 + z_to;
     int64_t s, end;
     if (self) {
-      s = cell_start[(uint64_t)col * m2];
-      end = cell_start[(uint64_t)(col + 1) * m2];
+      s = cell_start[from];
+      end = cell_start[to];
     } else {
-      s = warp_lower_bound(keys, n, (uint64_t)col * m2 * 8, lane);
-      end = warp_lower_bound(keys, n, (uint64_t)(col + 1) * m2 * 8, lane);
+      s = warp_lower_bound(keys, n, from * 8, lane);
+      end = warp_lower_bound(keys, n, to * 8, lane);
     }
     const int4 none = make_int4(0, 0, 0, 0);
     int64_t base = s;  // A holds queries [base, base + 32), B the 32 after them
@@ -533,10 +541,11 @@ int build_units(abx_context *ctx, PairLayout &L, const Split &split) {
   ABX_CHECK_CUDA(cudaMemsetAsync(L.counts.ptr, 0, COUNTS * sizeof(int), ctx->stream));
   if (n == 0) return ABX_OK;
   const uint32_t ncol = (uint32_t)L.fg.m[0] * L.fg.m[1];
-  const unsigned blocks = std::min(ceil_div(ncol, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
+  const int segs = ncol <= FEW_COLUMNS ? (int)ceil_div(L.fg.m[2], SEG_CELLS) : 1;
+  const unsigned blocks = std::min(ceil_div((size_t)ncol * segs, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
   k_units<<<blocks, UNIT_WARPS * 32, 0, ctx->stream>>>(
-      Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, L.fg, n, split, L.units.ptr,
-      L.singles.ptr, L.counts.ptr);
+      Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, L.fg, n, segs, split,
+      L.units.ptr, L.singles.ptr, L.counts.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
@@ -2027,9 +2036,11 @@ int fill_fixed(abx_context *ctx, PointLayout &P, const fx::Unit &U) {
 
 // Build a layout for cols (a searchable particle set) and a query set given as
 // SoA FP64 (qsrc, nq, stride) -- or the column set itself when qsrc == null.
-// All on the context's stream, nothing waited for; norm and thr as KParams'.
+// All on the context's stream, nothing waited for; norm and thr as KParams'; units
+// false: the points and cells alone.
 int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *qsrc, int64_t nq,
-                 int64_t qstride, PairLayout &L, const Split &split, int norm = 2) {
+                 int64_t qstride, PairLayout &L, const Split &split, int norm = 2,
+                 bool units = true) {
   GridDesc g;
   ABX_TRY(particles_grid_desc(cols, &g));
   L.r = r;
@@ -2041,6 +2052,7 @@ int layout_build(abx_context *ctx, abx_particles *cols, double r, const double *
   if (!L.self) ABX_TRY(reserve_points(nq, qsrc, qstride, false, L.rows_own, sets.s[1]));
   ABX_TRY(build_points(ctx, sets, L.cols, L.self ? nullptr : &L.rows_own, L.fg));
   ABX_TRY(build_cell_start(ctx, L));
+  if (!units) return ABX_OK;
   ABX_TRY(build_units(ctx, L, split));
   ABX_TRY(build_tables(ctx, L, norm, norm == 2 ? r * r : std::fabs(r)));
   return ABX_OK;
@@ -2457,7 +2469,7 @@ int knn_device(abx_particles *p, int k, int32_t *idx, double *d2) {
   const double h = std::pow(std::max(1.0, k / 4.0) * vol / (double)n, 1.0 / p->dim);
   std::lock_guard<std::mutex> hold(p->search->m);
   PairLayout &L = p->search->L;
-  ABX_TRY(layout_build(ctx, p, 3.0 * h, nullptr, n, n, L, SPLIT_COUNT));
+  ABX_TRY(layout_build(ctx, p, 3.0 * h, nullptr, n, n, L, SPLIT_NONE, 2, false));
   KParams P = base_params(L);
   k_knn<<<ceil_div(n, 128), 128, 0, ctx->stream>>>(P, k, n, idx, d2);
   ABX_CHECK_CUDA(cudaGetLastError());
