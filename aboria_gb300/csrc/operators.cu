@@ -77,12 +77,9 @@ template <int KIND> __device__ __forceinline__ float dk32(float d2, float p0f, f
 // chunks (blockIdx.y) as in k_dense_fix: with one CTA per 256 rows, 460 x 1484
 // took 2.0 ms, the latency of 1,484 values one after the other; with
 // chunks 124 us.
-struct DenseFix;
-__device__ bool dense_fix_done(const DenseFix *F);
 template <int KIND>
-__global__ void __launch_bounds__(DT) k_dense_fp64(DenseParams P, const DenseFix *F,
-                                                   int64_t chunk_cols, double *__restrict__ partial) {
-  if (F && dense_fix_done(F)) return;
+__device__ __forceinline__ void dense_rows_fp64(const DenseParams &P, int64_t chunk_cols,
+                                                double *__restrict__ partial) {
   __shared__ double sx[DT], sy[DT], sz[DT], sb[DT], ss[DT];
   const int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x;
   const bool act = i < P.nr;
@@ -126,6 +123,14 @@ __global__ void __launch_bounds__(DT) k_dense_fp64(DenseParams P, const DenseFix
   if (!act) return;
   if (partial) partial[(int64_t)blockIdx.y * P.nr + i] = acc;
   else P.c[i] = acc;
+}
+struct DenseFix;
+__device__ bool dense_fix_done(const DenseFix *F);
+template <int KIND>
+__global__ void __launch_bounds__(DT) k_dense_fp64(DenseParams P, const DenseFix *F,
+                                                   int64_t chunk_cols, double *__restrict__ partial) {
+  if (F && dense_fix_done(F)) return;
+  dense_rows_fp64<KIND>(P, chunk_cols, partial);
 }
 
 // Kernel values of two pairs: packed FP32x2 where the formula allows.
@@ -234,19 +239,18 @@ __device__ __forceinline__ double from_ordered(unsigned long long k) {
   return __longlong_as_double((long long)((k >> 63) ? k & 0x7fffffffffffffffull : ~k));
 }
 
-// Maxima of x_d and -x_d over a point set, on the bits in an order-preserving
-// form: a NaN of either sign sorts beyond the infinities and is caught with
-// them (floating-point negation and comparison would lose its sign).
-__global__ void __launch_bounds__(DT) k_dense_range(const double *__restrict__ a, int64_t na,
-                                                    const double *__restrict__ b, int64_t nb,
-                                                    int dim, DenseFix *__restrict__ F) {
+// Maxima of x_d and -x_d over every step-th point of two sets from `first` on, for the
+// whole CTA, to `out` (thread 0), on the bits in an order-preserving form: a NaN of
+// either sign sorts beyond the infinities and is caught with them (floating-point
+// negation and comparison would lose its sign).
+template <class Out>
+__device__ __forceinline__ void dense_range(const DenseParams &P, int64_t first, int64_t step, Out out) {
   __shared__ unsigned long long red[DT / 32];
-  const int64_t step = (int64_t)gridDim.x * DT;
-  for (int d = 0; d < dim; ++d) {
+  for (int d = 0; d < P.dim; ++d) {
     unsigned long long hi = 0, lo = 0;
-    for (int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x; i < na + nb; i += step) {
+    for (int64_t i = first + threadIdx.x; i < P.nr + P.nc; i += step) {
       const unsigned long long u = (unsigned long long)__double_as_longlong(
-          i < na ? a[d * na + i] : b[d * nb + (i - na)]);
+          i < P.nr ? P.rpos[d * P.nr + i] : P.cpos[d * P.nc + (i - P.nr)]);
       hi = max(hi, ordered_bits(u));
       lo = max(lo, ordered_bits(u ^ 0x8000000000000000ull));
     }
@@ -257,11 +261,15 @@ __global__ void __launch_bounds__(DT) k_dense_range(const double *__restrict__ a
       __syncthreads();
       if (threadIdx.x == 0) {
         for (int w = 1; w < DT / 32; ++w) v = max(v, red[w]);
-        atomicMax(&F->range[3 * s + d], v);
+        out(3 * s + d, v);
       }
       __syncthreads();
     }
   }
+}
+__global__ void __launch_bounds__(DT) k_dense_range(DenseParams P, DenseFix *__restrict__ F) {
+  dense_range(P, (int64_t)blockIdx.x * DT, (int64_t)gridDim.x * DT,
+              [&](int k, unsigned long long v) { atomicMax(&F->range[k], v); });
 }
 
 // The kernel's unit from the ranges (one thread's work, done by every CTA that
@@ -281,6 +289,16 @@ template <int KIND> __device__ fx::Unit dense_unit(const DenseParams &P,
 }
 
 template <int KIND>
+__device__ __forceinline__ FixCol fix_col(const DenseParams &P, const fx::Unit &U, int64_t j) {
+  FixCol c;
+  c.x = fx::fixed<KIND>(P.cpos[j], U);
+  c.y = P.dim > 1 ? fx::fixed<KIND>(P.cpos[P.nc + j], U) : 0;
+  c.z = P.dim > 2 ? fx::fixed<KIND>(P.cpos[2 * P.nc + j], U) : 0;
+  c.b = P.b[j];
+  return c;
+}
+
+template <int KIND>
 __global__ void __launch_bounds__(DT) k_dense_prep(DenseParams P, DenseFix *__restrict__ Fg,
                                                    FixCol *__restrict__ cols) {
   __shared__ fx::Unit U;
@@ -290,29 +308,22 @@ __global__ void __launch_bounds__(DT) k_dense_prep(DenseParams P, DenseFix *__re
   }
   __syncthreads();
   const int64_t j = (int64_t)blockIdx.x * DT + threadIdx.x;
-  if (!U.ok || j >= P.nc) return;
-  FixCol c;
-  c.x = fx::fixed<KIND>(P.cpos[j], U);
-  c.y = P.dim > 1 ? fx::fixed<KIND>(P.cpos[P.nc + j], U) : 0;
-  c.z = P.dim > 2 ? fx::fixed<KIND>(P.cpos[2 * P.nc + j], U) : 0;
-  c.b = P.b[j];
-  cols[j] = c;
+  if (U.ok && j < P.nc) cols[j] = fix_col<KIND>(P, U, j);
 }
 
+// `cols` null: the columns are put into fixed point as they are staged.
 template <int KIND, int DIM>
-__global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix *__restrict__ Fg,
-                                                  const FixCol *__restrict__ cols,
-                                                  int64_t chunk_cols, double *__restrict__ partial) {
+__device__ __forceinline__ void dense_rows_fix(const DenseParams &P, const fx::Unit &U,
+                                               const FixCol *__restrict__ cols, int64_t chunk_cols,
+                                               double *__restrict__ partial) {
   __shared__ FixCol sc[DT];
   __shared__ fx::u64 tab[fx::EXP_TAB];
-  if (!Fg->U.ok) return;
   if (KIND == ABX_K_GAUSSIAN) tab[threadIdx.x] = fx::exp_table.v[threadIdx.x];
-  const fx::Consts C = fx::consts(Fg->U, 1.0 / P.p0);
+  const fx::Consts C = fx::consts(U, 1.0 / P.p0);
   const int64_t i = (int64_t)blockIdx.x * DT + threadIdx.x;
   const bool act = i < P.nr;
   long long x = 0, y = 0, z = 0;
   if (act) {
-    const fx::Unit U = Fg->U;
     x = fx::biased(fx::fixed<KIND>(P.rpos[i], U));
     if (DIM > 1) y = fx::biased(fx::fixed<KIND>(P.rpos[P.nr + i], U));
     if (DIM > 2) z = fx::biased(fx::fixed<KIND>(P.rpos[2 * P.nr + i], U));
@@ -322,7 +333,8 @@ __global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix 
   const int64_t c1 = c0 + chunk_cols < P.nc ? c0 + chunk_cols : P.nc;
   for (int64_t t = c0; t < c1; t += DT) {
     __syncthreads();
-    if (t + threadIdx.x < c1) sc[threadIdx.x] = cols[t + threadIdx.x];
+    if (t + threadIdx.x < c1)
+      sc[threadIdx.x] = cols ? cols[t + threadIdx.x] : fix_col<KIND>(P, U, t + threadIdx.x);
     __syncthreads();
     const int nt = (int)((c1 - t) < DT ? (c1 - t) : DT);
 #pragma unroll 2
@@ -347,6 +359,33 @@ __global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix 
     if (partial) partial[(int64_t)blockIdx.y * P.nr + i] = acc;
     else P.c[i] = acc;
   }
+}
+template <int KIND, int DIM>
+__global__ void __launch_bounds__(DT) k_dense_fix(DenseParams P, const DenseFix *__restrict__ Fg,
+                                                  const FixCol *__restrict__ cols,
+                                                  int64_t chunk_cols, double *__restrict__ partial) {
+  if (!Fg->U.ok) return;
+  const fx::Unit U = Fg->U;
+  dense_rows_fix<KIND, DIM>(P, U, cols, chunk_cols, partial);
+}
+
+// The whole product of two small sets in one launch: every CTA goes over all points
+// for the ranges (L2 holds them) and puts its own columns into fixed point, or takes
+// the FP64 formula.  Four launches, of which one does the work, are what such a
+// product took: 1 x 1 37 us, 25 so; 300 x 300 Gaussian 101, 84.
+constexpr int64_t DENSE_SMALL = 2048;  // points
+template <int KIND, int DIM>
+__global__ void __launch_bounds__(DT) k_dense_small(DenseParams P, int64_t chunk_cols,
+                                                    double *__restrict__ partial) {
+  __shared__ unsigned long long range[6];
+  __shared__ fx::Unit U;
+  dense_range(P, 0, DT, [&](int k, unsigned long long v) { range[k] = v; });
+  if (threadIdx.x == 0) U = dense_unit<KIND>(P, range);
+  __syncthreads();
+  if (U.ok)
+    dense_rows_fix<KIND, DIM>(P, U, nullptr, chunk_cols, partial);
+  else
+    dense_rows_fp64<KIND>(P, chunk_cols, partial);
 }
 
 __global__ void k_dense_reduce(const double *__restrict__ partial, int64_t nr, int chunks,
@@ -392,11 +431,22 @@ int launch_dense_fix(abx_context *ctx, const DenseParams &P, abx_operator *op) {
   DenseFix *F = reinterpret_cast<DenseFix *>(op->partial.ptr);
   FixCol *cols = reinterpret_cast<FixCol *>(op->partial.ptr + (nf / 4) * 4);
   double *partial = used > 1 ? op->partial.ptr + (nf / 4) * 4 + nb : nullptr;
+  const dim3 grid(blocks, used);
+  if (P.nr + P.nc <= DENSE_SMALL) {
+    if (P.dim == 3)
+      k_dense_small<KIND, 3><<<grid, DT, 0, s>>>(P, chunk_cols, partial);
+    else if (P.dim == 2)
+      k_dense_small<KIND, 2><<<grid, DT, 0, s>>>(P, chunk_cols, partial);
+    else
+      k_dense_small<KIND, 1><<<grid, DT, 0, s>>>(P, chunk_cols, partial);
+    if (partial) k_dense_reduce<<<ceil_div(P.nr, 256), 256, 0, s>>>(partial, P.nr, used, P.c);
+    ABX_CHECK_CUDA(cudaGetLastError());
+    return ABX_OK;
+  }
   ABX_CHECK_CUDA(cudaMemsetAsync(F, 0, sizeof(DenseFix), s));
   const unsigned rb = std::min(ceil_div(P.nr + P.nc, DT), 2u * (unsigned)std::max(ctx->num_sms, 1));
-  k_dense_range<<<rb, DT, 0, s>>>(P.rpos, P.nr, P.cpos, P.nc, P.dim, F);
+  k_dense_range<<<rb, DT, 0, s>>>(P, F);
   k_dense_prep<KIND><<<std::max(1u, ceil_div(P.nc, DT)), DT, 0, s>>>(P, F, cols);
-  const dim3 grid(blocks, used);
   if (P.dim == 3)
     k_dense_fix<KIND, 3><<<grid, DT, 0, s>>>(P, F, cols, chunk_cols, partial);
   else if (P.dim == 2)
