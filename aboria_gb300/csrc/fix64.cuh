@@ -202,12 +202,15 @@ FX_HD int clz32(u32 x) {
 // correction is d - d^2 / (2 q0), d = res / (2 q0): D1 is d in units of 2^-50
 // to FP32 accuracy, R1 what D1 leaves of res (exact), and the last FP32 term
 // carries R1's and d^2's share.  u = 0 gives 0.
-FX_HD u64 sqrt60(u64 u) {
+// SMALL: for any u, to 2^-60 / sqrt(u 2^-60) below 2^40.  The residual is shifted with
+// rounding: the floor of -1 / 2^11 is -1, a correction by 2^11 / (2 q0), which for u
+// below 2^22 was more than the root.
+template <bool SMALL = false> FX_HD u64 sqrt60(u64 u) {
   const float uf = fma32((float)hi32(u), 4294967296.0f, (float)(u32)u);
   const float rs = rsqrt32(fmaxf(uf, 1.0f));
   const int q0 = f2i(uf * rs);
   const i64 res = (i64)u - (i64)q0 * q0;
-  const float d1 = (float)(int32_t)(res >> 11) * (rs * 1073741824.0f);  // 2^11 2^20 / 2
+  const float d1 = (float)(int32_t)((SMALL ? res + 1024 : res) >> 11) * (rs * 1073741824.0f);  // 2^11 2^20 / 2
   const int D1 = f2i(d1);
   const i64 R1 = (i64)((u64)res << 20) - (i64)q0 * (2 * D1);
   const float r1 = (float)(int32_t)(R1 >> 10);
@@ -306,7 +309,7 @@ FX_HD double exp2_neg(u64 t, const u64 *tab) {
 // accuracy where t is small.
 FX_HD double wendland(u64 q2) {
   if (q2 >= (1ull << 60)) return 0.0;
-  const i64 td = (i64)(1ull << 62) - (i64)sqrt60(q2);
+  const i64 td = (i64)(1ull << 62) - (i64)sqrt60<true>(q2);
   const u64 t = ((u64)td << 1) - (u64)(td >> 62);  // units of 2^-63, below 2^63
   const u32 th = hi32(t);
   if (td <= 0 || th == 0) return 0.0;  // t < 2^-31: the value is below 2^-121
