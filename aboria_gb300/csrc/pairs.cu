@@ -116,6 +116,7 @@ struct PairLayout {
   // queries once more as a list (k_units).
   DevBuf<int2> units;
   DevBuf<int> singles;
+  DevBuf<uint8_t> exits;  // of the units' chunks, and their entries (k_unit_exits)
   Split split = SPLIT_NONE;
   // full units, small units, their queries, stencil rows; work counters of a
   // count or product (4, 5) and of a list search (6, 7); small units and single
@@ -156,7 +157,7 @@ struct SearchSpace {
   void trim(int64_t nq, int64_t n) {
     if (nq > std::max(n, KEEP_QUERIES)) {
       L.rows_own.release();
-      L.units.release(), L.singles.release();
+      L.units.release(), L.singles.release(), L.exits.release();
       queries.buf.release(), qsoa.release(), cnt.release();
       rowptr.release(), rpk.release(), sums.release();
     }
@@ -420,31 +421,94 @@ int build_cell_start(abx_context *ctx, PairLayout &L) {
 // density, where a warp of 32 lanes would hold few queries), to the back, and
 // its queries to `singles`, which k_pairs_thread walks.  Built on the host before,
 // from a 16 B/point copy of the cells: 14 of the 39 ms of a search at N = 4M.
-// Few columns (1-D: one) are walked in `segs` segments of cells, where units end: one
-// warp took 620 us for 50,000 points, 64 take less than 10.
+//
+// Few columns (1-D: one) are walked by a warp per chunk of queries: where the first
+// unit of a chunk starts depends on all before it, but is one of 32 places, from each
+// of which a lane follows the chunk's units (k_unit_exits); going through the chunks
+// with these answers is short (k_unit_entries).  A count of 1,000,000 points in 1-D:
+// 13.2 ms with one warp, 1.0 so.
 constexpr int UNIT_WARPS = 4;
 constexpr uint32_t FEW_COLUMNS = 4;
-constexpr int SEG_CELLS = 16;  // at least
+constexpr int64_t MIN_CHUNK = 128, MOST_CHUNKS = 1024;
+
+struct UnitQueries {
+  const int4 *cell;
+  const uint32_t *keys, *cell_start;
+  bool self;
+  int64_t n, chunk;  // queries a chunk
+  int chunks;        // a column; 1: whole columns
+  int m2;
+};
+// Queries of a column (whole warps).
+__device__ __forceinline__ void column_range(const UnitQueries &Q, uint32_t col, int lane, int64_t &s,
+                                             int64_t &end) {
+  if (Q.self) {
+    s = Q.cell_start[(uint64_t)col * Q.m2];
+    end = Q.cell_start[(uint64_t)(col + 1) * Q.m2];
+  } else {
+    s = warp_lower_bound(Q.keys, Q.n, (uint64_t)col * Q.m2 * 8, lane);
+    end = warp_lower_bound(Q.keys, Q.n, (uint64_t)(col + 1) * Q.m2 * 8, lane);
+  }
+}
+// exits[item][e]: how far beyond the end of chunk `item` the units reach if one starts
+// at its e-th query.
 __global__ void __launch_bounds__(UNIT_WARPS * 32)
-    k_units(const int4 *__restrict__ cell, const uint32_t *__restrict__ keys,
-            const uint32_t *__restrict__ cell_start, bool self, int64_t n, FineGrid fg, int64_t cap,
-            int segs, Split split, int2 *__restrict__ units, int *__restrict__ singles,
-            int *__restrict__ counts) {
+    k_unit_exits(UnitQueries Q, uint32_t items, uint8_t *__restrict__ exits) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t item = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5);
+  if (item >= items) return;
+  int64_t s, end;
+  column_range(Q, item / Q.chunks, lane, s, end);
+  s += (int64_t)(item % Q.chunks) * Q.chunk;
+  const int64_t stop = min(s + Q.chunk, end);
+  s += lane;
+  while (s < stop) {
+    const int4 c0 = Q.cell[s];
+    int run = 1;
+    for (; run < 32 && s + run < end; ++run) {
+      const int4 c = Q.cell[s + run];
+      if (c.x != c0.x || c.y != c0.y || c.z < c0.z || c.z - c0.z >= GROUP_E2) break;
+    }
+    s += run;
+  }
+  exits[(size_t)item * 32 + lane] = (uint8_t)(s > stop ? min(s - stop, (int64_t)31) : 0);
+}
+// entries[item]: where the first unit of a chunk starts, from the chunk's first query.
+__global__ void __launch_bounds__(32) k_unit_entries(int chunks, const uint8_t *__restrict__ exits,
+                                                     uint8_t *__restrict__ entries) {
+  const int lane = threadIdx.x;
+  const size_t first = (size_t)blockIdx.x * chunks;
+  int e = 0;
+  for (int k0 = 0; k0 < chunks; k0 += 8) {
+    int row[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) row[k] = k0 + k < chunks ? exits[(first + k0 + k) * 32 + lane] : 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (lane == 0 && k0 + k < chunks) entries[first + k0 + k] = (uint8_t)e;
+      e = __shfl_sync(0xffffffffu, row[k], e);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(UNIT_WARPS * 32)
+    k_units(UnitQueries Q, const uint8_t *__restrict__ entries, FineGrid fg, int64_t cap, Split split,
+            int2 *__restrict__ units, int *__restrict__ singles, int *__restrict__ counts) {
   const int lane = threadIdx.x & 31, m2 = fg.m[2], K2 = fg.K[2];
-  const uint32_t ncol = (uint32_t)fg.m[0] * fg.m[1];
+  const int4 *__restrict__ cell = Q.cell;
+  const uint32_t *__restrict__ cell_start = Q.cell_start;
+  const uint32_t items = (uint32_t)fg.m[0] * fg.m[1] * Q.chunks;
   const uint32_t warps = gridDim.x * UNIT_WARPS;
-  const int len = (m2 + segs - 1) / segs;
-  for (uint32_t item = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); item < ncol * segs; item += warps) {
-    const uint32_t col = item / segs;
-    const int z_from = min((int)(item % segs) * len, m2), z_to = min(z_from + len, m2);
-    const uint64_t from = (uint64_t)col * m2 + z_from, to = (uint64_t)col * m2 + z_to;
+  for (uint32_t item = blockIdx.x * UNIT_WARPS + (threadIdx.x >> 5); item < items; item += warps) {
+    const uint32_t col = item / Q.chunks;
     int64_t s, end;
-    if (self) {
-      s = cell_start[from];
-      end = cell_start[to];
-    } else {
-      s = warp_lower_bound(keys, n, from * 8, lane);
-      end = warp_lower_bound(keys, n, to * 8, lane);
+    column_range(Q, col, lane, s, end);
+    int64_t last = end;  // units start below it
+    if (Q.chunks > 1) {
+      s += (int64_t)(item % Q.chunks) * Q.chunk;
+      last = min(s + Q.chunk, end);
+      if (s >= end) continue;
+      s += entries[item];
     }
     const int4 none = make_int4(0, 0, 0, 0);
     int64_t base = s;  // A holds queries [base, base + 32), B the 32 after them
@@ -453,8 +517,8 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
     int2 mine = make_int2(0, 0);  // lane i keeps the i-th unit not written out yet
     int z_mine = 0;               // and its first cell along e2
     int held = 0;
-    while (s < end || held > 0) {
-      if (s < end) {
+    while (s < last || held > 0) {
+      if (s < last) {
         if (s - base >= 32) {
           base += 32;
           A = B;
@@ -478,7 +542,7 @@ __global__ void __launch_bounds__(UNIT_WARPS * 32)
         ++held;
         s += count;
       }
-      if (held == 32 || s >= end) {
+      if (held == 32 || s >= last) {
         bool small = lane < held && mine.y < split.queries;
         if (small) {
           const int z = min(max(z_mine, 0), m2 - 1);
@@ -541,11 +605,21 @@ int build_units(abx_context *ctx, PairLayout &L, const Split &split) {
   ABX_CHECK_CUDA(cudaMemsetAsync(L.counts.ptr, 0, COUNTS * sizeof(int), ctx->stream));
   if (n == 0) return ABX_OK;
   const uint32_t ncol = (uint32_t)L.fg.m[0] * L.fg.m[1];
-  const int segs = ncol <= FEW_COLUMNS ? (int)ceil_div(L.fg.m[2], SEG_CELLS) : 1;
-  const unsigned blocks = std::min(ceil_div((size_t)ncol * segs, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
+  UnitQueries U{Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, n, 1, L.fg.m[2]};
+  if (ncol <= FEW_COLUMNS && n > MIN_CHUNK) {
+    U.chunk = std::max(MIN_CHUNK, (n / MOST_CHUNKS + 32) / 32 * 32);
+    U.chunks = (int)ceil_div(n, U.chunk);
+    const uint32_t items = ncol * U.chunks;
+    ABX_TRY(L.exits.reserve((size_t)items * 33));
+    uint8_t *entries = L.exits.ptr + (size_t)items * 32;
+    k_unit_exits<<<ceil_div(items, UNIT_WARPS), UNIT_WARPS * 32, 0, ctx->stream>>>(U, items, L.exits.ptr);
+    k_unit_entries<<<ncol, 32, 0, ctx->stream>>>(U.chunks, L.exits.ptr, entries);
+  }
+  const uint32_t items = ncol * U.chunks;
+  const unsigned blocks = std::min(ceil_div(items, UNIT_WARPS), 8u * (unsigned)ctx->num_sms);
   k_units<<<blocks, UNIT_WARPS * 32, 0, ctx->stream>>>(
-      Q.cell.ptr, Q.keys.ptr, L.cell_start.ptr, L.self, n, L.fg, n, segs, split,
-      L.units.ptr, L.singles.ptr, L.counts.ptr);
+      U, U.chunks > 1 ? L.exits.ptr + (size_t)items * 32 : nullptr, L.fg, n, split, L.units.ptr,
+      L.singles.ptr, L.counts.ptr);
   ABX_CHECK_CUDA(cudaGetLastError());
   return ABX_OK;
 }
