@@ -1635,6 +1635,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
           }
           nt += __popc(km);
         }
+        if (nt == 0) continue;  // (in 1-D most tiles lie beyond the unit's reach)
         __syncwarp();
         if (lane == 0 && (nt & 1)) {  // an odd tail is paired with a candidate at infinity
           float *xy = reinterpret_cast<float *>(&sm.pxy[nt >> 1]);
