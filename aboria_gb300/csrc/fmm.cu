@@ -1569,13 +1569,17 @@ __global__ void __launch_bounds__(PT * WPL) k_p2p_fix(
             bool near;
             double v = fx::value<KIND>(fx::diff(s0.x, x), fx::diff(s0.y, y), fx::diff(s1.x, z), D, C,
                                        tab, near);
-            if (KIND == ABX_K_LAPLACE && near && i != j0 + q) {
-              double d2 = 0.0;
-              for (int d = 0; d < D; ++d) {
-                const double dx = pos[(int64_t)d * npos + j0 + q] - pos[(int64_t)d * npos + i];
-                d2 += dx * dx;
+            if (KIND == ABX_K_LAPLACE && near) {
+              int j = j0 + q;
+              asm volatile("" : "+r"(j));  // (compared in here, not for every pair: 2 %)
+              if (i != j) {
+                double d2 = 0.0;
+                for (int d = 0; d < D; ++d) {
+                  const double dx = pos[(int64_t)d * npos + j] - pos[(int64_t)d * npos + i];
+                  d2 += dx * dx;
+                }
+                v = fmm_k64<KIND>(d2, p0);
               }
-              v = fmm_k64<KIND>(d2, p0);
             }
             acc = fma(v, __longlong_as_double(s1.y), acc);
           }
