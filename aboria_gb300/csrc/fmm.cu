@@ -1923,12 +1923,14 @@ int launch_l2p_p2p(FmmPlan *P, cudaStream_t s, const double *pos, int64_t npos, 
 //          512        33 / 17 against 25 / 22             1,024  355 / 351 against 392 / 374
 //        1,024        75 / 49 against 38 / 34             1,536  855 / 849 against 875 / 869
 //        1,536       148 / 110 against 62 / 58            4,096  886 / 875 against 861 / 849
+// (orders 5 to 7; FP64's line is at 8 CTAs an SM because with few nodes one thread is the
+// faster before: 2-D, order 3, 2,048 CTAs, a product 1,398 us against 1,437).
 template <typename T, bool M2M>
 void launch_links(const FmmPlan *P, int lev, const T *mats, double *V, cudaStream_t s) {
   if (P->batch_cnt[lev] == 0) return;
   const dim3 grid(P->batch_cnt[lev], ceil_div(P->ncheb, FT));
   const int2 *bt = P->batches.ptr + P->batch_off[lev];
-  constexpr int64_t LINE = sizeof(T) == 4 ? 2 : 16;  // CTAs an SM
+  constexpr int64_t LINE = sizeof(T) == 4 ? 2 : 8;  // CTAs an SM
   if ((int64_t)grid.x * grid.y < LINE * P->sms)
     k_m2m_l2l<T, M2M, 4><<<grid, 4 * FT, 0, s>>>(P->ncheb, P->links.ptr, bt, mats, V);
   else
