@@ -1,10 +1,14 @@
 // Products of matrices of scaled 56-bit integers (fix64.cuh: whole56) on the
-// tensor cores: an integer is seven signed 8-bit digits, each exact in FP16, and of
-// the 49 products of digits those 28 with i + j >= 6 are formed, as much as three
-// 32x32+64-bit multiply-adds of two 28-bit halves give.  The products of one weight
-// i + j, summed over up to 128 terms, stay within 2^24: FP32 accumulators hold them
-// exactly, whatever the order.  28 FP16 multiply-adds take the place of three
-// integer ones at 25 a clock and SM.
+// tensor cores, by splitting them into exact products of short numbers (Ozaki, Ogita,
+// Oishi, Rump, Numerical Algorithms 59, 2012): an integer is seven signed 8-bit
+// digits, each exact in FP16, and of the 49 products of digits those 28 with
+// i + j >= 6 are formed.  The products of one weight i + j above 6, summed over up to
+// 128 terms, stay within 2^24: FP32 accumulators hold them exactly, whatever the
+// order.  Those of weight 6, of which a 256th goes into the result, reach 1.13 2^24
+// where all digits are at their limits, and may be rounded to even numbers there.
+// What is left out of a term is below 2^-55 of the two scales' product, and 2^-58 of
+// it root mean square.  28 FP16 multiply-adds take the place of three 32x32+64-bit
+// ones, of which an SM does 25 a clock.
 #pragma once
 
 #include <cuda_fp16.h>

@@ -1,8 +1,9 @@
 // FP64-accurate kernel values from integer and FP32 arithmetic.
 //
 // GB300 issues 2 FP64 operations per clock and SM (measured 1.7-1.8) against
-// 58 32x32+64-bit multiply-adds, 62 integer ALU operations and 115 FP32 FMAs,
-// so one double-precision operation costs as much as about 32 integer ones.
+// 62 integer ALU operations, 115 FP32 FMAs and 25 32x32+64-bit multiply-adds of three
+// registers (58 with a uniform operand), so one double-precision operation costs as
+// much as about 32 integer ones.
 // A pair's kernel value takes ~30 of the former (distance 6-8, sqrt or exp
 // 10-20, the rest the polynomial and the product); here everything but the
 // last multiply-add into the row's FP64 sum runs on the integer pipe:
@@ -14,8 +15,8 @@
 //    the kernel's own scale: sqrt(p0 log2(e)) for the Gaussian, p0 for the
 //    Wendland kernel, held to 100 bits (Unit);
 //  * each difference is split as h 2^32 + l with a signed low half; h^2 and h l
-//    are summed exactly, l^2 (below the unit of the sum) is left out except
-//    where the kernel is singular (sq_acc);
+//    are summed exactly; l^2, which is below the unit of the sum, counts for
+//    Laplace and multiquadric values and Gaussians beyond 2^-255 (sq_acc, sq_low);
 //  * sqrt starts from the hardware's FP32 reciprocal square root and takes
 //    two corrections from exact integer residuals (sqrt60);
 //  * 2^-t splits t into an exponent, an index of a 256-entry table and a rest
@@ -365,8 +366,7 @@ FX_HD double multiquadric(u64 v, int r) {
 // ------------------------------------------------- scaled 56-bit numbers ---
 // Operands of integer products of matrices (digits.cuh): x 2^(56 - e) as an
 // integer for |x| <= 2^e, and its seven signed 8-bit digits, the lowest first.
-// Of a product x y the digits' products below 256^6 are left out, which are below
-// the numbers' own 2^-57.
+// Of a product x y the digits' products below 256^6 are left out (digits.cuh).
 FX_HD u64 abs_bits(double x) { return bits_of(x) & 0x7fffffffffffffffull; }
 // e with |x| <= 2^e from the bits of the largest |x|; NOT_FINITE, which makes
 // every integer 0 and every scale NaN, if that is infinite or NaN

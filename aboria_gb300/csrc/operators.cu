@@ -4,10 +4,11 @@
 // specialisation generic_product_impl::scaleAndAddTo
 // (src/detail/Operators.h:207-229), which zero-initialises the destination and
 // calls KernelX::evaluate.  The dense kernel restates KernelDense::evaluate
-// (src/Kernels.h:212-239): for each row i, in column order j = 0..n-1,
-// c_i += f(a_i, b_j) * b_j.  Each thread owns one row and walks the columns in
-// exactly that order, so the FP64 mode reproduces the reference's summation
-// order; columns are staged through shared memory 256 at a time.
+// (src/Kernels.h:212-239): for each row i, c_i = sum over j of f(a_i, b_j) * b_j.
+// The reference adds the columns in order; here a thread owns a row and walks a
+// chunk of them in order, 256 staged in shared memory at a time, and the chunks, as
+// many as the rows leave SMs idle (dense_chunks), are added in order.  So the
+// roundings are not the reference's and may differ between GPUs of other sizes.
 #include <cmath>
 
 #include "common.cuh"
@@ -73,7 +74,8 @@ template <int KIND> __device__ __forceinline__ float dk32(float d2, float p0f, f
   return 0.f;
 }
 
-// `F` (may be null): leave at once where k_dense_fix has done the product.  Column
+// `F` (may be null): leave at once where k_dense_fix has done the product.  Constant
+// and scalar-sum kernels, which have no fixed-point values, come here only.  Column
 // chunks (blockIdx.y) as in k_dense_fix: with one CTA per 256 rows, 460 x 1484
 // took 2.0 ms, the latency of 1,484 values one after the other; with
 // chunks 124 us.

@@ -250,14 +250,18 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 
 // ------------------------------------------- LU with an integer update ---
 // The same factorisation (partial pivoting, LAPACK's pivot convention) for
-// blocks of kernel values of one size (Gaussian, Wendland: at most 1, 1 on the
-// diagonal), where the trailing update, n^3 / 3 multiply-adds, need not run at 2
+// blocks whose largest entries are the 1s of the diagonal (Gaussian, Wendland), where
+// the trailing update, n^3 / 3 multiply-adds, need not run at 2
 // FP64 operations a clock and SM: the rows of L21 and the columns of U12 become
 // scaled 56-bit integers (fix64.cuh), and an FP64 multiply-add (1.8 a clock and SM)
 // becomes 28 exact FP16 ones on the tensor cores (update_mma).
-// The scale is the largest entry of the row (column), so a product's error is
-// 2^-56 of the largest product of its row and column, where FP64's partial sums
-// round at 2^-53 of themselves.
+// The scale is the largest entry of a row's (column's) 64 terms, so a product is good
+// to 2^-55 of the largest one of its row and column, where FP64's is to 2^-53 of
+// itself: as stable for the matrix as a whole, not entry by entry.  One-block solves
+// of 120 to 1,000 points against extended precision, compact Gaussian / Wendland /
+// Gaussian cut at 0.04, geometric means of this kernel's values over k_lu_fp64's:
+// solution's error 0.92 / 1.02 / 0.85, residual over |A| |y| 0.93 / 1.00 / 0.79, the
+// same row by row 1.03 / 1.09 / 1.19.
 //
 // A cluster of CTAs a domain (more, the fewer domains there are: the largest
 // domain's time is the kernel's), two to an SM.  The first factorises the panels;
@@ -267,14 +271,13 @@ __global__ void __launch_bounds__(LU_T) k_lu_fp64(double *__restrict__ mat,
 // them, two FP64 operations an entry, so the trailing matrix is updated for 64
 // columns at a time and only the rows and columns of those 64 panel by panel.
 // Pivots are compared as integers.  256 domains of 703 rows on average (set-up and
-// one apply): 98 -> 36 ms, 31.9 with the largest domains first, 22.8 with tensor
-// cores; blocks of 1,700 rows (4,003 points): 592 -> 35 ms.
+// one apply): 97 ms with k_lu_fp64, 22.4 with this.
 constexpr int FL_T = 256;      // threads
 constexpr int FW = 16;         // panel width
 constexpr int FB = 64;         // columns of a trailing update
 constexpr int PLD = FW + 1;    // panel row stride
-// rows of a panel in shared memory, so that two CTAs share an SM (one leaves the
-// integer pipe waiting: 40 ms); the few rows of larger blocks stay in L2
+// rows of a panel in shared memory; larger blocks' other rows stay in L2.  Two CTAs
+// share an SM up to 784 rows (with one, 36 ms became 40).
 constexpr int FL_ROWS = 712;
 
 using fx::abs_bits;
@@ -286,8 +289,7 @@ using fx::scale_exp;
 // U's are 28 KB, two CTAs an SM; those within a block of columns or rows are 128 x
 // 16 and 16 x 128 with the FW terms of a panel.  A warp has 16 x 16 entries, 56
 // accumulators a thread.  With 32-bit multiply-adds (25 a clock and SM) the
-// trailing matrix took 14.3 of the 31.8 ms (set-up and one apply) of 256 domains of
-// 703 rows, now 7.1 of 24.3; with the others' multiply-adds here as well 22.8.
+// trailing matrix took 14.3 ms of 256 domains of 703 rows, with these 7.1.
 using dg::MD;
 template <int TR, int TC, int KW> constexpr size_t digit_bytes() { return (size_t)MD * (TR + TC) * KW * 2; }
 constexpr size_t MD_BYTES = digit_bytes<64, 32, FB>();
@@ -874,8 +876,8 @@ int schwarz_build(abx_operator *op, int precision, Schwarz *&out) {
     cudaMemcpyAsync(S->dom_mat.ptr, moff.data(), moff.size() * 8, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(S->idx.ptr, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, s);
     if ((st = launch_assemble(ctx, *S, p, op->k, op->radius, size))) return fail(st);
-    // blocks of kernel values of one size: integer update (k_lu_fix); kernels
-    // whose values span many magnitudes: FP64
+    // kernels whose largest value is the diagonal's 1: integer update (k_lu_fix);
+    // Laplace, multiquadric and constant ones: FP64
     const bool flat = op->k.kind == ABX_K_GAUSSIAN || op->k.kind == ABX_K_COMPACT_GAUSSIAN ||
                       op->k.kind == ABX_K_WENDLAND_C2;
     if (flat) {
