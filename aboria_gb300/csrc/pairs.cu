@@ -1757,7 +1757,7 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32, 6)
 enum { VAL_FP64 = 0, VAL_MIXED = 1, VAL_FIX = 2 };
 constexpr int QCAP = 16;   // queued pairs per lane
 constexpr int DRAIN = 22;  // lanes that make an evaluation worth its issue
-constexpr int FLUSH32 = 32;  // terms of an FP32 sum, which then goes to the FP64 one
+constexpr uint32_t FLUSH32 = 32;  // terms from which on an FP32 sum goes to the FP64 one (below twice that)
 
 template <int POL, int KIND, int VAL, int NORM = 2>
 __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
@@ -1805,7 +1805,8 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
     const double si = (QUEUE && KIND == ABX_K_SCALAR_SUM) ? P.s_row[qi] : 0.0;
     double acc = 0.0;
     float acc32 = 0.f;
-    int count = 0, nq = 0, steps = 0;
+    int count = 0, nq = 0;
+    uint32_t terms = 0;  // candidates since this lane's FP32 sum was handed on
     auto evaluate = [&]() {  // one queued pair of every lane that has one
       if (nq > 0) {
         --nq;
@@ -1875,48 +1876,54 @@ __global__ void __launch_bounds__(WARPS_PER_CTA * 32)
           }
           const float zs = (float)(-i2 * m2 - qc.z);
           const int code = i0 | (i1 << 2) | ((i2 + 1) << 4);
-          while (__any_sync(0xffffffffu, k < e)) {
-            if (k < e) {
-              const float4 cl = __ldg(&P.cloc[k]);
-              const float dx = cl.x + rx, dy = cl.y + ry,
-                          dz = fmaf(cl.w + zs, fg.hf[2], cl.z) - ql.z;
-              float dd = norm32<NORM>(dx, dy, dz);
-              if (WCUT) {
-                // the clamp is the cut-off (see K_WEND_CUT)
-                dd = fmaf(dd, p0f2, 1e-30f);
-                const float t = __saturatef(fmaf(-dd, rsqrt_approx(dd), 1.f));
-                const float t2 = t * t;
-                if (t > 0.f) acc32 = fmaf(t2 * t2 * fmaf(t, -4.f, 5.f), __ldg(&P.b32[k]), acc32);
-              } else {
-                bool in = dd <= r2lo;
-                if (!in && dd <= r2hi) {  // rare: the reference's FP64 test
-                  // (opaque: otherwise the image shifts' FP64 products are computed for
-                  // every row, ahead of this branch; 100,000 x 50 Gaussian 197 -> 192 us)
-                  int img[3] = {i0 - 1, i1 - 1, i2};
-                  asm volatile("" : "+r"(img[0]), "+r"(img[1]), "+r"(img[2]));
-                  in = !(exact_norm(P.qpos[qi], P.cpos[k], img, fg, NORM) > P.thr);
+          // mixed sums: at most FLUSH32 candidates of a row at a time, which may cross a
+          // cluster that the query is not in
+          constexpr bool SUM32 = VAL == VAL_MIXED && POL == POL_MATVEC;
+          for (;;) {
+            const uint32_t to = SUM32 ? min(e, k + FLUSH32) : e;
+            if (SUM32) terms += to - k;
+            while (__any_sync(0xffffffffu, k < to)) {
+              if (k < to) {
+                const float4 cl = __ldg(&P.cloc[k]);
+                const float dx = cl.x + rx, dy = cl.y + ry,
+                            dz = fmaf(cl.w + zs, fg.hf[2], cl.z) - ql.z;
+                float dd = norm32<NORM>(dx, dy, dz);
+                if (WCUT) {
+                  // the clamp is the cut-off (see K_WEND_CUT)
+                  dd = fmaf(dd, p0f2, 1e-30f);
+                  const float t = __saturatef(fmaf(-dd, rsqrt_approx(dd), 1.f));
+                  const float t2 = t * t;
+                  if (t > 0.f) acc32 = fmaf(t2 * t2 * fmaf(t, -4.f, 5.f), __ldg(&P.b32[k]), acc32);
+                } else {
+                  bool in = dd <= r2lo;
+                  if (!in && dd <= r2hi) {  // rare: the reference's FP64 test
+                    // (opaque: otherwise the image shifts' FP64 products are computed for
+                    // every row, ahead of this branch; 100,000 x 50 Gaussian 197 -> 192 us)
+                    int img[3] = {i0 - 1, i1 - 1, i2};
+                    asm volatile("" : "+r"(img[0]), "+r"(img[1]), "+r"(img[2]));
+                    in = !(exact_norm(P.qpos[qi], P.cpos[k], img, fg, NORM) > P.thr);
+                  }
+                  if (POL == POL_COUNT) count += in ? 1 : 0;
+                  if (POL == POL_MATVEC && VAL == VAL_MIXED && in)
+                    acc32 = fmaf(kern32<KIND>(dd, P), __ldg(&P.b32[k]), acc32);
+                  if (QUEUE && in) {
+                    const int c = NEAR && dd < P.near2 ? code | NEAR_CODE : code;
+                    qu[nq * 32] = (unsigned long long)k | ((unsigned long long)c << 32);
+                    ++nq;
+                  }
                 }
-                if (POL == POL_COUNT) count += in ? 1 : 0;
-                if (POL == POL_MATVEC && VAL == VAL_MIXED && in)
-                  acc32 = fmaf(kern32<KIND>(dd, P), __ldg(&P.b32[k]), acc32);
-                if (QUEUE && in) {
-                  const int c = NEAR && dd < P.near2 ? code | NEAR_CODE : code;
-                  qu[nq * 32] = (unsigned long long)k | ((unsigned long long)c << 32);
-                  ++nq;
-                }
+                ++k;
               }
-              ++k;
+              if (QUEUE && __any_sync(0xffffffffu, nq == QCAP)) {
+                do evaluate();
+                while (__popc(__ballot_sync(0xffffffffu, nq > 0)) >= DRAIN);
+              }
             }
-            // every FLUSH32 candidates, however many a row of the stencil holds: a row
-            // may cross a cluster that the query is not in
-            if (VAL == VAL_MIXED && POL == POL_MATVEC && (++steps & (FLUSH32 - 1)) == 0) {
-              acc += (double)acc32;
-              acc32 = 0.f;
-            }
-            if (QUEUE && __any_sync(0xffffffffu, nq == QCAP)) {
-              do evaluate();
-              while (__popc(__ballot_sync(0xffffffffu, nq > 0)) >= DRAIN);
-            }
+            if (!SUM32 || !__any_sync(0xffffffffu, terms >= FLUSH32)) break;
+            acc += (double)acc32;
+            acc32 = 0.f;
+            terms = 0;
+            if (!__any_sync(0xffffffffu, k < e)) break;
           }
         }
       }
