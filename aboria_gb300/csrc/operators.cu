@@ -345,14 +345,22 @@ __device__ __forceinline__ void dense_rows_fix(const DenseParams &P, const fx::U
       bool near;
       double v = fx::value<KIND>(fx::diff(q.x, x), fx::diff(q.y, y), fx::diff(q.z, z), DIM, C, tab,
                                  near);
-      if (KIND == ABX_K_LAPLACE && near) {
-        double d2 = 0.0;
-        if (act)
+      if (KIND == ABX_K_LAPLACE && near && act) {
+        double a[DIM], b[DIM];
+        bool same = true;  // two points in one place have the value at distance 0
+        for (int d = 0; d < DIM; ++d) {
+          a[d] = P.cpos[d * P.nc + t + jj];
+          b[d] = P.rpos[d * P.nr + i];
+          same = same && __double_as_longlong(a[d]) == __double_as_longlong(b[d]);
+        }
+        if (!same) {
+          double d2 = 0.0;
           for (int d = 0; d < DIM; ++d) {
-            const double dx = P.cpos[d * P.nc + t + jj] - P.rpos[d * P.nr + i];
+            const double dx = a[d] - b[d];
             d2 = __dadd_rn(d2, __dmul_rn(dx, dx));
           }
-        v = dk64<KIND>(d2, P.p0, 0.0, 0.0);
+          v = dk64<KIND>(d2, P.p0, 0.0, 0.0);
+        }
       }
       acc = fma(v, q.b, acc);
     }

@@ -1460,10 +1460,16 @@ __device__ __forceinline__ double pair64(const D4 &xq, D4 xj, int code, const KP
 }
 
 // The same for a Laplace pair that the fixed-point value leaves out (k0 for a point
-// with itself).
+// with itself, or with one in the same place).
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
 __device__ __forceinline__ double near_pair64(const D4 &xq, int qi, int k, int code, const KParams &P) {
-  if (P.self && k == qi && (code & 63) == CENTRE) return P.fixc.k0;
-  return pair64<ABX_K_LAPLACE>(xq, P.cpos[k], code, P, 0.0, 0.0);
+  const bool centre = (code & 63) == CENTRE;
+  if (P.self && k == qi && centre) return P.fixc.k0;
+  const D4 xj = P.cpos[k];
+  if (centre && same_bits(xj.x, xq.x) && same_bits(xj.y, xq.y) && same_bits(xj.z, xq.z)) return P.fixc.k0;
+  return pair64<ABX_K_LAPLACE>(xq, xj, code, P, 0.0, 0.0);
 }
 
 // FP64 sparse matvec: the reference's arithmetic for every accepted pair,
