@@ -507,11 +507,11 @@ FX_HD double value(i64 dx, i64 dy, i64 dz, int dims, const Consts &C, const u64 
     if (dims > 2) U += sq_low(dz);
   }
   if (KIND == LAPLACE) {
-    if ((S | T) == 0 && U == 0) {
-      near = C.c < SAME_PLACE_P0;
+    near = !laplace_far(S);
+    if (near) {  // (looked at in here, not for every pair: 3 %)
+      if ((S | T) == 0 && U == 0) near = C.c < SAME_PLACE_P0;
       return C.k0;
     }
-    near = !laplace_far(S);
     int z;
     const u64 n = norm_d2(S, T, U, z);
     return laplace(n, z, C.c, C.r);
